@@ -212,3 +212,34 @@ def test_prepare_weight_rejects_wrong_sizes():
         ctx().prepare_weight(H.Q4_K, np.zeros(144, dtype=np.uint8), 1, 255)
     with pytest.raises(ffi.ZqFailure):
         ctx().prepare_weight(10, np.zeros(84, dtype=np.uint8), 1, 256)  # Q2_K: not a type of this path
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 256), (9, 768), (77, 1024)])
+@pytest.mark.parametrize("kind", ["gauss", "ties", "tiny", "flat"])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_q4_k_encoder_at_rounding_ties_and_unaligned_buffers(rows, cols, kind, offset):
+    """Byte-for-byte against the CPU encoder: quotients on and next to the rounding boundaries (the encoder divides only
+    there), subnormal-sized and constant groups, and a source that is not 16-byte aligned."""
+    import ctypes as C
+
+    from zllm_b200 import ffi
+
+    rng = np.random.default_rng(rows + cols)
+    n = rows * cols
+    if kind == "gauss":
+        v = rng.standard_normal(n) * 0.02
+    elif kind == "ties":  # scale 1 / min 0 groups whose values sit on k + 1/2 and one ulp beside it
+        v = rng.integers(0, 15, n) + 0.5
+        v = np.nextafter(v.astype(np.float32), rng.choice([-100.0, 100.0], n).astype(np.float32)) if rows % 2 else v
+        v[::32], v[1::32] = 15.0, 0.0
+    elif kind == "tiny":
+        v = rng.standard_normal(n) * 1e-7
+    else:
+        v = np.where(rng.random(n // 32).repeat(32) < 0.5, 0.0, -0.37)
+    v = v.astype(np.float32)
+    src = torch.zeros(n + 4, device="cuda")
+    src[offset:offset + n] = torch.from_numpy(v).cuda()
+    out = torch.empty(n // 256 * 144, dtype=torch.uint8, device="cuda")
+    ffi.call("zq_quantize", ctx().handle, H.Q4_K, C.c_void_p(src.data_ptr() + 4 * offset), rows, cols, C.c_void_p(out.data_ptr()), out.numel())
+    ctx().sync()
+    assert np.array_equal(out.cpu().numpy(), np.asarray(orc.encode_q4_k(v)).reshape(-1))
