@@ -102,3 +102,40 @@ def test_prefill_full_width_slice():
     sel = np.random.default_rng(13).choice(m, size=24, replace=False)
     want = orc.linear(H.Q4_K, data, rows, cols, x.float().cpu().numpy()[sel])
     assert H.max_rel_error(got[sel], want) <= BOUND
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+@pytest.mark.parametrize("m,rows,cols", [
+    (17, 1, 256), (33, 129, 1280), (255, 255, 512), (257, 257, 768),  # edges of 32-token groups, 128 / 256-row tiles; shares of one tile
+    (40, 25600, 512),   # 100 tiles: every tile cut along K
+    (40, 43520, 512),   # 170 tiles: 96 of them cut, 74 whole
+])
+def test_prefill_tiles_and_shares(tensor_type, m, rows, cols):
+    """Edges of the pair's tile (32 tokens, 128 and 256 rows) and the three ways tiles are dealt (whole, cut, both), with a
+    residual; block-32 types on columns that end inside a k-block.  Bound as above: both operands are rounded to f16 once."""
+    if tensor_type in (H.Q4_0, H.IQ4_NL, H.Q8_0):
+        cols -= 160
+    # weights inside the f16 operand's range (|w| <= 65504): arbitrary scale bits give weights of 1e8 and an infinite operand
+    data = H.random_weight(tensor_type, rows, cols, seed=m + rows)
+    x = dev(np.random.default_rng(m).standard_normal((m, cols)).astype(np.float32), torch.bfloat16)
+    r = np.random.default_rng(m + 1).standard_normal((m, rows)).astype(np.float32)
+    w = ctx().prepare_weight(tensor_type, data, rows, cols)
+    got = host(ctx().linear(x, w, out_dtype=torch.float32, residual=dev(r)))
+    sel = np.unique(np.concatenate([np.random.default_rng(m + 2).choice(m, size=min(m, 9), replace=False), [0, m - 1]]))
+    want = orc.linear(tensor_type, data, rows, cols, x.float().cpu().numpy()[sel]) + r[sel]
+    assert H.max_rel_error(got[sel], want) <= BOUND
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0])
+@pytest.mark.parametrize("m,rows,cols", [(31, 63, 512), (260, 130, 1024)])
+def test_prefill_gated_edges(tensor_type, m, rows, cols):
+    """64 gate and 64 up rows share a tile: ragged row counts, one and two token tiles, shares of a tile.
+    Bound: the output is a product of two projections, each within BOUND of its own scale, through a SiLU of slope at most
+    1.1: |d(silu(g) u)| <= 1.1 |dg| |u| + |silu(g)| |du|, i.e. 2.1 BOUND."""
+    gate, up = H.random_weight(tensor_type, rows, cols, seed=rows), H.random_weight(tensor_type, rows, cols, seed=rows + 1)
+    x = dev(np.random.default_rng(rows).standard_normal((m, cols)).astype(np.float32), torch.float16)
+    wg, wu = ctx().prepare_weight(tensor_type, gate, rows, cols), ctx().prepare_weight(tensor_type, up, rows, cols)
+    got = host(ctx().gated_linear(x, wg, wu, out_dtype=torch.float32))
+    sel = [0, 1, m // 2, m - 1]
+    want = orc.gated_linear(tensor_type, gate, up, rows, cols, x.float().cpu().numpy()[sel])
+    assert H.max_rel_error(got[sel], want) <= 2.1 * BOUND

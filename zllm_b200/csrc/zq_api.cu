@@ -134,6 +134,7 @@ static int finish_prepare(zq_ctx *ctx, zq_weight *w, zq_error *err) {
     int rc = make_weight_map(w, 2 * f.unit_bytes / 4, 128, &w->gemv_map, err);
     if (!rc) rc = make_weight_map(w, 2 * f.unit_bytes / 4, 64, &w->gemv_map_half, err);
     if (!rc) rc = make_weight_map(w, f.unit_bytes / 4, 128, &w->qmv_map, err);
+    if (!rc) rc = make_weight_map(w, f.unit_bytes / 4, 64, &w->unit_map_half, err);
     if (rc) return rc;
     // device copies, in the tail of the weight's own allocation (see resident_alloc_bytes)
     const size_t tail = (w->rows * w->row_pitch + 255) & ~size_t(255);

@@ -197,8 +197,8 @@ __device__ __forceinline__ float decode_unit_element(uint32_t type, const uint8_
 // scale and the packed words are read once for the eight (an element-wise decode reads and unpacks them eight times, which
 // at 8 bytes of output per packed byte, not HBM, bounded the passes built on it).  The eight elements lie in one 32-element
 // group of every format and, in the re-laid formats, in two words of neighbouring pieces.
-// OPERAND: Q4_K and Q5_K values as the GEMM operand forms them, one fused multiply-add instead of the codec's
-// multiply-then-subtract (one rounding fewer; zq_gemm.cu forms the same bits).
+// OPERAND: Q4_K and Q5_K values as the GEMM operand forms them (zq_gemm_dq.cuh: one fused multiply-add on 128 + q; the two
+// paths of the GEMM then give the same bits) instead of the codec's multiply-then-subtract.
 __device__ __forceinline__ void bytes_to_f32(uint32_t w, float *v) {  // four unsigned bytes
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = (float)((w >> (8 * j)) & 0xFFu);
@@ -246,8 +246,9 @@ template <uint32_t TYPE, bool OPERAND> __device__ __forceinline__ void decode8(c
         }
         bytes_to_f32(a, v);
         bytes_to_f32(b, v + 4);
+        const float c = fmaf(-128.0f, dsc, -dm);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = OPERAND ? fmaf(dsc, v[j], -dm) : __fsub_rn(__fmul_rn(dsc, v[j]), dm);
+        for (int j = 0; j < 8; ++j) v[j] = OPERAND ? fmaf(dsc, 128.0f + v[j], c) : __fsub_rn(__fmul_rn(dsc, v[j]), dm);
     } else if constexpr (TYPE == ZQ_Q6_K) {  // columns 32 G + 16 h + 4 t + i: the eight are (t, 0..3) and (t + 1, 0..3) of one scale group
         const int G = i0 >> 5, h = (i0 >> 4) & 1, t = (i0 >> 2) & 3, x2 = 2 * (2 * (G & 1) + h);
         const float ds = __fmul_rn(__half2float(*reinterpret_cast<const __half *>(unit)), (float)(int8_t)unit[kQ6kScales + (i0 >> 4)]);

@@ -319,8 +319,9 @@ struct zq_weight {
     uint8_t *data = nullptr;     // resident layout, device
     bool owns_data = true;
     CUtensorMap gemv_map;        // u32 tensor [rows, row_pitch/4], box = (chunk words, 128 rows): decode GEMV
-    CUtensorMap qmv_map;         // same tensor, box of one unit x 128 rows: tcgen05 decode kernel
+    CUtensorMap qmv_map;         // same tensor, box of one unit x 128 rows: tcgen05 decode kernel, prefill GEMM
     CUtensorMap gemv_map_half;   // same tensor, box of 64 rows: gated GEMV (gate and up halves of one stage)
+    CUtensorMap unit_map_half;   // same tensor, box of one unit x 64 rows: gated prefill GEMM
     // Device copies {gemv_map, gemv_map_half, qmv_map} behind the resident bytes (same allocation), for kernels that
     // pick their weight from a table at run time; null for the types no decode kernel reads through TMA.
     CUtensorMap *d_maps = nullptr;
@@ -330,7 +331,7 @@ namespace zq {
 int use_device(zq_ctx *ctx, zq_error *err);
 int ensure_workspace(zq_ctx *ctx, size_t bytes, zq_error *err);
 int ensure_xq(zq_ctx *ctx, size_t bytes, zq_error *err);
-int launch_gemm_fused_grouped(zq_ctx *ctx, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, zq_error *err);
+int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, zq_error *err);
 int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const __half *x, size_t m, void *y, int y_dtype, zq_error *err);
 int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err);
 int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t mats, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, void *y, int y_dtype, zq_error *err);

@@ -5,27 +5,38 @@
 // arithmetic contract is ggml_quant::matmul / gated_silu_matmul (src/kernel/cpu/ggml_quant.rs:280-362):
 // Y[token, row] = sum_k X[token, k] * dequant(W)[row, k], f32 accumulation.
 //
-// Data flow of this version:
-//   1. dequantise the resident packed weight once into an f16 [rows, K] operand in the context workspace
-//      (f32 value rounded once to f16: 2^-12 relative, which keeps layer outputs inside the 2e-3 bound; bf16
-//      operands would not), and convert the activations to f16 (exact for bf16/f16 inputs in f16 range);
-//   2. persistent CTAs (one per SM) walk output tiles of 128 weight rows x 256 tokens: a TMA warp streams
-//      64-column K blocks of both operands (128-byte swizzle) through a 4-stage mbarrier ring; one thread issues
-//      tcgen05.mma (M=128, N=256, K=16, kind::f16, f32 accumulator in 256 TMEM columns); tcgen05.commit releases
-//      ring stages and signals the epilogue warps, which read the accumulator with tcgen05.ld and store
-//      Y (+ residual) in the requested dtype while the MMAs of the next tile fill the second accumulator.  For the
-//      gated form two accumulators (gate and up, all 512 TMEM columns) share the activation tile and the epilogue
-//      applies silu(gate) * up.
-// Every wait is bounded; a wait that runs out raises the CTA's abort flag, all roles fall through to the end,
-// TMEM is released and the context status word reports it.
-#include "zq_common.cuh"
+// One kernel in two forms of the weight operand A (f16 [rows, K]; every value rounded once to f16, 2^-12 relative, which
+// keeps layer outputs inside the 2e-3 bound; bf16 operands would not):
+//   SRC = 0     A was dequantised to memory before (launch_dequantize_f16) and arrives by TMA
+//   SRC = type  the packed rows arrive by TMA and dequantiser warps write A into the swizzled shared-memory tile
+//               (zq_gemm_dq.cuh): the weight crosses HBM once, packed, and no operand pass runs
+// Activations are f16 (exact for bf16 inputs in f16 range), converted before the kernel where they are not.
+//
+// The two SMs of a cluster work on one tile of 256 weight rows x up to 256 tokens (cta_group::2, M = 256): each holds half
+// of the weight rows, half of the tokens' operand and the accumulator of its own rows (two of 256 TMEM columns, so the
+// epilogue of a tile runs under the MMAs of the next).  Why a pair: an MMA of 128 rows x 256 tokens x 16 reads 12 KB of
+// shared memory per 128 cycles and its operands take as much again to arrive, more than one SM's 128 B/clk; with the token
+// operand split over the pair both figures fall to two thirds.
+//
+// Tiles are dealt whole to the pairs while there are many; what does not divide is cut along K into equal shares
+// (256-column steps), and the last contributor of a cut tile adds the f32 partials in pair order (deterministic) and
+// stores.  A gated tile is 64 gate and 64 up rows per SM (128 outputs per pair): gate and up of an output meet in the
+// epilogue through shared memory, and the accumulator still fits twice.
+//
+// Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..5
+// epilogue; SRC != 0: warp 6 TMA of packed boxes, warps 7..22 dequantisers.
+// Every wait is bounded; a wait that runs out raises the CTA's abort flag, all roles fall through to the end, TMEM is
+// released and the context status word reports it.
+#include "zq_gemm_dq.cuh"
 
 namespace zq {
 
-constexpr int kBM = 128;   // weight rows per CTA (UMMA M)
-constexpr int kBN = 256;   // tokens per CTA (UMMA N)
-constexpr int kBK = 64;    // K elements per ring stage (128 bytes of f16: one swizzle atom row)
-constexpr int kGemmThreads = 192;  // warp 0: TMA, warp 1: MMA + TMEM owner, warps 2..5: epilogue
+constexpr int kBM = 128;      // weight rows per SM (operand tile of one CTA)
+constexpr int kPairM = 256;   // weight rows per pair
+constexpr int kBN = 256;      // most tokens per tile
+constexpr int kBK = 64;       // K elements per ring stage (128 bytes of f16: one swizzle atom row)
+constexpr int kStepK = 256;   // K elements per step: one packed unit, the grain in which tiles are cut
+constexpr int kDqWarps = 16;  // thread = (row, k-block of a unit): four warps per k-block
 
 struct GemmParams {
     void *y;
@@ -33,48 +44,85 @@ struct GemmParams {
     uint32_t *status;
     int y_dtype;
     int m;       // tokens
-    int n_out;   // weight rows
+    int n_out;   // output features (weight rows; gated: rows of gate)
     int k;       // input columns
-    // Grouped form (MoE prefill): the work list replaces the tile grid.  Item = {weight matrix z of the 3-D weight
-    // operand, first row of the tile, first token row, end of the matrix's token rows}; tokens are rows of one
-    // activation operand shared by all matrices, outputs are rows of y with n_out columns.
+    int bn;      // tokens per tile (multiple of 32, at most 256)
+    int box_tok; // token rows of one activation box (half a tile)
+    int cut_tiles, cut_pairs;  // the first cut_tiles tiles are cut along K into cut_pairs equal shares
+    float *partials;           // [2 * pairs][2 SMs][256 columns][128 rows] f32
+    uint32_t *counters;        // arrivals per (pair that begins a cut tile, SM), zero between launches
+    // Grouped form (MoE prefill): the work list replaces the tile grid.  Item = {weight matrix z, first output row of the tile,
+    // first token row, end of the tile's token rows}; tokens are rows of one activation operand shared by all matrices,
+    // outputs are rows of y with n_out columns.
     const int4 *items;
     int n_items;
     const int *n_items_dev;  // when set, the item count is read from device memory (a plan kernel wrote it); n_items is then its upper bound
-    // fused Q4_K kernel, grouped form: per-matrix tensor maps of the packed weights (device table indexed by z)
+    // grouped form of a packed type: per-matrix tensor maps (device table indexed by z)
     const CUtensorMap *w_maps, *w2_maps;
 };
 
-// ---- tcgen05 wrappers -------------------------------------------------------------------------------------------
-__device__ __forceinline__ void tmem_alloc(uint32_t *smem_dst, uint32_t cols) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(cols) : "memory");
+// ---- tcgen05 wrappers (pairs of SMs) -------------------------------------------------------------------------------
+__device__ __forceinline__ void tmem_alloc2(uint32_t *smem_dst, uint32_t cols) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(cols) : "memory");
 }
-__device__ __forceinline__ void tmem_relinquish() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t cols) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory");
-}
+__device__ __forceinline__ void tmem_relinquish2() { asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_dealloc2(uint32_t taddr, uint32_t cols) { asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(cols) : "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+// arrives on the barrier at this shared offset in both SMs of the pair once the MMAs issued so far are done
+__device__ __forceinline__ void tc_commit2(uint64_t *bar) {
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3) : "memory");
 }
-// D[tmem] (+)= A[smem] * B[smem], both K-major, f16 inputs, f32 accumulate.
-__device__ __forceinline__ void umma_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+// D[tmem of both SMs] (+)= A[smem of both] * B[smem of both], K-major, f16 inputs, f32 accumulate; issued by the first SM
+__device__ __forceinline__ void umma2_f16_ss(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// Load and wait in one statement: between two the compiler may copy or spill the destination registers, which do not hold the
+// values before the wait.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\ttcgen05.wait::ld.sync.aligned;"
                  : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
                    "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                  : "r"(taddr)
                  : "memory");
 }
-__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// ---- pair plumbing
+__device__ __forceinline__ uint32_t pair_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+// cluster address of this shared address in the pair's first SM
+__device__ __forceinline__ uint32_t pair_first(uint32_t local) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(local));
+    return r;
+}
+__device__ __forceinline__ void pair_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Default (CTA) scope on purpose: what the arrival publishes is read by this SM's own tensor core (operands, behind
+// fence.proxy.async) or was ordered by a tcgen05 fence (accumulators).  A release at cluster scope drains all of the thread's
+// memory traffic first, which cost more than a k-block's MMAs at every stage.
+__device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
+// Loads into this SM's shared memory whose completion counts on a barrier of the pair's first SM.  No multicast.
+__device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t cluster_bar, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(cluster_bar), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, uint32_t cluster_bar, int x, int y, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(cluster_bar), "r"(x), "r"(y), "r"(z)
+                 : "memory");
+}
 
 // K-major operand tile in shared memory, rows of 128 bytes, 128-byte swizzle: 8-row groups are 1024 bytes apart.
 __device__ __forceinline__ uint64_t make_sw128_desc(uint32_t smem_addr) {
@@ -87,368 +135,175 @@ __device__ __forceinline__ uint64_t make_sw128_desc(uint32_t smem_addr) {
     return desc;
 }
 
-__device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t *status, uint32_t code) {
-    for (uint32_t i = 0; i < (1u << 22); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
+// One lane of a converged warp, always the same one.  The single-issuer roles below run their loops with the whole warp and
+// only issue under this predicate: loop state and descriptors then stay in uniform registers.  Inside `if (lane == 0)` every
+// operand of every tcgen05 or TMA instruction was moved there one by one, about 1000 cycles per k-block for the MMA warp,
+// more than its MMAs take.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
+// One poll without a suspend-time hint: the hardware parks the thread for its own limit; with a hint the compiler polls and
+// sleeps in a loop, which delays the wake-up.
+__device__ __forceinline__ bool pair_try_wait(uint64_t *bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// `sleep_ns` > 0: roles that share a scheduler with working warps back off between polls (a bare poll loop re-issues
+// every few tens of nanoseconds).
+__device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t abort_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
+    for (uint32_t i = 0; i < (1u << 23); ++i) {
+        if (pair_try_wait(bar, parity)) return true;
+        uint32_t gone;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gone) : "r"(abort_addr));
+        if (gone) return false;
+        if (sleep_ns) __nanosleep(sleep_ns);
     }
-    *abort_flag = 1;
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u));
     atomicMax(status, code);
     return false;
 }
 
-// Same, for roles that share a scheduler with working warps: a failed poll is followed by a short sleep, so that
-// the waiting warp does not take issue slots from the warps that are dequantising (a bare poll loop re-issues every
-// few tens of nanoseconds).
-__device__ __forceinline__ bool wait_flag_backoff(uint64_t *bar, uint32_t parity, volatile int *abort_flag, uint32_t *status, uint32_t code, unsigned sleep_ns) {
-    for (uint32_t i = 0; i < (1u << 22); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (*abort_flag) return false;
-        __nanosleep(sleep_ns);
-    }
-    *abort_flag = 1;
-    atomicMax(status, code);
-    return false;
+// AND over the four epilogue warps (named barrier 3)
+__device__ __forceinline__ bool epilogue_all(bool v) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 q, %1, 0;\n\t"
+        "barrier.cta.red.and.pred p, 3, 128, q;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(r)
+        : "r"((uint32_t)v)
+        : "memory");
+    return r != 0;
 }
 
-template <bool GATED> struct GemmSmem {
-    static constexpr int stages = GATED ? 3 : 4;
-    static constexpr int acc_bufs = GATED ? 1 : 2;  // 256-column accumulators that fit the 512 TMEM columns
-    static constexpr int a_bytes = kBM * kBK * 2;  // 16 KB
-    static constexpr int b_bytes = kBN * kBK * 2;  // 32 KB
-    static constexpr int stage_bytes = (GATED ? 2 : 1) * a_bytes + b_bytes;
-    static constexpr int off_bar = stages * stage_bytes;
-    static constexpr int total = off_bar + 256 + 1024;  // barriers, tmem slot, slack for 1024-byte alignment
+// Shared-memory plan: 32 KB per ring stage (16 KB of weights, 16 KB of tokens), as many as fit beside the packed boxes.
+template <uint32_t SRC> struct GemmSmem {
+    static constexpr int unit_bytes = SRC == ZQ_Q8_0 ? 272 : SRC == ZQ_Q6_K ? 224 : SRC == ZQ_Q5_K ? 176 : 144;
+    static constexpr int a_bytes = kBM * kBK * 2;
+    static constexpr int b_bytes = kBN / 2 * kBK * 2;
+    static constexpr int stage_bytes = a_bytes + b_bytes;
+    static constexpr int p_bytes = SRC ? kBM * unit_bytes : 0;  // one packed box
+    static constexpr int pstages = SRC == 0 ? 0 : unit_bytes <= 144 ? 3 : 2;
+    static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 ? 4 : 5;
+    static constexpr int off_p = stages * stage_bytes;
+    static constexpr int off_x = off_p + pstages * p_bytes;  // gate / up exchange of the gated epilogue
+    static constexpr int x_bytes = 2 * 2 * 16 * 32 * 4;      // 2 row halves x 2 buffers x 16 columns x 32 rows
+    static constexpr int off_bar = off_x + x_bytes;
+    static constexpr int total = off_bar + 256 + 1024;       // barriers, slack for 1024-byte alignment
+    static constexpr int threads = (SRC ? 7 + kDqWarps : 6) * 32;
+    static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
+    static_assert(off_p % 1024 == 0 && off_x % 16 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
 };
 
 constexpr int kTokGroup = 8;  // token tiles per raster group: a weight tile is reused by 8 token tiles while it is hot in L2
 
-// Persistent CTA (one per SM) over output tiles of 128 weight rows x 256 tokens.  Tiles are rastered in groups of
-// 8 token tiles x all row tiles (token tile fastest), so that the CTAs in flight share weight tiles and the group's
-// activation tiles stay in L2.  The plain form double-buffers the accumulator in tensor memory: the epilogue of tile
-// i runs while the MMAs of tile i+1 fill the other buffer, and the TMA ring never drains between tiles.
-template <bool GATED>
-__global__ void __launch_bounds__(kGemmThreads, 1) gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-    using S = GemmSmem<GATED>;
-    constexpr int STAGES = S::stages;
-    constexpr int ACC = S::acc_bufs;
-    constexpr uint32_t ACC_COLS = GATED ? 512 : 256;
-    constexpr uint32_t TMEM_COLS = 512;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::off_bar);
-    uint64_t *empty = full + STAGES;
-    uint64_t *acc_full = empty + STAGES;
-    uint64_t *acc_empty = acc_full + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
-    __shared__ int s_abort;
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int k_blocks = (p.k + kBK - 1) / kBK;
-    const int n_row_tiles = (p.n_out + kBM - 1) / kBM, n_tok_tiles = (p.m + kBN - 1) / kBN;
-    const bool grouped = p.items != nullptr;
-    const int total_tiles = grouped ? (p.n_items_dev ? *p.n_items_dev : p.n_items) : n_row_tiles * n_tok_tiles;
-    auto tile_coords = [&](int tile, int &row0, int &tok0, int &tok_end, int &z) {
-        if (grouped) {
-            const int4 it = p.items[tile];
-            z = it.x;
-            row0 = it.y;
-            tok0 = it.z;
-            tok_end = it.w;
-            return;
-        }
-        z = 0;
-        tok_end = p.m;
-        const int per_group = kTokGroup * n_row_tiles;
-        const int group = tile / per_group, in_group = tile - group * per_group;
-        const int group_toks = (n_tok_tiles - group * kTokGroup) < kTokGroup ? (n_tok_tiles - group * kTokGroup) : kTokGroup;
-        row0 = (in_group / group_toks) * kBM;
-        tok0 = (group * kTokGroup + in_group % group_toks) * kBN;
-    };
-
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full[s], 1);
-            mbar_init(&empty[s], 1);
-        }
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
-        }
-        fence_mbar_init();
-        s_abort = 0;
-        tma_prefetch_desc(&map_w);
-        tma_prefetch_desc(&map_x);
-        if (GATED) tma_prefetch_desc(&map_w2);
-    }
-    if (warp == 1) {
-        tmem_alloc(tmem_slot, TMEM_COLS);
-        tmem_relinquish();
-    }
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
-
-    if (warp == 0) {
-        // ------------------------------------------------ TMA producer
-        if (lane == 0) {
-            long long kg = 0;  // k-block counter over all tiles of this CTA: ring position
-            for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
-                int row0, tok0, tok_end, z;
-                tile_coords(tile, row0, tok0, tok_end, z);
-                for (int kb = 0; kb < k_blocks; ++kb, ++kg) {
-                    const int s = (int)(kg % STAGES);
-                    if (kg >= STAGES && !wait_flag(&empty[s], (uint32_t)((kg / STAGES) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout)) break;
-                    uint8_t *st = smem + (size_t)s * S::stage_bytes;
-                    mbar_expect_tx(&full[s], S::stage_bytes);
-                    if (grouped) {
-                        tma_load_3d(st, &map_w, &full[s], kb * kBK, row0, z);
-                        if (GATED) tma_load_3d(st + S::a_bytes, &map_w2, &full[s], kb * kBK, row0, z);
-                    } else {
-                        tma_load_2d(st, &map_w, &full[s], kb * kBK, row0);
-                        if (GATED) tma_load_2d(st + S::a_bytes, &map_w2, &full[s], kb * kBK, row0);
-                    }
-                    tma_load_2d(st + (GATED ? 2 : 1) * S::a_bytes, &map_x, &full[s], kb * kBK, tok0);
-                }
-                if (*(volatile int *)&s_abort) break;
-            }
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            long long kg = 0;
-            int iter = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++iter) {
-                // instruction descriptor: f32 accumulator, f16 A and B, both K-major, M = 128, N = the tile's token
-                // count rounded up to 16 (a ragged last tile of a matrix does not pay for 256 columns)
-                int row0, tok0, tok_end, z;
-                tile_coords(tile, row0, tok0, tok_end, z);
-                int n_eff = tok_end - tok0;
-                n_eff = n_eff >= kBN ? kBN : ((n_eff + 15) & ~15);
-                if (n_eff < 16) n_eff = 16;
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(n_eff >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-                const int b = iter % ACC;
-                if (iter >= ACC) ok = wait_flag(&acc_empty[b], (uint32_t)((iter / ACC) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t acc_addr = tmem_base + (uint32_t)b * ACC_COLS;
-                for (int kb = 0; kb < k_blocks && ok; ++kb, ++kg) {
-                    const int s = (int)(kg % STAGES);
-                    ok = wait_flag(&full[s], (uint32_t)(kg / STAGES) & 1, &s_abort, p.status, kStatusTmaTimeout);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t st = smem_u32(smem + (size_t)s * S::stage_bytes);
-                    const uint64_t da = make_sw128_desc(st);
-                    const uint64_t da2 = make_sw128_desc(st + S::a_bytes);
-                    const uint64_t db = make_sw128_desc(st + (GATED ? 2 : 1) * S::a_bytes);
-#pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) {
-                        const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-                        // 16 K elements = 32 bytes = 2 descriptor units along the swizzled row
-                        umma_f16_ss(acc_addr, da + 2 * k, db + 2 * k, idesc, acc);
-                        if (GATED) umma_f16_ss(acc_addr + kBN, da2 + 2 * k, db + 2 * k, idesc, acc);
-                    }
-                    tc_commit(&empty[s]);  // arrives once the MMAs above have read the stage
-                }
-                tc_commit(&acc_full[b]);   // arrives when every MMA of the tile has completed
-            }
-        }
-    } else {
-        // ------------------------------------------------ epilogue: warp q of 4 owns TMEM lanes 32q..32q+31
-        const int q = warp & 3;
-        int iter = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++iter) {
-            int row0, tok0, tok_end, z;
-            tile_coords(tile, row0, tok0, tok_end, z);
-            const int b = iter % ACC;
-            const int row = row0 + q * 32 + lane;
-            const bool ok = wait_flag(&acc_full[b], (uint32_t)(iter / ACC) & 1, &s_abort, p.status, kStatusMmaTimeout);
-            tc_fence_after();
-            if (ok) {
-                const uint32_t lane_base = tmem_base + (uint32_t)b * ACC_COLS + ((uint32_t)(q * 32) << 16);
-                for (int c0 = 0; c0 < kBN; c0 += 16) {
-                    if (tok0 + c0 >= tok_end) break;  // warp-uniform
-                    uint32_t v[16], u[16];
-                    tmem_ld16(lane_base + c0, v);
-                    if (GATED) tmem_ld16(lane_base + kBN + c0, u);
-                    tmem_ld_wait();
-                    if (row < p.n_out) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int tok = tok0 + c0 + j;
-                            if (tok < tok_end) {
-                                float val = __uint_as_float(v[j]);
-                                if (GATED) {
-                                    const float up = __uint_as_float(u[j]);
-                                    val = (val / (1.0f + expf(-val))) * up;  // src/kernel/cpu/ggml_quant.rs:352
-                                }
-                                const size_t o = (size_t)tok * p.n_out + row;
-                                if (p.residual) val += load_as_f32(p.residual, p.y_dtype, o);
-                                store_from_f32(p.y, p.y_dtype, o, val);
-                            }
-                        }
-                    }
-                }
-            }
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);  // this warp's quarter of the accumulator may be overwritten
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
-}
-
-// ---------------------------------------------------------------------------------------------------------------
-// Fused form for Q4_K: the packed weight tile is dequantised inside the kernel, straight into the swizzled shared-
-// memory operand the tensor core reads, so the weight crosses HBM once (0.56 bytes per weight instead of the
-// 0.56 + 2 + 2 of a separate f16 operand pass).  Same tile walk, MMA issue and epilogue as gemm_kernel; what differs is
-// the A side of the ring:
-//   warp 0        TMA: one packed box per 256 K columns (128 rows x 144 bytes) into a 2-deep ring, and the
-//                 activation k-blocks (256 tokens x 64 K, 128-byte swizzle) into the main ring
-//   warps 6..13   dequantisers: thread = (row, half of the 64-column k-block) = one 32-weight scale group; reads the
-//                 group's packed bytes and (once per super-block) the row's scales from the packed box, forms
-//                 fma(d*sc, q, -dmin*m) in f32, rounds once to f16 and stores its four
-//                 16-byte chunks at their 128-byte-swizzle positions (chunk c of row r sits at c ^ (r & 7)), then
-//                 fence.proxy.async and one arrival per warp on the stage's a_full barrier
-//   warp 1        waits for a_full and b_full of a stage, issues the four K=16 MMAs, commits the stage's `empty`
-// The operand bits are exactly those the separate operand pass writes (same formula), so both paths give identical
-// results.  A last warp issues the packed boxes on a ring of its own.
-// ---------------------------------------------------------------------------------------------------------------
-constexpr int kFusedDqWarps = 8;   // thread = (row, half of the k-block) = one 32-weight scale group
-constexpr int kFusedThreads = (7 + kFusedDqWarps) * 32;  // + TMA (activations), MMA, 4 epilogue, TMA (packed boxes)
-constexpr int kFusedPackedWarp = 6 + kFusedDqWarps;
-constexpr int kQ4kUnitBytes = 144;
-
-template <bool GATED> struct FusedSmem {
-    static constexpr int stages = GATED ? 2 : 3;
-    static constexpr int pstages = GATED ? 2 : 3;
-    static constexpr int acc_bufs = GATED ? 1 : 2;
-    static constexpr int a_bytes = kBM * kBK * 2;
-    static constexpr int b_bytes = kBN * kBK * 2;
-    static constexpr int p_bytes = kBM * kQ4kUnitBytes;  // one packed box
-    static constexpr int stage_bytes = (GATED ? 2 : 1) * a_bytes + b_bytes;
-    static constexpr int pstage_bytes = (GATED ? 2 : 1) * p_bytes;
-    static constexpr int off_p = stages * stage_bytes;
-    static constexpr int off_bar = off_p + pstages * pstage_bytes;
-    static constexpr int total = off_bar + 512 + 1024;
+// A piece of work of one pair: K steps [k0, k1) of a tile.
+struct GemmSeg {
+    int row0, tok0, tok_end, z, k0, k1, tile;
 };
-
-// One scale group (32 weights) of one row of a packed Q4_K box -> 32 f16 in the swizzled A tile.
-// Integer -> float without the conversion unit: byte q under the exponent of 2^23 is the float 2^23 + q, and
-// subtracting 2^23 is exact, so d*sc*q - dmin*m comes out with the codec's own two roundings.
-__device__ __forceinline__ float nib_to_float(uint32_t masked, int byte) {
-    uint32_t r;
-    switch (byte) {
-    case 0: asm("prmt.b32 %0, %1, %2, 0x7540;" : "=r"(r) : "r"(masked), "r"(0x4B000000u)); break;
-    case 1: asm("prmt.b32 %0, %1, %2, 0x7541;" : "=r"(r) : "r"(masked), "r"(0x4B000000u)); break;
-    case 2: asm("prmt.b32 %0, %1, %2, 0x7542;" : "=r"(r) : "r"(masked), "r"(0x4B000000u)); break;
-    default: asm("prmt.b32 %0, %1, %2, 0x7543;" : "=r"(r) : "r"(masked), "r"(0x4B000000u)); break;
-    }
-    return __fadd_rn(__uint_as_float(r), -8388608.0f);
-}
-
-// The f16 operand value of a Q4_K weight, as both GEMM paths form it: fma(d*sc, q, -(dmin*m)) in f32 (one rounding,
-// slightly closer to the exact value than the codec's multiply-then-subtract), rounded once to f16.
-__device__ __forceinline__ uint32_t q4k_pair_f16(float dsc, float ndm, float qa, float qb) { return h2_as_u32(__floats2half2_rn(fmaf(dsc, qa, ndm), fmaf(dsc, qb, ndm))); }
-
-// The 8 (d*sc, -dmin*m) pairs of one super-block header (src/weight/codec/ggml.rs:471-473).
-__device__ __forceinline__ void q4k_group_scales(const uint4 &hdr, int g, float &dsc, float &ndm) {
-    const __half2 dd = u32_as_h2(hdr.x);
-    const float d = __low2float(dd), dmin = __high2float(dd);
-    uint32_t sc, mn;
-    if (g < 4) {
-        sc = (hdr.y >> (8 * g)) & 63u;
-        mn = (hdr.z >> (8 * g)) & 63u;
-    } else {
-        const int j = 8 * (g - 4);
-        sc = ((hdr.w >> j) & 0x0Fu) | (((hdr.y >> (j + 6)) & 3u) << 4);
-        mn = ((hdr.w >> (j + 4)) & 0x0Fu) | (((hdr.z >> (j + 6)) & 3u) << 4);
-    }
-    dsc = __fmul_rn(d, (float)sc);
-    ndm = -__fmul_rn(dmin, (float)mn);
-}
-
-// One scale group (32 weights: low or high nibbles of the pair's 32 quant bytes) of one row of a packed Q4_K box ->
-// 32 f16 in the swizzled A tile (the four 16-byte chunks 4 half .. 4 half + 3 of row `row`).
-__device__ __forceinline__ void dequant_group_to_sw128(const uint8_t *unit, int pair, int half, float dsc, float ndm, uint8_t *a_tile, int row) {
-    const uint4 q0 = *reinterpret_cast<const uint4 *>(unit + 16 + pair * 32), q1 = *reinterpret_cast<const uint4 *>(unit + 16 + pair * 32 + 16);
-    const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-    const int shift = half * 4;
-    uint8_t *row_base = a_tile + (row >> 3) * 1024 + (row & 7) * 128;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {  // chunk = 8 consecutive K = 2 packed words
-        uint32_t h[4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const uint32_t m = (qw[2 * c + j] >> shift) & 0x0F0F0F0Fu;
-            h[2 * j] = q4k_pair_f16(dsc, ndm, nib_to_float(m, 0), nib_to_float(m, 1));
-            h[2 * j + 1] = q4k_pair_f16(dsc, ndm, nib_to_float(m, 2), nib_to_float(m, 3));
+// Walks a pair's share: first its part of the cut tiles, then its whole tiles.
+struct GemmWalk {
+    int q, q1, tile, stride, total, steps, row_tiles, tok_tiles, rows_per_tile;
+    __device__ __forceinline__ GemmWalk(const GemmParams &p, int pair, int pairs, int rows_per_tile_) {
+        rows_per_tile = rows_per_tile_;
+        steps = (p.k + kStepK - 1) / kStepK;
+        row_tiles = (p.n_out + rows_per_tile - 1) / rows_per_tile;
+        tok_tiles = (p.m + p.bn - 1) / p.bn;
+        total = p.items ? (p.n_items_dev ? *p.n_items_dev : p.n_items) : row_tiles * tok_tiles;
+        stride = pairs;
+        const long long cut = (long long)p.cut_tiles * steps;
+        q = q1 = 0;
+        if (pair < p.cut_pairs) {
+            q = (int)(pair * cut / p.cut_pairs);
+            q1 = (int)((pair + 1) * cut / p.cut_pairs);
         }
-        const int chunk = half * 4 + c;
-        *reinterpret_cast<uint4 *>(row_base + ((chunk ^ (row & 7)) << 4)) = make_uint4(h[0], h[1], h[2], h[3]);
+        tile = p.cut_tiles + pair;
     }
+    __device__ __forceinline__ bool next(const GemmParams &p, GemmSeg &s) {
+        if (q < q1) {
+            s.tile = q / steps;
+            s.k0 = q - s.tile * steps;
+            s.k1 = s.k0 + (q1 - q) < steps ? s.k0 + (q1 - q) : steps;
+            q += s.k1 - s.k0;
+        } else if (tile < total) {
+            s.tile = tile;
+            s.k0 = 0;
+            s.k1 = steps;
+            tile += stride;
+        } else {
+            return false;
+        }
+        if (p.items) {
+            const int4 it = p.items[s.tile];
+            s.z = it.x;
+            s.row0 = it.y;
+            s.tok0 = it.z;
+            s.tok_end = it.w < it.z + kBN ? it.w : it.z + kBN;
+            return true;
+        }
+        s.z = 0;
+        const int per_group = kTokGroup * row_tiles;
+        const int group = s.tile / per_group, in_group = s.tile - group * per_group;
+        const int group_toks = (tok_tiles - group * kTokGroup) < kTokGroup ? (tok_tiles - group * kTokGroup) : kTokGroup;
+        s.row0 = (in_group / group_toks) * rows_per_tile;
+        s.tok0 = (group * kTokGroup + in_group % group_toks) * p.bn;
+        s.tok_end = s.tok0 + p.bn < p.m ? s.tok0 + p.bn : p.m;
+        return true;
+    }
+};
+// columns the MMA of a tile computes: its tokens, rounded up to 32 (16 per SM)
+__device__ __forceinline__ int tile_cols(const GemmSeg &s) {
+    const int n = (s.tok_end - s.tok0 + 31) & ~31;
+    return n > kBN ? kBN : n < 32 ? 32 : n;
 }
 
-template <bool GATED>
-__global__ void __launch_bounds__(kFusedThreads, 1) gemm_q4k_fused_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-    using S = FusedSmem<GATED>;
-    constexpr int STAGES = S::stages;
-    constexpr int PST = S::pstages;
-    constexpr int ACC = S::acc_bufs;
-    constexpr uint32_t ACC_COLS = GATED ? 512 : 256;
-    constexpr uint32_t TMEM_COLS = 512;
+template <uint32_t SRC, bool GATED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threads, 1)
+    gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
+    using S = GemmSmem<SRC>;
+    constexpr int STAGES = S::stages, PST = S::pstages > 0 ? S::pstages : 1;
+    constexpr int kRows = GATED ? kPairM / 2 : kPairM;  // output rows of a tile
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *a_full = reinterpret_cast<uint64_t *>(smem + S::off_bar);
-    uint64_t *b_full = a_full + STAGES;
-    uint64_t *empty = b_full + STAGES;
-    uint64_t *p_full = empty + STAGES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::off_bar);  // first SM: a stage's operands, both SMs' bytes and dequantiser warps
+    uint64_t *empty = full + STAGES;                                   // each SM: the stage's MMAs are done
+    uint64_t *p_full = empty + STAGES;                                 // each SM: packed boxes
     uint64_t *p_empty = p_full + PST;
-    uint64_t *acc_full = p_empty + PST;
-    uint64_t *acc_empty = acc_full + 2;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(acc_empty + 2);
-    __shared__ int s_abort;
+    uint64_t *acc_full = p_empty + PST;                                // each SM
+    uint64_t *acc_empty = acc_full + 2;                                // first SM: both SMs' epilogue warps
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort, s_last;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int n_sb = p.k / kUnitWeights;  // Q4_K: K is a multiple of 256
-    const int n_row_tiles = (p.n_out + kBM - 1) / kBM, n_tok_tiles = (p.m + kBN - 1) / kBN;
-    const bool grouped = p.items != nullptr;
-    const int total_tiles = grouped ? (p.n_items_dev ? *p.n_items_dev : p.n_items) : n_row_tiles * n_tok_tiles;
-    auto tile_coords = [&](int tile, int &row0, int &tok0, int &tok_end, int &z) {
-        if (grouped) {
-            const int4 it = p.items[tile];
-            z = it.x;
-            row0 = it.y;
-            tok0 = it.z;
-            tok_end = it.w;
-            return;
-        }
-        z = 0;
-        tok_end = p.m;
-        const int per_group = kTokGroup * n_row_tiles;
-        const int group = tile / per_group, in_group = tile - group * per_group;
-        const int group_toks = (n_tok_tiles - group * kTokGroup) < kTokGroup ? (n_tok_tiles - group * kTokGroup) : kTokGroup;
-        row0 = (in_group / group_toks) * kBM;
-        tok0 = (group * kTokGroup + in_group % group_toks) * kBN;
-    };
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the shuffle tells the compiler that it is uniform
+    const uint32_t rank = pair_rank();
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+    // Packed rows end on whole units (zero blocks): their padding is multiplied like the rest, against columns the TMA unit fills
+    // with zeros, so that every dequantiser warp has its turn in every unit.  A warp that skipped turns could meet a stage
+    // barrier two phases behind, which its parity cannot tell from one phase ahead.
+    const int k_blocks = SRC ? 4 * ((p.k + kStepK - 1) / kStepK) : (p.k + kBK - 1) / kBK;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&a_full[s], kFusedDqWarps);
-            mbar_init(&b_full[s], 1);
+            mbar_init(&full[s], SRC ? 9 : 1);  // the TMA issuer, and four dequantiser warps of each SM
             mbar_init(&empty[s], 1);
         }
         for (int s = 0; s < PST; ++s) {
             mbar_init(&p_full[s], 1);
-            mbar_init(&p_empty[s], kFusedDqWarps);
+            mbar_init(&p_empty[s], kDqWarps);
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 4);
+            mbar_init(&acc_empty[b], 8);
         }
         fence_mbar_init();
         s_abort = 0;
@@ -457,189 +312,312 @@ __global__ void __launch_bounds__(kFusedThreads, 1) gemm_q4k_fused_kernel(const 
         if (GATED) tma_prefetch_desc(&map_w2);
     }
     if (warp == 1) {
-        tmem_alloc(tmem_slot, TMEM_COLS);
-        tmem_relinquish();
+        tmem_alloc2(&s_tmem, 512);
+        tmem_relinquish2();
     }
     tc_fence_before();
     __syncthreads();
+    pair_sync();  // both SMs' barriers and tensor memory exist
     tc_fence_after();
-    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(tmem_slot);
+    const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&s_tmem);
+    const uint32_t abort_addr = smem_u32(&s_abort);
+    GemmWalk walk(p, pair, pairs, kRows);
+    GemmSeg sg;
 
     if (warp == 0) {
-        // ------------------------------------------------ TMA producer: activation k-blocks
-        if (lane == 0) {
-            long long kg = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                int row0, tok0, tok_end, z;
-                tile_coords(tile, row0, tok0, tok_end, z);
-                for (int kb = 0; kb < n_sb * (kUnitWeights / kBK) && ok; ++kb, ++kg) {
-                    const int s = (int)(kg % STAGES);
-                    if (kg >= STAGES) ok = wait_flag(&empty[s], (uint32_t)((kg / STAGES) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout);
-                    if (!ok) break;
-                    uint8_t *st = smem + (size_t)s * S::stage_bytes;
-                    mbar_expect_tx(&b_full[s], S::b_bytes);
-                    tma_load_2d(st + (GATED ? 2 : 1) * S::a_bytes, &map_x, &b_full[s], kb * kBK, tok0);
+        // ------------------------------------------------ TMA: tokens (half a tile each), and the f16 weight operand
+        int s = 0;
+        uint32_t ph = 0;
+        bool ok = true, fresh = true;  // fresh: first turn of the ring
+        const uint32_t bytes = 2u * (uint32_t)((SRC ? 0 : S::a_bytes) + p.box_tok * kBK * 2);
+        while (ok && walk.next(p, sg)) {
+            const int tok = sg.tok0 + (int)rank * (tile_cols(sg) / 2);
+            const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
+            const int kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
+            for (int kb = sg.k0 * 4; kb < kb1; ++kb) {
+                if (!fresh && !wait_flag(&empty[s], ph ^ 1u, abort_addr, p.status, kStatusMmaTimeout)) {
+                    ok = false;
+                    break;
                 }
-            }
-        }
-    } else if (warp == kFusedPackedWarp) {
-        // ------------------------------------------------ TMA producer: packed boxes, a ring of their own, so that a box
-        // is requested as soon as the dequantisers free its slot, not when the activation ring gets round to it
-        if (lane == 0) {
-            long long pq = 0;
-            bool ok = true;
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-                int row0, tok0, tok_end, z;
-                tile_coords(tile, row0, tok0, tok_end, z);
-                const CUtensorMap *mw = grouped ? &p.w_maps[z] : &map_w;
-                const CUtensorMap *mw2 = grouped ? (GATED ? &p.w2_maps[z] : mw) : &map_w2;
-                for (int sb = 0; sb < n_sb && ok; ++sb, ++pq) {
-                    const int ps = (int)(pq % PST);
-                    if (pq >= PST) ok = wait_flag_backoff(&p_empty[ps], (uint32_t)((pq / PST) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout, 100);
-                    if (!ok) break;
-                    uint8_t *pst = smem + S::off_p + (size_t)ps * S::pstage_bytes;
-                    mbar_expect_tx(&p_full[ps], S::pstage_bytes);
-                    tma_load_2d(pst, mw, &p_full[ps], sb * (kQ4kUnitBytes / 4), row0);
-                    if (GATED) tma_load_2d(pst + S::p_bytes, mw2, &p_full[ps], sb * (kQ4kUnitBytes / 4), row0);
+                if (elect_one()) {
+                    uint8_t *st = smem + (size_t)s * S::stage_bytes;
+                    const uint32_t bar = pair_first(smem_u32(&full[s]));
+                    if (rank == 0) mbar_expect_tx(&full[s], bytes);
+                    if constexpr (SRC == 0) {
+                        if (p.items) {
+                            tma_load_3d_pair(st, &map_w, bar, kb * kBK, row, sg.z);
+                            if (GATED) tma_load_3d_pair(st + S::a_bytes / 2, &map_w2, bar, kb * kBK, row, sg.z);
+                        } else {
+                            tma_load_2d_pair(st, &map_w, bar, kb * kBK, row);
+                            if (GATED) tma_load_2d_pair(st + S::a_bytes / 2, &map_w2, bar, kb * kBK, row);
+                        }
+                    }
+                    tma_load_2d_pair(st + S::a_bytes, &map_x, bar, kb * kBK, tok);
+                }
+                __syncwarp();
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                    fresh = false;
                 }
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------ MMA issuer
-        if (lane == 0) {
-            long long kg = 0;
-            int iter = 0;
+        // ------------------------------------------------ MMA issue
+        if (rank == 0) {
+            int s = 0, iter = 0;
+            uint32_t ph = 0;
             bool ok = true;
-            const int k_blocks = n_sb * (kUnitWeights / kBK);
-            for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++iter) {
-                int row0, tok0, tok_end, z;
-                tile_coords(tile, row0, tok0, tok_end, z);
-                int n_eff = tok_end - tok0;
-                n_eff = n_eff >= kBN ? kBN : ((n_eff + 15) & ~15);
-                if (n_eff < 16) n_eff = 16;
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(n_eff >> 3) << 17) | ((uint32_t)(kBM >> 4) << 24);
-                const int b = iter % ACC;
-                if (iter >= ACC) ok = wait_flag(&acc_empty[b], (uint32_t)((iter / ACC) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout);
+            const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
+            for (; ok && walk.next(p, sg); ++iter) {
+                // f32 accumulator, f16 A and B, both K-major, M = 256, N = the tile's tokens
+                const uint32_t idesc = (1u << 4) | ((uint32_t)(tile_cols(sg) >> 3) << 17) | ((uint32_t)(kPairM >> 4) << 24);
+                const int b = iter & 1;
+                if (iter >= 2) ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, abort_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc_addr = tmem_base + (uint32_t)b * ACC_COLS;
-                for (int kb = 0; kb < k_blocks && ok; ++kb, ++kg) {
-                    const int s = (int)(kg % STAGES);
-                    ok = wait_flag(&b_full[s], (uint32_t)(kg / STAGES) & 1, &s_abort, p.status, kStatusTmaTimeout);
-                    if (ok) ok = wait_flag(&a_full[s], (uint32_t)(kg / STAGES) & 1, &s_abort, p.status, kStatusMmaTimeout);
+                const uint32_t acc = tmem_base + (uint32_t)b * kBN;
+                const int kb0 = sg.k0 * 4, kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
+                for (int kb = kb0; kb < kb1; ++kb) {
+                    ok = wait_flag(&full[s], ph, abort_addr, p.status, kStatusTmaTimeout);
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t st = smem_u32(smem + (size_t)s * S::stage_bytes);
-                    const uint64_t da = make_sw128_desc(st);
-                    const uint64_t da2 = make_sw128_desc(st + S::a_bytes);
-                    const uint64_t db = make_sw128_desc(st + (GATED ? 2 : 1) * S::a_bytes);
+                    if (elect_one()) {
+                        const uint64_t da = desc0 + (uint32_t)(s * (S::stage_bytes / 16)), db = da + S::a_bytes / 16;
 #pragma unroll
-                    for (int k = 0; k < kBK / 16; ++k) {
-                        const uint32_t acc = (kb > 0 || k > 0) ? 1u : 0u;
-                        umma_f16_ss(acc_addr, da + 2 * k, db + 2 * k, idesc, acc);
-                        if (GATED) umma_f16_ss(acc_addr + kBN, da2 + 2 * k, db + 2 * k, idesc, acc);
+                        for (int k = 0; k < kBK / 16; ++k)  // 16 K elements = 32 bytes = 2 descriptor units along the swizzled row
+                            umma2_f16_ss(acc, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        tc_commit2(&empty[s]);
+                        if (kb + 1 == kb1) tc_commit2(&acc_full[b]);
                     }
-                    tc_commit(&empty[s]);
+                    __syncwarp();
+                    if (++s == STAGES) {
+                        s = 0;
+                        ph ^= 1u;
+                    }
                 }
-                tc_commit(&acc_full[b]);
             }
         }
     } else if (warp < 6) {
-        // ------------------------------------------------ epilogue: warp q of 4 owns TMEM lanes 32q..32q+31
+        // ------------------------------------------------ epilogue: warp q of 4 owns TMEM lanes 32q..32q+31 = the SM's operand rows
         const int q = warp & 3;
+        float *xch = reinterpret_cast<float *>(smem + S::off_x) + (q & 1) * (2 * 16 * 32);
         int iter = 0;
-        for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++iter) {
-            int row0, tok0, tok_end, z;
-            tile_coords(tile, row0, tok0, tok_end, z);
-            const int b = iter % ACC;
-            const int row = row0 + q * 32 + lane;
-            const bool ok = wait_flag_backoff(&acc_full[b], (uint32_t)(iter / ACC) & 1, &s_abort, p.status, kStatusMmaTimeout, 400);
+        const int et = (warp - 2) * 32 + lane;
+        for (; walk.next(p, sg); ++iter) {
+            const int b = iter & 1;
+            const int n_tok = sg.tok_end - sg.tok0;
+            if (!GATED && p.residual) {
+                // bring the tile's residual rows into L2 while its MMAs run: a warp can only have a few KB of loads in flight below
+                const size_t esz = dtype_size(p.y_dtype), r0 = (size_t)sg.row0 + rank * kBM;
+                const size_t bytes = (size_t)p.n_out * esz;
+                for (int i = et; i < n_tok * (int)esz; i += 128) {  // 128 rows = esz lines of 128 bytes per token
+                    const size_t at = r0 * esz + (size_t)(i % (int)esz) * 128;
+                    if (at < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(p.residual) + (size_t)(sg.tok0 + i / (int)esz) * bytes + at));
+                }
+            }
+            // the four warps go on together or not at all: they meet at barriers below (and the exchange buffer is free again)
+            const bool ok = epilogue_all(wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, abort_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0));
             tc_fence_after();
-            if (ok) {
-                const uint32_t lane_base = tmem_base + (uint32_t)b * ACC_COLS + ((uint32_t)(q * 32) << 16);
-                for (int c0 = 0; c0 < kBN; c0 += 16) {
-                    if (tok0 + c0 >= tok_end) break;  // warp-uniform
-                    uint32_t v[16], u[16];
-                    tmem_ld16(lane_base + c0, v);
-                    if (GATED) tmem_ld16(lane_base + kBN + c0, u);
-                    tmem_ld_wait();
-                    if (row < p.n_out) {
+            const uint32_t acc = tmem_base + (uint32_t)b * kBN + ((uint32_t)(q * 32) << 16);
+            const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
+            // output row of this lane; gated: warps 0, 1 hold gate rows, warps 2, 3 the up rows of the same outputs
+            const int row = GATED ? sg.row0 + (int)rank * 64 + (q & 1) * 32 + lane : sg.row0 + (int)rank * kBM + q * 32 + lane;
+            // 16 columns of finished sums (f32 bits) -> y
+            auto store16 = [&](int c0, uint32_t (&v)[16]) {
+                if (GATED) {
+                    // the two warps of one row half trade: the gate warp finishes columns 0..7 of the chunk, the up warp 8..15
+                    float *xb = xch + ((c0 >> 4) & 1) * (16 * 32);  // [which half travels][8 columns][32 rows]; rewritten two chunks later, behind the barrier in between
+                    const bool is_up = q >= 2;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int tok = tok0 + c0 + j;
-                            if (tok < tok_end) {
-                                float val = __uint_as_float(v[j]);
-                                if (GATED) {
-                                    const float up = __uint_as_float(u[j]);
-                                    val = (val / (1.0f + expf(-val))) * up;  // src/kernel/cpu/ggml_quant.rs:352
-                                }
-                                const size_t o = (size_t)tok * p.n_out + row;
-                                if (p.residual) val += load_as_f32(p.residual, p.y_dtype, o);
-                                store_from_f32(p.y, p.y_dtype, o, val);
-                            }
+                    for (int j = 0; j < 8; ++j) xb[((is_up ? 0 : 8) + j) * 32 + lane] = __uint_as_float(is_up ? v[j] : v[8 + j]);
+                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+                    if (row >= p.n_out) return;
+                    const int cb = c0 + (is_up ? 8 : 0);
+                    const size_t o = (size_t)(sg.tok0 + cb) * p.n_out + row;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        const float other = xb[((is_up ? 8 : 0) + j) * 32 + lane], mine = __uint_as_float(is_up ? v[8 + j] : v[j]);
+                        const float g = is_up ? other : mine, u = is_up ? mine : other;
+                        if (cb + j < n_tok) store_from_f32(p.y, p.y_dtype, o + (size_t)j * p.n_out, (g / (1.0f + expf(-g))) * u);  // src/kernel/cpu/ggml_quant.rs:352
+                    }
+                    return;
+                }
+                if (row >= p.n_out) return;
+                const size_t o = (size_t)(sg.tok0 + c0) * p.n_out + row;
+                if (p.residual) {  // all loads of the chunk, unconverted, before anything uses one (and before the first store: y may be the residual's own buffer)
+                    uint32_t r[16];
+                    if (p.y_dtype == ZQ_F32) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[j] = c0 + j < n_tok ? reinterpret_cast<const uint32_t *>(p.residual)[o + (size_t)j * p.n_out] : 0u;
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[j] = c0 + j < n_tok ? reinterpret_cast<const uint16_t *>(p.residual)[o + (size_t)j * p.n_out] : 0u;
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) r[j] = p.y_dtype == ZQ_F16 ? __float_as_uint(__half2float(__ushort_as_half((unsigned short)r[j]))) : r[j] << 16;
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(r[j]));
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j)
+                    if (c0 + j < n_tok) store_from_f32(p.y, p.y_dtype, o + (size_t)j * p.n_out, __uint_as_float(v[j]));
+            };
+            if (ok && whole) {
+                for (int c0 = 0; c0 < n_tok; c0 += 16) {  // warp-uniform
+                    uint32_t v[16];
+                    tmem_ld16(acc + c0, v);
+                    store16(c0, v);
+                }
+            }
+            if (!whole) {
+                // A share of a cut tile.  Whoever comes last adds the other shares from their slots to its own, in pair order;
+                // everyone else leaves its share in its slot and goes on.
+                const long long Q = (long long)p.cut_tiles * walk.steps, G = p.cut_pairs, ts = (long long)sg.tile * walk.steps;
+                const int c_first = (int)(((ts + 1) * G - 1) / Q), c_last = (int)(((ts + walk.steps) * G - 1) / Q);  // pairs that own the tile's first and last step
+                uint32_t *counter = p.counters + 2 * c_first + rank;
+                const uint32_t others = (uint32_t)(c_last - c_first);
+                if (et == 0) s_last = *reinterpret_cast<volatile uint32_t *>(counter) == others;
+                asm volatile("bar.sync 3, 128;" ::: "memory");
+                bool last = s_last != 0;
+                if (!last) {
+                    float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * (kBN * kBM) + q * 32 + lane;
+                    if (ok) {
+                        for (int c0 = 0; c0 < n_tok; c0 += 16) {
+                            uint32_t v[16];
+                            tmem_ld16(acc + c0, v);
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) __stcg(slot + (size_t)(c0 + j) * kBM, __uint_as_float(v[j]));
                         }
                     }
+                    __threadfence();
+                    asm volatile("bar.sync 3, 128;" ::: "memory");
+                    if (et == 0) s_last = atomicAdd(counter, 1u) == others;
+                    asm volatile("bar.sync 3, 128;" ::: "memory");
+                    last = s_last != 0;
+                }
+                if (last && ok) {
+                    __threadfence();
+                    const float *base = p.partials + (size_t)rank * (kBN * kBM) + q * 32 + lane;
+                    for (int c0 = 0; c0 < n_tok; c0 += 16) {
+                        uint32_t v[16];
+                        for (int c = c_first; c <= c_last; ++c) {
+                            if (c == pair) {
+                                uint32_t own[16];
+                                tmem_ld16(acc + c0, own);
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) v[j] = c == c_first ? own[j] : __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(own[j]));
+                            } else {
+                                const float *src = base + (size_t)(2 * c + (c == c_first ? 1 : 0)) * 2 * (kBN * kBM) + (size_t)c0 * kBM;
+                                float n[16];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) n[j] = __ldcg(src + (size_t)j * kBM);
+#pragma unroll
+                                for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(c == c_first ? n[j] : __uint_as_float(v[j]) + n[j]);
+                            }
+                        }
+                        store16(c0, v);
+                    }
+                    if (et == 0) *counter = 0;  // ready for the next launch
                 }
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[b]);
+            if (lane == 0) pair_arrive(pair_first(smem_u32(&acc_empty[b])));  // this warp's part of the accumulator may be overwritten
         }
-    } else {
-        // ------------------------------------------------ dequantisers: thread = (row, half of the k-block)
-        const int t = threadIdx.x - 6 * 32;
-        const int row = t & (kBM - 1), half = t >> 7;
-        long long kg = 0, pq = 0;
-        bool ok = true;
-        for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-            for (int sb = 0; sb < n_sb && ok; ++sb, ++pq) {
-                const int ps = (int)(pq % PST);
-                ok = wait_flag_backoff(&p_full[ps], (uint32_t)(pq / PST) & 1, &s_abort, p.status, kStatusTmaTimeout, 60);
-                if (!ok) break;
-                const uint8_t *u0 = smem + S::off_p + (size_t)ps * S::pstage_bytes + (size_t)row * kQ4kUnitBytes;
-                const uint8_t *u1 = u0 + S::p_bytes;
-                // the four groups this thread will meet in this super-block: 2 kb + half
-                float dsc0[4], ndm0[4], dsc1[4], ndm1[4];
-                {
-                    const uint4 hdr = *reinterpret_cast<const uint4 *>(u0);
-#pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) q4k_group_scales(hdr, 2 * kb + half, dsc0[kb], ndm0[kb]);
-                }
-                if (GATED) {
-                    const uint4 hdr = *reinterpret_cast<const uint4 *>(u1);
-#pragma unroll
-                    for (int kb = 0; kb < 4; ++kb) q4k_group_scales(hdr, 2 * kb + half, dsc1[kb], ndm1[kb]);
-                }
-#pragma unroll
-                for (int kb = 0; kb < kUnitWeights / kBK; ++kb, ++kg) {
-                    if (!ok) break;
-                    const int s = (int)(kg % STAGES);
-                    if (kg >= STAGES) ok = wait_flag_backoff(&empty[s], (uint32_t)((kg / STAGES) - 1) & 1, &s_abort, p.status, kStatusMmaTimeout, 60);
-                    if (!ok) break;
-                    uint8_t *st = smem + (size_t)s * S::stage_bytes;
-                    dequant_group_to_sw128(u0, kb, half, dsc0[kb], ndm0[kb], st, row);
-                    if (GATED) dequant_group_to_sw128(u1, kb, half, dsc1[kb], ndm1[kb], st + S::a_bytes, row);
-                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy stores -> visible to the tensor core
+    } else if constexpr (SRC != 0) {
+        if (warp == 6) {
+            // ------------------------------------------------ TMA: packed boxes (one unit of every row) on a ring of their own
+            int ps = 0;
+            uint32_t pph = 0;
+            bool ok = true, fresh = true;
+            while (ok && walk.next(p, sg)) {
+                const CUtensorMap *mw = p.items ? &p.w_maps[sg.z] : &map_w;
+                const CUtensorMap *mw2 = p.items ? (GATED ? &p.w2_maps[sg.z] : mw) : &map_w2;
+                const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
+                for (int u = sg.k0; u < sg.k1; ++u) {
+                    if (!fresh && !wait_flag(&p_empty[ps], pph ^ 1u, abort_addr, p.status, kStatusMmaTimeout, 50)) {
+                        ok = false;
+                        break;
+                    }
+                    if (elect_one()) {
+                        uint8_t *pst = smem + S::off_p + (size_t)ps * S::p_bytes;
+                        mbar_expect_tx(&p_full[ps], S::p_bytes);
+                        tma_load_2d(pst, mw, &p_full[ps], u * (S::unit_bytes / 4), row);
+                        if (GATED) tma_load_2d(pst + S::p_bytes / 2, mw2, &p_full[ps], u * (S::unit_bytes / 4), row);
+                    }
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(&a_full[s]);
+                    if (++ps == PST) {
+                        ps = 0;
+                        pph ^= 1u;
+                        fresh = false;
+                    }
                 }
-                __syncwarp();
-                if (lane == 0 && ok) mbar_arrive(&p_empty[ps]);
+            }
+        } else {
+            // ------------------------------------------------ dequantisers: thread = (row, k-block of the unit)
+            const int t = threadIdx.x - 7 * 32, row = t & (kBM - 1), mine = t >> 7;  // mine: warp-uniform
+            const int sw = row & 7;
+            const uint32_t row0 = smem_u32(smem) + (uint32_t)((row >> 3) * 1024 + sw * 128), box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
+            int s = 0, ps = 0;  // ring positions: s walks the k-blocks of all warps, this warp serves one in four
+            uint32_t ph = 0, pph = 0;
+            bool ok = true, fresh = true;
+            DqBlock<SRC> dq;
+            auto advance = [&](int n) {
+                s += n;
+                if (s >= STAGES) {
+                    s -= STAGES;
+                    ph ^= 1u;
+                    fresh = false;
+                }
+            };
+            while (ok && walk.next(p, sg)) {
+                for (int u = sg.k0; u < sg.k1; ++u) {
+                    ok = wait_flag(&p_full[ps], pph, abort_addr, p.status, kStatusTmaTimeout, 20);
+                    if (!ok) break;
+                    dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
+                    // Everything the warp needs of the box is in registers once this vote has read them.  Without it the arrival
+                    // overtakes shared-memory loads still queued behind other warps' stores, and the next box lands under them.
+                    if (__any_sync(0xffffffffu, dq.mix() == 0x9E3779B9u)) __nanosleep(0);  // a no-op that keeps the vote
+                    if (lane == 0) mbar_arrive(&p_empty[ps]);
+                    if (++ps == PST) {
+                        ps = 0;
+                        pph ^= 1u;
+                    }
+                    advance(mine);
+                    if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, abort_addr, p.status, kStatusMmaTimeout, 20);
+                    if (!ok) break;
+                    dq.emit(row0 + (uint32_t)(s * S::stage_bytes), sw);
+                    fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores of the pair
+                    __syncwarp();
+                    if (lane == 0) pair_arrive(pair_first(smem_u32(&full[s])));
+                    advance(4 - mine);
+                }
             }
         }
     }
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, TMEM_COLS);
+    pair_sync();  // nobody leaves while the other SM may still signal here or read operands
+    if (warp == 1) tmem_dealloc2(tmem_base, 512);
 }
 
-// activations of any supported dtype -> f16 [m, k]
-__global__ void to_f16_kernel(const void *__restrict__ x, int x_dtype, __half *__restrict__ out, size_t n) {
-    for (size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 4; i < n; i += (size_t)gridDim.x * blockDim.x * 4) {
+// activations of any supported dtype -> f16; eight values per thread and step (one 16- or 32-byte load, one 16-byte store)
+__global__ void __launch_bounds__(256) to_f16_kernel(const void *__restrict__ x, int x_dtype, __half *__restrict__ out, size_t n8) {
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
+        uint32_t h[4];
+        if (x_dtype == ZQ_F32) {
+            const float4 a = __ldcs(reinterpret_cast<const float4 *>(x) + 2 * i), b = __ldcs(reinterpret_cast<const float4 *>(x) + 2 * i + 1);
+            h[0] = h2_as_u32(__floats2half2_rn(a.x, a.y)); h[1] = h2_as_u32(__floats2half2_rn(a.z, a.w));
+            h[2] = h2_as_u32(__floats2half2_rn(b.x, b.y)); h[3] = h2_as_u32(__floats2half2_rn(b.z, b.w));
+        } else {
+            const uint4 r = __ldcs(reinterpret_cast<const uint4 *>(x) + i);
+            const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (i + j < n) out[i + j] = __float2half_rn(load_as_f32(x, x_dtype, i + j));
+            for (int j = 0; j < 4; ++j) h[j] = x_dtype == ZQ_F16 ? w[j] : h2_as_u32(__floats2half2_rn(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u)));
+        }
+        reinterpret_cast<uint4 *>(out)[i] = make_uint4(h[0], h[1], h[2], h[3]);
     }
 }
 
@@ -656,126 +634,12 @@ static int make_f16_map(const void *base, size_t rows, size_t cols, int box_rows
     return ZQ_OK;
 }
 
-// y[m, n] = x[m, k] W^T (+ residual), or silu(x gate^T) * (x up^T) when w_up is given.
-int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const void *x, int x_dtype, size_t m, void *y, int y_dtype, const void *residual, zq_error *err) {
-    const bool gated = w_up != nullptr;
-    const size_t n = w->rows, k = w->cols;
-    if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM needs columns aligned to 8, got %zu", k);
-    // The fused kernel saves the operand pass (one read of the packed weight, one write and one read of its f16 form),
-    // which dominates for few tokens; with many tokens the pass is amortised and the plain kernel, whose shared-memory
-    // traffic per k-block is lower (no operand stores by threads), runs the tensor core at a higher duty.
-    const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || m <= 1024) && w->type == ZQ_Q4_K && (!gated || w_up->type == ZQ_Q4_K) && k % kUnitWeights == 0;
-    if (fused) {
-        // Q4_K: dequantisation fused into the kernel; the workspace only holds the f16 copy of the activations
-        const size_t xb = (m * k * 2 + 255) & ~size_t(255);
-        const __half *xin = reinterpret_cast<const __half *>(x);
-        if (x_dtype != ZQ_F16) {
-            int rc = ensure_workspace(ctx, xb, err);
-            if (rc) return rc;
-            rc = launch_to_f16(ctx, x, x_dtype, reinterpret_cast<__half *>(ctx->workspace), m * k, err);
-            if (rc) return rc;
-            xin = reinterpret_cast<const __half *>(ctx->workspace);
-        }
-        CUtensorMap map_x;
-        int rc = make_f16_map(xin, m, k, kBN, &map_x, err);
-        if (rc) return rc;
-        GemmParams p;
-        p.y = y;
-        p.residual = residual;
-        p.status = ctx->status_dev;
-        p.y_dtype = y_dtype;
-        p.m = (int)m;
-        p.n_out = (int)n;
-        p.k = (int)k;
-        p.items = nullptr;
-        p.n_items = 0;
-        p.n_items_dev = nullptr;
-        const size_t total_tiles = ((n + kBM - 1) / kBM) * ((m + kBN - 1) / kBN);
-        dim3 grid((unsigned)(total_tiles < (size_t)ctx->sm_count ? total_tiles : (size_t)ctx->sm_count));
-        static bool configured[2][64] = {};
-        if (gated) {
-            if (!configured[1][ctx->device & 63]) {
-                ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_q4k_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem<true>::total), err);
-                configured[1][ctx->device & 63] = true;
-            }
-            gemm_q4k_fused_kernel<true><<<grid, kFusedThreads, FusedSmem<true>::total, ctx->stream>>>(w->qmv_map, w_up->qmv_map, map_x, p);
-        } else {
-            if (!configured[0][ctx->device & 63]) {
-                ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_q4k_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem<false>::total), err);
-                configured[0][ctx->device & 63] = true;
-            }
-            gemm_q4k_fused_kernel<false><<<grid, kFusedThreads, FusedSmem<false>::total, ctx->stream>>>(w->qmv_map, w->qmv_map, map_x, p);
-        }
-        ctx->launches++;
-        ZQ_CUDA_CHECK(cudaGetLastError(), err);
-        return ZQ_OK;
-    }
-    const size_t w_bytes = (n * k * 2 + 255) & ~size_t(255);
-    const size_t x_bytes = (m * k * 2 + 255) & ~size_t(255);
-    int rc = ensure_workspace(ctx, (gated ? 2 : 1) * w_bytes + x_bytes, err);
-    if (rc) return rc;
-    uint8_t *ws = reinterpret_cast<uint8_t *>(ctx->workspace);
-    __half *w16 = reinterpret_cast<__half *>(ws);
-    __half *w16b = reinterpret_cast<__half *>(ws + w_bytes);
-    __half *x16 = reinterpret_cast<__half *>(ws + (gated ? 2 : 1) * w_bytes);
-    rc = launch_dequantize_f16(ctx, w, w16, err);
-    if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
-    if (rc) return rc;
-    const __half *xin = reinterpret_cast<const __half *>(x);
-    if (x_dtype != ZQ_F16) {
-        const size_t total = m * k;
-        size_t blocks = (total / 4 + 255) / 256;
-        if (blocks > (size_t)ctx->sm_count * 32) blocks = (size_t)ctx->sm_count * 32;
-        if (blocks == 0) blocks = 1;
-        to_f16_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(x, x_dtype, x16, total);
-        ctx->launches++;
-        ZQ_CUDA_CHECK(cudaGetLastError(), err);
-        xin = x16;
-    }
-    CUtensorMap map_w, map_w2, map_x;
-    rc = make_f16_map(w16, n, k, kBM, &map_w, err);
-    if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, kBM, &map_w2, err);
-    if (!rc) rc = make_f16_map(xin, m, k, kBN, &map_x, err);
-    if (rc) return rc;
-    GemmParams p;
-    p.y = y;
-    p.residual = residual;
-    p.status = ctx->status_dev;
-    p.y_dtype = y_dtype;
-    p.m = (int)m;
-    p.n_out = (int)n;
-    p.k = (int)k;
-    p.items = nullptr;
-    p.n_items = 0;
-    p.n_items_dev = nullptr;
-    p.w_maps = p.w2_maps = nullptr;
-    const size_t total_tiles = ((n + kBM - 1) / kBM) * ((m + kBN - 1) / kBN);
-    dim3 grid((unsigned)(total_tiles < (size_t)ctx->sm_count ? total_tiles : (size_t)ctx->sm_count));
-    static bool configured[2][64] = {};
-    if (gated) {
-        if (!configured[1][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<true>::total), err);
-            configured[1][ctx->device & 63] = true;
-        }
-        gemm_kernel<true><<<grid, kGemmThreads, GemmSmem<true>::total, ctx->stream>>>(map_w, map_w2, map_x, p);
-    } else {
-        if (!configured[0][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<false>::total), err);
-            configured[0][ctx->device & 63] = true;
-        }
-        gemm_kernel<false><<<grid, kGemmThreads, GemmSmem<false>::total, ctx->stream>>>(map_w, map_w2, map_x, p);
-    }
-    ctx->launches++;
-    ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    return ZQ_OK;
-}
-
-static int make_f16_map3(const void *base, size_t mats, size_t rows, size_t cols, CUtensorMap *out, zq_error *err) {
+static int make_f16_map3(const void *base, size_t mats, size_t rows, size_t cols, int box_rows, CUtensorMap *out, zq_error *err) {
     EncodeTiledFn encode = get_encode_tiled(err);
     if (!encode) return ZQ_ERR_CUDA;
     cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)mats};
     cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)rows * cols * 2};
-    cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)kBM, 1};
+    cuuint32_t box[3] = {(cuuint32_t)kBK, (cuuint32_t)box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -784,13 +648,140 @@ static int make_f16_map3(const void *base, size_t mats, size_t rows, size_t cols
 }
 
 int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err) {
-    size_t blocks = (n / 4 + 255) / 256;
-    if (blocks > (size_t)ctx->sm_count * 32) blocks = (size_t)ctx->sm_count * 32;
+    const size_t n8 = n / 8;  // rows are multiples of 8 columns wherever this runs
+    size_t blocks = (n8 + 255) / 256;
+    if (blocks > (size_t)ctx->sm_count * 16) blocks = (size_t)ctx->sm_count * 16;
     if (blocks == 0) blocks = 1;
-    to_f16_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(x, x_dtype, out, n);
+    to_f16_kernel<<<(unsigned)blocks, 256, 0, ctx->stream>>>(x, x_dtype, out, n8);
     ctx->launches++;
     ZQ_CUDA_CHECK(cudaGetLastError(), err);
     return ZQ_OK;
+}
+
+template <uint32_t SRC, bool GATED>
+static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const GemmParams &p, int pairs, zq_error *err) {
+    using S = GemmSmem<SRC>;
+    static bool configured[64] = {};
+    if (!configured[ctx->device & 63]) {
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
+        configured[ctx->device & 63] = true;
+    }
+    gemm_kernel<SRC, GATED><<<2 * pairs, S::threads, S::total, ctx->stream>>>(mw, mw2, mx, p);
+    ctx->launches++;
+    ZQ_CUDA_CHECK(cudaGetLastError(), err);
+    return ZQ_OK;
+}
+static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const GemmParams &p, int pairs, zq_error *err) {
+#define ZQ_GEMM_CASE(T) case T: return gated ? launch_one<T, true>(ctx, mw, mw2, mx, p, pairs, err) : launch_one<T, false>(ctx, mw, mw2, mx, p, pairs, err)
+    switch (src) {
+        ZQ_GEMM_CASE(0);
+        ZQ_GEMM_CASE(ZQ_Q4_K);
+        ZQ_GEMM_CASE(ZQ_Q5_K);
+        ZQ_GEMM_CASE(ZQ_Q6_K);
+        ZQ_GEMM_CASE(ZQ_Q4_0);
+        ZQ_GEMM_CASE(ZQ_IQ4_NL);
+        ZQ_GEMM_CASE(ZQ_Q8_0);
+    default: return set_error(err, ZQ_ERR_UNSUPPORTED, "prefill GEMM: no kernel for GGUF type %u", src);
+    }
+#undef ZQ_GEMM_CASE
+}
+
+static void clear_params(zq_ctx *ctx, GemmParams &p) {
+    memset(&p, 0, sizeof(p));
+    p.status = ctx->status_dev;
+    p.counters = ctx->gemv_counters;
+}
+
+// Token tiles of a dense GEMM: as few as 256-token tiles allow, of equal size (300 tokens are two tiles of 160, not 256 + 44).
+static void plan_tokens(size_t m, GemmParams &p) {
+    const size_t tiles = (m + kBN - 1) / kBN;
+    p.m = (int)m;
+    p.bn = (int)(((m + tiles - 1) / tiles + 31) & ~size_t(31));
+    p.box_tok = p.bn / 2;
+}
+
+// How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; where that leaves more than a fifth of the
+// rounds empty, the tiles beyond the full rounds and one round more are cut into equal shares instead (all of them when
+// there are fewer than two rounds).  A share costs its f32 partial (128 KB per SM at 256 tokens) out and in, so a share is at
+// least two steps and a tile at most eight shares.
+static int plan_cut(const zq_ctx *ctx, int tiles, int steps, GemmParams &p) {
+    const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+    const int rounds = (tiles + pairs - 1) / pairs;
+    p.cut_tiles = p.cut_pairs = 0;
+    if (5 * tiles >= 4 * rounds * pairs || steps < 2) return tiles < pairs ? tiles : pairs;
+    const int full = tiles / pairs;
+    p.cut_tiles = full >= 2 ? tiles - (full - 1) * pairs : tiles;
+    long long shares = (long long)p.cut_tiles * steps / 2;
+    if (shares > 8LL * p.cut_tiles) shares = 8LL * p.cut_tiles;
+    p.cut_pairs = shares < pairs ? (int)shares : pairs;
+    if (p.cut_tiles < tiles) p.cut_pairs = pairs;
+    return p.cut_pairs;
+}
+static size_t partial_bytes(const GemmParams &p) { return p.cut_tiles ? (size_t)p.cut_pairs * 2 * 2 * kBN * kBM * sizeof(float) : 0; }
+
+// y[m, n] = x[m, k] W^T (+ residual), or silu(x gate^T) * (x up^T) when w_up is given.
+int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const void *x, int x_dtype, size_t m, void *y, int y_dtype, const void *residual, zq_error *err) {
+    const bool gated = w_up != nullptr;
+    const size_t n = w->rows, k = w->cols;
+    if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM needs columns aligned to 8, got %zu", k);
+    // Dequantising inside the kernel saves the operand pass (one read of the packed weight, one write and one read of its f16
+    // form); with many tokens the pass is amortised and what counts is that every token tile dequantises the weight again.
+    const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || m <= 1024) && has_i8_decode(w->type) && (!gated || w_up->type == w->type);
+    GemmParams p;
+    clear_params(ctx, p);
+    plan_tokens(m, p);
+    p.y = y;
+    p.residual = residual;
+    p.y_dtype = y_dtype;
+    p.n_out = (int)n;
+    p.k = (int)k;
+    const int rows_per_tile = gated ? kPairM / 2 : kPairM;
+    const size_t tiles = ((n + rows_per_tile - 1) / rows_per_tile) * ((m + p.bn - 1) / p.bn);
+    if (tiles > (size_t)INT32_MAX / 4) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM: %zu rows x %zu tokens are too many for one call", n, m);
+    const int pairs = plan_cut(ctx, (int)tiles, (int)((k + kStepK - 1) / kStepK), p);
+    const size_t part = (partial_bytes(p) + 1023) & ~size_t(1023);
+    const size_t w_bytes = fused ? 0 : (n * k * 2 + 1023) & ~size_t(1023);
+    const size_t x_bytes = x_dtype == ZQ_F16 ? 0 : (m * k * 2 + 1023) & ~size_t(1023);
+    int rc = ensure_workspace(ctx, part + (gated ? 2 : 1) * w_bytes + x_bytes, err);
+    if (rc) return rc;
+    uint8_t *ws = reinterpret_cast<uint8_t *>(ctx->workspace);
+    p.partials = reinterpret_cast<float *>(ws);
+    const __half *xin = reinterpret_cast<const __half *>(x);
+    if (x_dtype != ZQ_F16) {
+        __half *x16 = reinterpret_cast<__half *>(ws + part + (gated ? 2 : 1) * w_bytes);
+        rc = launch_to_f16(ctx, x, x_dtype, x16, m * k, err);
+        if (rc) return rc;
+        xin = x16;
+    }
+    CUtensorMap map_x;
+    rc = make_f16_map(xin, m, k, p.box_tok, &map_x, err);
+    if (rc) return rc;
+    if (fused) return launch_src(ctx, w->type, gated, gated ? w->unit_map_half : w->qmv_map, gated ? w_up->unit_map_half : w->qmv_map, map_x, p, pairs, err);
+    __half *w16 = reinterpret_cast<__half *>(ws + part), *w16b = reinterpret_cast<__half *>(ws + part + w_bytes);
+    rc = launch_dequantize_f16(ctx, w, w16, err);
+    if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
+    if (rc) return rc;
+    CUtensorMap map_w, map_w2;
+    rc = make_f16_map(w16, n, k, gated ? 64 : kBM, &map_w, err);
+    if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, gated ? 64 : kBM, &map_w2, err);
+    if (rc) return rc;
+    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, p, pairs, err);
+}
+
+static int grouped_params(zq_ctx *ctx, size_t rows, size_t k, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, GemmParams &p) {
+    clear_params(ctx, p);
+    p.y = y;
+    p.y_dtype = y_dtype;
+    p.m = (int)x_rows;
+    p.bn = kBN;
+    p.box_tok = kBN / 2;
+    p.n_out = (int)rows;
+    p.k = (int)k;
+    p.items = items;
+    p.n_items = n_items;
+    p.n_items_dev = n_items_dev;
+    const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+    return n_items < pairs ? n_items : pairs;
 }
 
 // Grouped GEMM (MoE prefill): `mats` f16 weight matrices [rows, k] stacked in one buffer (and a second stack for the
@@ -801,115 +792,49 @@ int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t m
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "grouped GEMM needs columns aligned to 8, got %zu", k);
     const bool gated = w2 != nullptr;
     CUtensorMap map_w, map_w2, map_x;
-    int rc = make_f16_map3(w, mats, rows, k, &map_w, err);
-    if (!rc) rc = make_f16_map3(gated ? w2 : w, mats, rows, k, &map_w2, err);
-    if (!rc) rc = make_f16_map(x, x_rows, k, kBN, &map_x, err);
+    int rc = make_f16_map3(w, mats, rows, k, gated ? 64 : kBM, &map_w, err);
+    if (!rc) rc = make_f16_map3(gated ? w2 : w, mats, rows, k, gated ? 64 : kBM, &map_w2, err);
+    if (!rc) rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
     if (rc) return rc;
     GemmParams p;
-    p.y = y;
-    p.residual = nullptr;
-    p.status = ctx->status_dev;
-    p.y_dtype = y_dtype;
-    p.m = (int)x_rows;
-    p.n_out = (int)rows;
-    p.k = (int)k;
-    p.items = items;
-    p.n_items = n_items;
-    p.n_items_dev = nullptr;
-    p.w_maps = p.w2_maps = nullptr;
-    dim3 grid((unsigned)(n_items < ctx->sm_count ? n_items : ctx->sm_count));
-    static bool configured[2][64] = {};
-    if (gated) {
-        if (!configured[1][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<true>::total), err);
-            configured[1][ctx->device & 63] = true;
-        }
-        gemm_kernel<true><<<grid, kGemmThreads, GemmSmem<true>::total, ctx->stream>>>(map_w, map_w2, map_x, p);
-    } else {
-        if (!configured[0][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<false>::total), err);
-            configured[0][ctx->device & 63] = true;
-        }
-        gemm_kernel<false><<<grid, kGemmThreads, GemmSmem<false>::total, ctx->stream>>>(map_w, map_w2, map_x, p);
-    }
-    ctx->launches++;
-    ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    return ZQ_OK;
+    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, nullptr, y, y_dtype, p);
+    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, p, pairs, err);
 }
 
-// Plain f16 x f16 GEMM on raw operands: y[m, rows] = x[m, k] w[rows, k]^T, f32 accumulation (router logits).
+// Plain f16 x f16 GEMM on raw operands: y[m, rows] = x[m, k] w[rows, k]^T, f32 accumulation (router logits).  Whole tiles only:
+// it uses no workspace, which its caller may hold.
 int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const __half *x, size_t m, void *y, int y_dtype, zq_error *err) {
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "f16 GEMM needs columns aligned to 8, got %zu", k);
+    GemmParams p;
+    clear_params(ctx, p);
+    plan_tokens(m, p);
     CUtensorMap map_w, map_x;
     int rc = make_f16_map(w, rows, k, kBM, &map_w, err);
-    if (!rc) rc = make_f16_map(x, m, k, kBN, &map_x, err);
+    if (!rc) rc = make_f16_map(x, m, k, p.box_tok, &map_x, err);
     if (rc) return rc;
-    GemmParams p;
     p.y = y;
-    p.residual = nullptr;
-    p.status = ctx->status_dev;
     p.y_dtype = y_dtype;
-    p.m = (int)m;
     p.n_out = (int)rows;
     p.k = (int)k;
-    p.items = nullptr;
-    p.n_items = 0;
-    p.n_items_dev = nullptr;
-    p.w_maps = p.w2_maps = nullptr;
-    const size_t total_tiles = ((rows + kBM - 1) / kBM) * ((m + kBN - 1) / kBN);
-    dim3 grid((unsigned)(total_tiles < (size_t)ctx->sm_count ? total_tiles : (size_t)ctx->sm_count));
-    static bool configured[64] = {};
-    if (!configured[ctx->device & 63]) {
-        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmSmem<false>::total), err);
-        configured[ctx->device & 63] = true;
-    }
-    gemm_kernel<false><<<grid, kGemmThreads, GemmSmem<false>::total, ctx->stream>>>(map_w, map_w, map_x, p);
-    ctx->launches++;
-    ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    return ZQ_OK;
+    const size_t tiles = ((rows + kPairM - 1) / kPairM) * ((m + p.bn - 1) / p.bn);
+    const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+    return launch_src(ctx, 0, false, map_w, map_w, map_x, p, tiles < (size_t)pairs ? (int)tiles : pairs, err);
 }
 
-// Grouped fused form (MoE prefill, Q4_K experts): no f16 copy of the weights at all.  `w_maps` / `w2_maps`: device
-// tables of the experts' packed-weight tensor maps (one unit x 128 rows boxes), indexed by the work items' z.
-int launch_gemm_fused_grouped(zq_ctx *ctx, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype,
-                              zq_error *err) {
+// Grouped form for packed experts (MoE prefill): no f16 copy of the weights at all.  `w_maps` / `w2_maps`: device tables of the
+// experts' packed-weight tensor maps (one unit x 128 rows boxes, gated: 64 rows), indexed by the work items' z.
+int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev,
+                              void *y, int y_dtype, zq_error *err) {
     if (n_items <= 0) return ZQ_OK;
-    if (k % kUnitWeights) return set_error(err, ZQ_ERR_SHAPE, "fused Q4_K GEMM needs columns aligned to 256, got %zu", k);
-    const bool gated = w2_maps != nullptr;
+    if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "grouped GEMM needs columns aligned to 8, got %zu", k);
     CUtensorMap map_x;
-    int rc = make_f16_map(x, x_rows, k, kBN, &map_x, err);
+    int rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
     if (rc) return rc;
     GemmParams p;
-    p.y = y;
-    p.residual = nullptr;
-    p.status = ctx->status_dev;
-    p.y_dtype = y_dtype;
-    p.m = (int)x_rows;
-    p.n_out = (int)rows;
-    p.k = (int)k;
-    p.items = items;
-    p.n_items = n_items;
-    p.n_items_dev = n_items_dev;
+    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, n_items_dev, y, y_dtype, p);
     p.w_maps = w_maps;
     p.w2_maps = w2_maps;
-    dim3 grid((unsigned)(n_items < ctx->sm_count ? n_items : ctx->sm_count));
-    static bool configured[2][64] = {};
-    if (gated) {
-        if (!configured[1][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_q4k_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem<true>::total), err);
-            configured[1][ctx->device & 63] = true;
-        }
-        gemm_q4k_fused_kernel<true><<<grid, kFusedThreads, FusedSmem<true>::total, ctx->stream>>>(map_x, map_x, map_x, p);
-    } else {
-        if (!configured[0][ctx->device & 63]) {
-            ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_q4k_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, FusedSmem<false>::total), err);
-            configured[0][ctx->device & 63] = true;
-        }
-        gemm_q4k_fused_kernel<false><<<grid, kFusedThreads, FusedSmem<false>::total, ctx->stream>>>(map_x, map_x, map_x, p);
-    }
-    ctx->launches++;
-    ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    return ZQ_OK;
+    return launch_src(ctx, type, w2_maps != nullptr, map_x, map_x, map_x, p, pairs, err);
 }
 
 }  // namespace zq

@@ -322,7 +322,7 @@ __global__ void router_items_kernel(int chunks, int row_tiles, int tok_tiles, in
     const int n = chunks * row_tiles * tok_tiles;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int c = i / (row_tiles * tok_tiles), rem = i - c * row_tiles * tok_tiles, rt = rem / tok_tiles, tt = rem - rt * tok_tiles;
-        items[i] = make_int4(c, rt * 128, c * m + tt * 256, c * m + m);
+        items[i] = make_int4(c, rt * 256, c * m + tt * 256, c * m + min(m, tt * 256 + 256));
     }
 }
 
@@ -478,6 +478,10 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_count_kernel(const 
     for (int e = threadIdx.x; e < E; e += kGroupThreads) hist[(size_t)blockIdx.x * E + e] = s_cnt[e];
 }
 
+// Tokens per tile when `count` tokens of an expert take `tiles` (= ceil(count / 256)) tiles: equal shares in whole MMA column
+// groups of 32.  270 tokens are 160 + 110, not 256 + 14: a tile costs at least its dequantisation, whatever its tokens.
+__host__ __device__ inline uint32_t moe_tile_tokens(uint32_t count, uint32_t tiles) { return ((count + tiles - 1) / tiles + 31u) & ~31u; }
+
 // counts: [0] items of the gated launch, [1] items of the down launch, [2] routed rows in all
 __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_t *__restrict__ hist, int chunks, int E, uint32_t *__restrict__ offsets, int rt_gated, int rt_down, int4 *__restrict__ items_gated,
                                                                          int4 *__restrict__ items_down, int *__restrict__ counts) {
@@ -513,10 +517,11 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_
     const uint32_t first = base_c + sc - c, tfirst = base_t + st - nt;
     if (e < E) {
         offsets[e] = first;
+        const uint32_t per = nt ? moe_tile_tokens(c, nt) : 0u;
         for (uint32_t tt = 0; tt < nt; ++tt) {
-            const int t0 = (int)(first + tt * 256u), end = (int)(first + c);
+            const int t0 = (int)(first + tt * per), end = (int)min(first + c, first + (tt + 1) * per);
             for (int rt = 0; rt < rt_gated; ++rt) items_gated[(size_t)(tfirst + tt) * rt_gated + rt] = make_int4(e, rt * 128, t0, end);
-            for (int rt = 0; rt < rt_down; ++rt) items_down[(size_t)(tfirst + tt) * rt_down + rt] = make_int4(e, rt * 128, t0, end);
+            for (int rt = 0; rt < rt_down; ++rt) items_down[(size_t)(tfirst + tt) * rt_down + rt] = make_int4(e, rt * 256, t0, end);
         }
     }
     if (e == kGroupThreads - 1) {  // the last thread holds the totals
@@ -622,7 +627,7 @@ static int ensure_moe_ws(zq_ctx *ctx, size_t bytes, zq_error *err) {
     return ZQ_OK;
 }
 
-// MoE prefill with Q4_K experts, everything on the device: grouping (three small kernels), one gather that also
+// MoE prefill, everything on the device: grouping (three small kernels), one gather that also
 // converts to f16, the two grouped fused GEMMs (their item counts read from device memory), shared expert, combine.
 static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *shared_gate, const zq_weight *shared_up, const zq_weight *shared_down, const void *dev_x, int x_dtype, size_t m, const uint32_t *dev_ids,
                               const float *dev_weights, size_t top_k, void *dev_y, int y_dtype, const void *dev_residual, zq_error *err) {
@@ -630,7 +635,7 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     const bool has_shared = shared_gate != nullptr;
     const int tokens_per_chunk = (int)(kGroupThreads / top_k > 0 ? kGroupThreads / top_k : 1);
     const int chunks = (int)((m + tokens_per_chunk - 1) / tokens_per_chunk);
-    const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 127) / 128);
+    const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 255) / 256);  // 128 gated outputs or 256 rows per tile
     const size_t max_tiles = routes / 256 + E;  // sum over experts of ceil(count / 256)
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     // tables and f32 results
@@ -664,9 +669,9 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     gather_rows_f16_kernel<<<grid_for(ctx, routes * (H / 8), 256), 256, 0, ctx->stream>>>(dev_x, x_dtype, d_slot_token, d_counts + 2, (int)H, x16);
     ctx->launches += 4;
     ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    rc = launch_gemm_fused_grouped(ctx, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, x16, routes, d_items_g, (int)(max_tiles * rt_i), d_counts, act16, ZQ_F16, err);
+    rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, x16, routes, d_items_g, (int)(max_tiles * rt_i), d_counts, act16, ZQ_F16, err);
     if (rc) return rc;
-    rc = launch_gemm_fused_grouped(ctx, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items_d, (int)(max_tiles * rt_h), d_counts + 1, d_out, ZQ_F32, err);
+    rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items_d, (int)(max_tiles * rt_h), d_counts + 1, d_out, ZQ_F32, err);
     if (rc) return rc;
     if (has_shared) {
         rc = zq_gated_mlp(ctx, shared_gate, shared_up, shared_down, dev_x, x_dtype, m, d_shared, ZQ_F32, nullptr, err);
@@ -718,11 +723,11 @@ int zq_moe_route_topk(zq_ctx *ctx, int scoring, const void *dev_x, int x_dtype, 
     if (m >= 256 && hidden % 8 == 0) {
         auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
         // slices of K as separate tiles while the whole-K tiles would leave most SMs idle
-        const int row_tiles = (int)((num_experts + 127) / 128), tok_tiles = (int)((m + 255) / 256);
+        const int row_tiles = (int)((num_experts + 255) / 256), tok_tiles = (int)((m + 255) / 256);
         int chunks = 1;
         if (hidden % 64 == 0)
             for (int c = 16; c >= 2; --c)
-                if ((3 * hidden / 64) % c == 0 && row_tiles * tok_tiles * c <= 2 * ctx->sm_count) {
+                if ((3 * hidden / 64) % c == 0 && row_tiles * tok_tiles * c <= ctx->sm_count) {
                     chunks = c;
                     break;
                 }
@@ -860,8 +865,8 @@ int zq_moe_experts_create(zq_ctx *ctx, const zq_weight *const *gate, const zq_we
             hg[e] = gate[e]->gemv_map_half;
             hu[e] = up[e]->gemv_map_half;
             hd[e] = down[e]->gemv_map;
-            qg[e] = gate[e]->qmv_map;
-            qu[e] = up[e]->qmv_map;
+            qg[e] = gate[e]->unit_map_half;
+            qu[e] = up[e]->unit_map_half;
             qd[e] = down[e]->qmv_map;
         }
         const size_t bytes = num_experts * sizeof(CUtensorMap);
@@ -939,9 +944,9 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
         return ZQ_OK;
     }
 
-    // ---- prefill with Q4_K experts: grouping, gather and the two grouped GEMMs stay on the device
+    // ---- prefill with packed experts the GEMM can unpack: grouping, gather and the two grouped GEMMs stay on the device
     if (!ctx->force_moe_per_expert && !ctx->force_moe_host_grouping && !ctx->disable_fused_gemm && routes >= 32 * E && E <= (size_t)kGroupThreads && top_k <= 64 && experts->d_gate_qmaps &&
-        experts->gate_type == ZQ_Q4_K && experts->down_type == ZQ_Q4_K && H % kUnitWeights == 0 && I % kUnitWeights == 0)
+        has_i8_decode(experts->gate_type) && has_i8_decode(experts->down_type))
         return moe_prefill_device(ctx, experts, shared_gate, shared_up, shared_down, dev_x, x_dtype, m, dev_ids, dev_weights, top_k, dev_y, y_dtype, dev_residual, err);
 
     // ---- routing back to the host, token-major stable grouping (src/moe/routing.rs:136-156)
@@ -1016,26 +1021,24 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
 
     // ---- experts, ascending id (src/moe/routing.rs:180-213: gather rows, expert batch, weighted scatter)
     const bool grouped_gemm = !ctx->force_moe_per_expert && routes >= 32 * E && H % 8 == 0 && I % 8 == 0;
-    const bool fused_gemm = grouped_gemm && !ctx->disable_fused_gemm && experts->d_gate_qmaps && experts->gate_type == ZQ_Q4_K && experts->down_type == ZQ_Q4_K && H % kUnitWeights == 0 && I % kUnitWeights == 0;
+    const bool fused_gemm = grouped_gemm && !ctx->disable_fused_gemm && experts->d_gate_qmaps && has_i8_decode(experts->gate_type) && has_i8_decode(experts->down_type);
+    // work items of one expert: its tokens in equal tiles, its rows in tiles of `rows_per_tile` outputs
+    auto add_items = [](std::vector<int4> &items, int z, int first, int end, int row_tiles, int rows_per_tile) {
+        const int nt = (end - first + 255) / 256, per = nt ? (int)moe_tile_tokens((uint32_t)(end - first), (uint32_t)nt) : 0;
+        for (int t = 0; t < nt; ++t)
+            for (int rt = 0; rt < row_tiles; ++rt) items.push_back(make_int4(z, rt * rows_per_tile, first + t * per, std::min(end, first + (t + 1) * per)));
+    };
+    const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 255) / 256);
     if (fused_gemm) {
-        // Prefill, Q4_K experts: two launches for the whole layer.  The fused tensor-core GEMM dequantises the packed
+        // Prefill, experts of a type the GEMM unpacks: two launches for the whole layer.  The fused tensor-core GEMM dequantises the packed
         // tiles of whichever expert a work item names (per-expert tensor maps in a device table), so there is no f16
         // copy of any expert.  Work list: one item per (expert, 256-token tile, 128-row tile); tokens are the gathered
         // slot rows, so outputs land in slot order as the combine expects.
         auto al2 = [](size_t v) { return (v + 1023) & ~size_t(1023); };
         std::vector<int4> items;
-        const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 127) / 128);
-        for (size_t e = 0; e < E; ++e) {
-            const int first = (int)offsets[e], end = (int)offsets[e + 1];
-            for (int t0 = first; t0 < end; t0 += 256)
-                for (int rt = 0; rt < rt_i; ++rt) items.push_back(make_int4((int)e, rt * 128, t0, end));
-        }
+        for (size_t e = 0; e < E; ++e) add_items(items, (int)e, (int)offsets[e], (int)offsets[e + 1], rt_i, 128);
         const int n_gated = (int)items.size();
-        for (size_t e = 0; e < E; ++e) {
-            const int first = (int)offsets[e], end = (int)offsets[e + 1];
-            for (int t0 = first; t0 < end; t0 += 256)
-                for (int rt = 0; rt < rt_h; ++rt) items.push_back(make_int4((int)e, rt * 128, t0, end));
-        }
+        for (size_t e = 0; e < E; ++e) add_items(items, (int)e, (int)offsets[e], (int)offsets[e + 1], rt_h, 256);
         const int n_down = (int)items.size() - n_gated;
         const size_t x16_bytes = al2(routes * H * sizeof(__half)), act16_bytes = al2(routes * I * sizeof(__half)), items_bytes = al2(items.size() * sizeof(int4));
         rc = ensure_workspace(ctx, x16_bytes + act16_bytes + items_bytes, err);
@@ -1051,9 +1054,9 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
             if (rc) return rc;
             xin = x16;
         }
-        rc = launch_gemm_fused_grouped(ctx, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, xin, routes, d_items, n_gated, nullptr, act16, ZQ_F16, err);
+        rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, xin, routes, d_items, n_gated, nullptr, act16, ZQ_F16, err);
         if (rc) return rc;
-        rc = launch_gemm_fused_grouped(ctx, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items + n_gated, n_down, nullptr, d_out, ZQ_F32, err);
+        rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items + n_gated, n_down, nullptr, d_out, ZQ_F32, err);
         if (rc) return rc;
     } else if (grouped_gemm) {
         // Prefill: one grouped tensor-core GEMM per projection and chunk of experts instead of two launches per
@@ -1070,24 +1073,15 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
         std::vector<int4> items;
         struct ChunkPlan { size_t e0, e1; int gated_first, gated_n, down_first, down_n; };
         std::vector<ChunkPlan> plans;
-        const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 127) / 128);
         for (size_t e0 = 0; e0 < E; e0 += chunk) {
             ChunkPlan cp;
             cp.e0 = e0;
             cp.e1 = e0 + chunk < E ? e0 + chunk : E;
             cp.gated_first = (int)items.size();
-            for (size_t e = cp.e0; e < cp.e1; ++e) {
-                const int first = (int)offsets[e], end = (int)offsets[e + 1];
-                for (int t0 = first; t0 < end; t0 += 256)
-                    for (int rt = 0; rt < rt_i; ++rt) items.push_back(make_int4((int)(e - e0), rt * 128, t0, end));
-            }
+            for (size_t e = cp.e0; e < cp.e1; ++e) add_items(items, (int)(e - e0), (int)offsets[e], (int)offsets[e + 1], rt_i, 128);
             cp.gated_n = (int)items.size() - cp.gated_first;
             cp.down_first = (int)items.size();
-            for (size_t e = cp.e0; e < cp.e1; ++e) {
-                const int first = (int)offsets[e], end = (int)offsets[e + 1];
-                for (int t0 = first; t0 < end; t0 += 256)
-                    for (int rt = 0; rt < rt_h; ++rt) items.push_back(make_int4((int)(e - e0), rt * 128, t0, end));
-            }
+            for (size_t e = cp.e0; e < cp.e1; ++e) add_items(items, (int)(e - e0), (int)offsets[e], (int)offsets[e + 1], rt_h, 256);
             cp.down_n = (int)items.size() - cp.down_first;
             plans.push_back(cp);
         }
