@@ -300,3 +300,27 @@ def test_host_batch_is_a_whole_bracket_in_one_call():
         ctx().linear_host_batch([(xs[0], ws[0], ys[0])])  # a bracket is already open; like every error this closes it
     with pytest.raises(ffi.ZqFailure):
         ctx().finish_batch()
+
+
+def test_host_mirror_reports_bad_arguments():
+    """The native half of the host mirror raises what the Python methods always raised, before anything is launched."""
+    from zllm_b200.ffi import ZqFailure
+
+    w = ctx().prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 64, 256, seed=3), 64, 256)
+    x = torch.zeros((2, 256), device="cuda")
+    with pytest.raises(ZqFailure):
+        ctx().linear(torch.zeros((2, 128), device="cuda"), w)
+    with pytest.raises(ZqFailure):
+        ctx().linear(x, w, residual=torch.zeros((1, 64), device="cuda"))
+    with pytest.raises(TypeError):
+        ctx().linear(x.double(), w)
+    with pytest.raises(KeyError):
+        ctx().linear(x, w, out_dtype=torch.float64)
+    with pytest.raises(TypeError):
+        ctx().linear_batch([(x, w), (x.half(), w)])
+    with pytest.raises(ZqFailure):
+        ctx().rmsnorm_linear_multi(x, torch.ones(128, device="cuda"), 1e-6, [w])
+    assert ctx().linear_batch([]) == []
+    w.release()
+    with pytest.raises(ZqFailure):
+        ctx().linear(x, w)

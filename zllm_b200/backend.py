@@ -35,14 +35,17 @@ class Weight:
     def __init__(self, ctx: "B200Context", handle: C.c_void_p):
         self.ctx = ctx
         self.handle = handle
+        # what every call needs of a weight, read once (0 once released, as the ABI answers for a null handle)
+        lib = ffi.load()
+        self._h, self._rows, self._cols = handle.value or 0, lib.zq_weight_rows(handle), lib.zq_weight_cols(handle)
 
     @property
     def rows(self) -> int:
-        return ffi.load().zq_weight_rows(self.handle)
+        return self._rows
 
     @property
     def cols(self) -> int:
-        return ffi.load().zq_weight_cols(self.handle)
+        return self._cols
 
     @property
     def tensor_type(self) -> int:
@@ -56,6 +59,7 @@ class Weight:
         if self.handle:
             ffi.load().zq_weight_release(self.handle)
             self.handle = None
+            self._h = self._rows = self._cols = 0
 
     def __del__(self):
         try:
@@ -72,6 +76,8 @@ class B200Context:
         handle = C.c_void_p()
         ffi.call("zq_ctx_create", device, C.byref(handle))
         self.handle = handle
+        self._h = handle.value
+        self._native = ffi.native()
         self.device = torch.device("cuda", device)
         if use_torch_stream:
             self.set_stream(torch.cuda.current_stream(self.device).cuda_stream)
@@ -98,6 +104,7 @@ class B200Context:
         if self.handle:
             self.lib.zq_ctx_destroy(self.handle)
             self.handle = None
+            self._h = 0
 
     # ---- weights
     def prepare_weight(self, tensor_type: int, data, rows: int, cols: int) -> Weight:
@@ -148,16 +155,7 @@ class B200Context:
         return x.numel() // cols
 
     def linear(self, x: torch.Tensor, w: Weight, out_dtype=None, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
-        x = x.contiguous()
-        m = self._rows(x, w.cols)
-        out_dtype = out_dtype or x.dtype
-        y = torch.empty((m, w.rows), dtype=out_dtype, device=x.device)
-        if residual is not None:
-            residual = residual.contiguous()
-            if residual.numel() != y.numel() or residual.dtype != out_dtype:
-                raise ffi.ZqFailure(1, f"residual shape/dtype mismatch: {tuple(residual.shape)} {residual.dtype} vs {tuple(y.shape)} {out_dtype}")
-        ffi.call("zq_linear", self.handle, w.handle, _ptr(x), _dt(x), m, _ptr(y), _DTYPES[out_dtype], _ptr(residual))
-        return y
+        return self._native.linear(self._h, x, w, out_dtype, residual)
 
     def linear_add(self, x: torch.Tensor, w: Weight, residual: torch.Tensor, out_dtype=None) -> torch.Tensor:
         return self.linear(x, w, out_dtype=out_dtype or residual.dtype, residual=residual)
@@ -168,33 +166,7 @@ class B200Context:
         ``jobs`` is a list of ``(x, weight)``, ``(x, weight, residual)``, ``(x, gate, up, "gated")`` or
         ``(x, weight, residual_or_None, "row")`` tuples (the last form is a row-parallel job: its result is summed over the
         ranks of the peer group); all inputs share one dtype.  Returns the list of outputs."""
-        arr = (ffi.ZqLinearJob * len(jobs))()
-        ys, keep = [], []
-        x_dt = None
-        for i, job in enumerate(jobs):
-            x = job[0].contiguous()
-            gated = len(job) == 4 and job[3] == "gated"
-            w = job[1]
-            m = self._rows(x, w.cols)
-            x_dt = x_dt or x.dtype
-            if x.dtype != x_dt:
-                raise TypeError("linear_batch: all inputs must share one dtype")
-            od = out_dtype or x.dtype
-            y = torch.empty((m, w.rows), dtype=od, device=x.device)
-            row = len(job) == 4 and job[3] == "row"
-            residual = job[2].contiguous() if ((len(job) == 3 or row) and job[2] is not None) else None
-            arr[i].w = w.handle.value
-            arr[i].w_up = job[2].handle.value if gated else None
-            arr[i].dev_x = x.data_ptr()
-            arr[i].m = m
-            arr[i].dev_y = y.data_ptr()
-            arr[i].dev_residual = residual.data_ptr() if residual is not None else None
-            arr[i].flags = ffi.JOB_ROW_PARALLEL if row else 0
-            ys.append(y)
-            keep.append((x, residual))
-        if jobs:
-            ffi.call("zq_linear_batch", self.handle, arr, len(jobs), _DTYPES[x_dt], _DTYPES[out_dtype or x_dt])
-        return ys
+        return self._native.linear_batch(self._h, jobs, out_dtype)
 
     def linear_row_parallel(self, x: torch.Tensor, w: Weight, out_dtype=None, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
         """This rank's column slice of a weight against its slice of the input; the ranks' partial results are summed
@@ -235,29 +207,12 @@ class B200Context:
         ffi.call("zq_moe_ep_init", self.handle, self._exchange_blobs(blob, group))
 
     def linear_multi(self, x: torch.Tensor, weights: Sequence[Weight], out_dtype=None):
-        x = x.contiguous()
-        m = self._rows(x, weights[0].cols)
-        out_dtype = out_dtype or x.dtype
-        ys = [torch.empty((m, w.rows), dtype=out_dtype, device=x.device) for w in weights]
-        wa = (C.c_void_p * len(weights))(*[w.handle for w in weights])
-        ya = (C.c_void_p * len(weights))(*[y.data_ptr() for y in ys])
-        ffi.call("zq_linear_multi", self.handle, wa, len(weights), _ptr(x), _dt(x), m, ya, _DTYPES[out_dtype])
-        return ys
+        return self._native.linear_multi(self._h, x, weights, out_dtype, None, 0.0, 0.0)
 
     def rmsnorm_linear_multi(self, x: torch.Tensor, norm_weight: torch.Tensor, eps: float, weights: Sequence[Weight], out_dtype=None, weight_offset: float = 0.0):
         """RMSNorm of every row, then the projections (``Backend::rmsnorm_linear`` / ``rmsnorm_dual_linear``,
         src/backend/mod.rs:455-464); ``weight_offset`` 1.0 is the Gemma form of the norm."""
-        x = x.contiguous()
-        m = self._rows(x, weights[0].cols)
-        norm_weight = norm_weight.contiguous().float()
-        if norm_weight.numel() != weights[0].cols:
-            raise ffi.ZqFailure(1, f"norm weight has {norm_weight.numel()} elements, input width is {weights[0].cols}")
-        out_dtype = out_dtype or x.dtype
-        ys = [torch.empty((m, w.rows), dtype=out_dtype, device=x.device) for w in weights]
-        wa = (C.c_void_p * len(weights))(*[w.handle for w in weights])
-        ya = (C.c_void_p * len(weights))(*[y.data_ptr() for y in ys])
-        ffi.call("zq_rmsnorm_linear", self.handle, wa, len(weights), _ptr(x), _dt(x), m, _ptr(norm_weight), float(eps), float(weight_offset), ya, _DTYPES[out_dtype])
-        return ys
+        return self._native.linear_multi(self._h, x, weights, out_dtype, norm_weight, eps, weight_offset)
 
     def rmsnorm_linear(self, x, norm_weight, eps: float, w: Weight, out_dtype=None, weight_offset: float = 0.0):
         return self.rmsnorm_linear_multi(x, norm_weight, eps, [w], out_dtype, weight_offset)[0]
@@ -278,34 +233,14 @@ class B200Context:
                        interleaved: bool = False, suffix: bool = False):
         """``Backend::rope_prefix_qk`` (src/backend/mod.rs:567; ``suffix=True`` is ``rope``): rotates q and k in place,
         one launch; ``cos`` / ``sin`` are f32 device tables [positions, rotary_dim / 2]."""
-        rows = query.shape[0] if query.dim() > 1 else 1
-        head_dim = query.numel() // rows // num_heads
-        if key is not None and (key.dtype != query.dtype or key.numel() != rows * num_kv_heads * head_dim):
-            raise ffi.ZqFailure(1, "rope: key shape or dtype does not match the query's")
-        cos, sin = cos.contiguous().float(), sin.contiguous().float()
-        if cos.numel() != sin.numel():
-            raise ffi.ZqFailure(1, f"rope: cos and sin tables differ in length ({cos.numel()} / {sin.numel()})")
-        ffi.call("zq_rope_qk", self.handle, _ptr(query), num_heads, _ptr(key), num_kv_heads if key is not None else 0, _dt(query), rows, head_dim, rotary_dim, int(interleaved), int(suffix), position,
-                 _ptr(cos), _ptr(sin), cos.numel())
+        self._native.rope(self._h, query, key, num_heads, num_kv_heads, rotary_dim, position, cos, sin, interleaved, suffix)
         return query, key
 
     def gated_linear(self, x: torch.Tensor, gate: Weight, up: Weight, out_dtype=None) -> torch.Tensor:
-        x = x.contiguous()
-        m = self._rows(x, gate.cols)
-        out_dtype = out_dtype or x.dtype
-        y = torch.empty((m, gate.rows), dtype=out_dtype, device=x.device)
-        ffi.call("zq_gated_silu", self.handle, gate.handle, up.handle, _ptr(x), _dt(x), m, _ptr(y), _DTYPES[out_dtype])
-        return y
+        return self._native.gated(self._h, x, gate, up, None, out_dtype, None)
 
     def gated_mlp(self, x: torch.Tensor, gate: Weight, up: Weight, down: Weight, out_dtype=None, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
-        x = x.contiguous()
-        m = self._rows(x, gate.cols)
-        out_dtype = out_dtype or x.dtype
-        y = torch.empty((m, down.rows), dtype=out_dtype, device=x.device)
-        if residual is not None:
-            residual = residual.contiguous()
-        ffi.call("zq_gated_mlp", self.handle, gate.handle, up.handle, down.handle, _ptr(x), _dt(x), m, _ptr(y), _DTYPES[out_dtype], _ptr(residual))
-        return y
+        return self._native.gated(self._h, x, gate, up, down, out_dtype, residual)
 
     def gated_mlp_add_residual(self, x, gate, up, down, residual, out_dtype=None):
         return self.gated_mlp(x, gate, up, down, out_dtype=out_dtype or residual.dtype, residual=residual)
@@ -331,16 +266,7 @@ class B200Context:
     def linear_host_batch(self, jobs):
         """A whole bracket in one call (``zq_linear_host_batch``): ``jobs`` is a list of ``(x_host, weight, y_host)`` numpy
         triples sharing one input dtype and one output dtype."""
-        import numpy as np
-
-        dt = {np.dtype(np.float32): ffi.F32, np.dtype(np.float16): ffi.F16}
-        arr = (ffi.ZqLinearHostJob * len(jobs))()
-        for i, (x_host, w, y_host) in enumerate(jobs):
-            arr[i].w = w.handle.value
-            arr[i].host_x = x_host.ctypes.data
-            arr[i].m = x_host.size // w.cols
-            arr[i].host_y = y_host.ctypes.data
-        ffi.call("zq_linear_host_batch", self.handle, arr, len(jobs), dt[jobs[0][0].dtype], dt[jobs[0][2].dtype])
+        self._native.linear_host_batch(self._h, jobs)
 
 
 class GgufFile:

@@ -144,24 +144,11 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
     return r != 0;
 }
-// One poll without a suspend-time hint: the hardware parks the thread for its own limit; with a hint the compiler polls and
-// sleeps in a loop, which delays the wake-up.
-__device__ __forceinline__ bool pair_try_wait(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // `sleep_ns` > 0: roles that share a scheduler with working warps back off between polls (a bare poll loop re-issues
 // every few tens of nanoseconds).
 __device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t abort_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
     for (uint32_t i = 0; i < (1u << 23); ++i) {
-        if (pair_try_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         uint32_t gone;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gone) : "r"(abort_addr));
         if (gone) return false;

@@ -130,6 +130,30 @@ def load() -> C.CDLL:
     return _lib
 
 
+_native = None
+
+
+def native():
+    """The host mirror's native half (``csrc/zq_torch.cpp``); like the library itself it has no fallback."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+
+        load()
+        path = os.path.join(_HERE, "lib", "_zq_torch.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -m zllm_b200.build` (there is no fallback path)")
+        import torch  # noqa: F401  (its libraries must be loaded first)
+
+        loader = importlib.machinery.ExtensionFileLoader("_zq_torch", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_zq_torch", path, loader=loader))
+        loader.exec_module(module)
+        module.setup(ZqFailure)
+        _native = module
+    return _native
+
+
 def call(name: str, *args):
     """Call an entry point that returns a status code and takes a trailing ``zq_error*``."""
     err = ZqError()
