@@ -243,3 +243,23 @@ def test_q4_k_encoder_at_rounding_ties_and_unaligned_buffers(rows, cols, kind, o
     ffi.call("zq_quantize", ctx().handle, H.Q4_K, C.c_void_p(src.data_ptr() + 4 * offset), rows, cols, C.c_void_p(out.data_ptr()), out.numel())
     ctx().sync()
     assert np.array_equal(out.cpu().numpy(), np.asarray(orc.encode_q4_k(v)).reshape(-1))
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q8_0, H.Q4_0, H.IQ4_NL, H.Q4_K, H.Q5_K, H.Q6_K, H.Q5_0])
+@pytest.mark.parametrize("cols", [256, 1024 - 96, 2048 + 128])  # whole units; a tail of 160 columns; a tail of half a unit
+def test_f32_rows_are_written_in_whole_and_ragged_units(tensor_type, cols):
+    """Dequantised f32 rows bit for bit, nothing written past the last row."""
+    if tensor_type in (H.Q4_K, H.Q5_K, H.Q6_K):
+        cols = (cols + 255) // 256 * 256
+    rows = 11
+    data = H.random_weight(tensor_type, rows, cols, seed=cols)
+    w = ctx().prepare_weight(tensor_type, data, rows, cols)
+    from zllm_b200 import ffi
+    import ctypes as C
+
+    out = torch.full((rows * cols + 64,), 7.0, device="cuda")
+    ffi.call("zq_dequantize_f32", ctx().handle, w.handle, C.c_void_p(out.data_ptr()))
+    ctx().sync()
+    got = out.cpu().numpy()
+    assert np.array_equal(_bits(got[:rows * cols]), _bits(np.asarray(orc.dequantize(tensor_type, data, rows * cols), dtype=np.float32).reshape(-1)))
+    assert np.all(got[rows * cols:] == 7.0)

@@ -193,10 +193,10 @@ __device__ __forceinline__ float decode_unit_element(uint32_t type, const uint8_
     return __fmul_rn(d, (float)kIq4nlValues[nib]);
 }
 
-// Eight consecutive elements i0 .. i0 + 7 (i0 a multiple of 8) of a resident unit, the same bits as decode_unit_element: the
-// scale and the packed words are read once for the eight (an element-wise decode reads and unpacks them eight times, which
-// at 8 bytes of output per packed byte, not HBM, bounded the passes built on it).  The eight elements lie in one 32-element
-// group of every format and, in the re-laid formats, in two words of neighbouring pieces.
+// N = 8 or 4 consecutive elements from i0 (a multiple of N) of a resident unit, the same bits as decode_unit_element: the
+// scale and the packed words are read once for all (an element-wise decode reads and unpacks them eight times, which
+// at 8 bytes of output per packed byte, not HBM, bounded the passes built on it).  The elements lie in one 32-element
+// group of every format and, in the re-laid formats, in one word (of neighbouring pieces) per four.
 // OPERAND: Q4_K and Q5_K values as the GEMM operand forms them (zq_gemm_dq.cuh: one fused multiply-add on 128 + q; the two
 // paths of the GEMM then give the same bits) instead of the codec's multiply-then-subtract.
 __device__ __forceinline__ void bytes_to_f32(uint32_t w, float *v) {  // four unsigned bytes
@@ -230,64 +230,64 @@ __device__ __forceinline__ uint32_t iq4nl_bytes(uint32_t nibs) {  // four codebo
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(T2), "r"(T3), "r"(sel));
     return (hi & mask) | (lo & ~mask);
 }
-template <uint32_t TYPE, bool OPERAND> __device__ __forceinline__ void decode8(const uint8_t *unit, int i0, float (&v)[8]) {
+template <uint32_t TYPE, bool OPERAND, int N> __device__ __forceinline__ void decode_run(const uint8_t *unit, int i0, float (&v)[N]) {
+    static_assert(N == 4 || N == 8, "runs of 4 or 8 elements");
+    constexpr int W = N / 4;  // packed words
     if constexpr (TYPE == ZQ_Q4_K || TYPE == ZQ_Q5_K) {
         const uint4 hdr = *reinterpret_cast<const uint4 *>(unit);
         const int g = i0 >> 5, j0 = i0 & 31;
         float dsc, dm;
         kquant_group(hdr, g, dsc, dm);
-        const uint2 qw = *reinterpret_cast<const uint2 *>(unit + (TYPE == ZQ_Q5_K ? 48 : 16) + (g >> 1) * 32 + j0);
+        auto words = [](const uint8_t *at, uint32_t (&w)[W]) {
+            if constexpr (W == 2) {
+                const uint2 x = *reinterpret_cast<const uint2 *>(at);
+                w[0] = x.x;
+                w[W - 1] = x.y;
+            } else {
+                w[0] = *reinterpret_cast<const uint32_t *>(at);
+            }
+        };
         const int shift = (g & 1) * 4;
-        uint32_t a = (qw.x >> shift) & 0x0F0F0F0Fu, b = (qw.y >> shift) & 0x0F0F0F0Fu;
-        if constexpr (TYPE == ZQ_Q5_K) {
-            const uint2 hb = *reinterpret_cast<const uint2 *>(unit + 16 + j0);
-            a |= ((hb.x >> g) & 0x01010101u) << 4;
-            b |= ((hb.y >> g) & 0x01010101u) << 4;
+        uint32_t q[W], hb[W];
+        words(unit + (TYPE == ZQ_Q5_K ? 48 : 16) + (g >> 1) * 32 + j0, q);
+        if constexpr (TYPE == ZQ_Q5_K) words(unit + 16 + j0, hb);
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            uint32_t a = (q[w] >> shift) & 0x0F0F0F0Fu;
+            if constexpr (TYPE == ZQ_Q5_K) a |= ((hb[w] >> g) & 0x01010101u) << 4;
+            bytes_to_f32(a, v + 4 * w);
         }
-        bytes_to_f32(a, v);
-        bytes_to_f32(b, v + 4);
         const float c = fmaf(-128.0f, dsc, -dm);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = OPERAND ? fmaf(dsc, 128.0f + v[j], c) : __fsub_rn(__fmul_rn(dsc, v[j]), dm);
-    } else if constexpr (TYPE == ZQ_Q6_K) {  // columns 32 G + 16 h + 4 t + i: the eight are (t, 0..3) and (t + 1, 0..3) of one scale group
+        for (int j = 0; j < N; ++j) v[j] = OPERAND ? fmaf(dsc, 128.0f + v[j], c) : __fsub_rn(__fmul_rn(dsc, v[j]), dm);
+    } else if constexpr (TYPE == ZQ_Q6_K) {  // columns 32 G + 16 h + 4 t + i: eight are (t, 0..3) and (t + 1, 0..3) of one scale group
         const int G = i0 >> 5, h = (i0 >> 4) & 1, t = (i0 >> 2) & 3, x2 = 2 * (2 * (G & 1) + h);
         const float ds = __fmul_rn(__half2float(*reinterpret_cast<const __half *>(unit)), (float)(int8_t)unit[kQ6kScales + (i0 >> 4)]);
 #pragma unroll
-        for (int w = 0; w < 2; ++w) {
+        for (int w = 0; w < W; ++w) {
             const uint32_t lo = (*reinterpret_cast<const uint32_t *>(unit + kQ6kLow + 32 * (t + w) + 4 * G) >> (4 * h)) & 0x0F0F0F0Fu;
             const uint32_t hi = (*reinterpret_cast<const uint32_t *>(unit + kQ6kHigh + 16 * (t + w) + 4 * (G >> 1)) >> x2) & 0x03030303u;
             sbytes_to_f32((lo << 2) | (hi << 6), v + 4 * w);  // 4 (q - 32) as s8
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(ds, v[j] * 0.25f);
+        for (int j = 0; j < N; ++j) v[j] = __fmul_rn(ds, v[j] * 0.25f);
     } else if constexpr (TYPE == ZQ_Q8_0 || TYPE == ZQ_Q4_0 || TYPE == ZQ_IQ4_NL) {
         const int blk = i0 >> 5, e = i0 & 31;
         const float d = __half2float(reinterpret_cast<const __half *>(unit)[blk]);
         const uint32_t *src = reinterpret_cast<const uint32_t *>(unit + (unit_quant_offset(TYPE, i0) & ~3));  // the second word is one piece (16 bytes) on
-        uint32_t a = src[0], b = src[4];
-        if constexpr (TYPE != ZQ_Q8_0) {
-            const int shift = (e >> 4) * 4;
-            a = (a >> shift) & 0x0F0F0F0Fu;
-            b = (b >> shift) & 0x0F0F0F0Fu;
-        }
-        if constexpr (TYPE == ZQ_Q4_0) {
-            bytes_to_f32(a, v);
-            bytes_to_f32(b, v + 4);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(v[j] - 8.0f, d);
-        } else {
-            if constexpr (TYPE == ZQ_IQ4_NL) {
-                a = iq4nl_bytes(a);
-                b = iq4nl_bytes(b);
-            }
-            sbytes_to_f32(a, v);
-            sbytes_to_f32(b, v + 4);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = __fmul_rn(d, v[j]);
+        for (int w = 0; w < W; ++w) {
+            uint32_t a = src[4 * w];
+            if constexpr (TYPE != ZQ_Q8_0) a = (a >> ((e >> 4) * 4)) & 0x0F0F0F0Fu;
+            if constexpr (TYPE == ZQ_IQ4_NL) a = iq4nl_bytes(a);
+            if constexpr (TYPE == ZQ_Q4_0) bytes_to_f32(a, v + 4 * w);
+            else sbytes_to_f32(a, v + 4 * w);
         }
+#pragma unroll
+        for (int j = 0; j < N; ++j) v[j] = TYPE == ZQ_Q4_0 ? __fmul_rn(v[j] - 8.0f, d) : __fmul_rn(d, v[j]);
     } else {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = decode_unit_element(TYPE, unit, i0 + j);
+        for (int j = 0; j < N; ++j) v[j] = decode_unit_element(TYPE, unit, i0 + j);
     }
 }
 
@@ -308,8 +308,10 @@ template <class Fn> static int with_type(uint32_t type, zq_error *err, Fn fn) {
     }
 }
 
-// One warp per 256-weight unit, 8 consecutive elements per lane: the packed bytes are read with coalesced loads, the
-// 1 KB (f32) of output is one contiguous store of the warp, the index division is one per warp.
+// One warp per 256-weight unit: the packed bytes are read with coalesced loads, the index division is one per warp.  A lane
+// holds 8 consecutive elements of a 16-bit output, and of an f32 output columns 4 lane .. + 3 of each half of the unit, so that
+// every store of the warp is 512 contiguous bytes: with 8 f32 per lane each of its two stores wrote every other 16 bytes, and
+// the half-written sectors, not HBM, set the pace (Q8_0 17408 x 5120 to f32: 93 -> 68 us, 6.6 TB/s).
 template <uint32_t TYPE>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t *__restrict__ resident, size_t row_pitch, int unit_bytes, size_t total_rows, size_t cols, int units_per_row, const uint32_t *__restrict__ row_ids, size_t n_rows,
                                                          void *__restrict__ out, int out_dtype, uint32_t *status) {
@@ -323,16 +325,22 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t *__restri
             if (lane == 0) atomicMax(status, (uint32_t)kStatusBadIndex);
             continue;
         }
-        const size_t k0 = (size_t)ur * kUnitWeights + 8 * lane;
-        if (k0 >= cols) continue;  // columns are a multiple of 32: all eight elements or none
-        float v[8];
-        decode8<TYPE, false>(resident + srow * row_pitch + (size_t)ur * unit_bytes, 8 * lane, v);
-        const size_t o = orow * cols + k0;
+        const uint8_t *unit = resident + srow * row_pitch + (size_t)ur * unit_bytes;
+        const size_t u0 = (size_t)ur * kUnitWeights, o0 = orow * cols + u0;
         if (out_dtype == ZQ_F32) {
-            float4 *dst = reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + o);
-            dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-            dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int i0 = 128 * h + 4 * lane;
+                if (u0 + i0 >= cols) break;  // columns are a multiple of 32: all four elements or none
+                float v[4];
+                decode_run<TYPE, false>(unit, i0, v);
+                *reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + o0 + i0) = make_float4(v[0], v[1], v[2], v[3]);
+            }
         } else {
+            if (u0 + 8 * lane >= cols) continue;  // all eight elements or none
+            float v[8];
+            decode_run<TYPE, false>(unit, 8 * lane, v);
+            const size_t o = o0 + 8 * lane;
             uint32_t h[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(256) dequantize_f16_batch_kernel(const __grid_
         const int k0 = ur * kUnitWeights + 8 * lane;
         if (k0 >= cols) continue;  // padded tail of the last unit (cols is a multiple of 32, so all 8 or none)
         float v[8];
-        decode8<TYPE, true>(resident + (size_t)row * row_pitch + (size_t)ur * unit_bytes, 8 * lane, v);
+        decode_run<TYPE, true>(resident + (size_t)row * row_pitch + (size_t)ur * unit_bytes, 8 * lane, v);
         uint4 packed;
         packed.x = h2_as_u32(__floats2half2_rn(v[0], v[1]));
         packed.y = h2_as_u32(__floats2half2_rn(v[2], v[3]));
@@ -444,51 +452,96 @@ int launch_dequantize(zq_ctx *ctx, const zq_weight *w, const uint32_t *row_ids, 
 __device__ __forceinline__ float f16_round(float v) { return __half2float(__float2half_rn(v)); }
 __device__ __forceinline__ float clampf(float v, float lo, float hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
-// One code of the Q4_K encoder: clamp(round half away from zero((v + min) / scale), 0, 15).  The IEEE division is only needed
-// where the quotient is within its own error of a rounding boundary: the product with the reciprocal is off by less than
-// 4 ulp (1e-6 relative, 1.6e-5 at the largest code), so anything further than 1e-4 from a half-integer rounds the same.
-// NaN and infinite quotients fail the comparison and take the division.
-__device__ __forceinline__ uint32_t q4k_code(float shifted, float scale, float inv) {
-    const float t = __fmul_rn(shifted, inv), up = t + 0.5f, n = floorf(up), frac = up - n;
-    float r = n;
-    if (!(frac > 1e-4f && frac < 1.0f - 1e-4f) && !(t > 17.0f && t < 1e30f) && !(t < -1.0f && t > -1e30f)) r = roundf(__fdiv_rn(shifted, scale));
-    return (uint32_t)clampf(r, 0.0f, 15.0f);
+// Codes of 32 values under one scale: clamp(round half away from zero((v + shift) / scale), 0, 15), four codes per word.
+// The IEEE division is only needed where the quotient is within its own error of a rounding boundary.  t = shifted * inv with
+// inv = 1 / scale within 2 ulp is off by less than 4e-6 up to the largest code, the division by less than 1e-6, so a t further
+// than 2e-5 from a half-integer rounds the same; a larger t clamps the same.  t is rounded by adding 1.5 * 2^23 (the code is
+// then the low bits of the sum) and the distance to the rounded value is collected over the 32 values (max.NaN keeps a NaN or an
+// infinite quotient), so the fast path takes 8 instructions a value and one test a group; about 1 group in 800 is done again.
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void q4k_codes(const float (&v)[32], float scale, float shift, uint32_t (&q)[8]) {
+    constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+    const float inv = __fdividef(1.0f, scale);
+    float off = 0.0f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        uint32_t u[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float shifted = __fadd_rn(v[4 * w + j], shift);
+            const float up = __fmaf_rn(shifted, inv, kMagic);
+            off = max_nan(off, fabsf(__fmaf_rn(shifted, inv, -__fsub_rn(up, kMagic))));
+            u[j] = __float_as_uint(fminf(fmaxf(up, kMagic), kMagic + 15.0f));
+        }
+        q[w] = __byte_perm(__byte_perm(u[0], u[1], 0x0040), __byte_perm(u[2], u[3], 0x0040), 0x5410);
+    }
+    if (!(off < 0.5f - 2e-5f)) {
+#pragma unroll
+        for (int w = 0; w < 8; ++w) {
+            q[w] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) q[w] |= (uint32_t)clampf(roundf(__fdiv_rn(__fadd_rn(v[4 * w + j], shift), scale)), 0.0f, 15.0f) << (8 * j);
+        }
+    }
 }
 
-// encode_q4_k: one warp per super-block, eight consecutive values per lane (four lanes = one group); same operations in
-// f32 as the reference per value and per group (f16 rounding of d and dmin, round-half-away-from-zero codes), so the bytes
-// are the reference's.  Bound by HBM (4 bytes in, 0.56 out per value).  The thread-per-super-block form it replaces read
-// with a 1 KB stride between lanes, wrote byte by byte and divided for every value.
+// encode_q4_k: a lane holds one group of 32 values, eight lanes a super-block, a warp four super-blocks; same operations in f32
+// as the reference per value and per group (f16 rounding of d and dmin, round-half-away-from-zero codes), so the bytes are the
+// reference's.  Bound by HBM (4 bytes in, 0.56 out per value).  Why a group per lane: with eight values per lane the work per
+// group and per super-block was repeated by 4 and 32 lanes and the kernel was bound by issue (124 us for 17408 x 5120; this
+// form 78 us, 5.2 TB/s).  Values arrive coalesced by cp.async, two tiles of 4 KB per warp in flight, at the chunk position
+// c ^ (group & 7), which keeps both the arriving 16-byte chunks and a lane's reads of its own 128 bytes free of bank conflicts.
 // VEC: values and blocks are 16-byte aligned (a block is 144 bytes, so every block then is).
+constexpr int kEncWarps = 8, kEncTile = 4 * 1024;  // warps per CTA; bytes of a warp's tile (four super-blocks of f32)
+constexpr int kEncSmem = kEncWarps * 2 * kEncTile;
 template <bool VEC>
-__global__ void __launch_bounds__(256) quantize_q4_k_kernel(const float *__restrict__ values, uint8_t *__restrict__ out, size_t blocks) {
-    const int lane = threadIdx.x & 31, sub = lane & 3;
-    for (size_t b = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); b < blocks; b += (size_t)gridDim.x * 8) {
-        const float *src = values + b * 256 + 8 * lane;
-        float v[8];
-        if (VEC) {
-            const float4 f0 = __ldcs(reinterpret_cast<const float4 *>(src)), f1 = __ldcs(reinterpret_cast<const float4 *>(src) + 1);
-            v[0] = f0.x; v[1] = f0.y; v[2] = f0.z; v[3] = f0.w; v[4] = f1.x; v[5] = f1.y; v[6] = f1.z; v[7] = f1.w;
-        } else {
+__global__ void __launch_bounds__(kEncWarps * 32) quantize_q4_k_kernel(const float *__restrict__ values, uint8_t *__restrict__ out, size_t blocks) {
+    extern __shared__ __align__(128) uint8_t enc_smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
+    const uint32_t tiles = smem_u32(enc_smem) + (uint32_t)(warp * 2 * kEncTile);
+    const size_t step = (size_t)gridDim.x * kEncWarps * 4;
+    auto fetch = [&](size_t b0, uint32_t tile) {  // super-blocks b0 .. b0 + 3 of this warp
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = src[j];
+        for (int i = 0; i < 8; ++i) {  // 16-byte chunk i * 32 + lane: chunk lane & 7 of group 4 i + lane / 8
+            const int group = 4 * i + (lane >> 3);
+            const uint32_t dst = tile + (uint32_t)(group * 128 + ((sub ^ (group & 7)) * 16));
+            if (b0 + (i >> 1) < blocks) {
+                const float *src = values + b0 * 256 + (size_t)(i * 32 + lane) * 4;
+                if (VEC) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+                else asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "f"(src[0]), "f"(src[1]), "f"(src[2]), "f"(src[3]) : "memory");
+            }
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    size_t b0 = ((size_t)blockIdx.x * kEncWarps + warp) * 4;
+    if (b0 < blocks) fetch(b0, tiles);
+    for (int buf = 0; b0 < blocks; b0 += step, buf ^= 1) {  // warp-uniform
+        if (b0 + step < blocks) fetch(b0 + step, tiles + (uint32_t)((buf ^ 1) * kEncTile));
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        const uint32_t row = tiles + (uint32_t)(buf * kEncTile + lane * 128);
+        const bool live = b0 + (lane >> 3) < blocks;
+        float v[32];
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[4 * c]), "=f"(v[4 * c + 1]), "=f"(v[4 * c + 2]), "=f"(v[4 * c + 3]) : "r"(row + (uint32_t)((c ^ sub) * 16)) : "memory");
+        __syncwarp();  // every lane has its values: the tile may be filled again
         float minimum = INFINITY, maximum = -INFINITY;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
+        for (int j = 0; j < 32; ++j) {
             minimum = fminf(minimum, v[j]);
             maximum = fmaxf(maximum, v[j]);
-        }
-#pragma unroll
-        for (int s = 1; s <= 2; s <<= 1) {
-            minimum = fminf(minimum, __shfl_xor_sync(0xffffffffu, minimum, s));
-            maximum = fmaxf(maximum, __shfl_xor_sync(0xffffffffu, maximum, s));
         }
         const float group_min = fmaxf(-minimum, 0.0f);
         const float group_scale = __fdiv_rn(fmaxf(__fadd_rn(maximum, group_min), 0.0f), 15.0f);
         float max_scale = fmaxf(group_scale, 0.0f), max_min = fmaxf(group_min, 0.0f);
 #pragma unroll
-        for (int s = 4; s <= 16; s <<= 1) {
+        for (int s = 1; s <= 4; s <<= 1) {
             max_scale = fmaxf(max_scale, __shfl_xor_sync(0xffffffffu, max_scale, s));
             max_min = fmaxf(max_min, __shfl_xor_sync(0xffffffffu, max_min, s));
         }
@@ -496,43 +549,39 @@ __global__ void __launch_bounds__(256) quantize_q4_k_kernel(const float *__restr
         const float d = __half2float(dh), dmin = __half2float(dmh);
         const uint32_t sc = d == 0.0f ? 0 : (uint8_t)clampf(roundf(__fdiv_rn(group_scale, d)), 0.0f, 63.0f);
         const uint32_t mc = dmin == 0.0f ? 0 : (uint8_t)clampf(roundf(__fdiv_rn(group_min, dmin)), 0.0f, 63.0f);
-        // header: byte g of the three scale words comes from groups g and g + 4 (lanes 4 g and 4 g + 16)
-        const uint32_t sc4 = __shfl_down_sync(0xffffffffu, sc, 16), mc4 = __shfl_down_sync(0xffffffffu, mc, 16);
-        const int sh = 2 * (lane & 12);
+        // header: byte g of the three scale words comes from groups g and g + 4 (lanes g and g + 4 of the eight)
+        const uint32_t sc4 = __shfl_down_sync(0xffffffffu, sc, 4), mc4 = __shfl_down_sync(0xffffffffu, mc, 4);
+        const int sh = 8 * (lane & 3);
         uint32_t w1 = ((sc & 0x3fu) | ((sc4 >> 4) << 6)) << sh, w2 = ((mc & 0x3fu) | ((mc4 >> 4) << 6)) << sh, w3 = ((sc4 & 0x0fu) | ((mc4 & 0x0fu) << 4)) << sh;
 #pragma unroll
-        for (int s = 4; s <= 8; s <<= 1) {
+        for (int s = 1; s <= 2; s <<= 1) {
             w1 |= __shfl_xor_sync(0xffffffffu, w1, s);
             w2 |= __shfl_xor_sync(0xffffffffu, w2, s);
             w3 |= __shfl_xor_sync(0xffffffffu, w3, s);
         }
         const uint32_t w0 = (uint32_t)__half_as_ushort(dh) | ((uint32_t)__half_as_ushort(dmh) << 16);
-        // codes: this lane's eight, then the odd group's codes become the high nibbles of the even group's bytes
-        const float scale = __fmul_rn(d, (float)sc), shift = __fmul_rn(dmin, (float)mc), inv = __fdividef(1.0f, scale);
-        uint32_t q0 = 0, q1 = 0;
-        if (scale != 0.0f) {
+        const float scale = __fmul_rn(d, (float)sc), shift = __fmul_rn(dmin, (float)mc);
+        uint32_t q[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        if (scale != 0.0f) q4k_codes(v, scale, shift, q);
+        // the codes of an odd group are the high nibbles of the even group's bytes: the even lane stores bytes 0..15 of the pair's
+        // 32, the odd lane bytes 16..31
+        const bool odd = lane & 1;
+        uint32_t o[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                q0 |= q4k_code(__fadd_rn(v[j], shift), scale, inv) << (8 * j);
-                q1 |= q4k_code(__fadd_rn(v[4 + j], shift), scale, inv) << (8 * j);
-            }
+        for (int w = 0; w < 4; ++w) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? q[w] : q[4 + w], 1);
+            o[w] = odd ? (got | (q[4 + w] << 4)) : (q[w] | (got << 4));
         }
-        q0 |= __shfl_xor_sync(0xffffffffu, q0, 4) << 4;
-        q1 |= __shfl_xor_sync(0xffffffffu, q1, 4) << 4;
-        uint8_t *block = out + b * 144;
+        if (!live) continue;  // no shuffle below
+        uint8_t *block = out + (b0 + (lane >> 3)) * 144, *dst = block + 16 + 16 * sub;
         if (VEC) {
-            if (lane == 0) *reinterpret_cast<uint4 *>(block) = make_uint4(w0, w1, w2, w3);
-            if ((lane & 4) == 0) *reinterpret_cast<uint2 *>(block + 16 + (lane >> 3) * 32 + 8 * sub) = make_uint2(q0, q1);
+            if (sub == 0) *reinterpret_cast<uint4 *>(block) = make_uint4(w0, w1, w2, w3);
+            *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
         } else {
             const uint32_t hw[4] = {w0, w1, w2, w3};
-            if (lane == 0)
-                for (int j = 0; j < 16; ++j) block[j] = (uint8_t)(hw[j >> 2] >> (8 * (j & 3)));
-            if ((lane & 4) == 0) {
-                uint8_t *dst = block + 16 + (lane >> 3) * 32 + 8 * sub;
-                for (int j = 0; j < 4; ++j) {
-                    dst[j] = (uint8_t)(q0 >> (8 * j));
-                    dst[4 + j] = (uint8_t)(q1 >> (8 * j));
-                }
+            for (int j = 0; j < 16; ++j) {
+                if (sub == 0) block[j] = (uint8_t)(hw[j >> 2] >> (8 * (j & 3)));
+                dst[j] = (uint8_t)(o[j >> 2] >> (8 * (j & 3)));
             }
         }
     }
@@ -587,11 +636,12 @@ int launch_quantize(zq_ctx *ctx, uint32_t type, const float *values, size_t rows
     int threads = 128;
     unsigned grid = (unsigned)((blocks + threads - 1) / threads);
     if (type == ZQ_Q4_K) {
-        size_t ctas = (blocks + 7) / 8;
-        if (ctas > (size_t)ctx->sm_count * 64) ctas = (size_t)ctx->sm_count * 64;
+        size_t ctas = (blocks + 4 * kEncWarps - 1) / (4 * kEncWarps);
+        if (ctas > (size_t)ctx->sm_count * 3) ctas = (size_t)ctx->sm_count * 3;  // three CTAs of 64 KB fit an SM; they walk the tensor
         const bool vec = ((reinterpret_cast<uintptr_t>(values) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-        if (vec) quantize_q4_k_kernel<true><<<(unsigned)ctas, 256, 0, ctx->stream>>>(values, reinterpret_cast<uint8_t *>(out), blocks);
-        else quantize_q4_k_kernel<false><<<(unsigned)ctas, 256, 0, ctx->stream>>>(values, reinterpret_cast<uint8_t *>(out), blocks);
+        auto kernel = vec ? quantize_q4_k_kernel<true> : quantize_q4_k_kernel<false>;
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kEncSmem), err);
+        kernel<<<(unsigned)ctas, kEncWarps * 32, kEncSmem, ctx->stream>>>(values, reinterpret_cast<uint8_t *>(out), blocks);
     } else quantize_block32_kernel<<<grid, threads, 0, ctx->stream>>>(type, values, reinterpret_cast<uint8_t *>(out), blocks);
     ctx->launches++;
     ZQ_CUDA_CHECK(cudaGetLastError(), err);
