@@ -60,3 +60,24 @@ def test_rmsnorm_linear_rejects_bad_arguments():
         ctx().rmsnorm_linear(x, dev(np.ones(255, dtype=np.float32)), 1e-6, w)
     with pytest.raises(ffi.ZqFailure):
         ctx().rmsnorm_linear(x, dev(np.ones(256, dtype=np.float32)), -1.0, w)
+
+
+@pytest.mark.parametrize("cols", [32, 288, 3840, 4128, 16416])  # one block; a ragged unit; one turn; a second turn; past the columns held in registers
+@pytest.mark.parametrize("m,dtype,shift", [(1, torch.float32, 0), (16, torch.bfloat16, 0), (3, torch.float16, 1), (17, torch.float32, 1)])
+def test_rmsnorm_records_and_rows_at_edge_widths(cols, m, dtype, shift):
+    """Records written by the norm (up to 16 rows; both formats where the weights want both) and f32 rows (17), input and norm
+    weights also off a 16-byte boundary.  Bounds as above: 16-bit integer activations, f16 operands beyond 16 rows."""
+    rows, eps = 72, 1e-5
+    rng = np.random.default_rng(cols + m)
+    types = [H.Q8_0, H.Q4_K, H.Q6_K] if cols % 256 == 0 else [H.Q8_0, H.IQ4_NL]
+    data = [H.random_weight(t, rows, cols, seed=cols + t) for t in types]
+    ws = [ctx().prepare_weight(t, d, rows, cols) for t, d in zip(types, data)]
+    x = torch.zeros(m * cols + 1, device="cuda", dtype=dtype)[shift:shift + m * cols].view(m, cols)
+    x.copy_(torch.from_numpy((rng.standard_normal((m, cols)) * 2.0).astype(np.float32)))
+    nw = torch.zeros(cols + 1, device="cuda")[shift:shift + cols]
+    nw.copy_(torch.from_numpy((1.0 + 0.1 * rng.standard_normal(cols)).astype(np.float32)))
+    got = ctx().rmsnorm_linear_multi(x, nw, eps, ws, out_dtype=torch.float32)
+    ctx().sync()
+    xn = _rmsnorm(x.float().cpu().numpy(), nw.cpu().numpy(), eps, 0.0)
+    for t, d, y in zip(types, data, got):
+        assert H.max_rel_error(host(y), orc.linear(t, d, rows, cols, xn)) <= (3e-4 if m <= 16 else 2e-3)

@@ -494,6 +494,19 @@ int zq_rmsnorm_linear(zq_ctx *ctx, const zq_weight *const *w, size_t n_weights, 
     const size_t cols = w[0]->cols;
     rc = ensure_scratch_norm(ctx, m * cols * sizeof(float), err);
     if (rc) return rc;
+    // All projections on the work-list kernel (the routing of zq_linear_batch): the norm kernel writes their activation records.
+    WlHostJob listed[3];
+    bool all_listed = !ctx->disable_worklist && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv;
+    for (size_t i = 0; i < n_weights && all_listed; ++i) {
+        listed[i] = {w[i], nullptr, ctx->norm, m, dev_y[i], nullptr, -1};
+        all_listed = gemv_wl_supported(ctx, listed[i]);
+    }
+    if (all_listed) {
+        for (size_t i = 0; i < n_weights; ++i)
+            if ((rc = check_linear(ctx, w[i], ctx->norm, ZQ_F32, m, dev_y[i], y_dtype, err))) return rc;
+        const WlNorm norm = {dev_x, dev_norm_weight, x_dtype, eps, weight_offset};
+        return launch_gemv_wl(ctx, listed, n_weights, ZQ_F32, y_dtype, err, &norm);
+    }
     rc = launch_rmsnorm(ctx, dev_x, x_dtype, m, cols, dev_norm_weight, eps, weight_offset, reinterpret_cast<float *>(ctx->norm), err);
     if (rc) return rc;
     zq_linear_job jobs[3];

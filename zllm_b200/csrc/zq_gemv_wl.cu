@@ -561,7 +561,7 @@ bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &j) {
 
 // Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one record
 // pass per record format, then one decode launch per (weight type, column-tile count, plain / gated) class.
-int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err) {
+int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm) {
     if (n_jobs == 0) return ZQ_OK;
     // ---- records: one block per distinct (x, m, cols, record format)
     struct Src { const void *x; size_t m, cols; bool q4k; size_t rec_begin, units; };
@@ -584,7 +584,12 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
     int rc = ensure_xq(ctx, total_rec * kRec, err);
     if (rc) return rc;
     uint8_t *xq = reinterpret_cast<uint8_t *>(ctx->xq);
-    for (int cls = 0; cls < 2; ++cls) {
+    if (norm) {  // one input, at most one source per format: the norm kernel writes the records
+        uint8_t *rec[2] = {nullptr, nullptr};
+        for (const Src &s : srcs) rec[s.q4k ? 0 : 1] = xq + s.rec_begin * kRec;
+        if ((rc = launch_rmsnorm_records(ctx, *norm, srcs[0].m, srcs[0].cols, rec[0], rec[1], err))) return rc;
+    }
+    for (int cls = 0; cls < 2 && !norm; ++cls) {
         WlQuantArgs qa;
         qa.x_dtype = x_dtype;
         qa.n_src = 0;

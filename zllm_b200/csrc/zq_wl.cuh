@@ -20,6 +20,15 @@ struct WlHostJob {
 
 // True when the job can ride in a work-list launch (Q4_K / Q4_0 / Q8_0, up to 16 activation rows).
 bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &job);
-int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err);
+// An RMSNorm in front of the list: every job's input is norm(x), and the jobs' own `x` is only the name of that one input.
+struct WlNorm {
+    const void *x;
+    const float *weight;
+    int x_dtype;
+    float eps, weight_offset;
+};
+int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm = nullptr);
+// norm(x) as activation records of the K-quant and / or block-32 format (zq_norm.cu); null: format not wanted.
+int launch_rmsnorm_records(zq_ctx *ctx, const WlNorm &norm, size_t m, size_t cols, uint8_t *rec_k, uint8_t *rec_b, zq_error *err);
 
 }  // namespace zq
