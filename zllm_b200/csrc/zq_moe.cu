@@ -452,11 +452,11 @@ __global__ void gather_rows_checked_kernel(const void *__restrict__ x, int dtype
 //   count   per chunk, how many routes go to each expert
 //   scan    one CTA, thread per expert: the chunk's first slot inside each expert's range, the experts' ranges, and
 //           the two work lists of the grouped GEMMs (one item per expert, 256-token tile, 128-row tile) with their counts
-//   place   per chunk: slot of every route (the thread of an expert walks the chunk's routes in order), the
-//           slot -> token table, and each token's slots and weights in combine order
+//   place   per chunk: slot of every route, and each token's slots and weights in combine order
 // Nothing returns to the host: the GEMM kernels read their item counts from device memory.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr int kGroupThreads = 1024;
+constexpr uint32_t kNoSlot = 0xFFFFFFFFu;  // token_slots entry of an absent route
 
 __global__ void __launch_bounds__(kGroupThreads) moe_prefill_count_kernel(const uint32_t *__restrict__ ids, int m, int top_k, int E, int tokens_per_chunk, uint32_t *__restrict__ hist, uint32_t *status) {
     extern __shared__ uint32_t grp_smem[];
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_
 }
 
 __global__ void __launch_bounds__(kGroupThreads) moe_prefill_place_kernel(const uint32_t *__restrict__ ids, const float *__restrict__ wts, int m, int top_k, int E, int tokens_per_chunk, const uint32_t *__restrict__ hist,
-                                                                          const uint32_t *__restrict__ offsets, uint32_t *__restrict__ slot_token, uint32_t *__restrict__ token_slots, float *__restrict__ token_w) {
+                                                                          const uint32_t *__restrict__ offsets, uint32_t *__restrict__ token_slots, float *__restrict__ token_w) {
     extern __shared__ uint32_t grp_smem[];
     const int cap = tokens_per_chunk * top_k;
     uint32_t *s_ids = grp_smem;         // [cap]
@@ -546,7 +546,7 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_place_kernel(const 
     const int r0 = t0 * top_k, nr = (t1 - t0) * top_k;
     for (int r = threadIdx.x; r < nr; r += kGroupThreads) {
         uint32_t id = ids[r0 + r];
-        s_slot[r] = 0;
+        s_slot[r] = kNoSlot;
         if (id == ZQ_MOE_NO_ROUTE) {  // an absent route: no slot, weight 0 in the combine
             s_ids[r] = (uint32_t)E;
             continue;
@@ -565,9 +565,7 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_place_kernel(const 
         int r2 = 0;
         for (; r2 + 4 <= r; r2 += 4) before += (s_ids[r2] == id) + (s_ids[r2 + 1] == id) + (s_ids[r2 + 2] == id) + (s_ids[r2 + 3] == id);
         for (; r2 < r; ++r2) before += s_ids[r2] == id;
-        const uint32_t slot = offsets[id] + hist[(size_t)blockIdx.x * E + id] + before;
-        slot_token[slot] = (uint32_t)((r0 + r) / top_k);
-        s_slot[r] = slot;
+        s_slot[r] = offsets[id] + hist[(size_t)blockIdx.x * E + id] + before;
     }
     __syncthreads();
     for (int t = threadIdx.x; t < t1 - t0; t += kGroupThreads) {
@@ -590,20 +588,20 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_place_kernel(const 
     }
 }
 
-// out16[s] = f16(x[slot_token[s]]) for the slots that exist (their number is on the device); 8 elements per thread
-__global__ void gather_rows_f16_kernel(const void *__restrict__ x, int dtype, const uint32_t *__restrict__ slot_token, const int *__restrict__ n_rows_dev, int hidden, __half *__restrict__ out) {
-    const size_t vec_per_row = (size_t)hidden / 8, total = (size_t)*n_rows_dev * vec_per_row;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / vec_per_row, v = i - r * vec_per_row;
-        const size_t src = (size_t)slot_token[r] * hidden + v * 8;
-        __align__(16) __half h[8];
-        if (dtype == ZQ_F16) {
-            *reinterpret_cast<uint4 *>(h) = *reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(x) + src);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) h[j] = __float2half_rn(load_as_f32(x, dtype, src + j));
+// out16[slot] = f16(x[t]) for every slot of token t: a CTA reads a token's row once and stores it top_k times.  Bound by the stores
+// (routes x hidden x 2 bytes); the form in slot order read every row top_k times, element by element (8192 tokens x 7168, top 8: 378 -> 187 us).
+__global__ void __launch_bounds__(256) scatter_rows_f16_kernel(const void *__restrict__ x, int dtype, const uint32_t *__restrict__ token_slots, int m, int top_k, int hidden, __half *__restrict__ out) {
+    for (int t = blockIdx.x; t < m; t += gridDim.x) {
+        const uint32_t *slots = token_slots + (size_t)t * top_k;
+        for (int v = threadIdx.x; v < hidden / 8; v += 256) {
+            float f[8];
+            load_act8(x, dtype, (size_t)t * hidden + 8 * (size_t)v, true, f);
+            const uint4 h = make_uint4(h2_as_u32(__floats2half2_rn(f[0], f[1])), h2_as_u32(__floats2half2_rn(f[2], f[3])), h2_as_u32(__floats2half2_rn(f[4], f[5])), h2_as_u32(__floats2half2_rn(f[6], f[7])));
+            for (int j = 0; j < top_k; ++j) {
+                const uint32_t s = slots[j];
+                if (s != kNoSlot) reinterpret_cast<uint4 *>(out + (size_t)s * hidden)[v] = h;
+            }
         }
-        reinterpret_cast<uint4 *>(out)[i] = *reinterpret_cast<const uint4 *>(h);
     }
 }
 
@@ -639,12 +637,12 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     const size_t max_tiles = routes / 256 + E;  // sum over experts of ceil(count / 256)
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     // tables and f32 results
-    const size_t o_hist = 0, o_offsets = o_hist + al((size_t)chunks * E * 4), o_counts = o_offsets + al((E + 1) * 4), o_slot_token = o_counts + al(16), o_token_slots = o_slot_token + al(routes * 4);
+    const size_t o_hist = 0, o_offsets = o_hist + al((size_t)chunks * E * 4), o_counts = o_offsets + al((E + 1) * 4), o_token_slots = o_counts + al(16);
     const size_t o_token_w = o_token_slots + al(routes * 4), o_out = o_token_w + al(routes * 4), o_shared = o_out + al(routes * H * 4), total = o_shared + (has_shared ? al(m * H * 4) : 0);
     int rc = ensure_moe_ws(ctx, total, err);
     if (rc) return rc;
     uint8_t *ws = reinterpret_cast<uint8_t *>(ctx->moe_ws);
-    uint32_t *d_hist = reinterpret_cast<uint32_t *>(ws + o_hist), *d_offsets = reinterpret_cast<uint32_t *>(ws + o_offsets), *d_slot_token = reinterpret_cast<uint32_t *>(ws + o_slot_token);
+    uint32_t *d_hist = reinterpret_cast<uint32_t *>(ws + o_hist), *d_offsets = reinterpret_cast<uint32_t *>(ws + o_offsets);
     uint32_t *d_token_slots = reinterpret_cast<uint32_t *>(ws + o_token_slots);
     int *d_counts = reinterpret_cast<int *>(ws + o_counts);
     float *d_token_w = reinterpret_cast<float *>(ws + o_token_w), *d_out = reinterpret_cast<float *>(ws + o_out), *d_shared = has_shared ? reinterpret_cast<float *>(ws + o_shared) : nullptr;
@@ -665,8 +663,8 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     }
     moe_prefill_count_kernel<<<chunks, kGroupThreads, E * 4, ctx->stream>>>(dev_ids, (int)m, (int)top_k, (int)E, tokens_per_chunk, d_hist, ctx->status_dev);
     moe_prefill_scan_kernel<<<1, kGroupThreads, 0, ctx->stream>>>(d_hist, chunks, (int)E, d_offsets, rt_i, rt_h, d_items_g, d_items_d, d_counts);
-    moe_prefill_place_kernel<<<chunks, kGroupThreads, place_smem, ctx->stream>>>(dev_ids, dev_weights, (int)m, (int)top_k, (int)E, tokens_per_chunk, d_hist, d_offsets, d_slot_token, d_token_slots, d_token_w);
-    gather_rows_f16_kernel<<<grid_for(ctx, routes * (H / 8), 256), 256, 0, ctx->stream>>>(dev_x, x_dtype, d_slot_token, d_counts + 2, (int)H, x16);
+    moe_prefill_place_kernel<<<chunks, kGroupThreads, place_smem, ctx->stream>>>(dev_ids, dev_weights, (int)m, (int)top_k, (int)E, tokens_per_chunk, d_hist, d_offsets, d_token_slots, d_token_w);
+    scatter_rows_f16_kernel<<<(unsigned)(m < (size_t)ctx->sm_count * 32 ? m : (size_t)ctx->sm_count * 32), 256, 0, ctx->stream>>>(dev_x, x_dtype, d_token_slots, (int)m, (int)top_k, (int)H, x16);
     ctx->launches += 4;
     ZQ_CUDA_CHECK(cudaGetLastError(), err);
     rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, x16, routes, d_items_g, (int)(max_tiles * rt_i), d_counts, act16, ZQ_F16, err);
