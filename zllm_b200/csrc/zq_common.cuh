@@ -289,6 +289,7 @@ struct zq_ctx {
     std::vector<PendingOut> pending_out;
     std::vector<PendingLinear> pending_linear;
     std::vector<PendingIn> pending_in;
+    size_t pending_in_bytes = 0;  // copied in for the layers of pending_linear
     bool batch_active = false;
     // Diagnostics: 1 = always use the per-item activation staging GEMV (the variant for activations too large to
     // stay resident in shared memory), so that tests can cover it at small sizes.
