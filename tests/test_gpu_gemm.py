@@ -139,3 +139,29 @@ def test_prefill_gated_edges(tensor_type, m, rows, cols):
     sel = [0, 1, m // 2, m - 1]
     want = orc.gated_linear(tensor_type, gate, up, rows, cols, x.float().cpu().numpy()[sel])
     assert H.max_rel_error(got[sel], want) <= 2.1 * BOUND
+
+
+@pytest.mark.parametrize("m", [17, 48, 300])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_projections_that_feed_each_other_wait_for_each_other(m, dtype):
+    """A GEMM is set up under the kernel before it (operand conversion or another GEMM): a chain enqueued at once gives the bits of
+    the same chain with a wait behind every call."""
+    cols = 1024
+    ws = [ctx().prepare_weight(t, H.random_weight(t, cols, cols, seed=160 + i), cols, cols) for i, t in enumerate((H.Q4_K, H.Q8_0, H.IQ4_NL, H.Q6_K))]
+    x0 = torch.from_numpy(np.random.default_rng(161).standard_normal((m, cols)).astype(np.float32)).to("cuda", dtype)
+
+    def chain(wait):
+        x, outs = x0, []
+        for i in range(8):
+            y = ctx().linear(x, ws[i % 4], residual=x)
+            if wait:
+                ctx().sync()
+            x = (y * 0.5).to(dtype)
+            outs.append(ctx().gated_linear(x, ws[i % 4], ws[i % 4], out_dtype=torch.float32))
+        ctx().sync()
+        return [o.cpu().numpy() for o in outs]
+
+    want = chain(True)
+    for _ in range(3):
+        for a, b in zip(chain(False), want):
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
