@@ -156,9 +156,11 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     uint64_t *empty = full + 8;
     __shared__ uint32_t s_abort;
     __shared__ int s_nseg, s_last, s_c0, s_cl;
-    // Up to 8 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with
-    // 9..16 rows that warp would need longer than the consumers themselves, so they do it together (and wait for it).
-    constexpr bool kAsyncFix = NT < 4;
+    // Up to 4 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with
+    // more that warp would need longer than the consumers themselves, so they do it together (and wait for it).  5..8 rows,
+    // one warp -> all: gated Q4_K 5120 -> 10240 at 8 rows 32.5 -> 23.1 us, at 5 rows 27.8 -> 22.7; two plain projections of that
+    // shape 25.8 -> 23.4 at 8 rows, 23.6 -> 23.1 at 5 (the worst seen: IQ4_NL 3840 -> 15360 at 5 rows, 29.6 -> 30.7).
+    constexpr bool kAsyncFix = NT < 2;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long G = gridDim.x, Q = a.q_total;
