@@ -171,3 +171,46 @@ def test_argument_errors():
     x = dev(np.zeros((1, cols), dtype=np.float32))
     with pytest.raises(ffi.ZqFailure):
         ctx().linear_batch([(x, w, w2, "gated")])  # gate and up differ in shape
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.IQ4_NL])
+@pytest.mark.parametrize("m", [1, 5, 16])
+def test_gated_pair_whose_tiles_fill_half_the_machine(tensor_type, m):
+    """76 tiles of 15 ring items on 148 SMs: dealt out by the work-list kernel (record pass + list), the last tile one row high.
+    Against the CPU path by the contract; against the single-matrix kernel, which takes the same activation records and differs
+    in the order of its f32 sums only: 2 x 29 terms of one projection are off by 58 x 2^-24 of the sum of their magnitudes, which
+    is about sqrt(29) times the result's rms, twice (gate and up): 4e-5."""
+    rows, cols = 4801, 7424
+    gate, up = H.random_weight(tensor_type, rows, cols, seed=150), H.random_weight(tensor_type, rows, cols, seed=151)
+    x = np.random.default_rng(152 + m).standard_normal((m, cols)).astype(np.float32)
+    wg, wu = ctx().prepare_weight(tensor_type, gate, rows, cols), ctx().prepare_weight(tensor_type, up, rows, cols)
+    before = ctx().launch_count
+    got = host(ctx().gated_linear(dev(x), wg, wu))
+    assert ctx().launch_count - before == 2
+    _check(got, orc.gated_linear(tensor_type, gate, up, rows, cols, x), tight=BOUND)
+    ctx().set_option("disable_worklist", 1)
+    try:
+        alone = host(ctx().gated_linear(dev(x), wg, wu))
+    finally:
+        ctx().set_option("disable_worklist", 0)
+    assert H.max_rel_error(got, alone) <= 4e-5
+
+
+def test_first_gated_call_of_a_context_can_be_captured():
+    """The gated pair that goes to the work-list kernel finds its record buffer in place: no allocation under capture."""
+    from zllm_b200.backend import B200Context
+
+    rows, cols = 4801, 7424
+    data = H.random_weight(H.Q4_K, rows, cols, seed=170)
+    c = B200Context(0, use_torch_stream=False)
+    stream = torch.cuda.Stream()
+    w = c.prepare_weight(H.Q4_K, data, rows, cols)
+    x = dev(np.random.default_rng(171).standard_normal((4, cols)).astype(np.float32))
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        c.set_stream(torch.cuda.current_stream().cuda_stream)
+        y = c.gated_linear(x, w, w)
+    graph.replay()
+    torch.cuda.synchronize()
+    _check(host(y), orc.gated_linear(H.Q4_K, data, data, rows, cols, x.cpu().numpy()), tight=BOUND)

@@ -154,6 +154,10 @@ static int ctx_allocate(zq_ctx *ctx, zq_error *err) {
     ctx->stream = ctx->own_stream;
     ctx->gemv_partials_floats = (size_t)ctx->sm_count * 2 * 128 * 16;  // two partial-tile slots (128 rows x 16 activation rows) per CTA
     ZQ_CUDA_CHECK(cudaMalloc(&ctx->gemv_partials, ctx->gemv_partials_floats * sizeof(float)), err);
+    // a first MB of activation records (4 rows of 116 000 columns): a gated decode call of up to 4 rows allocates nothing, also when
+    // it is the first call of a context and is being captured
+    int rc_xq = ensure_xq(ctx, size_t(1) << 20, err);
+    if (rc_xq) return rc_xq;
     ctx->gemv_counters_n = 1 << 16;
     ZQ_CUDA_CHECK(cudaMalloc(&ctx->gemv_counters, ctx->gemv_counters_n * sizeof(uint32_t)), err);
     ZQ_CUDA_CHECK(cudaMemset(ctx->gemv_counters, 0, ctx->gemv_counters_n * sizeof(uint32_t)), err);
@@ -519,6 +523,8 @@ int zq_gated_silu(zq_ctx *ctx, const zq_weight *gate, const zq_weight *up, const
     if (rc) return rc;
     if (!up || up->ctx != ctx) return set_error(err, ZQ_ERR_ARG, "gated linear: bad up weight");
     if (gate->rows != up->rows || gate->cols != up->cols || gate->type != up->type) return set_error(err, ZQ_ERR_SHAPE, "gated linear: gate [%zu, %zu] type %u and up [%zu, %zu] type %u differ", gate->rows, gate->cols, gate->type, up->rows, up->cols, up->type);
+    const WlHostJob listed = {gate, up, dev_x, m, dev_y, nullptr, -1};
+    if (!ctx->disable_worklist && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv && gemv_wl_supported(ctx, listed) && gated_prefers_worklist(ctx, gate, m)) return launch_gemv_wl(ctx, &listed, 1, x_dtype, y_dtype, err);
     if (m <= 16 && (!is_operand_pass_only(gate->type) || ((gate->type == ZQ_Q5_K || gate->type == ZQ_Q6_K) && !ctx->force_f16_gemv && !ctx->force_staged_gemv))) return launch_gemv(ctx, gate, up, dev_x, x_dtype, m, dev_y, y_dtype, nullptr, err);
     return launch_gemm(ctx, gate, up, dev_x, x_dtype, m, dev_y, y_dtype, nullptr, err);
 }

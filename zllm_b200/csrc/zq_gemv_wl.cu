@@ -561,6 +561,24 @@ bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &j) {
     return true;
 }
 
+// A gated decode launch of gemv_i8_kernel walks ceil(tiles * slices / SMs) rounds of whole slices; the work-list kernel deals the
+// same ring items out evenly, for a record pass, a longer start and the hand-over of cut tiles, ~5 us together.  It is taken when
+// the busiest SM would walk at least 216 KB of weights less, those 5 us at ~43 GB/s per SM.  Measured at 1 row, gemv_i8 -> work
+// list: 5120 -> 10240 (20 items on the busiest SM against 11) Q4_K 22.4 -> 18.3 us, IQ4_NL 30.7 -> 23.1, Q8_0 29.0 -> 25.8 (at 8
+// rows 27.2 -> 23.0, 36.0 -> 27.8, 34.3 -> 29.4); 4096 -> 11008 (16 against 10, the smallest difference that passes in a 4-bit
+// type) 18.2 -> 16.2, 25.4 -> 20.7; on the other side 3840 -> 15360 (16 against 13) Q4_K 18.8 and 18.9, Q8_0 25.1 and 27.0.
+// Up to 4 rows gemv_i8_kernel needs no workspace, so the list is only taken there when the record buffer holds its records as it is.
+bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) {
+    if (m <= 4 && m * gate->units_per_row * kRec > ctx->xq_bytes) return false;
+    const size_t sms = (size_t)ctx->sm_count, tiles = (gate->rows + kTileRows / 2 - 1) / (kTileRows / 2), chunks = (gate->units_per_row + kChunkUnits - 1) / kChunkUnits;
+    size_t split = tiles ? sms / tiles : 1;
+    if (split > 8) split = 8;
+    if (split > chunks) split = chunks;
+    if (split < 1) split = 1;
+    const size_t single = (tiles * split + sms - 1) / sms * ((chunks + split - 1) / split), even = (tiles * chunks + sms - 1) / sms;
+    return single > even && (single - even) * kTileRows * kChunkUnits * format_info(gate->type).unit_bytes >= 216 * 1024;
+}
+
 // Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one record
 // pass per record format, then one decode launch per (weight type, column-tile count, plain / gated) class.
 int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm) {
