@@ -214,3 +214,26 @@ def test_first_gated_call_of_a_context_can_be_captured():
     graph.replay()
     torch.cuda.synchronize()
     _check(host(y), orc.gated_linear(H.Q4_K, data, data, rows, cols, x.cpu().numpy()), tight=BOUND)
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_bracket_that_sends_its_layers_out_in_several_batches(pinned):
+    """16 rows: the layers go out whenever their activations pass 1 MB, so this list is sent in parts; an input read before and after
+    a part goes out, inputs that arrive while one runs, a last layer below the limit.  Twice, with other inputs."""
+    m = 16
+    shapes = [(2048, 8192, 0), (1024, 16400, 1), (2048, 300, 0), (17408, 640, 2), (1024, 72, 1)]  # columns, rows, input
+    weights = [(_weight(H.Q4_0, rows, cols, 180 + i), cols, rows, k) for i, (cols, rows, k) in enumerate(shapes)]
+    for seed in (190, 191):
+        rng = np.random.default_rng(seed)
+
+        def buf(shape):
+            t = torch.zeros(shape)
+            return (t.pin_memory() if pinned else t)
+
+        xs = {k: buf((m, cols)) for _, cols, _, k in weights}
+        for t in xs.values():
+            t.copy_(torch.from_numpy(rng.standard_normal(tuple(t.shape)).astype(np.float32)))
+        ys = [buf((m, rows)) for _, _, rows, _ in weights]
+        ctx().linear_host_batch([(xs[k].numpy(), w, y.numpy()) for ((_, w), _, _, k), y in zip(weights, ys)])
+        for ((data, _), cols, rows, k), y in zip(weights, ys):
+            _check(y.numpy(), orc.linear(H.Q4_0, data, rows, cols, xs[k].numpy()))
