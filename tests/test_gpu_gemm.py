@@ -165,3 +165,24 @@ def test_projections_that_feed_each_other_wait_for_each_other(m, dtype):
     for _ in range(3):
         for a, b in zip(chain(False), want):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+def test_operand_is_the_dequantised_value_rounded_once(tensor_type):
+    """Rows of the identity as activations (exact in f16, one non-zero product per sum) read the weight operand back bit for bit:
+    the codec's f32 value rounded once to f16, for scale and minimum of any ratio, down to values that nearly cancel."""
+    rows, cols = 300, 512
+    e, b = orc.BLOCK[tensor_type]
+    data = H.random_bytes_weight(tensor_type, rows, cols, seed=17).reshape(-1, b)
+    rng = np.random.default_rng(18)
+    exponent = rng.integers(-14, -4, size=len(data))
+    scales = [np.ldexp(1.0 + rng.random(len(data)), exponent).astype(np.float16)]
+    if len(H.SCALE_OFFSETS[tensor_type]) == 2:  # minimum: 2^-9 .. 2^4 times the scale
+        scales.append(np.ldexp(1.0 + rng.random(len(data)), exponent + rng.integers(-9, 5, size=len(data))).astype(np.float16))
+    for off, v in zip(H.SCALE_OFFSETS[tensor_type], scales):
+        data[:, off:off + 2] = v.view(np.uint8).reshape(-1, 2)
+    data = data.reshape(-1)
+    want = orc.dequantize(tensor_type, data, rows * cols).reshape(rows, cols).astype(np.float16)
+    w = ctx().prepare_weight(tensor_type, data, rows, cols)
+    got = host(ctx().linear(torch.eye(cols, device="cuda", dtype=torch.float16), w, out_dtype=torch.float32)).T
+    assert np.array_equal(got, want.astype(np.float32))

@@ -197,8 +197,6 @@ __device__ __forceinline__ float decode_unit_element(uint32_t type, const uint8_
 // scale and the packed words are read once for all (an element-wise decode reads and unpacks them eight times, which
 // at 8 bytes of output per packed byte, not HBM, bounded the passes built on it).  The elements lie in one 32-element
 // group of every format and, in the re-laid formats, in one word (of neighbouring pieces) per four.
-// OPERAND: Q4_K and Q5_K values as the GEMM operand forms them (zq_gemm_dq.cuh: one fused multiply-add on 128 + q; the two
-// paths of the GEMM then give the same bits) instead of the codec's multiply-then-subtract.
 __device__ __forceinline__ void bytes_to_f32(uint32_t w, float *v) {  // four unsigned bytes
 #pragma unroll
     for (int j = 0; j < 4; ++j) v[j] = (float)((w >> (8 * j)) & 0xFFu);
@@ -230,7 +228,7 @@ __device__ __forceinline__ uint32_t iq4nl_bytes(uint32_t nibs) {  // four codebo
     asm("prmt.b32 %0, %1, %2, %3;" : "=r"(hi) : "r"(T2), "r"(T3), "r"(sel));
     return (hi & mask) | (lo & ~mask);
 }
-template <uint32_t TYPE, bool OPERAND, int N> __device__ __forceinline__ void decode_run(const uint8_t *unit, int i0, float (&v)[N]) {
+template <uint32_t TYPE, int N> __device__ __forceinline__ void decode_run(const uint8_t *unit, int i0, float (&v)[N]) {
     static_assert(N == 4 || N == 8, "runs of 4 or 8 elements");
     constexpr int W = N / 4;  // packed words
     if constexpr (TYPE == ZQ_Q4_K || TYPE == ZQ_Q5_K) {
@@ -257,9 +255,8 @@ template <uint32_t TYPE, bool OPERAND, int N> __device__ __forceinline__ void de
             if constexpr (TYPE == ZQ_Q5_K) a |= ((hb[w] >> g) & 0x01010101u) << 4;
             bytes_to_f32(a, v + 4 * w);
         }
-        const float c = fmaf(-128.0f, dsc, -dm);
 #pragma unroll
-        for (int j = 0; j < N; ++j) v[j] = OPERAND ? fmaf(dsc, 128.0f + v[j], c) : __fsub_rn(__fmul_rn(dsc, v[j]), dm);
+        for (int j = 0; j < N; ++j) v[j] = __fsub_rn(__fmul_rn(dsc, v[j]), dm);
     } else if constexpr (TYPE == ZQ_Q6_K) {  // columns 32 G + 16 h + 4 t + i: eight are (t, 0..3) and (t + 1, 0..3) of one scale group
         const int G = i0 >> 5, h = (i0 >> 4) & 1, t = (i0 >> 2) & 3, x2 = 2 * (2 * (G & 1) + h);
         const float ds = __fmul_rn(__half2float(*reinterpret_cast<const __half *>(unit)), (float)(int8_t)unit[kQ6kScales + (i0 >> 4)]);
@@ -333,13 +330,13 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t *__restri
                 const int i0 = 128 * h + 4 * lane;
                 if (u0 + i0 >= cols) break;  // columns are a multiple of 32: all four elements or none
                 float v[4];
-                decode_run<TYPE, false>(unit, i0, v);
+                decode_run<TYPE>(unit, i0, v);
                 *reinterpret_cast<float4 *>(reinterpret_cast<float *>(out) + o0 + i0) = make_float4(v[0], v[1], v[2], v[3]);
             }
         } else {
             if (u0 + 8 * lane >= cols) continue;  // all eight elements or none
             float v[8];
-            decode_run<TYPE, false>(unit, 8 * lane, v);
+            decode_run<TYPE>(unit, 8 * lane, v);
             const size_t o = o0 + 8 * lane;
             uint32_t h[4];
 #pragma unroll
@@ -362,8 +359,8 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t *__restri
     }
 }
 
-// Packed rows -> f16 [rows, cols]: the operand pass of the prefill GEMM.  Each value is the weight's f32 value rounded
-// once (Q4_K: through one fused multiply-add, i.e. at least as close to the exact value as the codec's two-step form).  Up to kDequantBatch matrices of one type and shape
+// Packed rows -> f16 [rows, cols]: the operand pass of the prefill GEMM.  Each value is the codec's f32 value rounded
+// once (zq_gemm_dq.cuh forms the same bits).  Up to kDequantBatch matrices of one type and shape
 // per launch (MoE prefill dequantises the experts of a chunk together).  One warp per 256-weight unit, 8 consecutive elements per lane: the
 // unit's packed bytes are read once with coalesced loads, the 512 output bytes are one coalesced store, and the only
 // index division is one per warp.
@@ -384,7 +381,7 @@ __global__ void __launch_bounds__(256) dequantize_f16_batch_kernel(const __grid_
         const int k0 = ur * kUnitWeights + 8 * lane;
         if (k0 >= cols) continue;  // padded tail of the last unit (cols is a multiple of 32, so all 8 or none)
         float v[8];
-        decode_run<TYPE, true>(resident + (size_t)row * row_pitch + (size_t)ur * unit_bytes, 8 * lane, v);
+        decode_run<TYPE>(resident + (size_t)row * row_pitch + (size_t)ur * unit_bytes, 8 * lane, v);
         uint4 packed;
         packed.x = h2_as_u32(__floats2half2_rn(v[0], v[1]));
         packed.y = h2_as_u32(__floats2half2_rn(v[2], v[3]));

@@ -7,13 +7,16 @@
 // register: an instruction that uses it has waited for the loads, so the box may be given back to the TMA unit behind it.  Shared memory is addressed
 // by 32-bit shared addresses: as generic accesses the stores cost the fence behind them several times as much.
 //
-// Arithmetic, all with ONE rounding to f16 of a value that carries f32 precision or is exact:
-//   Q4_K, Q5_K, Q6_K   a code byte placed under the exponent of 2^7 is the float 128 + q; fma(s, 128 + q, c) with
-//                      c = offset - 128 s gives s q + offset.  c is off by at most 2^-18 s, 2^-9 or less of the f16
-//                      rounding step of the values it is added to.  Two fused multiply-adds per instruction (fma.rn.f32x2).
+// Arithmetic: every operand is the codec's f32 value rounded once to f16.
+//   Q4_K, Q5_K   a code byte placed under the exponent of 2^7 is the float 128 + q; 128 is taken off again (exact) and
+//                fma(s, q, -m) rounds once to f32: s = d sc has at most 17 significant bits, so s q is exact in the codec's
+//                product too.  One multiply-add on 128 + q with 128 s folded into the offset is an instruction less per two weights,
+//                but rounds that offset at 2^-17 s and loses bits of m where it is small beside the scale.
+//   Q6_K         fma(s, 128 + q + 32, -160 s) = s q: 160 s is exact, there is no other offset.
+//                Two additions or multiply-adds per instruction (add.rn.f32x2, fma.rn.f32x2).
 //   Q4_0, IQ4_NL, Q8_0 d q with d an f16 and q an integer of at most 8 bits: an f16 multiply rounds the exact product once,
 //                      which is what multiplying in f32 (exact) and rounding does.
-// About 2.5 instructions per weight for Q4_K, half on the ALU pipe (byte permutes); the form before this one took a permute,
+// About 3 instructions per weight for Q4_K, a good third on the ALU pipe (byte permutes); the form before this one took a permute,
 // a subtraction and a multiply-add per weight (9 instructions with its waits).
 #pragma once
 #include "zq_common.cuh"
@@ -30,19 +33,20 @@ __device__ __forceinline__ uint64_t dq_pair(float v) {
     asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
     return r;
 }
-// codes in bytes J, J + 1 of `codes` -> f16x2 of s * q + (c + 128 s)
-template <int J> __device__ __forceinline__ uint32_t dq_fma2(uint32_t codes, uint64_t s2, uint64_t c2) {
+// codes in bytes J, J + 1 of `codes` -> f16x2 of s * q + c; BIASED: of s * (128 + q) + c
+template <int J, bool BIASED> __device__ __forceinline__ uint32_t dq_fma2(uint32_t codes, uint64_t s2, uint64_t c2) {
     const uint32_t a = dq_prmt(codes, 0x43000000u, 0x7044u + (J << 8)), b = dq_prmt(codes, 0x43000000u, 0x7044u + ((J + 1) << 8));
     uint64_t v;
     uint32_t lo, hi, r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a), "r"(b));
+    if constexpr (!BIASED) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(0xC3000000C3000000ull));  // - 128
     asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(v) : "l"(s2), "l"(c2));
     asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
     return r;
 }
-__device__ __forceinline__ uint4 dq_chunk_fma(uint32_t w0, uint32_t w1, uint64_t s2, uint64_t c2) {
-    return make_uint4(dq_fma2<0>(w0, s2, c2), dq_fma2<2>(w0, s2, c2), dq_fma2<0>(w1, s2, c2), dq_fma2<2>(w1, s2, c2));
+template <bool BIASED> __device__ __forceinline__ uint4 dq_chunk_fma(uint32_t w0, uint32_t w1, uint64_t s2, uint64_t c2) {
+    return make_uint4(dq_fma2<0, BIASED>(w0, s2, c2), dq_fma2<2, BIASED>(w0, s2, c2), dq_fma2<0, BIASED>(w1, s2, c2), dq_fma2<2, BIASED>(w1, s2, c2));
 }
 // unsigned bytes -> f16 (byte - bias) * d; bias2 = f16x2 of 1024 + bias, d2 = f16x2 of d
 __device__ __forceinline__ uint4 dq_chunk_mul(uint32_t w0, uint32_t w1, uint32_t bias2, uint32_t d2) {
@@ -73,7 +77,7 @@ __device__ __forceinline__ uint32_t dq_lds32(uint32_t addr) {
     return v;
 }
 
-// (d sc, -dmin m - 128 d sc) of scale groups 2 kb and 2 kb + 1 of a K-quant super-block header; kb is warp-uniform
+// (d sc, -dmin m) of scale groups 2 kb and 2 kb + 1 of a K-quant super-block header; kb is warp-uniform
 __device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2], float (&c)[2]) {
     const __half2 dd = u32_as_h2(hdr.x);
     const float d = __low2float(dd), dmin = __high2float(dd);
@@ -92,7 +96,7 @@ __device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         s[n] = __fmul_rn(d, (float)((scw >> (8 * n)) & 0xFFu));
-        c[n] = fmaf(-128.0f, s[n], -__fmul_rn(dmin, (float)((mnw >> (8 * n)) & 0xFFu)));
+        c[n] = -__fmul_rn(dmin, (float)((mnw >> (8 * n)) & 0xFFu));
     }
 }
 
@@ -137,7 +141,7 @@ template <bool Q5> struct DqBlockK {
                         m[i] |= ((hw >> (g + n)) << 4) & 0x10101010u;
                     }
                 }
-                dq_store(row_base, sw, 4 * n + c8, dq_chunk_fma(m[0], m[1], s2, c2));
+                dq_store(row_base, sw, 4 * n + c8, dq_chunk_fma<false>(m[0], m[1], s2, c2));
             }
         }
     }
@@ -176,7 +180,7 @@ template <> struct DqBlock<ZQ_Q6_K> {
                 const uint32_t l = (hh ? (lw >> 4) : lw) & 0x0F0F0F0Fu, u = (x2 >= 4 ? (hw >> (x2 - 4)) : (hw << (4 - x2))) & 0x30303030u;
                 m[w] = (l | u) ^ 0x20202020u;
             }
-            dq_store(row_base, sw, c8, dq_chunk_fma(m[0], m[1], s2, c2));
+            dq_store(row_base, sw, c8, dq_chunk_fma<true>(m[0], m[1], s2, c2));
         }
     }
 };
