@@ -572,7 +572,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     // overtakes shared-memory loads still queued behind other warps' stores, and the next box lands under them.
                     if (__any_sync(0xffffffffu, dq.mix() == 0x9E3779B9u)) __nanosleep(0);  // a no-op that keeps the vote
                     if (lane == 0) mbar_arrive(&p_empty[ps]);
-                    const bool folded = dq.folds();
                     if (++ps == PST) {
                         ps = 0;
                         pph ^= 1u;
@@ -580,7 +579,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     advance(mine);
                     if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, abort_addr, p.status, kStatusMmaTimeout, 20);
                     if (!ok) break;
-                    dq.emit(row0 + (uint32_t)(s * S::stage_bytes), sw, folded);
+                    dq.emit(row0 + (uint32_t)(s * S::stage_bytes), sw);
                     fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores of the pair
                     __syncwarp();
                     if (lane == 0) pair_arrive(pair_first(smem_u32(&full[s])));

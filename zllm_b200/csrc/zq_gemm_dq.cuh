@@ -4,17 +4,14 @@
 // DqBlock<TYPE>::load brings what it needs of the unit into registers (at the row pitches of these formats the eight rows of
 // a quarter-warp's 16-byte loads fall into eight different bank groups, Q6_K excepted), emit() turns it into eight 16-byte
 // chunks and stores them at their 128-byte-swizzle positions (chunk c of row r at c ^ (r & 7)).  mix() reads every loaded
-// register: an instruction that uses it has waited for the loads, so the box may be given back to the TMA unit behind it; folds() is
-// what emit() needs to know of the whole warp.  Shared memory is addressed
+// register: an instruction that uses it has waited for the loads, so the box may be given back to the TMA unit behind it.  Shared memory is addressed
 // by 32-bit shared addresses: as generic accesses the stores cost the fence behind them several times as much.
 //
 // Arithmetic: every operand is the codec's f32 value rounded once to f16.
-//   Q4_K, Q5_K   a code byte placed under the exponent of 2^7 is the float 128 + q; with c = -128 s - m, fma(s, 128 + q, c) is
-//                s q - m, rounded once, where c is exact.  s and m have at most 17 significant bits, so it is wherever the last
-//                bits of 128 s and m are at most 2^7 apart: in practice all of a tensor whose minima are a few scales large.  Where
-//                a lane's c is not exact (m small beside s), its warp takes 128 off first (exact) and uses fma(s, q, -m), an
-//                instruction more per two weights (MoE layer of 8192 tokens 8.07 -> 8.26 ms if done always).  s q is exact in the
-//                codec's own product, so this is its value.
+//   Q4_K, Q5_K   a code byte placed under the exponent of 2^7 is the float 128 + q; 128 is taken off again (exact) and
+//                fma(s, q, -m) rounds once to f32: s = d sc has at most 17 significant bits, so s q is exact in the codec's
+//                product too.  One multiply-add on 128 + q with 128 s folded into the offset is an instruction less per two weights,
+//                but rounds that offset at 2^-17 s and loses bits of m where it is small beside the scale.
 //   Q6_K         fma(s, 128 + q + 32, -160 s) = s q: 160 s is exact, there is no other offset.
 //                Two additions or multiply-adds per instruction (add.rn.f32x2, fma.rn.f32x2).
 //   Q4_0, IQ4_NL, Q8_0 d q with d an f16 and q an integer of at most 8 bits: an f16 multiply rounds the exact product once,
@@ -80,8 +77,8 @@ __device__ __forceinline__ uint32_t dq_lds32(uint32_t addr) {
     return v;
 }
 
-// d sc and -dmin m of scale groups 2 kb and 2 kb + 1 of a K-quant super-block header; kb is warp-uniform
-__device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2], float (&nm)[2]) {
+// (d sc, -dmin m) of scale groups 2 kb and 2 kb + 1 of a K-quant super-block header; kb is warp-uniform
+__device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2], float (&c)[2]) {
     const __half2 dd = u32_as_h2(hdr.x);
     const float d = __low2float(dd), dmin = __high2float(dd);
     uint32_t scw, mnw;  // the four groups of this half as bytes
@@ -99,7 +96,7 @@ __device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         s[n] = __fmul_rn(d, (float)((scw >> (8 * n)) & 0xFFu));
-        nm[n] = -__fmul_rn(dmin, (float)((mnw >> (8 * n)) & 0xFFu));
+        c[n] = -__fmul_rn(dmin, (float)((mnw >> (8 * n)) & 0xFFu));
     }
 }
 
@@ -108,7 +105,7 @@ template <uint32_t TYPE> struct DqBlock;
 template <bool Q5> struct DqBlockK {
     uint4 q[2];          // the k-block's 32 quant bytes
     uint4 hb[Q5 ? 2 : 1];  // Q5_K: the high-bit bytes
-    float s[2], nm[2];
+    float s[2], c[2];
     int g;
     __device__ __forceinline__ void load(uint32_t unit, int kb) {
         const uint4 hdr = dq_lds128(unit);
@@ -120,34 +117,18 @@ template <bool Q5> struct DqBlockK {
             hb[1] = dq_lds128(unit + 32);
         }
         g = 2 * kb;
-        dq_kscale(hdr, kb, s, nm);
+        dq_kscale(hdr, kb, s, c);
     }
     __device__ __forceinline__ uint32_t mix() const {
-        uint32_t m = q[0].x ^ q[0].y ^ q[0].z ^ q[0].w ^ q[1].x ^ q[1].y ^ q[1].z ^ q[1].w ^ __float_as_uint(nm[0]);
+        uint32_t m = q[0].x ^ q[0].y ^ q[0].z ^ q[0].w ^ q[1].x ^ q[1].y ^ q[1].z ^ q[1].w ^ __float_as_uint(c[0]);
         if constexpr (Q5) m ^= hb[0].x ^ hb[0].y ^ hb[0].z ^ hb[0].w ^ hb[1].x ^ hb[1].y ^ hb[1].z ^ hb[1].w;
         return m;
     }
-    // warp-uniform: c = -128 s - m is exact in all lanes.  Either term comes back from it: an error would be a multiple of the smaller
-    // last bit of 128 s and m, at least 2^7 ulp of that term (17 significant bits of 24), which therefore would not come back.
-    __device__ __forceinline__ bool folds() const {
-        bool exact = true;
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-            const float s128 = 128.0f * s[n], c = __fsub_rn(nm[n], s128);
-            exact &= __fadd_rn(c, s128) == nm[n] && __fsub_rn(nm[n], c) == s128;
-        }
-        return __all_sync(0xffffffffu, exact);
-    }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw, bool folded) const {
-        const float c[2] = {fmaf(-128.0f, s[0], nm[0]), fmaf(-128.0f, s[1], nm[1])};
-        if (folded) emit_as<true>(row_base, sw, c);
-        else emit_as<false>(row_base, sw, nm);
-    }
-    template <bool BIASED> __device__ __forceinline__ void emit_as(uint32_t row_base, int sw, const float (&off)[2]) const {
+    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
         const uint32_t w[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
 #pragma unroll
         for (int n = 0; n < 2; ++n) {  // low nibbles: group 2 kb, high nibbles: group 2 kb + 1
-            const uint64_t s2 = dq_pair(s[n]), c2 = dq_pair(off[n]);
+            const uint64_t s2 = dq_pair(s[n]), c2 = dq_pair(c[n]);
 #pragma unroll
             for (int c8 = 0; c8 < 4; ++c8) {
                 uint32_t m[2];
@@ -160,7 +141,7 @@ template <bool Q5> struct DqBlockK {
                         m[i] |= ((hw >> (g + n)) << 4) & 0x10101010u;
                     }
                 }
-                dq_store(row_base, sw, 4 * n + c8, dq_chunk_fma<BIASED>(m[0], m[1], s2, c2));
+                dq_store(row_base, sw, 4 * n + c8, dq_chunk_fma<false>(m[0], m[1], s2, c2));
             }
         }
     }
@@ -185,8 +166,7 @@ template <> struct DqBlock<ZQ_Q6_K> {
     __device__ __forceinline__ uint32_t mix() const {
         return lo[0].x ^ lo[0].y ^ lo[1].x ^ lo[1].y ^ lo[2].x ^ lo[2].y ^ lo[3].x ^ lo[3].y ^ hi[0] ^ hi[1] ^ hi[2] ^ hi[3] ^ sc ^ __float_as_uint(d);
     }
-    __device__ __forceinline__ bool folds() const { return true; }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw, bool) const {
+    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
 #pragma unroll
         for (int c8 = 0; c8 < 8; ++c8) {  // eight columns: block G = 2 kb + c8 / 4, scale group h = (c8 / 2) & 1, t = 2 (c8 & 1) and t + 1
             const int gb = c8 >> 2, hh = (c8 >> 1) & 1, x2 = 2 * (2 * gb + hh);
@@ -215,8 +195,7 @@ template <bool NL> struct DqBlock4 {
         for (int t = 0; t < 4; ++t) p[t] = dq_lds64(unit + 16 + 16 * (t + 4 * (kb >> 1)) + 8 * (kb & 1));
     }
     __device__ __forceinline__ uint32_t mix() const { return p[0].x ^ p[0].y ^ p[1].x ^ p[1].y ^ p[2].x ^ p[2].y ^ p[3].x ^ p[3].y ^ d; }
-    __device__ __forceinline__ bool folds() const { return true; }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw, bool) const {
+    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const uint32_t d2 = dq_prmt(d, 0u, b ? 0x3232u : 0x1010u);
@@ -263,8 +242,7 @@ template <> struct DqBlock<ZQ_Q8_0> {  // piece t of a k-block: words t (columns
         for (int t = 0; t < 4; ++t) m ^= p[t].x ^ p[t].y ^ p[t].z ^ p[t].w;
         return m;
     }
-    __device__ __forceinline__ bool folds() const { return true; }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw, bool) const {
+    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const uint32_t d2 = dq_prmt(d, 0u, b ? 0x3232u : 0x1010u);
