@@ -177,8 +177,8 @@ def test_operand_is_the_dequantised_value_rounded_once(tensor_type):
     rng = np.random.default_rng(18)
     exponent = rng.integers(-14, -4, size=len(data))
     scales = [np.ldexp(1.0 + rng.random(len(data)), exponent).astype(np.float16)]
-    if len(H.SCALE_OFFSETS[tensor_type]) == 2:  # minimum: 2^-9 .. 2^4 times the scale
-        scales.append(np.ldexp(1.0 + rng.random(len(data)), exponent + rng.integers(-9, 5, size=len(data))).astype(np.float16))
+    if len(H.SCALE_OFFSETS[tensor_type]) == 2:  # minimum: 2^-9 .. 2^15 times the scale, as far as f16 goes
+        scales.append(np.ldexp(1.0 + rng.random(len(data)), np.minimum(exponent + rng.integers(-9, 16, size=len(data)), 8)).astype(np.float16))
     for off, v in zip(H.SCALE_OFFSETS[tensor_type], scales):
         data[:, off:off + 2] = v.view(np.uint8).reshape(-1, 2)
     data = data.reshape(-1)
