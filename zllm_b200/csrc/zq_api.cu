@@ -68,6 +68,15 @@ int ensure_xq(zq_ctx *ctx, size_t bytes, zq_error *err) {
     return ZQ_OK;
 }
 
+int LaunchScratch::take(zq_ctx *ctx, size_t bytes, zq_error *err) {
+    stream = ctx->stream;
+    ZQ_CUDA_CHECK(cudaMallocFromPoolAsync(&p, bytes, ctx->scratch_pool, stream), err);
+    return ZQ_OK;
+}
+LaunchScratch::~LaunchScratch() {
+    if (p) cudaFreeAsync(p, stream);
+}
+
 int ensure_scratch_mid(zq_ctx *ctx, size_t bytes, zq_error *err) {
     if (bytes <= ctx->mid_bytes) return ZQ_OK;
     ZQ_CUDA_CHECK(cudaStreamSynchronize(ctx->stream), err);
@@ -154,6 +163,15 @@ static int ctx_allocate(zq_ctx *ctx, zq_error *err) {
     ctx->stream = ctx->own_stream;
     ctx->gemv_partials_floats = (size_t)ctx->sm_count * 2 * 128 * 16;  // two partial-tile slots (128 rows x 16 activation rows) per CTA
     ZQ_CUDA_CHECK(cudaMalloc(&ctx->gemv_partials, ctx->gemv_partials_floats * sizeof(float)), err);
+    cudaMemPoolProps pool = {};
+    pool.allocType = cudaMemAllocationTypePinned;
+    pool.location.type = cudaMemLocationTypeDevice;
+    pool.location.id = ctx->device;
+    ZQ_CUDA_CHECK(cudaMemPoolCreate(&ctx->scratch_pool, &pool), err);
+    uint64_t kept = kScratchKept;
+    int no = 0;  // streams of one context do not wait for each other over a piece of scratch
+    ZQ_CUDA_CHECK(cudaMemPoolSetAttribute(ctx->scratch_pool, cudaMemPoolAttrReleaseThreshold, &kept), err);
+    ZQ_CUDA_CHECK(cudaMemPoolSetAttribute(ctx->scratch_pool, cudaMemPoolReuseAllowInternalDependencies, &no), err);
     // a first MB of activation records (4 rows of 116 000 columns): a gated decode call of up to 4 rows allocates nothing, also when
     // it is the first call of a context and is being captured
     int rc_xq = ensure_xq(ctx, size_t(1) << 20, err);
@@ -200,6 +218,7 @@ void zq_ctx_destroy(zq_ctx *ctx) {
     if (ctx->own_stream || ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->gemv_partials) cudaFree(ctx->gemv_partials);
     if (ctx->gemv_counters) cudaFree(ctx->gemv_counters);
+    if (ctx->scratch_pool) cudaMemPoolDestroy(ctx->scratch_pool);
     if (ctx->workspace) cudaFree(ctx->workspace);
     if (ctx->mid) cudaFree(ctx->mid);
     if (ctx->norm) cudaFree(ctx->norm);

@@ -250,6 +250,9 @@ struct zq_ctx {
     uint32_t *gemv_counters = nullptr;
     size_t gemv_partials_floats = 0;
     size_t gemv_counters_n = 0;
+    // Scratch of single launches (zq::LaunchScratch).  Up to kScratchKept bytes stay with the pool over a synchronisation; the pool
+    // goes with the context.
+    cudaMemPool_t scratch_pool = nullptr;
     // General workspace (grows on demand, never shrinks): dequantised operands of the prefill GEMM, MoE buffers.
     void *workspace = nullptr;
     size_t workspace_bytes = 0;
@@ -332,9 +335,22 @@ namespace zq {
 int use_device(zq_ctx *ctx, zq_error *err);
 int ensure_workspace(zq_ctx *ctx, size_t bytes, zq_error *err);
 int ensure_xq(zq_ctx *ctx, size_t bytes, zq_error *err);
+// Device memory of one launch, taken and given back in stream order.  For calls that must not depend on memory that other
+// calls use or replace: a captured graph owns its own (an allocation node), two streams of one context never share it, and a first
+// call may be captured.  Contents are undefined.
+constexpr size_t kScratchKept = size_t(256) << 20;
+struct LaunchScratch {
+    void *p = nullptr;
+    cudaStream_t stream = nullptr;
+    int take(zq_ctx *ctx, size_t bytes, zq_error *err);
+    LaunchScratch() = default;
+    LaunchScratch(const LaunchScratch &) = delete;
+    LaunchScratch &operator=(const LaunchScratch &) = delete;
+    ~LaunchScratch();
+};
 int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, zq_error *err);
 int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const __half *x, size_t m, void *y, int y_dtype, zq_error *err);
-int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err);
+int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err, uint32_t *zero = nullptr, int n_zero = 0);
 int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t mats, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, void *y, int y_dtype, zq_error *err);
 int ensure_scratch_mid(zq_ctx *ctx, size_t bytes, zq_error *err);
 int ensure_scratch_norm(zq_ctx *ctx, size_t bytes, zq_error *err);

@@ -50,7 +50,7 @@ struct GemmParams {
     int box_tok; // token rows of one activation box (half a tile)
     int cut_tiles, cut_pairs;  // the first cut_tiles tiles are cut along K into cut_pairs equal shares
     float *partials;           // [2 * pairs][2 SMs][256 columns][128 rows] f32
-    uint32_t *counters;        // arrivals per (pair that begins a cut tile, SM), zero between launches
+    uint32_t *counters;        // arrivals per (pair that begins a cut tile, SM), zero at the start of the launch
     // Grouped form (MoE prefill): the work list replaces the tile grid.  Item = {weight matrix z, first output row of the tile,
     // first token row, end of the tile's token rows}; tokens are rows of one activation operand shared by all matrices,
     // outputs are rows of y with n_out columns.
@@ -510,7 +510,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                         }
                         store16(c0, v);
                     }
-                    if (et == 0) *counter = 0;  // ready for the next launch
                 }
             }
             tc_fence_before();
@@ -595,10 +594,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     if (warp == 1) tmem_dealloc2(tmem_base, 512);
 }
 
-// activations of any supported dtype -> f16; eight values per thread and step (one 16- or 32-byte load, one 16-byte store)
-__global__ void __launch_bounds__(256) to_f16_kernel(const void *__restrict__ x, int x_dtype, __half *__restrict__ out, size_t n8) {
+// activations of any supported dtype -> f16; eight values per thread and step (one 16- or 32-byte load, one 16-byte store);
+// `zero`: arrival counters of the GEMM behind it
+__global__ void __launch_bounds__(256) to_f16_kernel(const void *__restrict__ x, int x_dtype, __half *__restrict__ out, size_t n8, uint32_t *__restrict__ zero, int n_zero) {
     pdl_launch_dependents();
     pdl_wait_prior_grid();
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < n_zero; i += 256) zero[i] = 0;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
         uint32_t h[4];
         if (x_dtype == ZQ_F32) {
@@ -641,7 +643,8 @@ static int make_f16_map3(const void *base, size_t mats, size_t rows, size_t cols
     return ZQ_OK;
 }
 
-int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err) {
+// n = 0: only the counters
+int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err, uint32_t *zero, int n_zero) {
     const size_t n8 = n / 8;  // rows are multiples of 8 columns wherever this runs
     size_t blocks = (n8 + 255) / 256;
     if (blocks > (size_t)ctx->sm_count * 16) blocks = (size_t)ctx->sm_count * 16;
@@ -655,7 +658,7 @@ int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->disable_pdl ? 0 : 1;
-    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, to_f16_kernel, x, x_dtype, out, n8), err);
+    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, to_f16_kernel, x, x_dtype, out, n8, zero, n_zero), err);
     ctx->launches++;
     return ZQ_OK;
 }
@@ -700,7 +703,6 @@ static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &
 static void clear_params(zq_ctx *ctx, GemmParams &p) {
     memset(&p, 0, sizeof(p));
     p.status = ctx->status_dev;
-    p.counters = ctx->gemv_counters;
 }
 
 // Token tiles of a dense GEMM: as few as 256-token tiles allow, of equal size (300 tokens are two tiles of 160, not 256 + 44).
@@ -728,7 +730,19 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, GemmParams &p) {
     if (p.cut_tiles < tiles) p.cut_pairs = pairs;
     return p.cut_pairs;
 }
-static size_t partial_bytes(const GemmParams &p) { return p.cut_tiles ? (size_t)p.cut_pairs * 2 * 2 * kBN * kBM * sizeof(float) : 0; }
+// Shares and their counters are scratch of the launch and not context memory: the short prefill of f16 rows needs no other, so that
+// it may be captured first, replayed after any later call and run on two streams at once, and no call needs a larger workspace
+// than a longer one before it.  A launch that gave up on a wait leaves no counter behind for the next.  Taking it from the pool costs
+// nothing that can be measured (48 tokens of 5120 x 17408 up and down: 66.8 us, in the context's workspace 66.8 to 67.0).
+static int take_shares(zq_ctx *ctx, GemmParams &p, LaunchScratch &scratch, zq_error *err) {
+    if (!p.cut_tiles) return ZQ_OK;
+    const size_t head = ((size_t)2 * p.cut_pairs * sizeof(uint32_t) + 1023) & ~size_t(1023);
+    const int rc = scratch.take(ctx, head + (size_t)p.cut_pairs * 2 * 2 * kBN * kBM * sizeof(float), err);
+    if (rc) return rc;
+    p.counters = reinterpret_cast<uint32_t *>(scratch.p);
+    p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(scratch.p) + head);
+    return ZQ_OK;
+}
 
 // y[m, n] = x[m, k] W^T (+ residual), or silu(x gate^T) * (x up^T) when w_up is given.
 int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const void *x, int x_dtype, size_t m, void *y, int y_dtype, const void *residual, zq_error *err) {
@@ -750,25 +764,28 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     const size_t tiles = ((n + rows_per_tile - 1) / rows_per_tile) * ((m + p.bn - 1) / p.bn);
     if (tiles > (size_t)INT32_MAX / 4) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM: %zu rows x %zu tokens are too many for one call", n, m);
     const int pairs = plan_cut(ctx, (int)tiles, (int)((k + kStepK - 1) / kStepK), p);
-    const size_t part = (partial_bytes(p) + 1023) & ~size_t(1023);
     const size_t w_bytes = fused ? 0 : (n * k * 2 + 1023) & ~size_t(1023);
     const size_t x_bytes = x_dtype == ZQ_F16 ? 0 : (m * k * 2 + 1023) & ~size_t(1023);
-    int rc = ensure_workspace(ctx, part + (gated ? 2 : 1) * w_bytes + x_bytes, err);
+    int rc = ensure_workspace(ctx, (gated ? 2 : 1) * w_bytes + x_bytes, err);
+    if (rc) return rc;
+    LaunchScratch scratch;
+    rc = take_shares(ctx, p, scratch, err);
     if (rc) return rc;
     uint8_t *ws = reinterpret_cast<uint8_t *>(ctx->workspace);
-    p.partials = reinterpret_cast<float *>(ws);
     const __half *xin = reinterpret_cast<const __half *>(x);
     if (x_dtype != ZQ_F16) {
-        __half *x16 = reinterpret_cast<__half *>(ws + part + (gated ? 2 : 1) * w_bytes);
-        rc = launch_to_f16(ctx, x, x_dtype, x16, m * k, err);
-        if (rc) return rc;
+        __half *x16 = reinterpret_cast<__half *>(ws + (gated ? 2 : 1) * w_bytes);
+        rc = launch_to_f16(ctx, x, x_dtype, x16, m * k, err, p.counters, p.counters ? 2 * p.cut_pairs : 0);
         xin = x16;
+    } else if (p.counters) {
+        rc = launch_to_f16(ctx, nullptr, ZQ_F16, nullptr, 0, err, p.counters, 2 * p.cut_pairs);
     }
+    if (rc) return rc;
     CUtensorMap map_x;
     rc = make_f16_map(xin, m, k, p.box_tok, &map_x, err);
     if (rc) return rc;
     if (fused) return launch_src(ctx, w->type, gated, gated ? w->unit_map_half : w->qmv_map, gated ? w_up->unit_map_half : w->qmv_map, map_x, p, pairs, err);
-    __half *w16 = reinterpret_cast<__half *>(ws + part), *w16b = reinterpret_cast<__half *>(ws + part + w_bytes);
+    __half *w16 = reinterpret_cast<__half *>(ws), *w16b = reinterpret_cast<__half *>(ws + w_bytes);
     rc = launch_dequantize_f16(ctx, w, w16, err);
     if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
     if (rc) return rc;
