@@ -80,6 +80,35 @@ def test_missing_peer_runs_into_the_wait_limit_and_the_context_survives():
     c.close()
 
 
+@pytest.mark.parametrize("rows,cols,m", [(512, 4096, 48), (20480, 512, 17)])  # tiles cut along K; whole tiles
+def test_prefill_behind_a_reduce_that_waits_for_a_peer(rows, cols, m):
+    """The prefill kernel is set up, loads and unpacks its first weights under the reduce before it; its own bounded waits start when
+    the reduce is over, however long that waited (here a second, for a peer that never comes)."""
+    from zllm_b200 import ffi
+    from zllm_b200.backend import B200Context
+
+    c = B200Context(0)
+    blob = (C.c_uint8 * ffi.DIST_HANDLE_BYTES)()
+    ffi.call("zq_dist_export", c.handle, 1 << 20, blob)
+    both = (C.c_uint8 * (2 * ffi.DIST_HANDLE_BYTES))(*(list(blob) * 2))
+    ffi.call("zq_dist_init", c.handle, 0, 2, both)
+    ffi.call("zq_dist_set_wait_ms", c.handle, 1000)
+    small = c.prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 256, 512, seed=3), 256, 512)
+    w = c.prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, rows, cols, seed=5), rows, cols)
+    x = torch.randn((m, cols), device="cuda", dtype=torch.float16)
+    want = c.linear(x, w)
+    c.sync()
+    c.linear_row_parallel(torch.randn((1, 512), device="cuda"), small)
+    y = c.linear(x, w)
+    with pytest.raises(ffi.ZqFailure) as info:
+        c.sync()
+    assert info.value.code == 5 and "peer" in info.value.message
+    assert torch.equal(y, want)
+    small.release()
+    w.release()
+    c.close()
+
+
 EP = dict(experts=16, top_k=4, hidden=512, inter=256)
 
 

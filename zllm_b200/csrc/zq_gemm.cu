@@ -312,6 +312,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     // Programmatic dependent launch: everything up to here, and for packed dense weights (constants) also their first boxes and
     // their dequantisation, runs under the previous kernel's end; activations, f16 operands, work lists, results and partials
     // belong to earlier kernels until they complete.  5120 x 17408 up and down in Q4_K: 48 tokens 76 -> 65 us, 512 tokens 192 -> 188 us.
+    // The warps that run ahead (6 and up) take the same wait once their ring has gone round, that is before the first wait for
+    // something that only the MMAs set free: the previous kernel may itself wait for another rank, for longer than a bounded wait here.
     if (SRC == 0 || p.items || warp < 6) pdl_wait_prior_grid();
     GemmWalk walk(p, pair, pairs, kRows);
     GemmSeg sg;
@@ -541,6 +543,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     if (++ps == PST) {
                         ps = 0;
                         pph ^= 1u;
+                        if (fresh) pdl_wait_prior_grid();
                         fresh = false;
                     }
                 }
@@ -559,6 +562,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 if (s >= STAGES) {
                     s -= STAGES;
                     ph ^= 1u;
+                    if (fresh) pdl_wait_prior_grid();
                     fresh = false;
                 }
             };
