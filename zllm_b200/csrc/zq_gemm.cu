@@ -25,8 +25,8 @@
 //
 // Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..5
 // epilogue; SRC != 0: warp 6 TMA of packed boxes, warps 7..22 dequantisers.
-// Every wait is bounded; a wait that runs out raises the CTA's abort flag, all roles fall through to the end, TMEM is
-// released and the context status word reports it.
+// Every wait is bounded, counted from the end of the previous kernel; a wait that runs out sets the CTA's state, all roles fall
+// through to the end, TMEM is released and the context status word reports it.
 #include "zq_gemm_dq.cuh"
 
 namespace zq {
@@ -144,17 +144,22 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
     return r != 0;
 }
+// State of a CTA, read by every poll that fails: set up under the previous kernel, whose end it waits for (polls do not count yet);
+// running; a bounded wait has run out.  A poll counts only while the previous kernel is over: the warps that run ahead of its
+// end would otherwise give up because of it.  (Having them wait for its end themselves cost 3 of 65 us at 48 tokens.)
+enum : uint32_t { kStateRun = 0, kStateAbort = 1, kStateAhead = 2 };
 // `sleep_ns` > 0: roles that share a scheduler with working warps back off between polls (a bare poll loop re-issues
 // every few tens of nanoseconds).
-__device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t abort_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
-    for (uint32_t i = 0; i < (1u << 23); ++i) {
+__device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t state_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
+    for (uint32_t i = 0; i < (1u << 23);) {
         if (mbar_try_wait(bar, parity)) return true;
-        uint32_t gone;
-        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(gone) : "r"(abort_addr));
-        if (gone) return false;
+        uint32_t state;
+        asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(state) : "r"(state_addr));
+        if (state == kStateAbort) return false;
+        if (state == kStateRun) ++i;
         if (sleep_ns) __nanosleep(sleep_ns);
     }
-    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_addr), "r"(1u));
+    asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(state_addr), "r"((uint32_t)kStateAbort));
     atomicMax(status, code);
     return false;
 }
@@ -269,7 +274,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     uint64_t *acc_full = p_empty + PST;                                // each SM
     uint64_t *acc_empty = acc_full + 2;                                // first SM: both SMs' epilogue warps
     __shared__ uint32_t s_tmem;
-    __shared__ int s_abort, s_last;
+    __shared__ uint32_t s_state;
+    __shared__ int s_last;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the shuffle tells the compiler that it is uniform
     const uint32_t rank = pair_rank();
@@ -293,7 +299,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             mbar_init(&acc_empty[b], 8);
         }
         fence_mbar_init();
-        s_abort = 0;
+        s_state = kStateAhead;
         tma_prefetch_desc(&map_w);
         tma_prefetch_desc(&map_x);
         if (GATED) tma_prefetch_desc(&map_w2);
@@ -308,13 +314,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     pair_sync();  // both SMs' barriers and tensor memory exist
     tc_fence_after();
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(&s_tmem);
-    const uint32_t abort_addr = smem_u32(&s_abort);
+    const uint32_t state_addr = smem_u32(&s_state);
     // Programmatic dependent launch: everything up to here, and for packed dense weights (constants) also their first boxes and
     // their dequantisation, runs under the previous kernel's end; activations, f16 operands, work lists, results and partials
     // belong to earlier kernels until they complete.  5120 x 17408 up and down in Q4_K: 48 tokens 76 -> 65 us, 512 tokens 192 -> 188 us.
-    // The warps that run ahead (6 and up) take the same wait once their ring has gone round, that is before the first wait for
-    // something that only the MMAs set free: the previous kernel may itself wait for another rank, for longer than a bounded wait here.
+    // The warps that run ahead (6 and up) wait for stages that only the MMAs set free, but these waits count from the end of the
+    // previous kernel (kStateAhead), which may itself wait for another rank for longer than any bound here.
     if (SRC == 0 || p.items || warp < 6) pdl_wait_prior_grid();
+    if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(&s_state) = kStateRun;  // nobody gives up before this
+    __syncwarp();
     GemmWalk walk(p, pair, pairs, kRows);
     GemmSeg sg;
 
@@ -329,7 +337,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
             const int kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
             for (int kb = sg.k0 * 4; kb < kb1; ++kb) {
-                if (!fresh && !wait_flag(&empty[s], ph ^ 1u, abort_addr, p.status, kStatusMmaTimeout)) {
+                if (!fresh && !wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout)) {
                     ok = false;
                     break;
                 }
@@ -367,13 +375,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 // f32 accumulator, f16 A and B, both K-major, M = 256, N = the tile's tokens
                 const uint32_t idesc = (1u << 4) | ((uint32_t)(tile_cols(sg) >> 3) << 17) | ((uint32_t)(kPairM >> 4) << 24);
                 const int b = iter & 1;
-                if (iter >= 2) ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, abort_addr, p.status, kStatusMmaTimeout);
+                if (iter >= 2) ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)b * kBN;
                 const int kb0 = sg.k0 * 4, kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    ok = wait_flag(&full[s], ph, abort_addr, p.status, kStatusTmaTimeout);
+                    ok = wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one()) {
@@ -411,7 +419,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 }
             }
             // the four warps go on together or not at all: they meet at barriers below (and the exchange buffer is free again)
-            const bool ok = epilogue_all(wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, abort_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0));
+            const bool ok = epilogue_all(wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0));
             tc_fence_after();
             const uint32_t acc = tmem_base + (uint32_t)b * kBN + ((uint32_t)(q * 32) << 16);
             const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
@@ -529,7 +537,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 const CUtensorMap *mw2 = p.items ? (GATED ? &p.w2_maps[sg.z] : mw) : &map_w2;
                 const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
                 for (int u = sg.k0; u < sg.k1; ++u) {
-                    if (!fresh && !wait_flag(&p_empty[ps], pph ^ 1u, abort_addr, p.status, kStatusMmaTimeout, 50)) {
+                    if (!fresh && !wait_flag(&p_empty[ps], pph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 50)) {
                         ok = false;
                         break;
                     }
@@ -543,7 +551,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     if (++ps == PST) {
                         ps = 0;
                         pph ^= 1u;
-                        if (fresh) pdl_wait_prior_grid();
                         fresh = false;
                     }
                 }
@@ -562,13 +569,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 if (s >= STAGES) {
                     s -= STAGES;
                     ph ^= 1u;
-                    if (fresh) pdl_wait_prior_grid();
                     fresh = false;
                 }
             };
             while (ok && walk.next(p, sg)) {
                 for (int u = sg.k0; u < sg.k1; ++u) {
-                    ok = wait_flag(&p_full[ps], pph, abort_addr, p.status, kStatusTmaTimeout, 20);
+                    ok = wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
                     if (!ok) break;
                     dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
                     // Everything the warp needs of the box is in registers once this vote has read them.  Without it the arrival
@@ -580,7 +586,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                         pph ^= 1u;
                     }
                     advance(mine);
-                    if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, abort_addr, p.status, kStatusMmaTimeout, 20);
+                    if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
                     if (!ok) break;
                     dq.emit(row0 + (uint32_t)(s * S::stage_bytes), sw);
                     fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores of the pair
