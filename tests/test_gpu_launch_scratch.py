@@ -1,5 +1,6 @@
-"""Short prefill of f16 rows in capture, replay and on two streams: the shares of cut tiles are scratch of the launch, so that such a call
-depends on no memory of the context that another call uses or replaces.  Results are compared bit for bit with plain calls."""
+"""Calls that use no memory of the context, in capture, replay and on two streams: short prefill of f16 rows (the shares of cut tiles are
+scratch of the launch) and gated decode pairs of up to 4 rows, on whichever kernel they run.  Results are compared bit for bit with
+plain calls."""
 import numpy as np
 import pytest
 import torch
@@ -9,8 +10,9 @@ from tests.gpu_util import ctx
 
 pytestmark = pytest.mark.gpu
 
-# rows, columns, tokens, gated: every tile cut; some cut and some whole; a gated pair of few tiles
-CALLS = [(300, 4096, 48, False), (43520, 512, 40, False), (200, 2048, 33, True)]
+# rows, columns, tokens, gated: every tile cut; some cut and some whole; a gated pair of few tiles; decode pairs dealt out by the
+# work-list kernel (tiles that fill half the machine)
+CALLS = [(300, 4096, 48, False), (43520, 512, 40, False), (200, 2048, 33, True), (4801, 7424, 1, True), (4801, 7424, 4, True)]
 
 
 def _setup(c, rows, cols, m, gated, seed=200):
@@ -34,7 +36,7 @@ def _bits(t):
 
 
 @pytest.mark.parametrize("rows,cols,m,gated", CALLS)
-def test_first_short_prefill_of_a_context_can_be_captured(rows, cols, m, gated):
+def test_first_call_of_a_context_can_be_captured_and_replayed_after_any_other(rows, cols, m, gated):
     c, stream = _fresh(), torch.cuda.Stream()
     w, x = _setup(c, rows, cols, m, gated)
     torch.cuda.synchronize()
@@ -51,6 +53,7 @@ def test_first_short_prefill_of_a_context_can_be_captured(rows, cols, m, gated):
     wide = c.prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 512, 8192, seed=9), 512, 8192)
     for rows_in in (16, 600, 3000):
         c.linear(torch.zeros((rows_in, 8192), device="cuda"), wide)
+    c.linear_batch([(torch.zeros((16, 8192), device="cuda"), wide) for _ in range(8)])  # 8 inputs: more than the first MB of records
     y.zero_()
     for _ in range(3):
         graph.replay()
@@ -59,9 +62,10 @@ def test_first_short_prefill_of_a_context_can_be_captured(rows, cols, m, gated):
     assert np.array_equal(_bits(y), want)
 
 
-def test_short_prefill_on_two_streams_of_one_context():
+@pytest.mark.parametrize("calls", [CALLS[:2], CALLS[3:]])
+def test_two_streams_of_one_context(calls):
     c = _fresh()
-    jobs = [_setup(c, *call, seed=210 + 4 * i) for i, call in enumerate(CALLS[:2])]
+    jobs = [_setup(c, *call, seed=210 + 4 * i) for i, call in enumerate(calls)]
     streams = [torch.cuda.Stream() for _ in jobs]
     torch.cuda.synchronize()
     c.set_stream(torch.cuda.current_stream().cuda_stream)

@@ -50,7 +50,7 @@ struct WlArgs {
     int chunk_words;   // 32-bit words per chunk of a weight row
     int y_dtype;
     float *partials;   // [2 * grid][kSlotFloats]: slot 2c + 1 = the tile CTA c begins, slot 2c = the tile it continues
-    uint32_t *counters;  // [grid], zero between launches: arrivals at the cut tile that CTA c begins
+    uint32_t *counters;  // [grid], zero at the start of the launch: arrivals at the cut tile that CTA c begins
     uint32_t *status;
 };
 
@@ -63,6 +63,8 @@ struct WlQuantArgs {
     WlQuantSrc src[kWlMaxJobs];
     int n_src, total, x_dtype;
     uint8_t *out;
+    uint32_t *zero;  // arrival counters to set to zero for the launch behind this one, or null
+    int n_zero;
 };
 
 // Records of every distinct activation block of the list: one warp per (block, unit, row).
@@ -70,6 +72,8 @@ template <uint32_t TYPE>
 __global__ void __launch_bounds__(256) wl_quantize_kernel(const __grid_constant__ WlQuantArgs qa) {
     pdl_launch_dependents();
     pdl_wait_prior_grid();  // the record buffer may still be read by the previous launch
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < qa.n_zero; i += 256) qa.zero[i] = 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rec = blockIdx.x * 8 + warp;
     if (rec >= qa.total) return;  // warp-uniform
@@ -567,9 +571,7 @@ bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &j) {
 // list: 5120 -> 10240 (20 items on the busiest SM against 11) Q4_K 22.4 -> 18.3 us, IQ4_NL 30.7 -> 23.1, Q8_0 29.0 -> 25.8 (at 8
 // rows 27.2 -> 23.0, 36.0 -> 27.8, 34.3 -> 29.4); 4096 -> 11008 (16 against 10, the smallest difference that passes in a 4-bit
 // type) 18.2 -> 16.2, 25.4 -> 20.7; on the other side 3840 -> 15360 (16 against 13) Q4_K 18.8 and 18.9, Q8_0 25.1 and 27.0.
-// Up to 4 rows gemv_i8_kernel needs no workspace, so the list is only taken there when the record buffer holds its records as it is.
-bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) {
-    if (m <= 4 && m * gate->units_per_row * kRec > ctx->xq_bytes) return false;
+bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate) {
     const size_t sms = (size_t)ctx->sm_count, tiles = (gate->rows + kTileRows / 2 - 1) / (kTileRows / 2), chunks = (gate->units_per_row + kChunkUnits - 1) / kChunkUnits;
     size_t split = tiles ? sms / tiles : 1;
     if (split > 8) split = 8;
@@ -581,8 +583,12 @@ bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) 
 
 // Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one record
 // pass per record format, then one decode launch per (weight type, column-tile count, plain / gated) class.
-int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm) {
+// `own_scratch` (one job): records, partial tiles and counters are scratch of the call instead of context memory.  gemv_i8_kernel, the
+// other route of a gated pair, uses no context memory up to 4 rows: such a call may be replayed from a graph after any later call
+// and run on two streams of a context at once, on either route.
+int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm, bool own_scratch) {
     if (n_jobs == 0) return ZQ_OK;
+    if (own_scratch && (n_jobs != 1 || norm)) return set_error(err, ZQ_ERR_ARG, "decode work list: scratch of its own is for one job");
     // ---- records: one block per distinct (x, m, cols, record format)
     struct Src { const void *x; size_t m, cols; bool q4k; size_t rec_begin, units; };
     std::vector<Src> srcs;
@@ -601,9 +607,22 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
         src_of[i] = s;
     }
     if (total_rec > (size_t)INT32_MAX / kRec) return set_error(err, ZQ_ERR_SHAPE, "decode work list: %zu activation records are too many for one call", total_rec);
-    int rc = ensure_xq(ctx, total_rec * kRec, err);
-    if (rc) return rc;
-    uint8_t *xq = reinterpret_cast<uint8_t *>(ctx->xq);
+    LaunchScratch scratch;
+    uint8_t *xq = nullptr;
+    float *partials = ctx->gemv_partials;
+    uint32_t *counters = ctx->gemv_counters;
+    int rc;
+    if (own_scratch) {
+        const size_t head = ((size_t)ctx->sm_count * sizeof(uint32_t) + 1023) & ~size_t(1023), slots = (size_t)2 * ctx->sm_count * kSlotFloats * sizeof(float);
+        if ((rc = scratch.take(ctx, head + slots + total_rec * kRec, err))) return rc;
+        uint8_t *at = reinterpret_cast<uint8_t *>(scratch.p);
+        counters = reinterpret_cast<uint32_t *>(at);
+        partials = reinterpret_cast<float *>(at + head);
+        xq = at + head + slots;
+    } else {
+        if ((rc = ensure_xq(ctx, total_rec * kRec, err))) return rc;
+        xq = reinterpret_cast<uint8_t *>(ctx->xq);
+    }
     if (norm) {  // one input, at most one source per format: the norm kernel writes the records
         uint8_t *rec[2] = {nullptr, nullptr};
         for (const Src &s : srcs) rec[s.q4k ? 0 : 1] = xq + s.rec_begin * kRec;
@@ -613,6 +632,8 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
         WlQuantArgs qa;
         qa.x_dtype = x_dtype;
         qa.n_src = 0;
+        qa.zero = own_scratch ? counters : nullptr;
+        qa.n_zero = own_scratch ? ctx->sm_count : 0;
         auto flush = [&]() -> int {
             if (qa.n_src == 0) return ZQ_OK;
             // records of one launch are contiguous: the kernel's record index starts at the first block's
@@ -647,8 +668,8 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
         wa.q_total = 0;
         wa.chunk_words = kChunkUnits * format_info(type).unit_bytes / 4;
         wa.y_dtype = y_dtype;
-        wa.partials = ctx->gemv_partials;
-        wa.counters = ctx->gemv_counters;
+        wa.partials = partials;
+        wa.counters = counters;
         wa.status = ctx->status_dev;
         int min_chunks = INT32_MAX;
         auto flush = [&]() -> int {

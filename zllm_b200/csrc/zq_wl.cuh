@@ -21,7 +21,7 @@ struct WlHostJob {
 // True when the job can ride in a work-list launch (Q4_K / Q4_0 / Q8_0, up to 16 activation rows).
 bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &job);
 // True when one gated pair (supported) is better dealt out by this kernel than launched on gemv_i8_kernel.
-bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m);
+bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate);
 // An RMSNorm in front of the list: every job's input is norm(x), and the jobs' own `x` is only the name of that one input.
 struct WlNorm {
     const void *x;
@@ -29,7 +29,7 @@ struct WlNorm {
     int x_dtype;
     float eps, weight_offset;
 };
-int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm = nullptr);
+int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm = nullptr, bool own_scratch = false);
 // norm(x) as activation records of the K-quant and / or block-32 format (zq_norm.cu); null: format not wanted.
 int launch_rmsnorm_records(zq_ctx *ctx, const WlNorm &norm, size_t m, size_t cols, uint8_t *rec_k, uint8_t *rec_b, zq_error *err);
 
