@@ -567,18 +567,22 @@ bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &j) {
 
 // A gated decode launch of gemv_i8_kernel walks ceil(tiles * slices / SMs) rounds of whole slices; the work-list kernel deals the
 // same ring items out evenly, for a record pass, a longer start and the hand-over of cut tiles, ~5 us together.  It is taken when
-// the busiest SM would walk at least 216 KB of weights less, those 5 us at ~43 GB/s per SM.  Measured at 1 row, gemv_i8 -> work
-// list: 5120 -> 10240 (20 items on the busiest SM against 11) Q4_K 22.4 -> 18.3 us, IQ4_NL 30.7 -> 23.1, Q8_0 29.0 -> 25.8 (at 8
-// rows 27.2 -> 23.0, 36.0 -> 27.8, 34.3 -> 29.4); 4096 -> 11008 (16 against 10, the smallest difference that passes in a 4-bit
-// type) 18.2 -> 16.2, 25.4 -> 20.7; on the other side 3840 -> 15360 (16 against 13) Q4_K 18.8 and 18.9, Q8_0 25.1 and 27.0.
-bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate) {
+// the busiest SM would walk at least 216 KB of weights less, those 5 us at ~43 GB/s per SM; with 9..16 rows of Q4_K and Q5_K, where
+// arithmetic sets the pace of both kernels and the longer hand-over is not hidden, at least 300 KB.  Measured, gemv_i8 -> work list:
+//   5120 -> 10240 (20 items on the busiest SM against 11)  1 row: Q4_K 21.5 -> 18.7 us, Q5_K 25.4 -> 21.1, IQ4_NL 30.2 -> 23.5, Q8_0 28.1 -> 25.8;
+//     8 rows: 26.4 -> 23.4, 29.5 -> 25.7, 35.5 -> 28.2, 33.9 -> 29.6;  16 rows: 36.9 -> 36.2, 40.9 -> 38.8, 45.1 -> 35.2, 42.0 -> 35.6, Q6_K 50.0 -> 40.8
+//   3840 -> 10240 (16 against 9)  16 rows: Q4_K 29.8 and 31.0 (258 KB: not taken), Q5_K 33.0 and 33.1, Q4_0 30.0 -> 26.5, IQ4_NL 36.0 -> 29.8, Q8_0 34.2 -> 29.9
+//   4096 -> 11008 (16 against 10, the smallest difference that passes in a 4-bit type)  1 row: Q4_K 17.8 -> 16.5, IQ4_NL 25.1 -> 21.0, Q8_0 23.3 -> 22.4;
+//     4 rows: 21.1 -> 20.9, 28.1 -> 24.7, 28.6 -> 28.1;  16 rows: Q4_K 31.1 and 34.1, Q5_K 34.3 and 36.6 (not taken), Q4_0 31.1 -> 29.0, IQ4_NL 37.5 -> 33.0
+//   3840 -> 15360 (16 against 13, not taken)  1 row: Q4_K 18.8 and 18.9, Q8_0 25.1 and 27.0
+bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) {
     const size_t sms = (size_t)ctx->sm_count, tiles = (gate->rows + kTileRows / 2 - 1) / (kTileRows / 2), chunks = (gate->units_per_row + kChunkUnits - 1) / kChunkUnits;
     size_t split = tiles ? sms / tiles : 1;
     if (split > 8) split = 8;
     if (split > chunks) split = chunks;
     if (split < 1) split = 1;
     const size_t single = (tiles * split + sms - 1) / sms * ((chunks + split - 1) / split), even = (tiles * chunks + sms - 1) / sms;
-    return single > even && (single - even) * kTileRows * kChunkUnits * format_info(gate->type).unit_bytes >= 216 * 1024;
+    return single > even && (single - even) * kTileRows * kChunkUnits * format_info(gate->type).unit_bytes >= (m > 8 && is_kclass(gate->type) ? 300 : 216) * 1024;
 }
 
 // Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one record

@@ -21,7 +21,7 @@ struct WlHostJob {
 // True when the job can ride in a work-list launch (Q4_K / Q4_0 / Q8_0, up to 16 activation rows).
 bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &job);
 // True when one gated pair (supported) is better dealt out by this kernel than launched on gemv_i8_kernel.
-bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate);
+bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m);
 // An RMSNorm in front of the list: every job's input is norm(x), and the jobs' own `x` is only the name of that one input.
 struct WlNorm {
     const void *x;
