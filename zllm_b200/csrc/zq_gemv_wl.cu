@@ -49,6 +49,7 @@ struct WlArgs {
     int q_total;       // ring items of the whole launch
     int chunk_words;   // 32-bit words per chunk of a weight row
     int y_dtype;
+    int async_fix;     // 5..8 rows: the finisher warp completes cut tiles (otherwise the consumers together)
     float *partials;   // [2 * grid][kSlotFloats]: slot 2c + 1 = the tile CTA c begins, slot 2c = the tile it continues
     uint32_t *counters;  // [grid], zero at the start of the launch: arrivals at the cut tile that CTA c begins
     uint32_t *status;
@@ -160,11 +161,10 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     uint64_t *empty = full + 8;
     __shared__ uint32_t s_abort;
     __shared__ int s_nseg, s_last, s_c0, s_cl;
-    // Up to 4 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with
-    // more that warp would need longer than the consumers themselves, so they do it together (and wait for it).  5..8 rows,
-    // one warp -> all: gated Q4_K 5120 -> 10240 at 8 rows 32.5 -> 23.1 us, at 5 rows 27.8 -> 22.7; two plain projections of that
-    // shape 25.8 -> 23.4 at 8 rows, 23.6 -> 23.1 at 5 (the worst seen: IQ4_NL 3840 -> 15360 at 5 rows, 29.6 -> 30.7).
-    constexpr bool kAsyncFix = NT < 2;
+    // Up to 4 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with 9..16
+    // that warp would need longer than the consumers themselves, so they do it together (and wait for it); with 5..8 rows the host
+    // decides by the length of the launch.
+    const bool async_fix = NT < 2 || (NT == 2 && a.async_fix);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long G = gridDim.x, Q = a.q_total;
@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
         // have stored a cut piece's partial sums, publishes them (fence + arrival count) and, if this CTA was the last
         // contributor, adds all partials in CTA order and stores the tile.
         pdl_launch_dependents();
-        if (!kAsyncFix) return;
+        if (!async_fix) return;
         pdl_wait_prior_grid();  // outputs and the fix-up scratch belong to earlier kernels until they complete
         constexpr int G4 = 4 * NT;  // float4 groups per lane: 128 rows x (4 NT) activation rows / 4 / 32 lanes
         for (int k = 0; k < 2 && k < nseg; ++k) {
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                         }
                     }
                 }
-                if constexpr (kAsyncFix) {
+                if (async_fix) {
                     named_bar_arrive(kBarFix + cut_k, kWlConsumers + 32);  // over to the finisher warp; this warp goes on
                     ++cut_k;
                 } else {
@@ -675,13 +675,19 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
         wa.partials = partials;
         wa.counters = counters;
         wa.status = ctx->status_dev;
-        int min_chunks = INT32_MAX;
+        int min_chunks = INT32_MAX, max_chunks = 0, max_m = 0;
         auto flush = [&]() -> int {
             if (wa.n_jobs == 0) return ZQ_OK;
             // pieces per CTA: at most one per tile boundary inside a range, plus the two ends
             const int grid = ctx->sm_count < wa.q_total ? ctx->sm_count : wa.q_total;
             const long long per_cta = (wa.q_total + grid - 1) / grid;
             if (per_cta / min_chunks + 3 > kWlMaxSegs) return set_error(err, ZQ_ERR_UNSUPPORTED, "decode work list: a CTA would walk more than %d tiles", kWlMaxSegs);
+            // The finisher warp needs longer for more rows, and longer for a gated tile; behind it the CTA should have that much left
+            // to stream once its cut pieces are done, i.e. its range less a tile.  In ring items, at 5 / 8 rows, consumers together -> finisher warp:
+            //   Q4_K 3840 -> 15360 (6 items of 8-item tiles)  17.7 / 17.8 -> 20.2 / 22.9 us, two of them (12)  25.8 / 26.0 -> 25.2 / 26.8
+            //   two 5120 -> 17408 (18 of 10)  32.6 / 32.8 -> 29.2 / 31.3; IQ4_NL 41.7 / 41.9 -> 38.5 / 40.2;  q, k, v, o, gate and up of 4096 (16 of 8)  33 / 31.5 -> 28.3 / 29.4
+            //   gated 5120 -> 10240 (10 of 10)  23.2 / 23.4 -> 27.6 / 32.4, two 4096 -> 11008 (18 of 8)  33.5 / 34.1 -> 32.0 / 37.4, two 4096 -> 14336 (24 of 8)  40.0 / 40.3 -> 36.0 / 38.7
+            wa.async_fix = wa.q_total / grid - max_chunks >= 2 * max_m - (gated ? 0 : 8);
             int r;
             switch (type) {
             case ZQ_Q4_K: r = launch_wl_type<ZQ_Q4_K>(ctx, wa, nt, gated, err); break;
@@ -694,6 +700,7 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
             wa.n_jobs = 0;
             wa.q_total = 0;
             min_chunks = INT32_MAX;
+            max_chunks = max_m = 0;
             return r;
         };
         for (size_t k = i; k < n_jobs; ++k) {
@@ -723,6 +730,8 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
             d.pad = 0;
             wa.q_total += (int)(tiles * chunks);
             if ((int)chunks < min_chunks) min_chunks = (int)chunks;
+            if ((int)chunks > max_chunks) max_chunks = (int)chunks;
+            if (d.m > max_m) max_m = d.m;
         }
         if ((rc = flush())) return rc;
     }
