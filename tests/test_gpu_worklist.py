@@ -218,8 +218,8 @@ def test_first_gated_call_of_a_context_can_be_captured():
 
 @pytest.mark.parametrize("pinned", [True, False])
 def test_bracket_that_sends_its_layers_out_in_several_batches(pinned):
-    """16 rows: the layers go out whenever their activations pass 1 MB, so this list is sent in parts; an input read before and after
-    a part goes out, inputs that arrive while one runs, a last layer below the limit.  Twice, with other inputs."""
+    """16 rows: the fourth input takes longer to arrive than the layers before it to run, so this list is sent in parts; an input read
+    before and after a part goes out, inputs that arrive while one runs.  Twice, with other inputs."""
     m = 16
     shapes = [(2048, 8192, 0), (1024, 16400, 1), (2048, 300, 0), (17408, 640, 2), (1024, 72, 1)]  # columns, rows, input
     weights = [(_weight(H.Q4_0, rows, cols, 180 + i), cols, rows, k) for i, (cols, rows, k) in enumerate(shapes)]
@@ -237,3 +237,56 @@ def test_bracket_that_sends_its_layers_out_in_several_batches(pinned):
         ctx().linear_host_batch([(xs[k].numpy(), w, y.numpy()) for ((_, w), _, _, k), y in zip(weights, ys)])
         for ((data, _), cols, rows, k), y in zip(weights, ys):
             _check(y.numpy(), orc.linear(H.Q4_0, data, rows, cols, xs[k].numpy()))
+
+
+@pytest.mark.parametrize("pinned", [True, False])
+def test_bracket_collects_layers_while_the_gpu_is_busy(pinned):
+    """Results of 1.1 MB each, one small input: nothing that a layer waits for, so the layers collect while those before them run; the same
+    list runs as the same launches every time, and its results do not depend on what ran before."""
+    m, rows, cols = 16, 17408, 512
+    made = [_weight(H.Q4_0, rows, cols, 300 + i) for i in range(8)]
+
+    def buf(shape):
+        t = torch.zeros(shape)
+        return t.pin_memory() if pinned else t
+
+    x = buf((m, cols))
+    x.copy_(torch.from_numpy(np.random.default_rng(301).standard_normal((m, cols)).astype(np.float32)))
+    ys = [buf((m, rows)) for _ in made]
+    counts, bits = [], []
+    for _ in range(3):
+        before = ctx().launch_count
+        ctx().linear_host_batch([(x.numpy(), w, y.numpy()) for (_, w), y in zip(made, ys)])
+        counts.append(ctx().launch_count - before)
+        bits.append([y.numpy().view(np.uint32).copy() for y in ys])
+    assert counts == [counts[0]] * 3 and counts[0] <= 8  # 16: a record pass and a launch for every layer
+    assert all(np.array_equal(a, b) for run in bits[1:] for a, b in zip(run, bits[0]))
+    for (data, _), y in zip(made, ys):
+        _check(y.numpy(), orc.linear(H.Q4_0, data, rows, cols, x.numpy()))
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0, H.Q6_K])
+@pytest.mark.parametrize("gated,m,jobs,finisher", [(False, 5, 8, True), (False, 8, 8, True), (False, 8, 5, False), (True, 5, 6, True), (True, 7, 6, True), (True, 8, 3, False)])
+def test_lists_of_5_to_8_rows_on_both_sides_of_the_finisher_rule(tensor_type, gated, m, jobs, finisher):
+    """71 (gated 141) tiles of 3 ring items per job, ranges that cut them: long lists leave cut tiles to the finisher warp, short ones to
+    the consumers.  Against the CPU path, and against the jobs run alone on the single-matrix kernel (same records, other order of the
+    f32 sums: 2 x 11 terms, the bound of the gated pair above with room)."""
+    rows, cols = 9000, 1536
+    per_cta = jobs * (3 * 141 if gated else 3 * 71) // ctx().sm_count
+    assert (per_cta - 3 >= 2 * m - (0 if gated else 8)) == finisher
+    data = [H.random_weight(tensor_type, rows, cols, seed=310 + i) for i in range(2)]
+    ws = [ctx().prepare_weight(tensor_type, d, rows, cols) for d in data]
+    xs = [dev(np.random.default_rng(320 + i).standard_normal((m, cols)).astype(np.float32)) for i in range(jobs)]
+    listed = [(x, ws[0], ws[1], "gated") if gated else (x, ws[i % 2]) for i, x in enumerate(xs)]
+    got = [host(y) for y in ctx().linear_batch(listed)]
+    ctx().set_option("disable_worklist", 1)
+    try:
+        alone = [host(y) for y in ctx().linear_batch(listed)]
+    finally:
+        ctx().set_option("disable_worklist", 0)
+    for a, b in zip(got, alone):
+        assert H.max_rel_error(a, b) <= 4e-5
+    for i in (0, jobs - 1):
+        x = xs[i].cpu().numpy()
+        want = orc.gated_linear(tensor_type, data[0], data[1], rows, cols, x) if gated else orc.linear(tensor_type, data[i % 2], rows, cols, x)
+        _check(got[i], want, tight=BOUND)

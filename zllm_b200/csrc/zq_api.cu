@@ -627,10 +627,27 @@ static void batch_abandon(zq_ctx *ctx) {
     ctx->io_out_used = false;
     ctx->pending_out.clear();
     ctx->pending_linear.clear();
-    ctx->pending_in_bytes = 0;
+    ctx->line = {};
     ctx->pending_in.clear();
     for (auto &c : ctx->io_chunks) c.used = 0;
     ctx->batch_active = false;
+}
+
+// When pending layers of a bracket go out is decided on a time line made of byte counts alone, so that the same list always runs as
+// the same launches: a call costs the host 4 us and sending layers out 10 us more, copies in travel at 45 GB/s, weights stream at
+// 4.5 TB/s and a launch costs 8 us.  Layers go out when the GPU would otherwise stand idle for a launch's cost because of a copy in that
+// they do not need, or for half as long again because the host is still recording; while the GPU is busy they collect into
+// larger launches, also where their results are long.  A limit of 1 MB of pending activations, fitted to one list, split brackets
+// whose weights outweigh their copies.  End to end in turn, 1 MB -> this rule (everything at the end): 30 projections of the decode sweep
+// at 1, 4 and 16 rows 455 -> 440 us (440); the five of Q4_0 at 1 / 4 / 8 / 16 rows 103 / 114 / 117 / 145 -> 103 / 113 / 110 / 143 (- / - / 150 / 217),
+// of Q8_0 at 16 156 -> 150 (207); eight layers of five projections (4096 wide, Q4_K) at 1 / 16 rows 206 / 411 -> 190 / 417 (- / 463); the
+// worst of six drawn lists 72 -> 75 (96).
+constexpr double kBatchCallUs = 4, kBatchSendUs = 10, kBatchLaunchUs = 8, kBatchCopyBytesPerUs = 45e3, kBatchWeightBytesPerUs = 4.5e6;
+constexpr size_t kBatchWeightBytes = size_t(160) << 20;  // a launch's worth: tens of microseconds of streaming
+static bool batch_gpu_idles(const zq_ctx *ctx) {
+    const auto &t = ctx->line;
+    const double ready = std::max(t.run, t.pending_in) + kBatchLaunchUs;  // end of a launch's cost of standing idle
+    return (t.in >= ready && t.in >= t.host + kBatchLaunchUs) || t.host >= ready + kBatchLaunchUs / 2;
 }
 
 // Runs the bracket's deferred layers: one zq_linear_batch call per run of layers with the same dtypes (in call order),
@@ -642,12 +659,16 @@ static int batch_flush(zq_ctx *ctx, zq_error *err) {
         const int xd = ctx->pending_linear[i].x_dtype, yd = ctx->pending_linear[i].y_dtype;
         size_t e = i;
         jobs.clear();
+        size_t weights = 0;
         while (e < ctx->pending_linear.size() && ctx->pending_linear[e].x_dtype == xd && ctx->pending_linear[e].y_dtype == yd) {
             const zq_ctx::PendingLinear &p = ctx->pending_linear[e];
             zq_linear_job j = {p.w, nullptr, p.dev_x, p.m, p.dev_y, nullptr, 0};
             jobs.push_back(j);
+            weights += p.w->gguf_bytes;
             ++e;
         }
+        ctx->line.run = std::max(std::max(ctx->line.run, ctx->line.pending_in), ctx->line.host) + kBatchLaunchUs + (double)weights / kBatchWeightBytesPerUs;
+        ctx->line.host += kBatchSendUs;
         // the layers wait for their inputs (ev_in is recorded behind the copy of the last one); the copies out wait for the layers
         // and run beside the next batch
         ZQ_CUDA_CHECK(cudaStreamWaitEvent(ctx->stream, ctx->ev_in, 0), err);
@@ -663,7 +684,6 @@ static int batch_flush(zq_ctx *ctx, zq_error *err) {
         i = e;
     }
     ctx->pending_linear.clear();
-    ctx->pending_in_bytes = 0;
     return ZQ_OK;
 }
 
@@ -689,6 +709,7 @@ int zq_batch_finish(zq_ctx *ctx, zq_error *err) {
     }
     ctx->io_out_used = false;
     ctx->batch_active = false;
+    ctx->line = {};
     for (const auto &o : ctx->pending_out) memcpy(o.host, o.pinned, o.bytes);
     ctx->pending_out.clear();
     ctx->pending_in.clear();
@@ -736,21 +757,15 @@ int zq_linear_host(zq_ctx *ctx, const zq_weight *w, const void *host_x, int x_dt
             batch_abandon(ctx);
             return rc;
         }
-        // The GPU should not sit idle while the host records a long bracket: what is pending goes out as soon as it is a
-        // launch's worth, i.e. when the next layer is of another kernel class (weight type, row-count class, dtypes), when
-        // the pending weights pass ~160 MB (tens of microseconds of streaming), or when the pending activations pass 1 MB: that is
-        // ~18 us of copying in and out, against ~8 us for a launch of its own, and the layers then run between their own copies
-        // instead of between all copies in and all copies out (five projections of 16 rows, 5.6 MB in all: 224 -> 147 us).
+        // What is pending goes out before this layer is recorded when this one is of another kernel class (weight type, row-count class,
+        // dtypes) or when the GPU would stand idle (see batch_gpu_idles).  This call's copy in is already on its way: it runs
+        // under the launches, which do not wait for it.
         auto row_class = [](size_t rows) { return rows <= 4 ? 1 : rows <= 8 ? 2 : rows <= 16 ? 4 : 0; };
+        ctx->line.host += kBatchCallUs;
+        if (!dev_in) ctx->line.in = std::max(ctx->line.in, ctx->line.host) + (double)xb / kBatchCopyBytesPerUs;
         if (!ctx->pending_linear.empty()) {
             const zq_ctx::PendingLinear &last = ctx->pending_linear.back();
-            size_t weights = 0, moved = ctx->pending_in_bytes;
-            for (const auto &p : ctx->pending_linear) {
-                weights += p.w->gguf_bytes;
-                moved += p.y_bytes;
-            }
-            // this call's copy in is already on its way: it runs under the launches below, which do not wait for it
-            if (last.w->type != w->type || row_class(last.m) != row_class(m) || last.x_dtype != x_dtype || last.y_dtype != y_dtype || weights >= (size_t(160) << 20) || moved >= (size_t(1) << 20)) rc = batch_flush(ctx, err);
+            if (last.w->type != w->type || row_class(last.m) != row_class(m) || last.x_dtype != x_dtype || last.y_dtype != y_dtype || batch_gpu_idles(ctx)) rc = batch_flush(ctx, err);
         }
         if (!rc) {
             cudaError_t ce = cudaEventRecord(ctx->ev_in, ctx->io_in);
@@ -761,9 +776,15 @@ int zq_linear_host(zq_ctx *ctx, const zq_weight *w, const void *host_x, int x_dt
             return rc;
         }
         const size_t y_off = dev_in ? 0 : xb_al;
-        if (!dev_in) ctx->pending_in_bytes += xb;
+        ctx->line.pending_in = ctx->line.in;
         ctx->pending_linear.push_back({w, dev_in ? dev_in : dx, m, dx + y_off, y_pinned ? host_y : px + y_off, yb, x_dtype, y_dtype});
         if (!y_pinned) ctx->pending_out.push_back({host_y, px + y_off, yb});
+        size_t weights = 0;
+        for (const auto &p : ctx->pending_linear) weights += p.w->gguf_bytes;
+        if (weights >= kBatchWeightBytes && (rc = batch_flush(ctx, err))) {
+            batch_abandon(ctx);
+            return rc;
+        }
         return ZQ_OK;
     }
     if (ctx->host_io_bytes < xb_al + yb) {

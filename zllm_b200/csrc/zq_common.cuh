@@ -292,7 +292,9 @@ struct zq_ctx {
     std::vector<PendingOut> pending_out;
     std::vector<PendingLinear> pending_linear;
     std::vector<PendingIn> pending_in;
-    size_t pending_in_bytes = 0;  // copied in for the layers of pending_linear
+    // Time line of the open bracket as byte counts predict it, in us since it began (zq_api.cu: batch_gpu_idles): the host's calls, arrival
+    // of the last input copied and of the last one a pending layer needs, end of the layers launched so far.
+    struct { double host = 0, in = 0, pending_in = 0, run = 0; } line;
     bool batch_active = false;
     // Diagnostics: 1 = always use the per-item activation staging GEMV (the variant for activations too large to
     // stay resident in shared memory), so that tests can cover it at small sizes.
