@@ -324,3 +324,14 @@ def test_host_mirror_reports_bad_arguments():
     w.release()
     with pytest.raises(ZqFailure):
         ctx().linear(x, w)
+
+
+def test_an_output_that_does_not_fit_is_an_out_of_memory_error():
+    """The native half raises what torch raises (callers catch torch.OutOfMemoryError to make room), before anything is launched."""
+    class Huge:  # 4 PB of output for one row
+        _h, _rows, _cols = 1, 1 << 50, 256
+
+    with pytest.raises(torch.OutOfMemoryError):
+        ctx().linear(torch.zeros((1, 256), device="cuda"), Huge())
+    w = ctx().prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 64, 256, seed=4), 64, 256)
+    assert torch.equal(ctx().linear(torch.zeros((1, 256), device="cuda"), w), torch.zeros((1, 64), device="cuda"))

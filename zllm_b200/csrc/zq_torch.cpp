@@ -9,6 +9,7 @@
 
 #include <ATen/ATen.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <vector>
@@ -105,8 +106,8 @@ template <class Fn> PyObject *guarded(Fn fn) {
         return fn();
     } catch (const PyError &) {
         return nullptr;
-    } catch (const std::exception &e) {
-        PyErr_SetString(PyExc_RuntimeError, e.what());
+    } catch (...) {  // torch's own errors become the exceptions torch raises from Python (an allocation that fails: torch.OutOfMemoryError)
+        torch::translate_exception_to_python(std::current_exception());
         return nullptr;
     }
 }
