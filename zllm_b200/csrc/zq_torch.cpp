@@ -128,6 +128,16 @@ struct Items {
     PyObject *operator[](size_t i) const { return PySequence_Fast_GET_ITEM(fast, (Py_ssize_t)i); }
 };
 
+// KeyError(x.dtype): what a batch raises for inputs the library does not read
+[[noreturn]] void dtype_key_error(PyObject *x) {
+    PyObject *dtype = PyObject_GetAttrString(x, "dtype");
+    if (dtype) {
+        PyErr_SetObject(PyExc_KeyError, dtype);
+        Py_DECREF(dtype);
+    }
+    throw PyError();
+}
+
 // linear(ctx, x, weight, out_dtype, residual)
 PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t) {
     return guarded([&]() -> PyObject * {
@@ -176,6 +186,7 @@ PyObject *py_linear_batch(PyObject *, PyObject *const *a, Py_ssize_t) {
             const size_t m = rows_of(x, w.cols);
             if (i == 0) {
                 xt = x.scalar_type();
+                if (zq_dtype(xt) < 0) dtype_key_error(job[0]);
                 od = out_dtype_of(a[2], xt);
             }
             if (x.scalar_type() != xt) type_error("linear_batch: all inputs must share one dtype");
@@ -196,16 +207,11 @@ PyObject *py_linear_batch(PyObject *, PyObject *const *a, Py_ssize_t) {
             keep.push_back(x);
         }
         if (n) {
-            const int xd = zq_dtype(xt);
-            if (xd < 0) {
-                PyErr_SetString(PyExc_KeyError, dtype_name(xt).c_str());
-                throw PyError();
-            }
             zq_error err;
             int rc;
             {
                 NoGil g;
-                rc = zq_linear_batch(ctx, arr.data(), n, xd, zq_dtype(od), &err);
+                rc = zq_linear_batch(ctx, arr.data(), n, zq_dtype(xt), zq_dtype(od), &err);
             }
             check(rc, err);
         }
