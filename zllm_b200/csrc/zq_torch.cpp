@@ -346,7 +346,7 @@ PyObject *py_linear_host_batch(PyObject *, PyObject *const *a, Py_ssize_t) {
             const WeightRef w = weight_of(job[1]);
             for (int k = 0; k < 2; ++k) {
                 View &v = views[2 * i + k];
-                if (PyObject_GetBuffer(job[2 * k], &v.b, PyBUF_FORMAT | PyBUF_STRIDES | (k ? PyBUF_WRITABLE : 0))) throw PyError();
+                if (PyObject_GetBuffer(job[2 * k], &v.b, PyBUF_FORMAT | PyBUF_STRIDES)) throw PyError();
                 v.held = true;
                 if (i == 0) {
                     const char *f = v.b.format ? v.b.format : "";
