@@ -93,13 +93,23 @@ size_t rows_of(const at::Tensor &x, size_t cols) {
     if (cols == 0 || (size_t)last != cols) fail(1, "linear input cols=" + std::to_string(last) + ", weight cols=" + std::to_string(cols));
     return (size_t)x.numel() / cols;
 }
-at::Tensor new_rows(const at::Tensor &like, size_t m, size_t n, at::ScalarType t) { return at::empty({(int64_t)m, (int64_t)n}, like.options().dtype(t)); }
-at::Tensor contiguous(const at::Tensor &t) { return t.is_contiguous() ? t : t.contiguous(); }
-
-struct NoGil {  // the ABI may wait (workspace growth, host-buffer calls): let other threads run
+// Other threads run while torch allocates (which may wait for the device) and inside the ABI (workspace growth, host-buffer calls).
+struct NoGil {
     PyThreadState *s = PyEval_SaveThread();
     ~NoGil() { PyEval_RestoreThread(s); }
 };
+// without the GIL
+at::Tensor new_rows(const at::Tensor &like, size_t m, size_t n, at::ScalarType t) { return at::empty({(int64_t)m, (int64_t)n}, like.options().dtype(t)); }
+at::Tensor contiguous(const at::Tensor &t) {
+    if (t.is_contiguous()) return t;
+    NoGil g;
+    return t.contiguous();
+}
+at::Tensor as_f32(const at::Tensor &t) {
+    if (t.scalar_type() == at::kFloat) return t;
+    NoGil g;
+    return t.to(at::kFloat);
+}
 
 template <class Fn> PyObject *guarded(Fn fn) {
     try {
@@ -146,16 +156,17 @@ PyObject *py_linear(PyObject *, PyObject *const *a, Py_ssize_t) {
         const WeightRef w = weight_of(a[2]);
         const size_t m = rows_of(x, w.cols);
         const at::ScalarType od = out_dtype_of(a[3], x.scalar_type());
-        at::Tensor y = new_rows(x, m, w.rows, od), r;
+        at::Tensor y, r;
         if (!is_none(a[4])) {
             r = contiguous(tensor_of(a[4]));
-            if (r.numel() != y.numel() || r.scalar_type() != od) fail(1, "residual shape/dtype mismatch: " + std::to_string(r.numel()) + " values of " + dtype_name(r.scalar_type()) + " vs " + std::to_string(y.numel()) + " of " + dtype_name(od));
+            if ((size_t)r.numel() != m * w.rows || r.scalar_type() != od) fail(1, "residual shape/dtype mismatch: " + std::to_string(r.numel()) + " values of " + dtype_name(r.scalar_type()) + " vs " + std::to_string(m * w.rows) + " of " + dtype_name(od));
         }
         const int xd = in_dtype(x);
         zq_error err;
         int rc;
         {
             NoGil g;
+            y = new_rows(x, m, w.rows, od);
             rc = zq_linear(ctx, w.h, x.data_ptr(), xd, m, y.data_ptr(), zq_dtype(od), r.defined() ? r.data_ptr() : nullptr, &err);
         }
         check(rc, err);
@@ -170,8 +181,8 @@ PyObject *py_linear_batch(PyObject *, PyObject *const *a, Py_ssize_t) {
         Items jobs(a[1]);
         const size_t n = jobs.size();
         std::vector<zq_linear_job> arr(n);
-        std::vector<at::Tensor> ys(n), keep;
-        keep.reserve(2 * n);
+        std::vector<at::Tensor> ys(n), inputs(n), keep;
+        std::vector<size_t> rows(n);
         at::ScalarType xt = at::kFloat, od = at::kFloat;
         for (size_t i = 0; i < n; ++i) {
             Items job(jobs[i]);
@@ -190,27 +201,30 @@ PyObject *py_linear_batch(PyObject *, PyObject *const *a, Py_ssize_t) {
                 od = out_dtype_of(a[2], xt);
             }
             if (x.scalar_type() != xt) type_error("linear_batch: all inputs must share one dtype");
-            ys[i] = new_rows(x, m, w.rows, od);
             zq_linear_job &j = arr[i];
             j = {};
             j.w = w.h;
             j.w_up = gated ? weight_of(job[2]).h : nullptr;
             j.dev_x = x.data_ptr();
             j.m = m;
-            j.dev_y = ys[i].data_ptr();
+            rows[i] = w.rows;
+            inputs[i] = x;
             if ((job.size() == 3 || row) && !is_none(job[2])) {
                 const at::Tensor r = contiguous(tensor_of(job[2]));
                 j.dev_residual = r.data_ptr();
                 keep.push_back(r);
             }
             j.flags = row ? ZQ_JOB_ROW_PARALLEL : 0;
-            keep.push_back(x);
         }
         if (n) {
             zq_error err;
             int rc;
             {
                 NoGil g;
+                for (size_t i = 0; i < n; ++i) {
+                    ys[i] = new_rows(inputs[i], arr[i].m, rows[i], od);
+                    arr[i].dev_y = ys[i].data_ptr();
+                }
                 rc = zq_linear_batch(ctx, arr.data(), n, zq_dtype(xt), zq_dtype(od), &err);
             }
             check(rc, err);
@@ -233,19 +247,18 @@ PyObject *py_linear_multi(PyObject *, PyObject *const *a, Py_ssize_t) {
         std::vector<const zq_weight *> wh(n);
         std::vector<at::Tensor> ys(n);
         std::vector<void *> yp(n);
+        std::vector<size_t> rows(n);
         const size_t cols = weight_of(ws[0]).cols, m = rows_of(x, cols);
         at::Tensor norm;
         if (!is_none(a[4])) {
-            norm = contiguous(tensor_of(a[4]));
-            if (norm.scalar_type() != at::kFloat) norm = norm.to(at::kFloat);
+            norm = as_f32(contiguous(tensor_of(a[4])));
             if ((size_t)norm.numel() != cols) fail(1, "norm weight has " + std::to_string(norm.numel()) + " elements, input width is " + std::to_string(cols));
         }
         const at::ScalarType od = out_dtype_of(a[3], x.scalar_type());
         for (size_t i = 0; i < n; ++i) {
             const WeightRef w = weight_of(ws[i]);
             wh[i] = w.h;
-            ys[i] = new_rows(x, m, w.rows, od);
-            yp[i] = ys[i].data_ptr();
+            rows[i] = w.rows;
         }
         const int xd = in_dtype(x);
         const double eps = PyFloat_AsDouble(a[5]), offset = PyFloat_AsDouble(a[6]);
@@ -254,6 +267,10 @@ PyObject *py_linear_multi(PyObject *, PyObject *const *a, Py_ssize_t) {
         int rc;
         {
             NoGil g;
+            for (size_t i = 0; i < n; ++i) {
+                ys[i] = new_rows(x, m, rows[i], od);
+                yp[i] = ys[i].data_ptr();
+            }
             rc = norm.defined() ? zq_rmsnorm_linear(ctx, wh.data(), n, x.data_ptr(), xd, m, norm.data_ptr<float>(), (float)eps, (float)offset, yp.data(), zq_dtype(od), &err)
                                 : zq_linear_multi(ctx, wh.data(), n, x.data_ptr(), xd, m, yp.data(), zq_dtype(od), &err);
         }
@@ -272,13 +289,14 @@ PyObject *py_gated(PyObject *, PyObject *const *a, Py_ssize_t) {
         const WeightRef down = mlp ? weight_of(a[4]) : WeightRef{nullptr, gate.rows, 0};
         const size_t m = rows_of(x, gate.cols);
         const at::ScalarType od = out_dtype_of(a[5], x.scalar_type());
-        at::Tensor y = new_rows(x, m, down.rows, od), r;
+        at::Tensor y, r;
         if (!is_none(a[6])) r = contiguous(tensor_of(a[6]));
         const int xd = in_dtype(x);
         zq_error err;
         int rc;
         {
             NoGil g;
+            y = new_rows(x, m, down.rows, od);
             rc = mlp ? zq_gated_mlp(ctx, gate.h, up.h, down.h, x.data_ptr(), xd, m, y.data_ptr(), zq_dtype(od), r.defined() ? r.data_ptr() : nullptr, &err)
                      : zq_gated_silu(ctx, gate.h, up.h, x.data_ptr(), xd, m, y.data_ptr(), zq_dtype(od), &err);
         }
@@ -307,9 +325,7 @@ PyObject *py_rope(PyObject *, PyObject *const *a, Py_ssize_t) {
         }
         const int64_t head_dim = q.numel() / rows / v[0];
         if (k.defined() && (k.scalar_type() != q.scalar_type() || k.numel() != rows * v[1] * head_dim)) fail(1, "rope: key shape or dtype does not match the query's");
-        at::Tensor c = contiguous(tensor_of(a[7])), s = contiguous(tensor_of(a[8]));
-        if (c.scalar_type() != at::kFloat) c = c.to(at::kFloat);
-        if (s.scalar_type() != at::kFloat) s = s.to(at::kFloat);
+        const at::Tensor c = as_f32(contiguous(tensor_of(a[7]))), s = as_f32(contiguous(tensor_of(a[8])));
         if (c.numel() != s.numel()) fail(1, "rope: cos and sin tables differ in length (" + std::to_string(c.numel()) + " / " + std::to_string(s.numel()) + ")");
         const int d = in_dtype(q);
         zq_error err;
