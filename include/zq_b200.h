@@ -46,14 +46,19 @@ enum { ZQ_OK = 0, ZQ_ERR_SHAPE = 1, ZQ_ERR_UNSUPPORTED = 2, ZQ_ERR_CUDA = 3, ZQ_
 int zq_ctx_create(int device, zq_ctx **out, zq_error *err);
 void zq_ctx_destroy(zq_ctx *ctx);
 /* Run on a caller-owned cudaStream_t instead of the context's own stream.  NULL is a valid handle: it is the
- * legacy default stream.  zq_ctx_use_own_stream goes back to the stream the context created. */
+ * legacy default stream.  zq_ctx_use_own_stream goes back to the stream the context created.
+ * The context's buffers belong to its calls in the order they are issued; calls on two streams at once are safe where a call uses
+ * none of them: zq_linear and zq_gated_silu of up to 4 rows, and of f16 rows on packed weights (Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL,
+ * Q8_0) from 17 to 1024 rows.  The same calls may be captured first and replayed after any other; a graph of any other call must
+ * not be replayed after a later call that needed larger buffers.  Where such a call needs scratch it takes it in stream order, in a
+ * graph as an allocation node (a graph with one cannot be a child graph or be instantiated twice at a time). */
 int zq_ctx_set_stream(zq_ctx *ctx, void *cuda_stream, zq_error *err);
 int zq_ctx_use_own_stream(zq_ctx *ctx, zq_error *err);
 /* Waits for the stream and reports any status word a kernel left behind (bounded waits that ran out). */
 int zq_ctx_sync(zq_ctx *ctx, zq_error *err);
 /* Diagnostic switches (the counterpart of the reference's ZLLM_CUDA_* environment switches, kept per context).
  * Known keys (0/1): "force_staged_gemv", "force_f16_gemv" (decode on the f16 kernels instead of the integer-MMA kernel),
- * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_fused_gemm" / "force_fused_gemm" (Q4_K prefill never / always on the kernel that dequantises inside the GEMM; default: up to 1024 tokens and MoE prefill). */
+ * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_fused_gemm" / "force_fused_gemm" (prefill of Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL and Q8_0 never / always with the dequantisation inside the GEMM; default: up to 1024 tokens and MoE prefill). */
 int zq_ctx_set_option(zq_ctx *ctx, const char *key, int value, zq_error *err);
 int zq_ctx_sm_count(const zq_ctx *ctx);
 /* Number of kernels this library has launched on the context since creation (bench accounting). */
@@ -95,8 +100,8 @@ int zq_linear_multi(zq_ctx *ctx, const zq_weight *const *w, size_t n_weights, co
  * decode launch gguf_dual_gemv_q4k_f16 (src/kernel/metal/gguf/mod.rs:1787-1824) to any number of weights and inputs:
  * the projections of a decode step that are ready together (q, k, v; gate and up; the layers of several sequences)
  * stream through one persistent kernel whose TMA ring never drains between matrices.  Per job: y = W x (+ residual),
- * or y = silu(gate x) * (up x) when `w_up` is given (then `w` is the gate; no residual).  Jobs of Q4_K / Q4_0 / Q8_0
- * weights with up to 16 rows share launches (one per weight type, row-count class 1-4 / 5-8 / 9-16 and plain / gated);
+ * or y = silu(gate x) * (up x) when `w_up` is given (then `w` is the gate; no residual).  Jobs of Q4_K / Q5_K / Q6_K /
+ * Q4_0 / IQ4_NL / Q8_0 weights with up to 16 rows share launches (one per weight type, row-count class 1-4 / 5-8 / 9-16 and plain / gated);
  * every other job runs as its own zq_linear / zq_gated_silu call.  All jobs share x_dtype and y_dtype.  Results do not
  * depend on how the jobs are grouped beyond f32 rounding of the split-tile sums, and are the same from run to run. */
 enum { ZQ_JOB_ROW_PARALLEL = 1 };  /* zq_linear_job.flags: sum this job's result over the ranks of the peer group (zq_dist_init) */

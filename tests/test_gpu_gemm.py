@@ -18,8 +18,8 @@ BOUND = 2e-3
 
 @pytest.fixture(autouse=True, params=["fused", "operand_pass"])
 def gemm_variant(request):
-    """Q4_K runs on the kernel that dequantises inside the GEMM and on the separate f16 operand pass + plain GEMM (what
-    the other formats use); both must produce the same bits, so every case runs on both."""
+    """Every decode type runs on the kernel that dequantises inside the GEMM and on the separate f16 operand pass + plain GEMM;
+    both must produce the same bits, so every case runs on both."""
     ctx().set_option("disable_fused_gemm", 1 if request.param == "operand_pass" else 0)
     ctx().set_option("force_fused_gemm", 1 if request.param == "fused" else 0)
     yield request.param
@@ -186,3 +186,59 @@ def test_operand_is_the_dequantised_value_rounded_once(tensor_type):
     w = ctx().prepare_weight(tensor_type, data, rows, cols)
     got = host(ctx().linear(torch.eye(cols, device="cuda", dtype=torch.float16), w, out_dtype=torch.float32)).T
     assert np.array_equal(got, want.astype(np.float32))
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+@pytest.mark.parametrize("gated", [False, True])
+def test_both_operand_forms_agree_bit_for_bit_for_every_type(tensor_type, gated, gemm_variant):
+    if gemm_variant == "operand_pass":
+        pytest.skip("compares a fused variant with the operand pass in one go")
+    rows, m = 300, 530
+    cols = 1024 if tensor_type in (H.Q4_K, H.Q5_K, H.Q6_K) else 1024 - 96
+    ws = [ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=177 + i), rows, cols) for i in range(2)]
+    x = dev(np.random.default_rng(178).standard_normal((m, cols)).astype(np.float32), torch.bfloat16)
+
+    def run():
+        return host(ctx().gated_linear(x, *ws, out_dtype=torch.float32) if gated else ctx().linear(x, ws[0], out_dtype=torch.float32)).copy()
+
+    a = run()
+    ctx().set_option("force_fused_gemm", 0)
+    ctx().set_option("disable_fused_gemm", 1)
+    assert np.array_equal(a.view(np.uint32), run().view(np.uint32))
+
+
+@pytest.mark.parametrize("m", [17, 48, 300, 1100])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_a_call_reads_what_the_call_directly_before_it_wrote(m, dtype):
+    """No torch operator between the calls: every result is the next call's input (f16: no conversion between them either) and residual, the
+    gated result too, and a decode call reads the last; the same bits as with a wait behind every call."""
+    cols = 1024  # weights of 0.01: a projection scales by 0.32, the gated product stays small, so 24 calls stay inside f16
+    ws = [ctx().prepare_weight(t, H.random_weight(t, cols, cols, seed=260 + i, std=0.01), cols, cols) for i, t in enumerate((H.Q4_K, H.Q8_0, H.IQ4_NL, H.Q4_0))]
+    x0 = torch.from_numpy(np.random.default_rng(261).standard_normal((m, cols)).astype(np.float32)).to("cuda", dtype)
+
+    def chain(wait):
+        x, outs = x0, []
+        for i in range(8):
+            x = ctx().linear(x, ws[i % 4], residual=x)
+            if wait:
+                ctx().sync()
+            outs.append(x)
+            g = ctx().gated_linear(x, ws[(i + 1) % 4], ws[(i + 1) % 4])
+            if wait:
+                ctx().sync()
+            outs.append(g)
+            x = ctx().linear(g, ws[(i + 2) % 4], residual=x)
+            if wait:
+                ctx().sync()
+            outs.append(x)
+            outs.append(ctx().linear(x[:4], ws[(i + 3) % 4]))
+            if wait:
+                ctx().sync()
+        ctx().sync()
+        return [o.float().cpu().numpy() for o in outs]
+
+    want = chain(True)
+    assert all(np.isfinite(o).all() for o in want)
+    for _ in range(3):
+        for a, b in zip(chain(False), want):
+            assert np.array_equal(a.view(np.uint32), b.view(np.uint32))

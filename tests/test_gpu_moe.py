@@ -288,3 +288,53 @@ def test_gather_and_scatter_add_rows_on_their_own():
     with pytest.raises(ffi.ZqFailure):
         ctx().sync()
     ctx().sync()
+
+
+@pytest.mark.parametrize("gate_type,down_type,hidden,inter", [
+    (H.Q4_0, H.Q4_0, 544, 352), (H.IQ4_NL, H.IQ4_NL, 544, 352), (H.Q8_0, H.Q4_0, 288, 1120),  # widths that end inside a 256-column unit, and inside a k-block
+    (H.Q5_K, H.Q6_K, 512, 768), (H.Q6_K, H.Q5_K, 256, 512), (H.Q4_K, H.Q8_0, 512, 352)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+def test_moe_prefill_takes_every_packed_type(gate_type, down_type, hidden, inter, dtype):
+    """Grouped GEMMs on packed experts of every type they unpack, mixed gate / down types, tiles of equal token shares, absent routes:
+    the same bits as grouping on the host, and token by token the values of the same arithmetic in 64 bits: operands (the codec's values,
+    the activations, the intermediate) rounded to f16 once, everything else exact.  Bound: an intermediate whose f32 sums fall on
+    the other side of a rounding boundary is off by one f16 step, 2^-10 of its value at most, so a token by 2^-10 of its norm; f16 and
+    bf16 results add 2^-12 and 2^-9.  (Against unrounded operands the error is that of the rounding, which for unscaled random codes
+    is 1.1e-3 of a token's norm, computed and measured alike.)  The activations are bf16 values in every dtype."""
+    from zllm_b200 import ffi
+    from zllm_b200.backend import MoeExperts, moe_forward
+
+    n_exp, top_k, m = 4, 2, 530
+    gates = [H.random_weight(gate_type, inter, hidden, seed=840 + 3 * e) for e in range(n_exp)]
+    ups = [H.random_weight(gate_type, inter, hidden, seed=841 + 3 * e) for e in range(n_exp)]
+    downs = [H.random_weight(down_type, hidden, inter, seed=842 + 3 * e, std=0.05) for e in range(n_exp)]
+    rng = np.random.default_rng(84)
+    x = torch.from_numpy(rng.standard_normal((m, hidden)).astype(np.float32)).to("cuda", torch.bfloat16).to(dtype)
+    ids_np = np.stack([rng.permutation(n_exp)[:top_k] for _ in range(m)]).astype(np.uint32)
+    w_np = rng.random((m, top_k)).astype(np.float32)
+    absent = rng.random((m, top_k)) < 0.1
+    ids_np[absent] = ffi.MOE_NO_ROUTE
+    c = ctx()
+    table = MoeExperts(c, [c.prepare_weight(gate_type, g, inter, hidden) for g in gates], [c.prepare_weight(gate_type, u, inter, hidden) for u in ups],
+                       [c.prepare_weight(down_type, d, hidden, inter) for d in downs])
+    ids, wd = torch.from_numpy(ids_np.view(np.int32)).cuda(), dev(w_np)
+    got = host(moe_forward(c, table, x, ids, wd)).copy()
+    c.set_option("force_moe_host_grouping", 1)
+    try:
+        on_host = host(moe_forward(c, table, x, ids, wd)).copy()
+    finally:
+        c.set_option("force_moe_host_grouping", 0)
+    assert np.array_equal(got.view(np.uint32), on_host.view(np.uint32))
+    def f16(a):
+        return a.astype(np.float16).astype(np.float64)
+
+    mats = [[f16(orc.dequantize(t, d, r * k).reshape(r, k)) for d in side] for t, side, r, k in ((gate_type, gates, inter, hidden), (gate_type, ups, inter, hidden), (down_type, downs, hidden, inter))]
+    rows, sel = x.float().cpu().numpy().astype(np.float64), np.arange(0, m, 7)
+    for t in sel:
+        want = np.zeros(hidden)
+        for e, weight in zip(ids_np[t], w_np[t]):
+            if e != ffi.MOE_NO_ROUTE:
+                g, u = mats[0][e] @ rows[t], mats[1][e] @ rows[t]
+                want += weight * (mats[2][e] @ f16(g / (1.0 + np.exp(-g)) * u))
+        error = np.linalg.norm(got[t] - want)
+        assert error <= (2.0 ** -10 + (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12 if dtype == torch.float16 else 0.0)) * np.linalg.norm(want)

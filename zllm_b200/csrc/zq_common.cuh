@@ -62,8 +62,8 @@ __host__ __device__ inline FormatInfo format_info(uint32_t t) {
 }
 
 // Types without an unpacker in the f16 decode kernels and without an encoder.  Of these, Q5_K and Q6_K
-// (src/weight/codec/ggml.rs:425-469) decode on the integer-MMA kernels (has_i8_decode); with more than 16 rows, or with a
-// diagnostic switch that turns those kernels off, they take the f16 operand pass + tensor-core GEMM like the rest.
+// (src/weight/codec/ggml.rs:425-469) decode on the integer-MMA kernels (has_i8_decode); with more than 16 rows the tensor-core GEMM
+// unpacks them itself or takes the f16 operand pass, and so does every row count under a diagnostic switch that turns the decode kernels off.
 __host__ __device__ inline bool is_operand_pass_only(uint32_t type) { return type == ZQ_Q5_K || type == ZQ_Q6_K || type == ZQ_Q5_0 || type == ZQ_Q5_1 || type == ZQ_Q3_K || type == ZQ_IQ4_XS; }
 // Q5_0, Q5_1, Q3_K and IQ4_XS (src/weight/codec/ggml.rs:111-130, 246-261, 384-406) are resident in GGUF layout, dequantise
 // bit-exactly, and run every projection through the f16 operand pass and the tensor-core GEMM.
@@ -167,11 +167,6 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, u
 __device__ __forceinline__ void bulk_load_1d(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(src)), "r"(bytes),
                  "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, uint64_t *bar, int x, int y, int z) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
-                 "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 
@@ -304,10 +299,10 @@ struct zq_ctx {
     int enable_tcgen05_gemv = 0;
     int force_f16_gemv = 0;  // skip the integer-MMA decode kernel (tests of the f16 kernels)
     int narrow_gemv_tiles = 0;  // integer-MMA decode, up to 4 rows: 64-row tiles, two CTAs per SM (measured slower; off)
-    int disable_pdl = 0;     // launch decode kernels without programmatic dependent launch
+    int disable_pdl = 0;     // launch decode and prefill kernels without programmatic dependent launch
     int disable_worklist = 0;  // zq_linear_batch and the multi-weight entries: one launch per job instead of the work-list kernel
-    int force_fused_gemm = 0;      // Q4_K prefill: the fused kernel for every token count (tests)
-    int disable_fused_gemm = 0;    // Q4_K prefill: separate f16 operand pass + plain GEMM instead of the fused kernel
+    int force_fused_gemm = 0;      // prefill of the decode types: dequantisation inside the GEMM for every token count (tests)
+    int disable_fused_gemm = 0;    // prefill: always the separate f16 operand pass
     int force_moe_per_expert = 0;  // MoE forward: always the host-grouped per-expert path (tests)
     const void *moe_row_sink = nullptr;  // zq::PeerRowSink of the expert-parallel forward while it runs its local experts, else null
     int force_moe_host_grouping = 0;  // MoE prefill: group the routes on the host instead of on the device (tests, A/B)

@@ -451,7 +451,7 @@ __global__ void gather_rows_checked_kernel(const void *__restrict__ x, int dtype
 // ascending expert id, src/backend/cpu/moe.rs:107-141).  A stable counting sort over chunks of whole tokens:
 //   count   per chunk, how many routes go to each expert
 //   scan    one CTA, thread per expert: the chunk's first slot inside each expert's range, the experts' ranges, and
-//           the two work lists of the grouped GEMMs (one item per expert, 256-token tile, 128-row tile) with their counts
+//           the two work lists of the grouped GEMMs (one item per expert, tile of up to 256 tokens, tile of 128 gated outputs or 256 rows) with their counts
 //   place   per chunk: slot of every route, and each token's slots and weights in combine order
 // Nothing returns to the host: the GEMM kernels read their item counts from device memory.
 // ---------------------------------------------------------------------------------------------------------------
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_count_kernel(const 
 // groups of 32.  270 tokens are 160 + 110, not 256 + 14: a tile costs at least its dequantisation, whatever its tokens.
 __host__ __device__ inline uint32_t moe_tile_tokens(uint32_t count, uint32_t tiles) { return ((count + tiles - 1) / tiles + 31u) & ~31u; }
 
-// counts: [0] items of the gated launch, [1] items of the down launch, [2] routed rows in all
+// counts: [0] items of the gated launch, [1] items of the down launch
 __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_t *__restrict__ hist, int chunks, int E, uint32_t *__restrict__ offsets, int rt_gated, int rt_down, int4 *__restrict__ items_gated,
                                                                          int4 *__restrict__ items_down, int *__restrict__ counts) {
     __shared__ uint32_t warp_tot[2][32];
@@ -529,7 +529,6 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_
         const uint32_t tiles = base_t + st;
         counts[0] = (int)(tiles * (uint32_t)rt_gated);
         counts[1] = (int)(tiles * (uint32_t)rt_down);
-        counts[2] = (int)(base_c + sc);
     }
 }
 
@@ -1030,7 +1029,7 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
     if (fused_gemm) {
         // Prefill, experts of a type the GEMM unpacks: two launches for the whole layer.  The fused tensor-core GEMM dequantises the packed
         // tiles of whichever expert a work item names (per-expert tensor maps in a device table), so there is no f16
-        // copy of any expert.  Work list: one item per (expert, 256-token tile, 128-row tile); tokens are the gathered
+        // copy of any expert.  Work list: one item per (expert, tile of up to 256 tokens, tile of 128 gated outputs or 256 rows); tokens are the gathered
         // slot rows, so outputs land in slot order as the combine expects.
         auto al2 = [](size_t v) { return (v + 1023) & ~size_t(1023); };
         std::vector<int4> items;
