@@ -48,8 +48,8 @@ void zq_ctx_destroy(zq_ctx *ctx);
 /* Run on a caller-owned cudaStream_t instead of the context's own stream.  NULL is a valid handle: it is the
  * legacy default stream.  zq_ctx_use_own_stream goes back to the stream the context created.
  * The context's buffers belong to its calls in the order they are issued; calls on two streams at once are safe where a call uses
- * none of them: zq_linear and zq_gated_silu of up to 4 rows, and of f16 rows on packed weights (Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL,
- * Q8_0) from 17 to 1024 rows.  The same calls may be captured first and replayed after any other; a graph of any other call must
+ * none of them: zq_linear and zq_gated_silu of up to 4 rows (and up to 8192 columns), and of 17 to 1024 f16 rows, on Q4_K, Q5_K,
+ * Q6_K, Q4_0, IQ4_NL and Q8_0 weights.  The same calls may be captured first and replayed after any other; a graph of any other call must
  * not be replayed after a later call that needed larger buffers.  Where such a call needs scratch it takes it in stream order, in a
  * graph as an allocation node (a graph with one cannot be a child graph or be instantiated twice at a time). */
 int zq_ctx_set_stream(zq_ctx *ctx, void *cuda_stream, zq_error *err);
