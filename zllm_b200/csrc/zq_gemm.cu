@@ -743,7 +743,8 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, GemmParams &p) {
 // Shares and their counters are scratch of the launch and not context memory: the short prefill of f16 rows needs no other, so that
 // it may be captured first, replayed after any later call and run on two streams at once, and no call needs a larger workspace
 // than a longer one before it.  A launch that gave up on a wait leaves no counter behind for the next.  Taking it from the pool costs
-// nothing that can be measured (48 tokens of 5120 x 17408 up and down: 66.8 us, in the context's workspace 66.8 to 67.0).
+// nothing that can be measured (two builds in turn that differed in this alone, 48 tokens of 5120 x 17408 up and down: 66.8 us from the
+// pool, 66.8 to 67.0 from the context's workspace).
 static int take_shares(zq_ctx *ctx, GemmParams &p, LaunchScratch &scratch, zq_error *err) {
     if (!p.cut_tiles) return ZQ_OK;
     const size_t head = ((size_t)2 * p.cut_pairs * sizeof(uint32_t) + 1023) & ~size_t(1023);
