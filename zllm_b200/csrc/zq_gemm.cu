@@ -164,6 +164,25 @@ __device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32
     return false;
 }
 
+template <int DT> struct DtypeTag {
+    static constexpr int value = DT;
+};
+// f32 bits -> one element of the output type, and an element's bits as they are loaded -> f32
+template <int DT> __device__ __forceinline__ void store_as(uint8_t *at, uint32_t f32_bits) {
+    if constexpr (DT == ZQ_F32) *reinterpret_cast<uint32_t *>(at) = f32_bits;
+    else if constexpr (DT == ZQ_F16) *reinterpret_cast<__half *>(at) = __float2half_rn(__uint_as_float(f32_bits));
+    else *reinterpret_cast<__nv_bfloat16 *>(at) = __float2bfloat16_rn(__uint_as_float(f32_bits));
+}
+template <int DT> __device__ __forceinline__ uint32_t load_raw(const uint8_t *at) {
+    if constexpr (DT == ZQ_F32) return *reinterpret_cast<const uint32_t *>(at);
+    else return *reinterpret_cast<const uint16_t *>(at);
+}
+template <int DT> __device__ __forceinline__ float raw_as_f32(uint32_t r) {
+    if constexpr (DT == ZQ_F32) return __uint_as_float(r);
+    else if constexpr (DT == ZQ_F16) return __half2float(__ushort_as_half((unsigned short)r));
+    else return __uint_as_float(r << 16);
+}
+
 // AND over the four epilogue warps (named barrier 3)
 __device__ __forceinline__ bool epilogue_all(bool v) {
     uint32_t r;
@@ -425,8 +444,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
             // output row of this lane; gated: warps 0, 1 hold gate rows, warps 2, 3 the up rows of the same outputs
             const int row = GATED ? sg.row0 + (int)rank * 64 + (q & 1) * 32 + lane : sg.row0 + (int)rank * kBM + q * 32 + lane;
-            // 16 columns of finished sums (f32 bits) -> y
-            auto store16 = [&](int c0, uint32_t (&v)[16]) {
+            // 16 columns of finished sums (f32 bits) -> y.  With the output type known at compile time and one wide multiply-add per address
+            // an element takes about 4 instructions.
+            auto store16 = [&](auto dt, int c0, uint32_t (&v)[16]) {
+                constexpr int DT = decltype(dt)::value;
+                const size_t at = ((size_t)(sg.tok0 + c0) * p.n_out + row) * dtype_size(DT);
+                uint8_t *const yb = reinterpret_cast<uint8_t *>(p.y) + at;
+                auto token = [&](int j) { return (uint64_t)(uint32_t)p.n_out * (uint32_t)(j * (int)dtype_size(DT)); };  // bytes from one token's row to the j-th after it
                 if (GATED) {
                     // the two warps of one row half trade: the gate warp finishes columns 0..7 of the chunk, the up warp 8..15
                     float *xb = xch + ((c0 >> 4) & 1) * (16 * 32);  // [which half travels][8 columns][32 rows]; rewritten two chunks later, behind the barrier in between
@@ -435,42 +459,49 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     for (int j = 0; j < 8; ++j) xb[((is_up ? 0 : 8) + j) * 32 + lane] = __uint_as_float(is_up ? v[j] : v[8 + j]);
                     asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
                     if (row >= p.n_out) return;
-                    const int cb = c0 + (is_up ? 8 : 0);
-                    const size_t o = (size_t)(sg.tok0 + cb) * p.n_out + row;
+                    const int cb = is_up ? 8 : 0, left = n_tok - c0 - cb;
+                    uint8_t *const yc = yb + token(cb);
 #pragma unroll
                     for (int j = 0; j < 8; ++j) {
-                        const float other = xb[((is_up ? 8 : 0) + j) * 32 + lane], mine = __uint_as_float(is_up ? v[8 + j] : v[j]);
+                        const float other = xb[(cb + j) * 32 + lane], mine = __uint_as_float(is_up ? v[8 + j] : v[j]);
                         const float g = is_up ? other : mine, u = is_up ? mine : other;
-                        if (cb + j < n_tok) store_from_f32(p.y, p.y_dtype, o + (size_t)j * p.n_out, (g / (1.0f + expf(-g))) * u);  // src/kernel/cpu/ggml_quant.rs:352
+                        v[j] = __float_as_uint((g / (1.0f + expf(-g))) * u);  // src/kernel/cpu/ggml_quant.rs:352
                     }
+#pragma unroll
+                    for (int j = 0; j < 8; ++j)
+                        if (j < left) store_as<DT>(yc + token(j), v[j]);
                     return;
                 }
                 if (row >= p.n_out) return;
-                const size_t o = (size_t)(sg.tok0 + c0) * p.n_out + row;
+                const int left = n_tok - c0;
                 if (p.residual) {  // all loads of the chunk, unconverted, before anything uses one (and before the first store: y may be the residual's own buffer)
+                    const uint8_t *const rb = reinterpret_cast<const uint8_t *>(p.residual) + at;
                     uint32_t r[16];
-                    if (p.y_dtype == ZQ_F32) {
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) r[j] = c0 + j < n_tok ? reinterpret_cast<const uint32_t *>(p.residual)[o + (size_t)j * p.n_out] : 0u;
-                    } else {
+                    for (int j = 0; j < 16; ++j) r[j] = j < left ? load_raw<DT>(rb + token(j)) : 0u;
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) r[j] = c0 + j < n_tok ? reinterpret_cast<const uint16_t *>(p.residual)[o + (size_t)j * p.n_out] : 0u;
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) r[j] = p.y_dtype == ZQ_F16 ? __float_as_uint(__half2float(__ushort_as_half((unsigned short)r[j]))) : r[j] << 16;
-                    }
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(r[j]));
+                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + raw_as_f32<DT>(r[j]));
                 }
+                if (left >= 16) {
 #pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (c0 + j < n_tok) store_from_f32(p.y, p.y_dtype, o + (size_t)j * p.n_out, __uint_as_float(v[j]));
+                    for (int j = 0; j < 16; ++j) store_as<DT>(yb + token(j), v[j]);
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        if (j < left) store_as<DT>(yb + token(j), v[j]);
+                }
             };
-            if (ok && whole) {
+            auto store_tile = [&](auto dt) {
                 for (int c0 = 0; c0 < n_tok; c0 += 16) {  // warp-uniform
                     uint32_t v[16];
                     tmem_ld16(acc + c0, v);
-                    store16(c0, v);
+                    store16(dt, c0, v);
                 }
+            };
+            if (ok && whole) {
+                if (p.y_dtype == ZQ_F32) store_tile(DtypeTag<ZQ_F32>());
+                else if (p.y_dtype == ZQ_F16) store_tile(DtypeTag<ZQ_F16>());
+                else store_tile(DtypeTag<ZQ_BF16>());
             }
             if (!whole) {
                 // A share of a cut tile.  Whoever comes last adds the other shares from their slots to its own, in pair order;
@@ -518,7 +549,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                                 for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(c == c_first ? n[j] : __uint_as_float(v[j]) + n[j]);
                             }
                         }
-                        store16(c0, v);
+                        if (p.y_dtype == ZQ_F32) store16(DtypeTag<ZQ_F32>(), c0, v);
+                        else if (p.y_dtype == ZQ_F16) store16(DtypeTag<ZQ_F16>(), c0, v);
+                        else store16(DtypeTag<ZQ_BF16>(), c0, v);
                     }
                 }
             }
