@@ -188,6 +188,24 @@ def test_operand_is_the_dequantised_value_rounded_once(tensor_type):
     assert np.array_equal(got, want.astype(np.float32))
 
 
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K])
+def test_k_quant_operand_at_the_edges_of_the_scale_range(tensor_type):
+    """Scale and minimum that are zero, negative, subnormal f16 or as large as the operand's range allows (31 * 63 * 32 < 65504): the operand is
+    the codec's value rounded once, bit for bit (a zero's sign does not survive the sum)."""
+    rows, cols = 96, 256
+    e, b = orc.BLOCK[tensor_type]
+    data = H.random_bytes_weight(tensor_type, rows, cols, seed=19).reshape(-1, b)
+    edges = np.array([0.0, -0.0, 2.0 ** -24, -3 * 2.0 ** -24, 1023 * 2.0 ** -24, 2.0 ** -14, 0.3, -0.3, 31.0, -32.0], np.float16)
+    rng = np.random.default_rng(20)
+    for off in H.SCALE_OFFSETS[tensor_type]:
+        data[:, off:off + 2] = rng.choice(edges, size=len(data)).view(np.uint8).reshape(-1, 2)
+    data = data.reshape(-1)
+    want = orc.dequantize(tensor_type, data, rows * cols).reshape(rows, cols).astype(np.float16)
+    w = ctx().prepare_weight(tensor_type, data, rows, cols)
+    got = host(ctx().linear(torch.eye(cols, device="cuda", dtype=torch.float16), w, out_dtype=torch.float32)).T
+    assert np.isfinite(want).all() and np.array_equal(got, want.astype(np.float32))
+
+
 @pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
 @pytest.mark.parametrize("gated", [False, True])
 def test_both_operand_forms_agree_bit_for_bit_for_every_type(tensor_type, gated, gemm_variant):

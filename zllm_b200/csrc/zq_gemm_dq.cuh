@@ -8,18 +8,18 @@
 // by 32-bit shared addresses: as generic accesses the stores cost the fence behind them several times as much.
 //
 // Arithmetic: every operand is the codec's f32 value rounded once to f16.
-//   Q4_K, Q5_K   a code byte placed under the exponent of 2^7 is the float 128 + q; 128 is taken off again (exact) and
-//                fma(s, q, -m) rounds once to f32: s = d sc has at most 17 significant bits, so s q is exact in the codec's
-//                product too.  One multiply-add on 128 + q with -128 s folded into the offset is an instruction less per two weights,
-//                but rounds that offset at 2^-17 s and loses bits of m where it is small beside the scale.  Measured in turn, folded
-//                and not: 48 / 512 tokens of 5120 x 17408 up and down 65.2 / 190.3 and 64.7 / 191.0 us, MoE layer of 8192 tokens
-//                8.19 and 8.34 ms; both forms behind a vote on whether the offset is exact: 66.7 / 191.2 us, 8.27 ms.
-//   Q6_K         fma(s, 128 + q + 32, -160 s) = s q: 160 s is exact, there is no other offset.
-//                Two additions or multiply-adds per instruction (add.rn.f32x2, fma.rn.f32x2).
+//   Q4_K, Q5_K   the codec's d sc q - dmin m: sc q is at most 31 * 63, an integer f16 holds exactly, so one f16 multiply-add on the code
+//                (biased by 1024 to sit in the mantissa, sc (1024 + q) - 1024 sc, for two weights) gives it without rounding, and one
+//                mixed-precision multiply-add (f16 d times f16 sc q plus the f32 minimum term, rounded once to f32) does the rest: d sc has 17
+//                significant bits, so the codec's products are exact too.
+//                What bounds it is the ALU pipe, which takes a byte permute, a logic operation or a conversion in two cycles: 1.1 such
+//                operations per weight of about 2.6 instructions.  With codes permuted under an f32 exponent (fma(s, 128 + q - 128, -m)) it were
+//                1.9 of 2.9: 48 tokens of 5120 x 17408 up and down 63.1 us, now 58.0.  (A bias that stays in the product would save an
+//                instruction there, but rounds the minimum away where it is small beside the scale.)
+//   Q6_K         fma(s, 128 + q + 32, -160 s) = s q: 160 s is exact, there is no other offset.  Two multiply-adds per instruction
+//                (fma.rn.f32x2).
 //   Q4_0, IQ4_NL, Q8_0 d q with d an f16 and q an integer of at most 8 bits: an f16 multiply rounds the exact product once,
 //                      which is what multiplying in f32 (exact) and rounding does.
-// About 3 instructions per weight for Q4_K, a good third on the ALU pipe (byte permutes); the form before this one took a permute,
-// a subtraction and a multiply-add per weight (9 instructions with its waits).
 #pragma once
 #include "zq_common.cuh"
 
@@ -35,21 +35,49 @@ __device__ __forceinline__ uint64_t dq_pair(float v) {
     asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
     return r;
 }
-// codes in bytes J, J + 1 of `codes` -> f16x2 of s * q + c; BIASED: of s * (128 + q) + c
-template <int J, bool BIASED> __device__ __forceinline__ uint32_t dq_fma2(uint32_t codes, uint64_t s2, uint64_t c2) {
+// f32 sums f16 * f16 + f32, rounded once: the mixed-precision multiply-add of this architecture takes either half of a register
+// pair, at the rate of an f32 one.
+__device__ __forceinline__ void dq_fma_halves(uint32_t t2, unsigned short d, float c, float &lo, float &hi) {
+    asm("{\n\t.reg .b16 l, h;\n\t"
+        "mov.b32 {l, h}, %2;\n\t"
+        "fma.rn.f32.f16 %0, l, %3, %4;\n\t"
+        "fma.rn.f32.f16 %1, h, %3, %4;\n\t}"
+        : "=f"(lo), "=f"(hi)
+        : "r"(t2), "h"(d), "f"(c));
+}
+__device__ __forceinline__ float dq_fma_half(unsigned short a, unsigned short b, float c) {
+    float r;
+    asm("fma.rn.f32.f16 %0, %1, %2, %3;" : "=f"(r) : "h"(a), "h"(b), "f"(c));
+    return r;
+}
+__device__ __forceinline__ uint32_t dq_pack(float lo, float hi) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
+}
+__device__ __forceinline__ uint32_t dq_hfma2(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+// (a & b) | c
+__device__ __forceinline__ uint32_t dq_and_or(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
+    return r;
+}
+// codes in bytes J, J + 1 of `codes` -> f16x2 of s * (128 + q) + c
+template <int J> __device__ __forceinline__ uint32_t dq_fma2(uint32_t codes, uint64_t s2, uint64_t c2) {
     const uint32_t a = dq_prmt(codes, 0x43000000u, 0x7044u + (J << 8)), b = dq_prmt(codes, 0x43000000u, 0x7044u + ((J + 1) << 8));
     uint64_t v;
     uint32_t lo, hi, r;
     asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(a), "r"(b));
-    if constexpr (!BIASED) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(v) : "l"(0xC3000000C3000000ull));  // - 128
     asm("fma.rn.f32x2 %0, %0, %1, %2;" : "+l"(v) : "l"(s2), "l"(c2));
     asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(v));
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(__uint_as_float(hi)), "f"(__uint_as_float(lo)));
     return r;
 }
-template <bool BIASED> __device__ __forceinline__ uint4 dq_chunk_fma(uint32_t w0, uint32_t w1, uint64_t s2, uint64_t c2) {
-    return make_uint4(dq_fma2<0, BIASED>(w0, s2, c2), dq_fma2<2, BIASED>(w0, s2, c2), dq_fma2<0, BIASED>(w1, s2, c2), dq_fma2<2, BIASED>(w1, s2, c2));
-}
+__device__ __forceinline__ uint4 dq_chunk_fma(uint32_t w0, uint32_t w1, uint64_t s2, uint64_t c2) { return make_uint4(dq_fma2<0>(w0, s2, c2), dq_fma2<2>(w0, s2, c2), dq_fma2<0>(w1, s2, c2), dq_fma2<2>(w1, s2, c2)); }
 // unsigned bytes -> f16 (byte - bias) * d; bias2 = f16x2 of 1024 + bias, d2 = f16x2 of d
 __device__ __forceinline__ uint4 dq_chunk_mul(uint32_t w0, uint32_t w1, uint32_t bias2, uint32_t d2) {
     uint4 r;
@@ -79,37 +107,16 @@ __device__ __forceinline__ uint32_t dq_lds32(uint32_t addr) {
     return v;
 }
 
-// (d sc, -dmin m) of scale groups 2 kb and 2 kb + 1 of a K-quant super-block header; kb is warp-uniform
-__device__ __forceinline__ void dq_kscale(const uint4 &hdr, int kb, float (&s)[2], float (&c)[2]) {
-    const __half2 dd = u32_as_h2(hdr.x);
-    const float d = __low2float(dd), dmin = __high2float(dd);
-    uint32_t scw, mnw;  // the four groups of this half as bytes
-    if (kb < 2) {
-        scw = hdr.y & 0x3F3F3F3Fu;
-        mnw = hdr.z & 0x3F3F3F3Fu;
-    } else {
-        scw = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
-        mnw = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
-    }
-    if (kb & 1) {
-        scw >>= 16;
-        mnw >>= 16;
-    }
-#pragma unroll
-    for (int n = 0; n < 2; ++n) {
-        s[n] = __fmul_rn(d, (float)((scw >> (8 * n)) & 0xFFu));
-        c[n] = -__fmul_rn(dmin, (float)((mnw >> (8 * n)) & 0xFFu));
-    }
-}
-
 template <uint32_t TYPE> struct DqBlock;
 
 template <bool Q5> struct DqBlockK {
     uint4 q[2];          // the k-block's 32 quant bytes
     uint4 hb[Q5 ? 2 : 1];  // Q5_K: the high-bit bytes
-    float s[2], c[2];
+    uint32_t sc;         // f16x2: 6-bit scales of groups 2 kb and 2 kb + 1
+    unsigned short d;    // f16
+    float c[2];          // -dmin m of the two groups
     int g;
-    __device__ __forceinline__ void load(uint32_t unit, int kb) {
+    __device__ __forceinline__ void load(uint32_t unit, int kb) {  // kb is warp-uniform
         const uint4 hdr = dq_lds128(unit);
         const uint32_t qs = unit + (Q5 ? 48 : 16) + 32 * kb;
         q[0] = dq_lds128(qs);
@@ -119,31 +126,62 @@ template <bool Q5> struct DqBlockK {
             hb[1] = dq_lds128(unit + 32);
         }
         g = 2 * kb;
-        dq_kscale(hdr, kb, s, c);
+        uint32_t scw, mnw;  // the four groups of this half as bytes
+        if (kb < 2) {
+            scw = hdr.y & 0x3F3F3F3Fu;
+            mnw = hdr.z & 0x3F3F3F3Fu;
+        } else {
+            scw = (hdr.w & 0x0F0F0F0Fu) | ((hdr.y >> 2) & 0x30303030u);
+            mnw = ((hdr.w >> 4) & 0x0F0F0F0Fu) | ((hdr.z >> 2) & 0x30303030u);
+        }
+        const uint32_t pick = (kb & 1) ? 0x4342u : 0x4140u;  // bytes -> f16 1024 + byte
+        sc = hsub2_u32(dq_prmt(scw, 0x64646464u, pick), 0x64006400u);
+        const uint32_t mn = hsub2_u32(dq_prmt(mnw, 0x64646464u, pick), 0x64006400u);
+        d = (unsigned short)(hdr.x & 0xFFFFu);
+        const unsigned short minus_dmin = (unsigned short)((hdr.x >> 16) ^ 0x8000u);
+        c[0] = dq_fma_half(minus_dmin, (unsigned short)(mn & 0xFFFFu), -0.0f);
+        c[1] = dq_fma_half(minus_dmin, (unsigned short)(mn >> 16), -0.0f);
     }
     __device__ __forceinline__ uint32_t mix() const {
         uint32_t m = q[0].x ^ q[0].y ^ q[0].z ^ q[0].w ^ q[1].x ^ q[1].y ^ q[1].z ^ q[1].w ^ __float_as_uint(c[0]);
         if constexpr (Q5) m ^= hb[0].x ^ hb[0].y ^ hb[0].z ^ hb[0].w ^ hb[1].x ^ hb[1].y ^ hb[1].z ^ hb[1].w;
         return m;
     }
+    // f16x2 operands of columns (0, 1) and (2, 3) from the f16x2 codes of columns (0, 2) and (1, 3), biased by 1024
+    __device__ __forceinline__ uint2 four(uint32_t even, uint32_t odd, uint32_t s2, uint32_t k2, float cn) const {
+        float v0, v1, v2, v3;
+        dq_fma_halves(dq_hfma2(even, s2, k2), d, cn, v0, v2);
+        dq_fma_halves(dq_hfma2(odd, s2, k2), d, cn, v1, v3);
+        return make_uint2(dq_pack(v0, v1), dq_pack(v2, v3));
+    }
     __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
         const uint32_t w[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
 #pragma unroll
         for (int n = 0; n < 2; ++n) {  // low nibbles: group 2 kb, high nibbles: group 2 kb + 1
-            const uint64_t s2 = dq_pair(s[n]), c2 = dq_pair(c[n]);
+            uint32_t s2 = dq_prmt(sc, 0u, n ? 0x3232u : 0x1010u);
+            if (n && !Q5) s2 = hmul2_u32(s2, 0x2C002C00u);  // high nibbles stay in place, as 16 q
+            const uint32_t k2 = hmul2_u32(s2, 0xE400E400u);   // takes the bias 1024 off again
 #pragma unroll
             for (int c8 = 0; c8 < 4; ++c8) {
-                uint32_t m[2];
+                uint2 r[2];
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    m[i] = (n ? (w[2 * c8 + i] >> 4) : w[2 * c8 + i]) & 0x0F0F0F0Fu;
+                    const uint32_t x = w[2 * c8 + i];
+                    uint32_t even, odd;
                     if constexpr (Q5) {  // bit g + n of every high-bits byte -> bit 4 of the code
                         const uint4 &h4 = hb[c8 >> 1];
                         const uint32_t hw = (c8 & 1) ? (i ? h4.w : h4.z) : (i ? h4.y : h4.x);
-                        m[i] |= ((hw >> (g + n)) << 4) & 0x10101010u;
+                        const uint32_t code = ((n ? (x >> 4) : x) & 0x0F0F0F0Fu) | (((hw >> (g + n)) << 4) & 0x10101010u);
+                        even = dq_prmt(code, 0x64646464u, 0x4240u);
+                        odd = dq_prmt(code, 0x64646464u, 0x4341u);
+                    } else {
+                        const uint32_t mask = n ? 0x00F000F0u : 0x000F000Fu;
+                        even = dq_and_or(x, mask, 0x64006400u);
+                        odd = dq_and_or(x >> 8, mask, 0x64006400u);
                     }
+                    r[i] = four(even, odd, s2, k2, c[n]);
                 }
-                dq_store(row_base, sw, 4 * n + c8, dq_chunk_fma<false>(m[0], m[1], s2, c2));
+                dq_store(row_base, sw, 4 * n + c8, make_uint4(r[0].x, r[0].y, r[1].x, r[1].y));
             }
         }
     }
@@ -182,7 +220,7 @@ template <> struct DqBlock<ZQ_Q6_K> {
                 const uint32_t l = (hh ? (lw >> 4) : lw) & 0x0F0F0F0Fu, u = (x2 >= 4 ? (hw >> (x2 - 4)) : (hw << (4 - x2))) & 0x30303030u;
                 m[w] = (l | u) ^ 0x20202020u;
             }
-            dq_store(row_base, sw, c8, dq_chunk_fma<true>(m[0], m[1], s2, c2));
+            dq_store(row_base, sw, c8, dq_chunk_fma(m[0], m[1], s2, c2));
         }
     }
 };
