@@ -278,6 +278,77 @@ __device__ __forceinline__ int tile_cols(const GemmSeg &s) {
     return n > kBN ? kBN : n < 32 ? 32 : n;
 }
 
+// A cut tile whose shares have all arrived.
+struct GemmCut {
+    int row0, tok0, n_tok, c_first, c_last;
+};
+
+// Adds the shares of an SM's half of a cut tile in pair order and stores it: all warps together, once their roles are over.  Reading
+// the shares is a matter of bytes in flight (several times 128 KB per SM at some 1000 cycles of latency): a thread takes four rows of
+// several tokens at a time.  The four epilogue warps alone, 16 columns of one share at a time, took most of the launch where
+// every tile is cut: 17408 -> 5120 in Q4_K YYY
+template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(const GemmParams &p, const GemmCut &t, uint32_t rank) {
+    constexpr int OUT = GATED ? kBM / 2 : kBM, QUADS = OUT / 4, PARTS = GATED ? 2 : 1, LANES = THREADS / QUADS;  // LANES: columns that the CTA takes side by side
+    constexpr int COLS = (THREADS > 256 ? 4 : 16) / PARTS;
+    const int quad = (int)threadIdx.x % QUADS, lane_col = (int)threadIdx.x / QUADS, row = t.row0 + (int)rank * OUT + 4 * quad;
+    const int rows = p.n_out - row < 4 ? p.n_out - row : 4, esz = (int)dtype_size(p.y_dtype);
+    if (rows <= 0 || lane_col >= LANES) return;
+    for (int c0 = lane_col; c0 < t.n_tok; c0 += LANES * COLS) {
+        float4 sum[PARTS][COLS];
+        for (int c = t.c_first; c <= t.c_last; ++c) {
+            const float *share = p.partials + ((size_t)(2 * c + (c == t.c_first ? 1 : 0)) * 2 + rank) * (kBN * kBM) + 4 * quad;
+            float4 v[PARTS][COLS];
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+                for (int k = 0; k < COLS; ++k) {
+                    const int col = c0 + k * LANES;
+                    v[part][k] = col < t.n_tok ? __ldcg(reinterpret_cast<const float4 *>(share + col * kBM + part * OUT)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part)
+#pragma unroll
+                for (int k = 0; k < COLS; ++k) {
+                    const float4 n = v[part][k];
+                    float4 &s = sum[part][k];
+                    s = c == t.c_first ? n : make_float4(s.x + n.x, s.y + n.y, s.z + n.z, s.w + n.w);
+                }
+        }
+#pragma unroll
+        for (int k = 0; k < COLS; ++k) {
+            const int col = c0 + k * LANES;
+            if (col >= t.n_tok) break;
+            const size_t at = (size_t)(t.tok0 + col) * p.n_out + row;
+            float o[4] = {sum[0][k].x, sum[0][k].y, sum[0][k].z, sum[0][k].w};
+            if (GATED) {
+                const float u[4] = {sum[PARTS - 1][k].x, sum[PARTS - 1][k].y, sum[PARTS - 1][k].z, sum[PARTS - 1][k].w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) o[j] = (o[j] / (1.0f + expf(-o[j]))) * u[j];
+            }
+            if (p.residual) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (j < rows) o[j] += load_as_f32(p.residual, p.y_dtype, at + j);
+            }
+            if ((p.n_out & 3) == 0) {  // four whole rows, and y (16-byte aligned) is aligned to them
+                uint8_t *const yb = reinterpret_cast<uint8_t *>(p.y) + at * esz;
+                if (p.y_dtype == ZQ_F32) {
+                    *reinterpret_cast<float4 *>(yb) = make_float4(o[0], o[1], o[2], o[3]);
+                } else if (p.y_dtype == ZQ_F16) {
+                    *reinterpret_cast<uint2 *>(yb) = make_uint2(h2_as_u32(__floats2half2_rn(o[0], o[1])), h2_as_u32(__floats2half2_rn(o[2], o[3])));
+                } else {
+                    const __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+                    *reinterpret_cast<uint2 *>(yb) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    if (j < rows) store_from_f32(p.y, p.y_dtype, at + j, o[j]);
+            }
+        }
+    }
+}
+
 template <uint32_t SRC, bool GATED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
@@ -294,7 +365,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     uint64_t *acc_empty = acc_full + 2;                                // first SM: both SMs' epilogue warps
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_state;
-    __shared__ int s_last;
+    __shared__ GemmCut s_cut[2];  // cut tiles that this SM adds up: a pair's shares touch two at most
+    __shared__ int s_cuts;
 
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;  // the shuffle tells the compiler that it is uniform
     const uint32_t rank = pair_rank();
@@ -319,6 +391,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
         }
         fence_mbar_init();
         s_state = kStateAhead;
+        s_cuts = 0;
         tma_prefetch_desc(&map_w);
         tma_prefetch_desc(&map_x);
         if (GATED) tma_prefetch_desc(&map_w2);
@@ -504,56 +577,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 else store_tile(DtypeTag<ZQ_BF16>());
             }
             if (!whole) {
-                // A share of a cut tile.  Whoever comes last adds the other shares from their slots to its own, in pair order;
-                // everyone else leaves its share in its slot and goes on.
+                // A share of a cut tile goes to its slot; the SM that comes last takes the tile down for the end of the kernel.
                 const long long Q = (long long)p.cut_tiles * walk.steps, G = p.cut_pairs, ts = (long long)sg.tile * walk.steps;
                 const int c_first = (int)(((ts + 1) * G - 1) / Q), c_last = (int)(((ts + walk.steps) * G - 1) / Q);  // pairs that own the tile's first and last step
-                uint32_t *counter = p.counters + 2 * c_first + rank;
-                const uint32_t others = (uint32_t)(c_last - c_first);
-                if (et == 0) s_last = *reinterpret_cast<volatile uint32_t *>(counter) == others;
-                asm volatile("bar.sync 3, 128;" ::: "memory");
-                bool last = s_last != 0;
-                if (!last) {
-                    float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * (kBN * kBM) + q * 32 + lane;
-                    if (ok) {
-                        for (int c0 = 0; c0 < n_tok; c0 += 16) {
-                            uint32_t v[16];
-                            tmem_ld16(acc + c0, v);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) __stcg(slot + (size_t)(c0 + j) * kBM, __uint_as_float(v[j]));
-                        }
-                    }
-                    __threadfence();
-                    asm volatile("bar.sync 3, 128;" ::: "memory");
-                    if (et == 0) s_last = atomicAdd(counter, 1u) == others;
-                    asm volatile("bar.sync 3, 128;" ::: "memory");
-                    last = s_last != 0;
-                }
-                if (last && ok) {
-                    __threadfence();
-                    const float *base = p.partials + (size_t)rank * (kBN * kBM) + q * 32 + lane;
+                float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * (kBN * kBM) + q * 32 + lane;
+                if (ok) {
                     for (int c0 = 0; c0 < n_tok; c0 += 16) {
                         uint32_t v[16];
-                        for (int c = c_first; c <= c_last; ++c) {
-                            if (c == pair) {
-                                uint32_t own[16];
-                                tmem_ld16(acc + c0, own);
+                        tmem_ld16(acc + c0, v);
 #pragma unroll
-                                for (int j = 0; j < 16; ++j) v[j] = c == c_first ? own[j] : __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(own[j]));
-                            } else {
-                                const float *src = base + (size_t)(2 * c + (c == c_first ? 1 : 0)) * 2 * (kBN * kBM) + (size_t)c0 * kBM;
-                                float n[16];
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) n[j] = __ldcg(src + (size_t)j * kBM);
-#pragma unroll
-                                for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(c == c_first ? n[j] : __uint_as_float(v[j]) + n[j]);
-                            }
-                        }
-                        if (p.y_dtype == ZQ_F32) store16(DtypeTag<ZQ_F32>(), c0, v);
-                        else if (p.y_dtype == ZQ_F16) store16(DtypeTag<ZQ_F16>(), c0, v);
-                        else store16(DtypeTag<ZQ_BF16>(), c0, v);
+                        for (int j = 0; j < 16; ++j) __stcg(slot + (size_t)(c0 + j) * kBM, __uint_as_float(v[j]));
                     }
                 }
+                __threadfence();
+                asm volatile("bar.sync 3, 128;" ::: "memory");
+                if (et == 0 && ok && atomicAdd(p.counters + 2 * c_first + rank, 1u) == (uint32_t)(c_last - c_first)) s_cut[s_cuts++] = {sg.row0, sg.tok0, n_tok, c_first, c_last};
             }
             tc_fence_before();
             __syncwarp();
@@ -635,6 +673,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     __syncthreads();
     pair_sync();  // nobody leaves while the other SM may still signal here or read operands
     if (warp == 1) tmem_dealloc2(tmem_base, 512);
+    if (s_cuts) __threadfence();  // behind the arrivals that this SM has seen
+    for (int i = 0; i < s_cuts; ++i) add_up_cut<GATED, S::threads>(p, s_cut[i], rank);
 }
 
 // activations of any supported dtype -> f16; eight values per thread and step (one 16- or 32-byte load, one 16-byte store);
