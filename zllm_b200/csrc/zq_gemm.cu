@@ -19,12 +19,15 @@
 // operand split over the pair both figures fall to two thirds.
 //
 // Tiles are dealt whole to the pairs while there are many; what does not divide is cut along K into equal shares
-// (256-column steps), and the last contributor of a cut tile adds the f32 partials in pair order (deterministic) and
-// stores.  A gated tile is 64 gate and 64 up rows per SM (128 outputs per pair): gate and up of an output meet in the
-// epilogue through shared memory, and the accumulator still fits twice.
+// (256-column steps), and the SM that finishes a cut tile's last share adds the f32 partials in pair order (deterministic) and
+// stores.  A gated tile is 64 gate and 64 up rows per SM (128 outputs per pair), 16 of one and 16 of the other in turn: gate and up of
+// an output meet in one warp of the epilogue, and the accumulator still fits twice.
 //
-// Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..5
-// epilogue; SRC != 0: warp 6 TMA of packed boxes, warps 7..22 dequantisers.
+// Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..9
+// epilogue; SRC != 0: warp 10 TMA of packed boxes, warps 11..26 dequantisers.  Eight epilogue warps and not four, because a tile's epilogue is
+// a chain of some 5 (gated: 50) instructions per element in each, which short tiles (few columns of K) do not hide and which the
+// last tile of a pair shows in full: Q4_K gated 1536 -> 3840 at 256 tokens 95 us, now 26; 4096 -> 11008 at 256 tokens 75 us, now 47 (with the
+// exchange of gate and up inside a warp; before, through shared memory and a barrier per 16 columns).
 // Every wait is bounded, counted from the end of the previous kernel; a wait that runs out sets the CTA's state, all roles fall
 // through to the end, TMEM is released and the context status word reports it.
 #include "zq_gemm_dq.cuh"
@@ -36,6 +39,7 @@ constexpr int kPairM = 256;   // weight rows per pair
 constexpr int kBN = 256;      // most tokens per tile
 constexpr int kBK = 64;       // K elements per ring stage (128 bytes of f16: one swizzle atom row)
 constexpr int kStepK = 256;   // K elements per step: one packed unit, the grain in which tiles are cut
+constexpr int kEpi = 8;       // epilogue warps
 constexpr int kDqWarps = 16;  // thread = (row, k-block of a unit): four warps per k-block
 
 struct GemmParams {
@@ -112,6 +116,9 @@ __device__ __forceinline__ void pair_sync() {
 // fence.proxy.async) or was ordered by a tcgen05 fence (accumulators).  A release at cluster scope drains all of the thread's
 // memory traffic first, which cost more than a k-block's MMAs at every stage.
 __device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
+// Operand row of row r of a gated box (64 gate rows, then 64 up rows): 16 gate rows and the 16 up rows of the same outputs alternate, so
+// that they meet in one epilogue warp.
+__device__ __forceinline__ int gated_row(int r) { return ((r & 63) >> 4) * 32 + (r >> 6) * 16 + (r & 15); }
 // Loads into this SM's shared memory whose completion counts on a barrier of the pair's first SM.  No multicast.
 __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t cluster_bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)),
@@ -183,20 +190,6 @@ template <int DT> __device__ __forceinline__ float raw_as_f32(uint32_t r) {
     else return __uint_as_float(r << 16);
 }
 
-// AND over the four epilogue warps (named barrier 3)
-__device__ __forceinline__ bool epilogue_all(bool v) {
-    uint32_t r;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\t"
-        "setp.ne.u32 q, %1, 0;\n\t"
-        "barrier.cta.red.and.pred p, 3, 128, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(r)
-        : "r"((uint32_t)v)
-        : "memory");
-    return r != 0;
-}
-
 // Shared-memory plan: 32 KB per ring stage (16 KB of weights, 16 KB of tokens), as many as fit beside the packed boxes.
 template <uint32_t SRC> struct GemmSmem {
     static constexpr int unit_bytes = SRC == ZQ_Q8_0 ? 272 : SRC == ZQ_Q6_K ? 224 : SRC == ZQ_Q5_K ? 176 : 144;
@@ -207,13 +200,11 @@ template <uint32_t SRC> struct GemmSmem {
     static constexpr int pstages = SRC == 0 ? 0 : unit_bytes <= 144 ? 3 : 2;
     static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 ? 4 : 5;
     static constexpr int off_p = stages * stage_bytes;
-    static constexpr int off_x = off_p + pstages * p_bytes;  // gate / up exchange of the gated epilogue
-    static constexpr int x_bytes = 2 * 2 * 16 * 32 * 4;      // 2 row halves x 2 buffers x 16 columns x 32 rows
-    static constexpr int off_bar = off_x + x_bytes;
+    static constexpr int off_bar = off_p + pstages * p_bytes;
     static constexpr int total = off_bar + 256 + 1024;       // barriers, slack for 1024-byte alignment
-    static constexpr int threads = (SRC ? 7 + kDqWarps : 6) * 32;
+    static constexpr int threads = (2 + kEpi + (SRC ? 1 + kDqWarps : 0)) * 32;
     static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
-    static_assert(off_p % 1024 == 0 && off_x % 16 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
+    static_assert(off_p % 1024 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
 };
 
 constexpr int kTokGroup = 8;  // token tiles per raster group: a weight tile is reused by 8 token tiles while it is hot in L2
@@ -286,24 +277,25 @@ struct GemmCut {
 // Adds the shares of an SM's half of a cut tile in pair order and stores it: all warps together, once their roles are over.  Reading
 // the shares is a matter of bytes in flight (several times 128 KB per SM at some 1000 cycles of latency): a thread takes four rows of
 // several tokens at a time.  The four epilogue warps alone, 16 columns of one share at a time, took most of the launch where
-// every tile is cut: 17408 -> 5120 in Q4_K YYY
+// every tile is cut: 17408 -> 5120 in Q4_K, 48 / 256 / 512 tokens 40 / 88 / 89 us, now 32 / 47 / 75.
 template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(const GemmParams &p, const GemmCut &t, uint32_t rank) {
     constexpr int OUT = GATED ? kBM / 2 : kBM, QUADS = OUT / 4, PARTS = GATED ? 2 : 1, LANES = THREADS / QUADS;  // LANES: columns that the CTA takes side by side
     constexpr int COLS = (THREADS > 256 ? 4 : 16) / PARTS;
     const int quad = (int)threadIdx.x % QUADS, lane_col = (int)threadIdx.x / QUADS, row = t.row0 + (int)rank * OUT + 4 * quad;
+    const int at0 = GATED ? gated_row(4 * quad) : 4 * quad;  // operand row; gated: of gate, up lies 16 rows on
     const int rows = p.n_out - row < 4 ? p.n_out - row : 4, esz = (int)dtype_size(p.y_dtype);
     if (rows <= 0 || lane_col >= LANES) return;
     for (int c0 = lane_col; c0 < t.n_tok; c0 += LANES * COLS) {
         float4 sum[PARTS][COLS];
         for (int c = t.c_first; c <= t.c_last; ++c) {
-            const float *share = p.partials + ((size_t)(2 * c + (c == t.c_first ? 1 : 0)) * 2 + rank) * (kBN * kBM) + 4 * quad;
+            const float *share = p.partials + ((size_t)(2 * c + (c == t.c_first ? 1 : 0)) * 2 + rank) * (kBN * kBM) + at0;
             float4 v[PARTS][COLS];
 #pragma unroll
             for (int part = 0; part < PARTS; ++part)
 #pragma unroll
                 for (int k = 0; k < COLS; ++k) {
                     const int col = c0 + k * LANES;
-                    v[part][k] = col < t.n_tok ? __ldcg(reinterpret_cast<const float4 *>(share + col * kBM + part * OUT)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[part][k] = col < t.n_tok ? __ldcg(reinterpret_cast<const float4 *>(share + col * kBM + part * 16)) : make_float4(0.f, 0.f, 0.f, 0.f);
                 }
 #pragma unroll
             for (int part = 0; part < PARTS; ++part)
@@ -355,6 +347,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     using S = GemmSmem<SRC>;
     constexpr int STAGES = S::stages, PST = S::pstages > 0 ? S::pstages : 1;
     constexpr int kRows = GATED ? kPairM / 2 : kPairM;  // output rows of a tile
+    constexpr int kPackedWarp = 2 + kEpi;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::off_bar);  // first SM: a stage's operands, both SMs' bytes and dequantiser warps
@@ -387,7 +380,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 8);
+            mbar_init(&acc_empty[b], 2 * kEpi);
         }
         fence_mbar_init();
         s_state = kStateAhead;
@@ -410,9 +403,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     // Programmatic dependent launch: everything up to here, and for packed dense weights (constants) also their first boxes and
     // their dequantisation, runs under the previous kernel's end; activations, f16 operands, work lists, results and partials
     // belong to earlier kernels until they complete.  5120 x 17408 up and down in Q4_K: 48 tokens 76 -> 65 us, 512 tokens 192 -> 188 us.
-    // The warps that run ahead (6 and up) wait for stages that only the MMAs set free, but these waits count from the end of the
+    // The warps that run ahead (packed boxes, dequantisers) wait for stages that only the MMAs set free, but these waits count from the end of the
     // previous kernel (kStateAhead), which may itself wait for another rank for longer than any bound here.
-    if (SRC == 0 || p.items || warp < 6) pdl_wait_prior_grid();
+    if (SRC == 0 || p.items || warp < kPackedWarp) pdl_wait_prior_grid();
     if (threadIdx.x == 0) *reinterpret_cast<volatile uint32_t *>(&s_state) = kStateRun;  // nobody gives up before this
     __syncwarp();
     GemmWalk walk(p, pair, pairs, kRows);
@@ -438,12 +431,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     const uint32_t bar = pair_first(smem_u32(&full[s]));
                     if (rank == 0) mbar_expect_tx(&full[s], bytes);
                     if constexpr (SRC == 0) {
-                        if (p.items) {
-                            tma_load_3d_pair(st, &map_w, bar, kb * kBK, row, sg.z);
-                            if (GATED) tma_load_3d_pair(st + S::a_bytes / 2, &map_w2, bar, kb * kBK, row, sg.z);
-                        } else {
-                            tma_load_2d_pair(st, &map_w, bar, kb * kBK, row);
-                            if (GATED) tma_load_2d_pair(st + S::a_bytes / 2, &map_w2, bar, kb * kBK, row);
+#pragma unroll
+                        for (int h = 0; h < (GATED ? 8 : 1); ++h) {  // gated: 16 rows of gate, 16 of up, and so on
+                            const CUtensorMap *m = GATED && (h & 1) ? &map_w2 : &map_w;
+                            if (p.items) tma_load_3d_pair(st + h * (S::a_bytes / 8), m, bar, kb * kBK, row + (h >> 1) * 16, sg.z);
+                            else tma_load_2d_pair(st + h * (S::a_bytes / 8), m, bar, kb * kBK, row + (h >> 1) * 16);
                         }
                     }
                     tma_load_2d_pair(st + S::a_bytes, &map_x, bar, kb * kBK, tok);
@@ -492,10 +484,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 }
             }
         }
-    } else if (warp < 6) {
-        // ------------------------------------------------ epilogue: warp q of 4 owns TMEM lanes 32q..32q+31 = the SM's operand rows
-        const int q = warp & 3;
-        float *xch = reinterpret_cast<float *>(smem + S::off_x) + (q & 1) * (2 * 16 * 32);
+    } else if (warp < kPackedWarp) {
+        // ------------------------------------------------ epilogue: a warp owns TMEM lanes 32 q .. 32 q + 31 = those operand rows of the SM, and
+        // every second group of 16 columns
+        const int q = warp & 3, part = (warp - 2) >> 2;
         int iter = 0;
         const int et = (warp - 2) * 32 + lane;
         for (; walk.next(p, sg); ++iter) {
@@ -505,18 +497,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 // bring the tile's residual rows into L2 while its MMAs run: a warp can only have a few KB of loads in flight below
                 const size_t esz = dtype_size(p.y_dtype), r0 = (size_t)sg.row0 + rank * kBM;
                 const size_t bytes = (size_t)p.n_out * esz;
-                for (int i = et; i < n_tok * (int)esz; i += 128) {  // 128 rows = esz lines of 128 bytes per token
+                for (int i = et; i < n_tok * (int)esz; i += 32 * kEpi) {  // 128 rows = esz lines of 128 bytes per token
                     const size_t at = r0 * esz + (size_t)(i % (int)esz) * 128;
                     if (at < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(p.residual) + (size_t)(sg.tok0 + i / (int)esz) * bytes + at));
                 }
             }
-            // the four warps go on together or not at all: they meet at barriers below (and the exchange buffer is free again)
-            const bool ok = epilogue_all(wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0));
+            const bool ok = wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0);
             tc_fence_after();
             const uint32_t acc = tmem_base + (uint32_t)b * kBN + ((uint32_t)(q * 32) << 16);
             const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
-            // output row of this lane; gated: warps 0, 1 hold gate rows, warps 2, 3 the up rows of the same outputs
-            const int row = GATED ? sg.row0 + (int)rank * 64 + (q & 1) * 32 + lane : sg.row0 + (int)rank * kBM + q * 32 + lane;
+            // output row of this lane; gated: lanes 0..15 hold gate rows, lanes 16..31 the up rows of the same outputs
+            const int row = GATED ? sg.row0 + (int)rank * 64 + q * 16 + (lane & 15) : sg.row0 + (int)rank * kBM + q * 32 + lane;
             // 16 columns of finished sums (f32 bits) -> y.  With the output type known at compile time and one wide multiply-add per address
             // an element takes about 4 instructions.
             auto store16 = [&](auto dt, int c0, uint32_t (&v)[16]) {
@@ -525,21 +516,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 uint8_t *const yb = reinterpret_cast<uint8_t *>(p.y) + at;
                 auto token = [&](int j) { return (uint64_t)(uint32_t)p.n_out * (uint32_t)(j * (int)dtype_size(DT)); };  // bytes from one token's row to the j-th after it
                 if (GATED) {
-                    // the two warps of one row half trade: the gate warp finishes columns 0..7 of the chunk, the up warp 8..15
-                    float *xb = xch + ((c0 >> 4) & 1) * (16 * 32);  // [which half travels][8 columns][32 rows]; rewritten two chunks later, behind the barrier in between
-                    const bool is_up = q >= 2;
+                    // the two lanes of an output trade: the gate lane finishes columns 0..7 of the group, the up lane 8..15
+                    const bool is_up = lane >= 16;
+                    float g[8], u[8];
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) xb[((is_up ? 0 : 8) + j) * 32 + lane] = __uint_as_float(is_up ? v[j] : v[8 + j]);
-                    asm volatile("bar.sync %0, 64;" ::"r"(1 + (q & 1)) : "memory");
+                    for (int j = 0; j < 8; ++j) {
+                        const uint32_t mine = is_up ? v[8 + j] : v[j], other = __shfl_xor_sync(0xffffffffu, is_up ? v[j] : v[8 + j], 16);
+                        g[j] = __uint_as_float(is_up ? other : mine);
+                        u[j] = __uint_as_float(is_up ? mine : other);
+                    }
                     if (row >= p.n_out) return;
                     const int cb = is_up ? 8 : 0, left = n_tok - c0 - cb;
                     uint8_t *const yc = yb + token(cb);
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) {
-                        const float other = xb[(cb + j) * 32 + lane], mine = __uint_as_float(is_up ? v[8 + j] : v[j]);
-                        const float g = is_up ? other : mine, u = is_up ? mine : other;
-                        v[j] = __float_as_uint((g / (1.0f + expf(-g))) * u);  // src/kernel/cpu/ggml_quant.rs:352
-                    }
+                    for (int j = 0; j < 8; ++j) v[j] = __float_as_uint((g[j] / (1.0f + expf(-g[j]))) * u[j]);  // src/kernel/cpu/ggml_quant.rs:352
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
                         if (j < left) store_as<DT>(yc + token(j), v[j]);
@@ -565,7 +555,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 }
             };
             auto store_tile = [&](auto dt) {
-                for (int c0 = 0; c0 < n_tok; c0 += 16) {  // warp-uniform
+                for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {  // warp-uniform
                     uint32_t v[16];
                     tmem_ld16(acc + c0, v);
                     store16(dt, c0, v);
@@ -582,7 +572,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 const int c_first = (int)(((ts + 1) * G - 1) / Q), c_last = (int)(((ts + walk.steps) * G - 1) / Q);  // pairs that own the tile's first and last step
                 float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * (kBN * kBM) + q * 32 + lane;
                 if (ok) {
-                    for (int c0 = 0; c0 < n_tok; c0 += 16) {
+                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {
                         uint32_t v[16];
                         tmem_ld16(acc + c0, v);
 #pragma unroll
@@ -590,7 +580,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                     }
                 }
                 __threadfence();
-                asm volatile("bar.sync 3, 128;" ::: "memory");
+                asm volatile("bar.sync 3, %0;" ::"n"(32 * kEpi) : "memory");
                 if (et == 0 && ok && atomicAdd(p.counters + 2 * c_first + rank, 1u) == (uint32_t)(c_last - c_first)) s_cut[s_cuts++] = {sg.row0, sg.tok0, n_tok, c_first, c_last};
             }
             tc_fence_before();
@@ -598,7 +588,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             if (lane == 0) pair_arrive(pair_first(smem_u32(&acc_empty[b])));  // this warp's part of the accumulator may be overwritten
         }
     } else if constexpr (SRC != 0) {
-        if (warp == 6) {
+        if (warp == kPackedWarp) {
             // ------------------------------------------------ TMA: packed boxes (one unit of every row) on a ring of their own
             int ps = 0;
             uint32_t pph = 0;
@@ -628,9 +618,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             }
         } else {
             // ------------------------------------------------ dequantisers: thread = (row, k-block of the unit)
-            const int t = threadIdx.x - 7 * 32, row = t & (kBM - 1), mine = t >> 7;  // mine: warp-uniform
-            const int sw = row & 7;
-            const uint32_t row0 = smem_u32(smem) + (uint32_t)((row >> 3) * 1024 + sw * 128), box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
+            const int t = threadIdx.x - (kPackedWarp + 1) * 32, row = t & (kBM - 1), mine = t >> 7;  // row of the box; mine: warp-uniform
+            const int a_row = GATED ? gated_row(row) : row, sw = a_row & 7;
+            const uint32_t row0 = smem_u32(smem) + (uint32_t)((a_row >> 3) * 1024 + sw * 128), box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
             int s = 0, ps = 0;  // ring positions: s walks the k-blocks of all warps, this warp serves one in four
             uint32_t ph = 0, pph = 0;
             bool ok = true, fresh = true;
@@ -880,8 +870,8 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
     if (rc) return rc;
     CUtensorMap map_w, map_w2;
-    rc = make_f16_map(w16, n, k, gated ? 64 : kBM, &map_w, err);
-    if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, gated ? 64 : kBM, &map_w2, err);
+    rc = make_f16_map(w16, n, k, gated ? 16 : kBM, &map_w, err);
+    if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, gated ? 16 : kBM, &map_w2, err);
     if (rc) return rc;
     return launch_src(ctx, 0, gated, map_w, map_w2, map_x, p, pairs, err);
 }
@@ -910,8 +900,8 @@ int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t m
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "grouped GEMM needs columns aligned to 8, got %zu", k);
     const bool gated = w2 != nullptr;
     CUtensorMap map_w, map_w2, map_x;
-    int rc = make_f16_map3(w, mats, rows, k, gated ? 64 : kBM, &map_w, err);
-    if (!rc) rc = make_f16_map3(gated ? w2 : w, mats, rows, k, gated ? 64 : kBM, &map_w2, err);
+    int rc = make_f16_map3(w, mats, rows, k, gated ? 16 : kBM, &map_w, err);
+    if (!rc) rc = make_f16_map3(gated ? w2 : w, mats, rows, k, gated ? 16 : kBM, &map_w2, err);
     if (!rc) rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
     if (rc) return rc;
     GemmParams p;
