@@ -126,6 +126,33 @@ def test_prefill_tiles_and_shares(tensor_type, m, rows, cols):
     assert H.max_rel_error(got[sel], want) <= BOUND
 
 
+@pytest.mark.parametrize("tensor_type,m,rows,cols,gated,dtype", [
+    (H.Q4_K, 40, 2100, 3072, False, torch.float32), (H.Q5_K, 40, 2100, 3072, False, torch.bfloat16), (H.Q6_K, 40, 2100, 3072, False, torch.float16),
+    (H.Q4_0, 40, 2100, 3072, False, torch.float32), (H.IQ4_NL, 40, 2100, 3072, False, torch.bfloat16), (H.Q8_0, 40, 2100, 3072, False, torch.float16),
+    (H.Q4_K, 300, 333, 8192, False, torch.float16),   # two token tiles, rows that are no multiple of 4
+    (H.Q4_K, 256, 511, 8192, False, torch.float32),   # whole 256-token tiles
+    (H.Q4_K, 40, 43520, 3072, False, torch.float32),  # 170 tiles: 96 of them cut, 74 whole
+    (H.Q4_K, 70, 700, 3072, True, torch.float32), (H.Q8_0, 256, 77, 8192, True, torch.float16), (H.IQ4_NL, 33, 1030, 4096, True, torch.bfloat16),
+])
+def test_prefill_cut_tiles(tensor_type, m, rows, cols, gated, dtype):
+    """Long rows and few tiles: cut along K and added up at the end, with residual, every output type, ragged rows and tokens.
+    Bounds as in the tests around this one, plus the rounding of a 16-bit output (2^-9 bf16, 2^-12 f16)."""
+    ws = [H.random_weight(tensor_type, rows, cols, seed=m + rows + i) for i in range(2 if gated else 1)]
+    x = dev(np.random.default_rng(m).standard_normal((m, cols)).astype(np.float32), torch.float16)
+    wd = [ctx().prepare_weight(tensor_type, w, rows, cols) for w in ws]
+    sel = np.unique(np.concatenate([np.random.default_rng(m + 2).choice(m, size=min(m, 7), replace=False), [0, m - 1]]))
+    xs = x.float().cpu().numpy()[sel]
+    rounding = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    if gated:
+        got = host(ctx().gated_linear(x, *wd, out_dtype=dtype).float())
+        assert H.max_rel_error(got[sel], orc.gated_linear(tensor_type, *ws, rows, cols, xs)) <= 2.1 * BOUND + rounding
+        return
+    r = dev(np.random.default_rng(m + 1).standard_normal((m, rows)).astype(np.float32), dtype)
+    got = host(ctx().linear(x, wd[0], out_dtype=dtype, residual=r).float())
+    want = orc.linear(tensor_type, ws[0], rows, cols, xs) + r.float().cpu().numpy()[sel]
+    assert H.max_rel_error(got[sel], want) <= BOUND + rounding
+
+
 @pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0])
 @pytest.mark.parametrize("m,rows,cols", [(31, 63, 512), (260, 130, 1024)])
 def test_prefill_gated_edges(tensor_type, m, rows, cols):

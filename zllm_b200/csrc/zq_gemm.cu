@@ -30,6 +30,8 @@
 // exchange of gate and up inside a warp; before, through shared memory and a barrier per 16 columns).
 // Every wait is bounded, counted from the end of the previous kernel; a wait that runs out sets the CTA's state, all roles fall
 // through to the end, TMEM is released and the context status word reports it.
+#include <algorithm>
+
 #include "zq_gemm_dq.cuh"
 
 namespace zq {
@@ -786,22 +788,31 @@ static void plan_tokens(size_t m, GemmParams &p) {
     p.box_tok = p.bn / 2;
 }
 
-// How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; where that leaves more than a fifth of the
-// rounds empty, the tiles beyond the full rounds and one round more are cut into equal shares instead (all of them when
-// there are fewer than two rounds).  A share costs its f32 partial (128 KB per SM at 256 tokens) out and in, so a share is at
-// least two steps and a tile at most eight shares.
-static int plan_cut(const zq_ctx *ctx, int tiles, int steps, GemmParams &p) {
+// How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; cut, the tiles beyond the full rounds and one
+// round more (all of them when there are fewer than two rounds) take equal shares of at least two steps, at most eight of a tile.
+// Cutting saves the steps that the busiest pair is ahead of the average one, at 0.85 us (a dequantised step of up to 152 tokens) or 5.6 ns
+// per token each; it costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the
+// addition by all warps takes the place of an epilogue that eight of them compute).  From operands in memory it also costs what the pairs
+// then read at different depths of K and no longer share in L2: three times as much, and nothing is cut past L2's size.  Of 127
+// random shapes of 17 to 1024 tokens (256 to 20000 rows, 512 to 17408 columns, three types, plain and gated) the rule is 1.5 % behind the
+// better choice on average, never cutting 15 %, always 12 %.  Whole and cut, us:
+//   Q4_K 5120 -> 5120, 64 tokens 23.5 / 18.0;  11008 -> 4096, 300 tokens 67.5 / 48.6;  2048 -> 8192, 700 tokens 29.4 / 34.3;  5120 -> 17408, 512 tokens 64.8 / 74.3
+//   operands in memory: 16896 -> 576, 1900 tokens 113 / 87;  15360 -> 3840, 3001 tokens 345 / 431
+static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool gated, size_t operand_bytes, GemmParams &p) {
     const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
-    const int rounds = (tiles + pairs - 1) / pairs;
+    const int rounds = (tiles + pairs - 1) / pairs, whole = tiles < pairs ? tiles : pairs;
     p.cut_tiles = p.cut_pairs = 0;
-    if (5 * tiles >= 4 * rounds * pairs || steps < 2) return tiles < pairs ? tiles : pairs;
-    const int full = tiles / pairs;
-    p.cut_tiles = full >= 2 ? tiles - (full - 1) * pairs : tiles;
-    long long shares = (long long)p.cut_tiles * steps / 2;
-    if (shares > 8LL * p.cut_tiles) shares = 8LL * p.cut_tiles;
-    p.cut_pairs = shares < pairs ? (int)shares : pairs;
-    if (p.cut_tiles < tiles) p.cut_pairs = pairs;
-    return p.cut_pairs;
+    if (steps < 2 || tiles % pairs == 0 || (!fused && operand_bytes > (size_t(128) << 20))) return whole;
+    const int full = tiles / pairs, cut = full >= 2 ? tiles - (full - 1) * pairs : tiles;
+    long long shares = (long long)cut * steps / 2;
+    if (shares > 8LL * cut) shares = 8LL * cut;
+    const int cut_pairs = shares < pairs && cut == tiles ? (int)shares : pairs;
+    const long long saved = (long long)(rounds - (tiles - cut) / pairs) * steps - ((long long)cut * steps + cut_pairs - 1) / cut_pairs;
+    const long long step_ns = std::max(fused ? 850LL : 500LL, 56LL * p.bn / 10), cost_ns = 3000 + (fused ? (gated ? 30LL : 50LL) : 160LL) * p.bn;
+    if (saved * step_ns <= cost_ns) return whole;
+    p.cut_tiles = cut;
+    p.cut_pairs = cut_pairs;
+    return cut_pairs;
 }
 // Shares and their counters are scratch of the launch and not context memory: the short prefill of f16 rows needs no other, so that
 // it may be captured first, replayed after any later call and run on two streams at once, and no call needs a larger workspace
@@ -843,7 +854,7 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     const int rows_per_tile = gated ? kPairM / 2 : kPairM;
     const size_t tiles = ((n + rows_per_tile - 1) / rows_per_tile) * ((m + p.bn - 1) / p.bn);
     if (tiles > (size_t)INT32_MAX / 4) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM: %zu rows x %zu tokens are too many for one call", n, m);
-    const int pairs = plan_cut(ctx, (int)tiles, (int)((k + kStepK - 1) / kStepK), p);
+    const int pairs = plan_cut(ctx, (int)tiles, (int)((k + kStepK - 1) / kStepK), fused, gated, ((gated ? 2 : 1) * n + m) * k * 2, p);
     const size_t w_bytes = fused ? 0 : (n * k * 2 + 1023) & ~size_t(1023);
     const size_t x_bytes = x_dtype == ZQ_F16 ? 0 : (m * k * 2 + 1023) & ~size_t(1023);
     int rc = ensure_workspace(ctx, (gated ? 2 : 1) * w_bytes + x_bytes, err);
