@@ -245,6 +245,29 @@ def test_q4_k_encoder_at_rounding_ties_and_unaligned_buffers(rows, cols, kind, o
     assert np.array_equal(out.cpu().numpy(), np.asarray(orc.encode_q4_k(v)).reshape(-1))
 
 
+@pytest.mark.parametrize("blocks", [1, 3, 4, 5, 4 * 8 * 148 * 3 + 7])  # a warp's tile of four super-blocks, more than one turn of the grid
+@pytest.mark.parametrize("spread", [0.0, 2.0, 7.0])  # decades between the groups of a super-block
+def test_q4_k_encoder_with_groups_of_very_different_size(blocks, spread):
+    """Byte-for-byte: a group beside one a million times its size has a minimum rounded far past its own scale, or no
+    scale at all; every number of super-blocks a warp can be left with."""
+    import ctypes as C
+
+    from zllm_b200 import ffi
+
+    rng = np.random.default_rng(blocks + int(spread))
+    size = 10.0 ** rng.uniform(-spread, 0.0, (blocks, 8, 1))
+    v = (size * (rng.standard_normal((blocks, 8, 32)) + rng.choice([0.0, -9.0, 9.0], (blocks, 8, 1)))).astype(np.float32)
+    if blocks > 64:
+        v[8:] = v[rng.integers(0, 8, blocks - 8)]  # few distinct super-blocks: the CPU encoder sees eight
+    out = torch.empty(blocks * 144, dtype=torch.uint8, device="cuda")
+    src = torch.from_numpy(v.reshape(-1)).cuda()
+    ffi.call("zq_quantize", ctx().handle, H.Q4_K, C.c_void_p(src.data_ptr()), blocks, 256, C.c_void_p(out.data_ptr()), out.numel())
+    ctx().sync()
+    _, first, inverse = np.unique(v.reshape(blocks, -1), axis=0, return_index=True, return_inverse=True)
+    want = np.asarray(orc.encode_q4_k(v.reshape(blocks, -1)[first])).reshape(-1, 144)[inverse.reshape(-1)]
+    assert np.array_equal(out.cpu().numpy().reshape(-1, 144), want)
+
+
 @pytest.mark.parametrize("tensor_type", [H.Q8_0, H.Q4_0, H.IQ4_NL, H.Q4_K, H.Q5_K, H.Q6_K, H.Q5_0])
 @pytest.mark.parametrize("cols", [256, 1024 - 96, 2048 + 128])  # whole units; a tail of 160 columns; a tail of half a unit
 def test_f32_rows_are_written_in_whole_and_ragged_units(tensor_type, cols):

@@ -493,6 +493,8 @@ __device__ __forceinline__ void q4k_codes(const float (&v)[32], float scale, flo
 // form 78 us, 5.2 TB/s).  Values arrive coalesced by cp.async, two tiles of 4 KB per warp in flight, at the chunk position
 // c ^ (group & 7), which keeps both the arriving 16-byte chunks and a lane's reads of its own 128 bytes free of bank conflicts.
 // VEC: values and blocks are 16-byte aligned (a block is 144 bytes, so every block then is).
+// Super-blocks are taken from the last to the first: what wrote the values (a dequantisation, usually) wrote the last of them last, and
+// some of those need not come back from HBM.  17408 x 5120 (356 MB of values) behind a dequantisation: 150.9 us for both, now 148.2.
 constexpr int kEncWarps = 8, kEncTile = 4 * 1024;  // warps per CTA; bytes of a warp's tile (four super-blocks of f32)
 constexpr int kEncSmem = kEncWarps * 2 * kEncTile;
 template <bool VEC>
@@ -500,7 +502,7 @@ __global__ void __launch_bounds__(kEncWarps * 32) quantize_q4_k_kernel(const flo
     extern __shared__ __align__(128) uint8_t enc_smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane & 7;
     const uint32_t tiles = smem_u32(enc_smem) + (uint32_t)(warp * 2 * kEncTile);
-    const size_t step = (size_t)gridDim.x * kEncWarps * 4;
+    const size_t step = (size_t)gridDim.x * kEncWarps * 4, end = (blocks + 3) & ~size_t(3);
     auto fetch = [&](size_t b0, uint32_t tile) {  // super-blocks b0 .. b0 + 3 of this warp
 #pragma unroll
         for (int i = 0; i < 8; ++i) {  // 16-byte chunk i * 32 + lane: chunk lane & 7 of group 4 i + lane / 8
@@ -514,10 +516,11 @@ __global__ void __launch_bounds__(kEncWarps * 32) quantize_q4_k_kernel(const flo
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    size_t b0 = ((size_t)blockIdx.x * kEncWarps + warp) * 4;
-    if (b0 < blocks) fetch(b0, tiles);
-    for (int buf = 0; b0 < blocks; b0 += step, buf ^= 1) {  // warp-uniform
-        if (b0 + step < blocks) fetch(b0 + step, tiles + (uint32_t)((buf ^ 1) * kEncTile));
+    size_t turn = ((size_t)blockIdx.x * kEncWarps + warp) * 4;
+    if (turn < end) fetch(end - 4 - turn, tiles);
+    for (int buf = 0; turn < end; turn += step, buf ^= 1) {  // warp-uniform
+        const size_t b0 = end - 4 - turn;
+        if (turn + step < end) fetch(b0 - step, tiles + (uint32_t)((buf ^ 1) * kEncTile));
         else asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncwarp();
