@@ -290,3 +290,72 @@ def test_lists_of_5_to_8_rows_on_both_sides_of_the_finisher_rule(tensor_type, ga
         x = xs[i].cpu().numpy()
         want = orc.gated_linear(tensor_type, data[0], data[1], rows, cols, x) if gated else orc.linear(tensor_type, data[i % 2], rows, cols, x)
         _check(got[i], want, tight=BOUND)
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+@pytest.mark.parametrize("specs", [
+    [(200, 1536, 1), (130, 256, 4), (257, 2560, 3)],                   # odd units, one unit, ragged rows
+    [(3840, 3840, 1), (3840, 512, 1), (15000, 1024, 2)],               # ranges that hold parts of two inputs
+    [(640, 17408, 1), (300, 16384, 4), (129, 8192, 4)],                # records that leave a short ring, or none: the record pass then
+])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_records_in_shared_memory_give_the_bits_of_the_record_pass(tensor_type, specs, dtype):
+    """Lists of up to 4 rows quantise their inputs inside the decode kernel.  A result that lies over an input (here: the first job's over the
+    last one's) sends the same list through the record pass: same ranges, same order of every sum."""
+    from zllm_b200 import ffi
+
+    rng = np.random.default_rng(400 + len(specs) + specs[0][1])
+    ws = [ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=401 + i), rows, cols) for i, (rows, cols, _) in enumerate(specs)]
+    xs = [dev(rng.standard_normal((m, cols)).astype(np.float32), dtype) for _, cols, m in specs]
+
+    def run(over):
+        jobs = (ffi.ZqLinearJob * len(specs))()
+        ys = [torch.zeros(m * rows, device="cuda") for rows, _, m in specs]
+        inputs = [x.clone() for x in xs]
+        for j, (rows, cols, m), w, x, y in zip(jobs, specs, ws, inputs, ys):
+            j.w, j.dev_x, j.m, j.dev_y = w.handle, x.data_ptr(), m, y.data_ptr()
+        if over:  # the last input inside the first result's buffer: read before anything is written
+            need = xs[-1].numel() * xs[-1].element_size()
+            buf = torch.zeros(max(specs[0][0] * specs[0][2] * 4, need), dtype=torch.uint8, device="cuda")
+            buf[:need] = xs[-1].reshape(-1).view(torch.uint8)
+            jobs[len(specs) - 1].dev_x = jobs[0].dev_y = buf.data_ptr()
+            ys[0] = buf[: specs[0][0] * specs[0][2] * 4].view(torch.float32)
+        before = ctx().launch_count
+        code = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}[dtype]
+        ffi.call("zq_linear_batch", ctx().handle, jobs, len(specs), code, 0)
+        ctx().sync()
+        return [host(y).copy() for y in ys], ctx().launch_count - before
+
+    (inside, n_inside), (passed, n_passed) = run(False), run(True)
+    assert n_passed == 2 and n_inside <= 2
+    for a, b in zip(inside, passed):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("types,m", [((H.Q4_K, H.Q6_K), 1), ((H.Q4_K, H.Q6_K), 4), ((H.Q8_0, H.Q5_K, H.IQ4_NL), 1), ((H.Q4_0, H.Q8_0, H.Q4_K, H.Q5_K, H.Q6_K, H.IQ4_NL), 1)])
+def test_lists_of_several_types_in_one_launch(types, m):
+    rng = np.random.default_rng(430 + m)
+    made = [(t, rows, cols, *_weight(t, rows, cols, 431 + i)) for i, (t, rows, cols) in enumerate((t, 130 + 257 * i, 256 * (1 + 3 * (i % 3))) for i, t in enumerate(types))]
+    xs = [rng.standard_normal((m, cols)).astype(np.float32) for _, _, cols, _, _ in made]
+    before = ctx().launch_count
+    ys = ctx().linear_batch([(dev(x), w) for x, (*_, w) in zip(xs, made)])
+    assert ctx().launch_count - before == 1
+    for y, x, (t, rows, cols, data, _) in zip(ys, xs, made):
+        _check(host(y), orc.linear(t, data, rows, cols, x))
+
+
+@pytest.mark.parametrize("types", [(H.Q4_K,), (H.Q4_K, H.Q8_0)])
+def test_norm_inside_the_decode_kernel_and_before_it(types):
+    """One row: norm and projections in one launch, the bits of the norm kernel in front (which a second row brings back)."""
+    cols, rows = 3840, 300
+    ws = [_weight(t, rows + i, cols, 440 + i)[1] for i, t in enumerate(types)]
+    x = dev(np.random.default_rng(441).standard_normal((1, cols)).astype(np.float32) * 2.0)
+    nw = dev((1.0 + 0.1 * np.random.default_rng(442).standard_normal(cols)).astype(np.float32))
+    before = ctx().launch_count
+    one = [host(y) for y in ctx().rmsnorm_linear_multi(x, nw, 1e-5, ws)]
+    assert ctx().launch_count - before == 1
+    two = [host(y) for y in ctx().rmsnorm_linear_multi(torch.cat([x, x]), nw, 1e-5, ws)]
+    for a, b in zip(one, two):
+        if len(types) == 1:
+            assert np.array_equal(a[0].view(np.uint32), b[0].view(np.uint32))
+        assert H.max_rel_error(a, b[:1]) <= 1e-5  # two types share a launch in one case: other ranges, other order of the f32 sums

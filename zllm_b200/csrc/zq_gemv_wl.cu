@@ -20,6 +20,8 @@
 // (src/kernel/cpu/ggml_quant.rs:189-277) for a list of weights, as Backend::dual_linear / triple_linear
 // (src/backend/mod.rs:444-451) and the Metal backend's gguf_dual_gemv_q4k_f16 (src/kernel/metal/gguf/mod.rs:1787-1824)
 // do for two or three.
+#include <algorithm>
+
 #include "zq_i8.cuh"
 #include "zq_wl.cuh"
 
@@ -40,7 +42,21 @@ struct WlJob {
     int tiles;                 // row tiles
     int q_begin;               // first ring item of the job in the launch's (job, tile, chunk) order
     int y_dtype;               // output (and residual) dtype of this job
-    int pad;
+    int src;                   // resident records: index into WlArgs::src
+    uint32_t type;             // GGUF type (mixed lists)
+};
+
+// Resident records: a distinct input block of the list in one record format.
+struct WlSrc {
+    const void *x;
+    int m, cols;
+    bool kclass;
+};
+// Resident records behind an RMSNorm: the one input row is norm(x).
+struct WlNormArgs {
+    const float *weight;  // null: no norm
+    float eps, weight_offset;
+    bool x_wide, w_wide;  // 16-byte aligned row / weights
 };
 
 struct WlArgs {
@@ -50,6 +66,10 @@ struct WlArgs {
     int chunk_words;   // 32-bit words per chunk of a weight row
     int y_dtype;
     int async_fix;     // 5..8 rows: the finisher warp completes cut tiles (otherwise the consumers together)
+    int stages, stage_stride, off_rec;  // resident records: ring stages, bytes of one, where the records start
+    int n_src, x_dtype;
+    WlSrc src[kWlMaxJobs];
+    WlNormArgs norm;
     float *partials;   // [2 * grid][kSlotFloats]: slot 2c + 1 = the tile CTA c begins, slot 2c = the tile it continues
     uint32_t *counters;  // [grid], zero at the start of the launch: arrivals at the cut tile that CTA c begins
     uint32_t *status;
@@ -112,13 +132,30 @@ template <uint32_t TYPE, int NT> struct WlSmem {
     static_assert(STRIDE % 128 == 0 && STAGE_W % 256 == 0, "ring stages must keep TMA destinations 128-byte aligned");
 };
 
+// Resident records (up to 4 rows, plain jobs): no record pass and no records in the ring.  Every CTA quantises the slices that its own
+// range needs, each once, into shared memory, while the first weights are on their way; an RMSNorm in front of the list (one
+// row) is computed there too, by every CTA for itself: a row is a few KB out of L2.  That takes a launch (of 4 to 5 us in a chain of
+// small ones) and the records' way through memory off a decode step; lists of several types go out as one launch instead of one per
+// type (TYPE 0).  Decode step of 12 layers of 1536 columns, q, k, v in Q4_K and Q6_K behind a norm: 434 us (81 launches), now 382 (62); 4 layers of
+// 3840 columns: 324, now 315; five Q4_K projections of five inputs: 38.7, now 37.9.
+// The ring gets what the records leave, five stages at most.
+template <uint32_t TYPE> struct WlResSmem {
+    static constexpr int XCH_FLOATS = 16 * 32 * 2;
+    static constexpr int LIMIT = 232448 - 2048;  // opt-in maximum minus static shared memory
+    static constexpr int OFF_XCH = (LIMIT - (2 * XCH_FLOATS * 4 + kWlMaxSegs * 16 + 256)) & ~127;
+    static constexpr int OFF_SEG = OFF_XCH + 2 * XCH_FLOATS * 4;
+    static constexpr int OFF_BAR = OFF_SEG + kWlMaxSegs * 16;
+    static constexpr int TOTAL = OFF_BAR + 128 + 128;
+};
+
 constexpr int kWlConsumers = kI8Threads;        // 16 consumer warps: 8 row sub-tiles x 2 units
 constexpr int kWlThreads = kWlConsumers + 64;   // + the producer warp and the finisher warp
+constexpr int kWlNormTurns = 4;                 // a norm inside the kernel holds its row in registers: up to 16 384 columns
 // Named barriers (0 is left to __syncthreads, which this kernel never uses: the producer warp runs its own loop).
 constexpr int kBarQuad = 1;    // 1..4: the four warps that hold gate and up sums of the same 16 output rows (gated tiles)
 constexpr int kBarPair = 5;    // 5..12: the two warps (unit halves) of one row sub-tile
 constexpr int kBarFix = 13;    // 13, 14: the 16 consumer warps hand a cut tile's partial sums to the finisher warp (first / second cut piece)
-constexpr int kBarAll = 15;    // the 16 consumer warps among themselves (9..16 activation rows: they finish cut tiles on their own)
+constexpr int kBarAll = 15;    // the 16 consumer warps among themselves (9..16 activation rows: they finish cut tiles on their own; resident records)
 
 __device__ __forceinline__ void named_bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
 // Release / acquire fence at GPU scope: orders this thread's (and, after a CTA barrier, its CTA's) earlier accesses before
@@ -141,26 +178,128 @@ __device__ __forceinline__ void wl_wait(uint64_t *bar, uint32_t parity, uint32_t
     atomicMax(status, (uint32_t)kStatusTmaTimeout);
 }
 
+__device__ __forceinline__ int wl_unit_bytes(uint32_t type) { return type == ZQ_Q8_0 ? 272 : type == ZQ_Q6_K ? 224 : type == ZQ_Q5_K ? 176 : 144; }
+
+// One record into shared memory (the warp's lanes hold 8 columns each).
+template <bool KCLASS> __device__ __forceinline__ void wl_store_record(uint8_t *dst, const float (&v)[8], int lane) {
+    constexpr uint32_t T = KCLASS ? (uint32_t)ZQ_Q4_K : (uint32_t)ZQ_Q4_0;
+    const RecLane o = quantize_record<T>(v, lane);
+    *reinterpret_cast<uint4 *>(dst + o.slot) = make_uint4(o.ph0, o.ph1, o.pl0, o.pl1);
+    if (KCLASS && (lane & 7) == 0) *reinterpret_cast<uint2 *>(dst + kRecSums + (lane >> 3) * 8) = make_uint2(o.sw0, o.sw1);
+    if (lane == 0) *reinterpret_cast<float *>(dst + kRecScale) = o.scale;
+}
+
+// The records of this CTA's range, by the 16 consumer warps.
+template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(const WlArgs &a, uint8_t *records, const int *s_lo, const int *s_hi, const int *s_rec0, float *s_partial) {
+    constexpr bool MIX = TYPE == 0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto store = [&](const WlSrc &src, int rec, const float (&v)[8]) {
+        uint8_t *dst = records + rec * kRec;
+        if (MIX ? src.kclass : is_kclass(MIX ? (uint32_t)ZQ_Q4_K : TYPE)) wl_store_record<true>(dst, v, lane);
+        else wl_store_record<false>(dst, v, lane);
+    };
+    if (a.norm.weight) {
+        // the arithmetic of rmsnorm_kernel (zq_norm.cu), thread for thread: thread t holds columns 8 (t + 512 i)
+        const WlSrc &s0 = a.src[0];
+        float v[kWlNormTurns][8], w[kWlNormTurns][8];
+        const int turns = ((s0.cols + 255) / 256 * 32 + kWlConsumers - 1) / kWlConsumers;
+        auto load = [&](const void *p, int dtype, bool wide, int c, float (&o)[8]) {
+            const bool valid = 8 * c < s0.cols;
+            if (wide) {
+                load_act8(p, dtype, 8 * (size_t)c, valid, o);
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) o[j] = valid ? load_as_f32(p, dtype, 8 * (size_t)c + j) : 0.f;
+            }
+        };
+        float acc = 0.f;
+#pragma unroll
+        for (int i = 0; i < kWlNormTurns; ++i) {
+            if (i < turns) {
+                load(s0.x, a.x_dtype, a.norm.x_wide, tid + i * kWlConsumers, v[i]);
+                load(a.norm.weight, ZQ_F32, a.norm.w_wide, tid + i * kWlConsumers, w[i]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kWlNormTurns; ++i) {
+            if (i < turns) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc = fmaf(v[i][j], v[i][j], acc);
+            }
+        }
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, s);
+        if (lane == 0) s_partial[warp] = acc;
+        named_bar_sync(kBarAll, kWlConsumers);
+        float total = s_partial[lane & 15];
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, s);
+        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)s0.cols), a.norm.eps)));
+#pragma unroll
+        for (int i = 0; i < kWlNormTurns; ++i) {
+            const int unit = warp + 16 * i;
+            if (i >= turns) break;
+            bool scaled = false;
+            for (int s = 0; s < a.n_src; ++s) {  // the same row in one or both record formats
+                if (unit < s_lo[s] || unit >= s_hi[s]) continue;  // warp-uniform
+                if (!scaled) {
+                    scaled = true;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) v[i][j] = 8 * (tid + i * kWlConsumers) < s0.cols ? __fmul_rn(__fmul_rn(v[i][j], inv), a.norm.weight_offset == 0.0f ? w[i][j] : __fadd_rn(a.norm.weight_offset, w[i][j])) : 0.f;
+                }
+                store(a.src[s], s_rec0[s] + unit - s_lo[s], v[i]);
+            }
+        }
+    } else {
+        for (int s = 0; s < a.n_src; ++s) {
+            const WlSrc &src = a.src[s];
+            const int count = s_hi[s] > s_lo[s] ? (s_hi[s] - s_lo[s]) * src.m : 0;
+            constexpr int kBatch = 4;  // all loads of four records first, so that their latencies overlap
+            for (int base = warp; base < count; base += 16 * kBatch) {
+                float v[kBatch][8];
+#pragma unroll
+                for (int b = 0; b < kBatch; ++b) {
+                    const int k = base + 16 * b, u = k / src.m, row = k - u * src.m, k0 = (s_lo[s] + u) * kUnitWeights + 8 * lane;
+                    load_act8(src.x, a.x_dtype, (size_t)row * src.cols + k0, k < count && k0 < src.cols, v[b]);
+                }
+#pragma unroll
+                for (int b = 0; b < kBatch; ++b)
+                    if (base + 16 * b < count) store(src, s_rec0[s] + base + 16 * b, v[b]);  // warp-uniform
+            }
+        }
+    }
+    named_bar_sync(kBarAll, kWlConsumers);
+}
+
 // Warp-specialised: warp 16 is the producer (it alone waits for free ring stages and issues the TMA copies, so no
 // consumer ever stalls on another consumer's progress); warps 0..15 consume.  At the end of a tile only the warps
 // that hold sums of the same output rows meet (named barriers of 64 or 128 threads): the two unit halves of a row
 // sub-tile, plus the gate / up partners of a gated tile.  The accumulators of partner warps sit in the same lanes, so
 // the exchange buffer is indexed by lane and the owning warp stores its 16 rows straight from its fragments.
-template <uint32_t TYPE, int NT, bool GATED>
+// RES: resident records.  TYPE 0 (with RES): the jobs' types differ, each brings its own.
+template <uint32_t TYPE, int NT, bool GATED, bool RES>
 __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_constant__ WlArgs a) {
-    using S = WlSmem<TYPE, NT>;
-    constexpr int STAGES = S::STAGES, STRIDE = S::STRIDE, STAGE_W = S::STAGE_W, PITCH = S::PITCH, UB = S::UB;
+    static_assert(!RES || (NT == 1 && !GATED), "resident records: up to 4 rows, plain jobs");
+    constexpr bool MIX = TYPE == 0;
+    using S = WlSmem<MIX ? (uint32_t)ZQ_Q4_K : TYPE, NT>;
+    using R = WlResSmem<TYPE>;
+    const int STAGES = RES ? a.stages : S::STAGES, STRIDE = RES ? a.stage_stride : S::STRIDE;
+    constexpr int STAGE_W = S::STAGE_W;  // not in a mixed list
+    constexpr int OFF_XCH = RES ? R::OFF_XCH : S::OFF_XCH, OFF_SEG = RES ? R::OFF_SEG : S::OFF_SEG, OFF_BAR = RES ? R::OFF_BAR : S::OFF_BAR;
     constexpr int XCH_FLOATS = S::XCH_FLOATS, NACC = NT * 2;
+    auto unit_bytes = [&](const WlJob &jb) -> int { return MIX ? wl_unit_bytes(jb.type) : S::UB; };
     constexpr int out_rows = GATED ? kTileRows / 2 : kTileRows;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
     uint8_t *ws = smem;
-    float *xch = reinterpret_cast<float *>(smem + S::OFF_XCH);
-    int4 *segs = reinterpret_cast<int4 *>(smem + S::OFF_SEG);  // {job, tile, first chunk | end chunk << 16, first item (CTA-relative)}
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::OFF_BAR);
+    float *xch = reinterpret_cast<float *>(smem + OFF_XCH);
+    int4 *segs = reinterpret_cast<int4 *>(smem + OFF_SEG);  // {job, tile, first chunk | end chunk << 16, first item (CTA-relative)}
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + OFF_BAR);
     uint64_t *empty = full + 8;
     __shared__ uint32_t s_abort;
     __shared__ int s_nseg, s_last, s_c0, s_cl;
+    __shared__ int s_lo[RES ? kWlMaxJobs : 1], s_hi[RES ? kWlMaxJobs : 1], s_rec0[RES ? kWlMaxJobs : 1];  // units of a source that this CTA needs, index of their first record
+    __shared__ float s_partial[16];
     // Up to 4 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with 9..16
     // that warp would need longer than the consumers themselves, so they do it together (and wait for it); with 5..8 rows the host
     // decides by the length of the launch.
@@ -203,6 +342,23 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
             }
         }
         if (q < q1) atomicMax(a.status, (uint32_t)kStatusBadIndex);  // the host sizes launches so that this never happens
+        if constexpr (RES) {
+            for (int i = 0; i < a.n_src; ++i) {
+                s_lo[i] = INT32_MAX;
+                s_hi[i] = 0;
+            }
+            for (int k = 0; k < n; ++k) {
+                const WlJob &jb = a.jobs[segs[k].x];
+                const int lo = (segs[k].z & 0xFFFF) * kChunkUnits, hi = min((segs[k].z >> 16) * kChunkUnits, jb.units);
+                s_lo[jb.src] = min(s_lo[jb.src], lo);
+                s_hi[jb.src] = max(s_hi[jb.src], hi);
+            }
+            int at = 0;
+            for (int i = 0; i < a.n_src; ++i) {
+                s_rec0[i] = at;
+                if (s_hi[i] > s_lo[i]) at += (s_hi[i] - s_lo[i]) * a.src[i].m;
+            }
+        }
         // Cut tiles first: a piece of a tile that a range boundary cuts (only the first and the last piece of a range can
         // be one) is finished by whichever contributor arrives last, so every CTA does its cut pieces at the start and
         // the hand-over completes under the streaming of the whole tiles instead of at the very end of the kernel.
@@ -315,9 +471,15 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 int nu = jb.units - chunk * kChunkUnits;
                 if (nu > kChunkUnits) nu = kChunkUnits;
                 uint8_t *dst = ws + (size_t)stage * STRIDE;
-                mbar_expect_tx(&full[stage], (uint32_t)(STAGE_W + nu * jb.m * kRec));
-                tma_load_2d(dst, jb.map_a, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
-                if (GATED) tma_load_2d(dst + STAGE_W / 2, jb.map_b, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
+                if constexpr (RES) {
+                    const int words = kChunkUnits * unit_bytes(jb) / 4;
+                    mbar_expect_tx(&full[stage], (uint32_t)(kTileRows * words * 4));
+                    tma_load_2d(dst, jb.map_a, &full[stage], chunk * words, sg.y * out_rows);
+                } else {
+                    mbar_expect_tx(&full[stage], (uint32_t)(STAGE_W + nu * jb.m * kRec));
+                    tma_load_2d(dst, jb.map_a, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
+                    if (GATED) tma_load_2d(dst + STAGE_W / 2, jb.map_b, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
+                }
             };
             auto issue_x = [&](int i, int stage) {
                 const int4 sg = segs[psi];
@@ -333,11 +495,13 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 issue_w(s, s);  // weights are constants: they may stream while the previous kernel still runs
             }
             pdl_launch_dependents();
-            pdl_wait_prior_grid();  // the records belong to the record pass, which waits for everything before it
-            psi = 0;
-            for (int s = 0; s < pre; ++s) {
-                locate(s);
-                issue_x(s, s);
+            if constexpr (!RES) {
+                pdl_wait_prior_grid();  // the records belong to the record pass, which waits for everything before it
+                psi = 0;
+                for (int s = 0; s < pre; ++s) {
+                    locate(s);
+                    issue_x(s, s);
+                }
             }
             int stage = 0;
             uint32_t phase = 0;
@@ -348,7 +512,7 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 if (f) break;  // never start a copy nobody will wait for
                 locate(i);
                 issue_w(i, stage);
-                issue_x(i, stage);
+                if constexpr (!RES) issue_x(i, stage);
                 if (++stage == STAGES) {
                     stage = 0;
                     phase ^= 1u;
@@ -366,12 +530,15 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     const int g = lane >> 2, t = lane & 3;
     const int rs = warp & 7, ul = warp >> 3;
     const int r0 = 16 * rs + frag_row(g);
-    const uint32_t w_first = smem_u32(ws) + (uint32_t)(r0 * PITCH + ul * UB);
+    int ub = S::UB;  // unit bytes of the piece's weight
+    uint32_t w_first = smem_u32(ws) + (uint32_t)((r0 * kChunkUnits + ul) * S::UB);
     const uint32_t rec_base = smem_u32(ws) + STAGE_W;
     const uint32_t xoff = (uint32_t)(16 * t + 8 * (g & 1));
+    if constexpr (RES) wl_resident_records<TYPE>(a, smem + a.off_rec, s_lo, s_hi, s_rec0, s_partial);
 
     float yacc[NT][2];
     uint32_t moff[NT], soff[NT];
+    uint32_t jtype = TYPE;
     int si = -1, seg_end = 0, chunk = 0, units = 0, M = 1, buf = 0, cut_k = 0;
     uint32_t rec_unit = 0;  // byte offset of this warp's unit inside a stage's records
     int stage = 0;
@@ -395,22 +562,38 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 yacc[nt][0] = yacc[nt][1] = 0.f;
             }
             rec_unit = (uint32_t)(ul * M * kRec);
+            if constexpr (RES) rec_unit = smem_u32(smem) + (uint32_t)(a.off_rec + (s_rec0[jb.src] + (chunk * kChunkUnits + ul - s_lo[jb.src]) * M) * kRec);
+            if constexpr (MIX) {
+                jtype = jb.type;
+                ub = unit_bytes(jb);
+                w_first = smem_u32(ws) + (uint32_t)((r0 * kChunkUnits + ul) * ub);
+            }
         }
         wl_wait(&full[stage], phase, abort_addr, a.status);
         if (chunk * kChunkUnits + ul < units) {
             const uint32_t soffs = (uint32_t)(stage * STRIDE);
-            const uint32_t wq0 = w_first + soffs, wq1 = wq0 + 8 * PITCH;
-            const uint32_t rb = rec_base + soffs + rec_unit;
+            const uint32_t wq0 = w_first + soffs, wq1 = wq0 + (uint32_t)(8 * kChunkUnits * ub);
+            const uint32_t rb = RES ? rec_unit : rec_base + soffs + rec_unit;
             uint32_t rec[NT], srec[NT];
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
                 rec[nt] = rb + moff[nt];
                 srec[nt] = rb + soff[nt];
             }
-            if constexpr (TYPE == ZQ_Q6_K) consume_q6k_i8<NT>(wq0, wq1, t, rec, srec, xoff, yacc);
+            if constexpr (MIX) {
+                switch (jtype) {
+                case ZQ_Q4_K: consume_q4k_i8<NT, false>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                case ZQ_Q5_K: consume_q4k_i8<NT, true>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                case ZQ_Q6_K: consume_q6k_i8<NT>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                case ZQ_Q4_0: consume_b32_i8<ZQ_Q4_0, NT>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                case ZQ_IQ4_NL: consume_b32_i8<ZQ_IQ4_NL, NT>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                default: consume_b32_i8<ZQ_Q8_0, NT>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+                }
+            } else if constexpr (TYPE == ZQ_Q6_K) consume_q6k_i8<NT>(wq0, wq1, t, rec, srec, xoff, yacc);
             else if constexpr (is_kclass(TYPE)) consume_q4k_i8<NT, TYPE == ZQ_Q5_K>(wq0, wq1, t, rec, srec, xoff, yacc);
             else consume_b32_i8<TYPE, NT>(wq0, wq1, t, rec, srec, xoff, yacc);
         }
+        if constexpr (RES) rec_unit += (uint32_t)(kChunkUnits * M * kRec);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == STAGES) {
@@ -523,20 +706,20 @@ static int launch_wl_quantize(zq_ctx *ctx, const WlQuantArgs &qa, zq_error *err)
     return ZQ_OK;
 }
 
-template <uint32_t TYPE, int NT, bool GATED>
+template <uint32_t TYPE, int NT, bool GATED, bool RES = false>
 static int launch_wl_one(zq_ctx *ctx, const WlArgs &wa, zq_error *err) {
-    using S = WlSmem<TYPE, NT>;
-    auto kernel = gemv_wl_kernel<TYPE, NT, GATED>;
+    constexpr int smem = RES ? WlResSmem<TYPE>::TOTAL : WlSmem<TYPE ? TYPE : (uint32_t)ZQ_Q4_K, NT>::TOTAL;
+    auto kernel = gemv_wl_kernel<TYPE, NT, GATED, RES>;
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        ZQ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL), err);
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem), err);
         configured[ctx->device & 63] = true;
     }
     int grid = ctx->sm_count < wa.q_total ? ctx->sm_count : wa.q_total;  // every CTA gets at least one item
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(kWlThreads);
-    cfg.dynamicSmemBytes = S::TOTAL;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -553,6 +736,109 @@ static int launch_wl_type(zq_ctx *ctx, const WlArgs &wa, int nt, bool gated, zq_
     if (nt == 1) return gated ? launch_wl_one<TYPE, 1, true>(ctx, wa, err) : launch_wl_one<TYPE, 1, false>(ctx, wa, err);
     if (nt == 2) return gated ? launch_wl_one<TYPE, 2, true>(ctx, wa, err) : launch_wl_one<TYPE, 2, false>(ctx, wa, err);
     return gated ? launch_wl_one<TYPE, 4, true>(ctx, wa, err) : launch_wl_one<TYPE, 4, false>(ctx, wa, err);
+}
+
+static int launch_wl_resident(zq_ctx *ctx, uint32_t type, const WlArgs &wa, zq_error *err) {
+    switch (type) {
+    case 0: return launch_wl_one<0, 1, false, true>(ctx, wa, err);
+    case ZQ_Q4_K: return launch_wl_one<ZQ_Q4_K, 1, false, true>(ctx, wa, err);
+    case ZQ_Q5_K: return launch_wl_one<ZQ_Q5_K, 1, false, true>(ctx, wa, err);
+    case ZQ_Q6_K: return launch_wl_one<ZQ_Q6_K, 1, false, true>(ctx, wa, err);
+    case ZQ_Q4_0: return launch_wl_one<ZQ_Q4_0, 1, false, true>(ctx, wa, err);
+    case ZQ_IQ4_NL: return launch_wl_one<ZQ_IQ4_NL, 1, false, true>(ctx, wa, err);
+    default: return launch_wl_one<ZQ_Q8_0, 1, false, true>(ctx, wa, err);
+    }
+}
+
+// A list of plain jobs of up to 4 rows in one launch with resident records; `taken` says whether it was.  It is where the records that a
+// CTA's range can need leave the ring three stages (Q8_0: two), and no result lies over an input (CTAs read inputs while others write results;
+// the record pass reads them all first).  A list of one input without a norm keeps the record pass: callers count on its two launches.
+static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, const WlNorm *norm, bool &taken, zq_error *err) {
+    taken = false;
+    if (n_jobs > (size_t)kWlMaxJobs || (norm && (jobs[0].m != 1 || jobs[0].w->cols > (size_t)kWlNormTurns * kWlConsumers * 8))) return ZQ_OK;
+    if (!norm && std::all_of(jobs, jobs + n_jobs, [&](const WlHostJob &j) { return j.x == jobs[0].x; })) return ZQ_OK;
+    WlArgs wa;
+    wa.n_jobs = (int)n_jobs;
+    wa.n_src = 0;
+    uint32_t type = jobs[0].w->type;
+    int unit_bytes = 0, min_chunks = INT32_MAX;
+    long long q_total = 0;
+    int src_units[kWlMaxJobs];
+    for (size_t k = 0; k < n_jobs; ++k) {
+        const WlHostJob &j = jobs[k];
+        if (j.m > 4 || j.w_up) return ZQ_OK;
+        if (j.w->type != type) type = 0;
+        unit_bytes = std::max(unit_bytes, format_info(j.w->type).unit_bytes);
+        const bool kclass = is_kclass(j.w->type);
+        const void *x = norm ? norm->x : j.x;
+        int s = 0;
+        for (; s < wa.n_src; ++s)
+            if (wa.src[s].x == x && wa.src[s].m == (int)j.m && wa.src[s].cols == (int)j.w->cols && wa.src[s].kclass == kclass) break;
+        if (s == wa.n_src) {
+            src_units[s] = (int)j.w->units_per_row;
+            wa.src[wa.n_src++] = {x, (int)j.m, (int)j.w->cols, kclass};
+        }
+        const long long tiles = (long long)((j.w->rows + kTileRows - 1) / kTileRows), chunks = (long long)((j.w->units_per_row + kChunkUnits - 1) / kChunkUnits);
+        if (q_total + tiles * chunks > (long long)INT32_MAX / 512) return ZQ_OK;
+        WlJob &d = wa.jobs[k];
+        d.map_a = d.map_b = j.w->d_maps;
+        d.xq = nullptr;
+        d.y = j.y;
+        d.residual = j.residual;
+        d.m = (int)j.m;
+        d.n_out = (int)j.w->rows;
+        d.units = (int)j.w->units_per_row;
+        d.chunks = (int)chunks;
+        d.tiles = (int)tiles;
+        d.q_begin = (int)q_total;
+        d.y_dtype = j.y_dtype >= 0 ? j.y_dtype : y_dtype;
+        d.src = s;
+        d.type = j.w->type;
+        q_total += tiles * chunks;
+        min_chunks = std::min(min_chunks, d.chunks);
+    }
+    const auto apart = [](const void *a, size_t an, const void *b, size_t bn) {
+        const uintptr_t a0 = reinterpret_cast<uintptr_t>(a), b0 = reinterpret_cast<uintptr_t>(b);
+        return a0 + an <= b0 || b0 + bn <= a0;
+    };
+    const size_t xe = dtype_size(norm ? norm->x_dtype : x_dtype);
+    for (size_t k = 0; k < n_jobs; ++k) {
+        const size_t y_bytes = (size_t)wa.jobs[k].m * wa.jobs[k].n_out * dtype_size(wa.jobs[k].y_dtype);
+        for (int s = 0; s < wa.n_src; ++s)
+            if (!apart(wa.jobs[k].y, y_bytes, wa.src[s].x, (size_t)wa.src[s].m * wa.src[s].cols * xe)) return ZQ_OK;
+        if (norm && !apart(wa.jobs[k].y, y_bytes, norm->weight, (size_t)wa.src[0].cols * sizeof(float))) return ZQ_OK;
+    }
+    wa.q_total = (int)q_total;
+    const int grid = ctx->sm_count < wa.q_total ? ctx->sm_count : wa.q_total, per_cta = (wa.q_total + grid - 1) / grid;
+    if (per_cta / min_chunks + 3 > kWlMaxSegs) return ZQ_OK;
+    // records a range can need: the sources of neighbouring jobs that one range reaches
+    int most = 0;
+    for (size_t i = 0; i < n_jobs; ++i) {
+        int need = 0, between = 0;
+        uint32_t seen = 0;
+        for (size_t k = i; k < n_jobs && between < per_cta; ++k) {
+            if (!(seen >> wa.jobs[k].src & 1)) need += src_units[wa.jobs[k].src] * wa.jobs[k].m;
+            seen |= 1u << wa.jobs[k].src;
+            if (k > i) between += wa.jobs[k].tiles * wa.jobs[k].chunks;
+        }
+        most = std::max(most, need);
+    }
+    wa.stage_stride = kTileRows * kChunkUnits * unit_bytes;
+    const long long left = (long long)WlResSmem<0>::OFF_XCH - (long long)most * kRec;
+    wa.stages = left < 0 ? 0 : (int)std::min<long long>(5, left / wa.stage_stride);
+    if (wa.stages < (unit_bytes == 272 ? 2 : 3)) return ZQ_OK;  // with Q8_0 the ring of the record pass has two stages as well
+    wa.off_rec = wa.stages * wa.stage_stride;
+    wa.chunk_words = 0;
+    wa.y_dtype = y_dtype;
+    wa.x_dtype = norm ? norm->x_dtype : x_dtype;
+    wa.async_fix = 1;
+    wa.norm = {};
+    if (norm) wa.norm = {norm->weight, norm->eps, norm->weight_offset, (reinterpret_cast<uintptr_t>(norm->x) & 15) == 0, (reinterpret_cast<uintptr_t>(norm->weight) & 15) == 0};
+    wa.partials = ctx->gemv_partials;
+    wa.counters = ctx->gemv_counters;
+    wa.status = ctx->status_dev;
+    taken = true;
+    return launch_wl_resident(ctx, type, wa, err);
 }
 
 static bool wl_type_ok(uint32_t t) { return t == ZQ_Q4_K || t == ZQ_Q4_0 || t == ZQ_Q8_0 || t == ZQ_IQ4_NL || t == ZQ_Q5_K || t == ZQ_Q6_K; }
@@ -593,6 +879,11 @@ bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) 
 int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, zq_error *err, const WlNorm *norm, bool own_scratch) {
     if (n_jobs == 0) return ZQ_OK;
     if (own_scratch && (n_jobs != 1 || norm)) return set_error(err, ZQ_ERR_ARG, "decode work list: scratch of its own is for one job");
+    if (!own_scratch) {
+        bool taken = false;
+        const int rc = launch_gemv_wl_resident(ctx, jobs, n_jobs, x_dtype, y_dtype, norm, taken, err);
+        if (taken || rc) return rc;
+    }
     // ---- records: one block per distinct (x, m, cols, record format)
     struct Src { const void *x; size_t m, cols; bool q4k; size_t rec_begin, units; };
     std::vector<Src> srcs;
@@ -727,7 +1018,8 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
             d.tiles = (int)tiles;
             d.q_begin = wa.q_total;
             d.y_dtype = j.y_dtype >= 0 ? j.y_dtype : y_dtype;
-            d.pad = 0;
+            d.src = 0;
+            d.type = type;
             wa.q_total += (int)(tiles * chunks);
             if ((int)chunks < min_chunks) min_chunks = (int)chunks;
             if ((int)chunks > max_chunks) max_chunks = (int)chunks;
