@@ -153,6 +153,32 @@ def test_prefill_cut_tiles(tensor_type, m, rows, cols, gated, dtype):
     assert H.max_rel_error(got[sel], want) <= BOUND + rounding
 
 
+@pytest.mark.parametrize("tensor_type,rows,m,gated,dtype", [
+    (H.Q4_K, 17300, 257, False, torch.float32),   # one wide tile of 9 chunks, one pair per tile; ragged rows
+    (H.Q6_K, 17408, 320, False, torch.bfloat16),  # full width, 10 chunks
+    (H.Q4_K, 17408, 900, False, torch.float16),   # three wide tiles per pair: their accumulators overlap
+    (H.Q8_0, 11008, 830, False, torch.float32),   # the last of three tiles is not wide
+    (H.Q5_K, 17408, 300, False, torch.float16), (H.IQ4_NL, 17408, 289, False, torch.float32), (H.Q4_0, 17408, 290, False, torch.float32),
+    (H.IQ4_NL, 3840, 560, True, torch.float16),   # gated
+])
+def test_prefill_wide_tiles(tensor_type, rows, m, gated, dtype, gemm_variant):
+    """Tiles of 257 to 320 tokens give the bits of the operand pass, whose tiles end at 256 (whole tiles on both sides: no sum is split)."""
+    if gemm_variant == "operand_pass":
+        pytest.skip("compares the two in one go")
+    cols = 512
+    ws = [ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=500 + i), rows, cols) for i in range(2 if gated else 1)]
+    x = dev(np.random.default_rng(501).standard_normal((m, cols)).astype(np.float32), torch.float16)
+    r = None if gated else dev(np.random.default_rng(502).standard_normal((m, rows)).astype(np.float32), dtype)
+
+    def run():
+        return (ctx().gated_linear(x, *ws, out_dtype=dtype) if gated else ctx().linear(x, ws[0], out_dtype=dtype, residual=r)).clone()
+
+    a = run()
+    ctx().set_option("force_fused_gemm", 0)
+    ctx().set_option("disable_fused_gemm", 1)
+    assert torch.equal(a, run())
+
+
 @pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0])
 @pytest.mark.parametrize("m,rows,cols", [(31, 63, 512), (260, 130, 1024)])
 def test_prefill_gated_edges(tensor_type, m, rows, cols):

@@ -329,6 +329,7 @@ struct zq_weight {
 };
 
 namespace zq {
+constexpr int kGemmTileTokens = 256, kGemmWideTokens = 320;  // most tokens per item of a grouped GEMM; 320 for packed types, where asked for
 int use_device(zq_ctx *ctx, zq_error *err);
 int ensure_workspace(zq_ctx *ctx, size_t bytes, zq_error *err);
 int ensure_xq(zq_ctx *ctx, size_t bytes, zq_error *err);
@@ -345,7 +346,7 @@ struct LaunchScratch {
     LaunchScratch &operator=(const LaunchScratch &) = delete;
     ~LaunchScratch();
 };
-int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, zq_error *err);
+int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, bool wide, void *y, int y_dtype, zq_error *err);
 int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const __half *x, size_t m, void *y, int y_dtype, zq_error *err);
 int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n, zq_error *err, uint32_t *zero = nullptr, int n_zero = 0);
 int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t mats, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, void *y, int y_dtype, zq_error *err);

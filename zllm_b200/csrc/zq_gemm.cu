@@ -38,7 +38,9 @@ namespace zq {
 
 constexpr int kBM = 128;      // weight rows per SM (operand tile of one CTA)
 constexpr int kPairM = 256;   // weight rows per pair
-constexpr int kBN = 256;      // most tokens per tile
+constexpr int kBN = kGemmTileTokens;      // 256: most tokens per MMA, and per tile of operands in memory
+constexpr int kWideBN = kGemmWideTokens;  // 320: most tokens per wide tile (packed types): two MMAs (pieces) of up to 160 share a dequantised operand
+constexpr int kChunk = 32, kChunks = 512 / kChunk;  // accumulator columns of wide tiles are given back in chunks of 32
 constexpr int kBK = 64;       // K elements per ring stage (128 bytes of f16: one swizzle atom row)
 constexpr int kStepK = 256;   // K elements per step: one packed unit, the grain in which tiles are cut
 constexpr int kEpi = 8;       // epilogue warps
@@ -53,9 +55,10 @@ struct GemmParams {
     int n_out;   // output features (weight rows; gated: rows of gate)
     int k;       // input columns
     int bn;      // tokens per tile (multiple of 32, at most 256)
-    int box_tok; // token rows of one activation box (half a tile)
+    int box_tok; // token rows of one activation box (half a tile's)
+    int wide;    // tiles may have up to kWideBN tokens; those with more than kBN take two boxes of 80 token rows
     int cut_tiles, cut_pairs;  // the first cut_tiles tiles are cut along K into cut_pairs equal shares
-    float *partials;           // [2 * pairs][2 SMs][256 columns][128 rows] f32
+    float *partials;           // [2 * pairs][2 SMs][bn columns][128 rows] f32
     uint32_t *counters;        // arrivals per (pair that begins a cut tile, SM), zero at the start of the launch
     // Grouped form (MoE prefill): the work list replaces the tile grid.  Item = {weight matrix z, first output row of the tile,
     // first token row, end of the tile's token rows}; tokens are rows of one activation operand shared by all matrices,
@@ -192,18 +195,18 @@ template <int DT> __device__ __forceinline__ float raw_as_f32(uint32_t r) {
     else return __uint_as_float(r << 16);
 }
 
-// Shared-memory plan: 32 KB per ring stage (16 KB of weights, 16 KB of tokens), as many as fit beside the packed boxes.
-template <uint32_t SRC> struct GemmSmem {
+// Shared-memory plan: a ring stage is 16 KB of weights and half a tile's tokens (16 KB, WIDE 20 KB); packed boxes take what the stages leave.
+template <uint32_t SRC, bool WIDE> struct GemmSmem {
     static constexpr int unit_bytes = SRC == ZQ_Q8_0 ? 272 : SRC == ZQ_Q6_K ? 224 : SRC == ZQ_Q5_K ? 176 : 144;
     static constexpr int a_bytes = kBM * kBK * 2;
-    static constexpr int b_bytes = kBN / 2 * kBK * 2;
-    static constexpr int stage_bytes = a_bytes + b_bytes;
+    static constexpr int stage_bytes = a_bytes + (WIDE ? kWideBN : kBN) / 2 * kBK * 2;
     static constexpr int p_bytes = SRC ? kBM * unit_bytes : 0;  // one packed box
-    static constexpr int pstages = SRC == 0 ? 0 : unit_bytes <= 144 ? 3 : 2;
-    static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 ? 4 : 5;
+    static constexpr int pstages = SRC == 0 ? 0 : unit_bytes <= 144 && !WIDE ? 3 : 2;
+    static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 || (SRC == ZQ_Q6_K && WIDE) ? 4 : 5;
     static constexpr int off_p = stages * stage_bytes;
     static constexpr int off_bar = off_p + pstages * p_bytes;
-    static constexpr int total = off_bar + 256 + 1024;       // barriers, slack for 1024-byte alignment
+    static constexpr int bar_bytes = 256 + (WIDE ? kChunks * 8 : 0);
+    static constexpr int total = off_bar + bar_bytes + 1024;    // barriers, slack for 1024-byte alignment
     static constexpr int threads = (2 + kEpi + (SRC ? 1 + kDqWarps : 0)) * 32;
     static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
     static_assert(off_p % 1024 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
@@ -252,7 +255,8 @@ struct GemmWalk {
             s.z = it.x;
             s.row0 = it.y;
             s.tok0 = it.z;
-            s.tok_end = it.w < it.z + kBN ? it.w : it.z + kBN;
+            const int most = p.wide ? kWideBN : kBN;
+            s.tok_end = it.w < it.z + most ? it.w : it.z + most;
             return true;
         }
         s.z = 0;
@@ -265,11 +269,17 @@ struct GemmWalk {
         return true;
     }
 };
-// columns the MMA of a tile computes: its tokens, rounded up to 32 (16 per SM)
-__device__ __forceinline__ int tile_cols(const GemmSeg &s) {
-    const int n = (s.tok_end - s.tok0 + 31) & ~31;
-    return n > kBN ? kBN : n < 32 ? 32 : n;
+// Accumulator columns of a tile, in chunks: its tokens rounded up to 32 (16 per SM).
+__device__ __forceinline__ int tile_chunks(const GemmSeg &s) {
+    const int n = (s.tok_end - s.tok0 + kChunk - 1) / kChunk;
+    return n < 1 ? 1 : n;
 }
+// Tiles take the low and the high end of the 512 accumulator columns in turn.  Two that do not fit beside each other (both wide)
+// overlap in the middle, where the epilogue begins: it gives a tile's chunks back from the middle outwards, and the MMAs of
+// the next tile start as soon as those they share with it are free.
+__device__ __forceinline__ int tile_column(int iter, int chunks) { return (iter & 1) ? (kChunks - chunks) * kChunk : 0; }
+// Chunks of the first of a tile's two pieces (of its only one).
+__device__ __forceinline__ int first_piece(int chunks) { return chunks > kBN / kChunk ? (chunks + 1) / 2 : chunks; }
 
 // A cut tile whose shares have all arrived.
 struct GemmCut {
@@ -290,7 +300,7 @@ template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(co
     for (int c0 = lane_col; c0 < t.n_tok; c0 += LANES * COLS) {
         float4 sum[PARTS][COLS];
         for (int c = t.c_first; c <= t.c_last; ++c) {
-            const float *share = p.partials + ((size_t)(2 * c + (c == t.c_first ? 1 : 0)) * 2 + rank) * (kBN * kBM) + at0;
+            const float *share = p.partials + ((size_t)(2 * c + (c == t.c_first ? 1 : 0)) * 2 + rank) * ((size_t)p.bn * kBM) + at0;
             float4 v[PARTS][COLS];
 #pragma unroll
             for (int part = 0; part < PARTS; ++part)
@@ -343,10 +353,14 @@ template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(co
     }
 }
 
-template <uint32_t SRC, bool GATED>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threads, 1)
-    gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const GemmParams p) {
-    using S = GemmSmem<SRC>;
+// WIDE: tiles of up to 320 tokens.  What they are for: a tile of a packed type costs its dequantisation whatever its tokens, and an expert that
+// got 257 to 320 tokens was two tiles (256 experts of 7168 x 2048 in Q4_K, 8192 tokens, 256 +- 16 to an expert: MoE layer 8.2 ms, now 7.1).
+// A form of its own because the second piece costs the issuing warp instructions in every k-block: with one form for both, 48
+// tokens of 5120 x 17408 up and down took 61.2 us instead of 56.7.
+template <uint32_t SRC, bool GATED, bool WIDE>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>::threads, 1)
+    gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const GemmParams p) {
+    using S = GemmSmem<SRC, WIDE>;
     constexpr int STAGES = S::stages, PST = S::pstages > 0 ? S::pstages : 1;
     constexpr int kRows = GATED ? kPairM / 2 : kPairM;  // output rows of a tile
     constexpr int kPackedWarp = 2 + kEpi;
@@ -358,6 +372,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
     uint64_t *p_empty = p_full + PST;
     uint64_t *acc_full = p_empty + PST;                                // each SM
     uint64_t *acc_empty = acc_full + 2;                                // first SM: both SMs' epilogue warps
+    uint64_t *step_free = acc_empty + 2;                               // WIDE, first SM: both SMs' epilogue warps are through with the k-th chunk of a tile; once per tile each
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_state;
     __shared__ GemmCut s_cut[2];  // cut tiles that this SM adds up: a pair's shares touch two at most
@@ -384,6 +399,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 2 * kEpi);
         }
+        for (int c = 0; WIDE && c < kChunks; ++c) mbar_init(&step_free[c], 2 * kEpi);
         fence_mbar_init();
         s_state = kStateAhead;
         s_cuts = 0;
@@ -418,9 +434,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
         int s = 0;
         uint32_t ph = 0;
         bool ok = true, fresh = true;  // fresh: first turn of the ring
-        const uint32_t bytes = 2u * (uint32_t)((SRC ? 0 : S::a_bytes) + p.box_tok * kBK * 2);
         while (ok && walk.next(p, sg)) {
-            const int tok = sg.tok0 + (int)rank * (tile_cols(sg) / 2);
+            const int columns = tile_chunks(sg) * kChunk, first = first_piece(columns / kChunk) * kChunk;
+            const bool two = WIDE && columns > first;
+            const int tok = sg.tok0 + (int)rank * (first / 2), tok2 = sg.tok0 + first + (int)rank * ((columns - first) / 2);
+            const uint32_t bytes = 2u * (uint32_t)((SRC ? 0 : S::a_bytes) + (two ? kWideBN / 2 : p.box_tok) * kBK * 2);
             const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
             const int kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
             for (int kb = sg.k0 * 4; kb < kb1; ++kb) {
@@ -440,7 +458,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                             else tma_load_2d_pair(st + h * (S::a_bytes / 8), m, bar, kb * kBK, row + (h >> 1) * 16);
                         }
                     }
-                    tma_load_2d_pair(st + S::a_bytes, &map_x, bar, kb * kBK, tok);
+                    tma_load_2d_pair(st + S::a_bytes, two ? &map_x2 : &map_x, bar, kb * kBK, tok);
+                    if (two) tma_load_2d_pair(st + S::a_bytes + kWideBN / 4 * kBK * 2, &map_x2, bar, kb * kBK, tok2);
                 }
                 __syncwarp();
                 if (++s == STAGES) {
@@ -457,14 +476,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             uint32_t ph = 0;
             bool ok = true;
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
+            int before = 0;  // chunks of the tile before
             for (; ok && walk.next(p, sg); ++iter) {
-                // f32 accumulator, f16 A and B, both K-major, M = 256, N = the tile's tokens
-                const uint32_t idesc = (1u << 4) | ((uint32_t)(tile_cols(sg) >> 3) << 17) | ((uint32_t)(kPairM >> 4) << 24);
+                // f32 accumulator, f16 A and B, both K-major, M = 256, N = the piece's tokens
+                const int chunks = tile_chunks(sg), first = first_piece(chunks), second = chunks - first, shared = before + chunks - kChunks;
+                before = chunks;
+                const uint32_t idesc0 = (1u << 4) | ((uint32_t)(kPairM >> 4) << 24), idesc = idesc0 | ((uint32_t)(first * (kChunk >> 3)) << 17), idesc2 = idesc0 | ((uint32_t)(second * (kChunk >> 3)) << 17);
                 const int b = iter & 1;
                 if (iter >= 2) ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
+                if (WIDE && ok && shared > 0) ok = wait_flag(&step_free[shared - 1], (uint32_t)(iter - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem_base + (uint32_t)b * kBN;
+                const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * kBN), acc2 = acc + (uint32_t)(first * kChunk);
                 const int kb0 = sg.k0 * 4, kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     ok = wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout);
@@ -475,6 +498,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
 #pragma unroll
                         for (int k = 0; k < kBK / 16; ++k)  // 16 K elements = 32 bytes = 2 descriptor units along the swizzled row
                             umma2_f16_ss(acc, da + 2 * k, db + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+                        if (WIDE && second) {
+                            const uint64_t db2 = db + kWideBN / 4 * kBK * 2 / 16;
+#pragma unroll
+                            for (int k = 0; k < kBK / 16; ++k) umma2_f16_ss(acc2, da + 2 * k, db2 + 2 * k, idesc2, (kb > kb0 || k > 0) ? 1u : 0u);
+                        }
                         tc_commit2(&empty[s]);
                         if (kb + 1 == kb1) tc_commit2(&acc_full[b]);
                     }
@@ -494,7 +522,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
         const int et = (warp - 2) * 32 + lane;
         for (; walk.next(p, sg); ++iter) {
             const int b = iter & 1;
-            const int n_tok = sg.tok_end - sg.tok0;
+            const int n_tok = sg.tok_end - sg.tok0, chunks = tile_chunks(sg);
             if (!GATED && p.residual) {
                 // bring the tile's residual rows into L2 while its MMAs run: a warp can only have a few KB of loads in flight below
                 const size_t esz = dtype_size(p.y_dtype), r0 = (size_t)sg.row0 + rank * kBM;
@@ -506,7 +534,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
             }
             const bool ok = wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0);
             tc_fence_after();
-            const uint32_t acc = tmem_base + (uint32_t)b * kBN + ((uint32_t)(q * 32) << 16);
+            const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * kBN) + ((uint32_t)(q * 32) << 16);
+            auto free_step = [&](int k) {  // this warp is through with the k-th chunk
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) pair_arrive(pair_first(smem_u32(&step_free[k])));
+            };
             const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
             // output row of this lane; gated: lanes 0..15 hold gate rows, lanes 16..31 the up rows of the same outputs
             const int row = GATED ? sg.row0 + (int)rank * 64 + q * 16 + (lane & 15) : sg.row0 + (int)rank * kBM + q * 32 + lane;
@@ -557,10 +590,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 }
             };
             auto store_tile = [&](auto dt) {
-                for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {  // warp-uniform
-                    uint32_t v[16];
-                    tmem_ld16(acc + c0, v);
-                    store16(dt, c0, v);
+                if constexpr (WIDE) {
+                    for (int k = 0; k < chunks; ++k) {  // warp-uniform; from the middle of the columns outwards
+                        const int c0 = ((iter & 1) ? k : chunks - 1 - k) * kChunk + 16 * part;
+                        uint32_t v[16];
+                        if (c0 < n_tok) tmem_ld16(acc + c0, v);
+                        free_step(k);
+                        if (c0 < n_tok) store16(dt, c0, v);
+                    }
+                } else {
+                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {  // walked as above, 48 tokens of 5120 x 17408 up and down take 63.8 us instead of 57.7
+                        uint32_t v[16];
+                        tmem_ld16(acc + c0, v);
+                        store16(dt, c0, v);
+                    }
                 }
             };
             if (ok && whole) {
@@ -572,7 +615,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 // A share of a cut tile goes to its slot; the SM that comes last takes the tile down for the end of the kernel.
                 const long long Q = (long long)p.cut_tiles * walk.steps, G = p.cut_pairs, ts = (long long)sg.tile * walk.steps;
                 const int c_first = (int)(((ts + 1) * G - 1) / Q), c_last = (int)(((ts + walk.steps) * G - 1) / Q);  // pairs that own the tile's first and last step
-                float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * (kBN * kBM) + q * 32 + lane;
+                float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * ((size_t)p.bn * kBM) + q * 32 + lane;
                 if (ok) {
                     for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {
                         uint32_t v[16];
@@ -585,6 +628,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC>::threa
                 asm volatile("bar.sync 3, %0;" ::"n"(32 * kEpi) : "memory");
                 if (et == 0 && ok && atomicAdd(p.counters + 2 * c_first + rank, 1u) == (uint32_t)(c_last - c_first)) s_cut[s_cuts++] = {sg.row0, sg.tok0, n_tok, c_first, c_last};
             }
+            if (WIDE)
+                for (int k = whole && ok ? chunks : 0; k < kChunks; ++k) free_step(k);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) pair_arrive(pair_first(smem_u32(&acc_empty[b])));  // this warp's part of the accumulator may be overwritten
@@ -738,12 +783,12 @@ int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n
     return ZQ_OK;
 }
 
-template <uint32_t SRC, bool GATED>
-static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const GemmParams &p, int pairs, zq_error *err) {
-    using S = GemmSmem<SRC>;
+template <uint32_t SRC, bool GATED, bool WIDE>
+static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
+    using S = GemmSmem<SRC, WIDE>;
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
         configured[ctx->device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -756,12 +801,17 @@ static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->disable_pdl ? 0 : 1;
-    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED>, mw, mw2, mx, p), err);
+    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED, WIDE>, mw, mw2, mx, mx2, p), err);
     ctx->launches++;
     return ZQ_OK;
 }
-static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const GemmParams &p, int pairs, zq_error *err) {
-#define ZQ_GEMM_CASE(T) case T: return gated ? launch_one<T, true>(ctx, mw, mw2, mx, p, pairs, err) : launch_one<T, false>(ctx, mw, mw2, mx, p, pairs, err)
+template <uint32_t SRC> static int launch_form(zq_ctx *ctx, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
+    constexpr bool W = SRC != 0;  // operands in memory have no wide tiles
+    if (W && p.wide) return gated ? launch_one<SRC, true, W>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, W>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    return gated ? launch_one<SRC, true, false>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, false>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+}
+static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
+#define ZQ_GEMM_CASE(T) case T: return launch_form<T>(ctx, gated, mw, mw2, mx, mx2, p, pairs, err)
     switch (src) {
         ZQ_GEMM_CASE(0);
         ZQ_GEMM_CASE(ZQ_Q4_K);
@@ -780,12 +830,21 @@ static void clear_params(zq_ctx *ctx, GemmParams &p) {
     p.status = ctx->status_dev;
 }
 
-// Token tiles of a dense GEMM: as few as 256-token tiles allow, of equal size (300 tokens are two tiles of 160, not 256 + 44).
-static void plan_tokens(size_t m, GemmParams &p) {
-    const size_t tiles = (m + kBN - 1) / kBN;
+// Token tiles of a dense GEMM: as few as tiles of `cap` tokens allow, of equal size (300 tokens in tiles of up to 256 are two of
+// 160, not 256 + 44).
+static void plan_tokens(size_t m, size_t cap, GemmParams &p) {
+    const size_t tiles = (m + cap - 1) / cap;
     p.m = (int)m;
     p.bn = (int)(((m + tiles - 1) / tiles + 31) & ~size_t(31));
-    p.box_tok = p.bn / 2;
+    p.wide = p.bn > kBN;
+    p.box_tok = p.wide ? kBN / 2 : p.bn / 2;
+}
+// Boxes of half a tile's tokens, and (wide tiles) of half a piece's.
+static int make_token_maps(const __half *x, size_t rows, size_t k, const GemmParams &p, CUtensorMap *map_x, CUtensorMap *map_x2, zq_error *err) {
+    int rc = make_f16_map(x, rows, k, p.box_tok, map_x, err);
+    if (!rc && p.wide) rc = make_f16_map(x, rows, k, kWideBN / 4, map_x2, err);
+    if (!p.wide) *map_x2 = *map_x;
+    return rc;
 }
 
 // How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; cut, the tiles beyond the full rounds and one
@@ -822,7 +881,7 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool ga
 static int take_shares(zq_ctx *ctx, GemmParams &p, LaunchScratch &scratch, zq_error *err) {
     if (!p.cut_tiles) return ZQ_OK;
     const size_t head = ((size_t)2 * p.cut_pairs * sizeof(uint32_t) + 1023) & ~size_t(1023);
-    const int rc = scratch.take(ctx, head + (size_t)p.cut_pairs * 2 * 2 * kBN * kBM * sizeof(float), err);
+    const int rc = scratch.take(ctx, head + (size_t)p.cut_pairs * 2 * 2 * p.bn * kBM * sizeof(float), err);
     if (rc) return rc;
     p.counters = reinterpret_cast<uint32_t *>(scratch.p);
     p.partials = reinterpret_cast<float *>(reinterpret_cast<uint8_t *>(scratch.p) + head);
@@ -845,7 +904,18 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || m <= 1024) && has_i8_decode(w->type) && (!gated || w_up->type == w->type);
     GemmParams p;
     clear_params(ctx, p);
-    plan_tokens(m, p);
+    const int row_tiles = (int)((n + (gated ? kPairM / 2 : kPairM) - 1) / (gated ? kPairM / 2 : kPairM));
+    plan_tokens(m, kBN, p);
+    // Wide tiles where the rounds of whole tiles, at a step's time each (see plan_cut), come out no longer.  us, tiles of up to 256 and of up to 320:
+    //   Q4_K 5120 -> 17408  270 tokens 48.4 / 39.5, 560 80.8 / 76.3, 800 124 / 117;  4096 -> 4096  300 tokens 31.4 / 50.9 (not taken)
+    //   4096 -> 11008  Q6_K 270 tokens 54.1 / 45.2, 900 94.6 / 70.9;  Q8_0 560 tokens 41.6 / 55.1 (not taken), 800 72.2 / 66.2;  gated Q4_K 300 tokens 70.5 / 80.0 (not taken)
+    if (fused && m > kBN) {
+        const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
+        const auto time = [&](const GemmParams &g) { return (((long long)row_tiles * ((g.m + g.bn - 1) / g.bn) + pairs - 1) / pairs) * std::max(850, 56 * g.bn / 10); };
+        GemmParams wide = p;
+        plan_tokens(m, kWideBN, wide);
+        if (wide.wide && time(wide) <= time(p)) p = wide;
+    }
     p.y = y;
     p.residual = residual;
     p.y_dtype = y_dtype;
@@ -872,10 +942,10 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
         rc = launch_to_f16(ctx, nullptr, ZQ_F16, nullptr, 0, err, p.counters, 2 * p.cut_pairs);
     }
     if (rc) return rc;
-    CUtensorMap map_x;
-    rc = make_f16_map(xin, m, k, p.box_tok, &map_x, err);
+    CUtensorMap map_x, map_x2;
+    rc = make_token_maps(xin, m, k, p, &map_x, &map_x2, err);
     if (rc) return rc;
-    if (fused) return launch_src(ctx, w->type, gated, gated ? w->unit_map_half : w->qmv_map, gated ? w_up->unit_map_half : w->qmv_map, map_x, p, pairs, err);
+    if (fused) return launch_src(ctx, w->type, gated, gated ? w->unit_map_half : w->qmv_map, gated ? w_up->unit_map_half : w->qmv_map, map_x, map_x2, p, pairs, err);
     __half *w16 = reinterpret_cast<__half *>(ws), *w16b = reinterpret_cast<__half *>(ws + w_bytes);
     rc = launch_dequantize_f16(ctx, w, w16, err);
     if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
@@ -884,11 +954,12 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     rc = make_f16_map(w16, n, k, gated ? 16 : kBM, &map_w, err);
     if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, gated ? 16 : kBM, &map_w2, err);
     if (rc) return rc;
-    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, p, pairs, err);
+    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, map_x2, p, pairs, err);
 }
 
-static int grouped_params(zq_ctx *ctx, size_t rows, size_t k, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, void *y, int y_dtype, GemmParams &p) {
+static int grouped_params(zq_ctx *ctx, size_t rows, size_t k, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, bool wide, void *y, int y_dtype, GemmParams &p) {
     clear_params(ctx, p);
+    p.wide = wide;
     p.y = y;
     p.y_dtype = y_dtype;
     p.m = (int)x_rows;
@@ -916,8 +987,8 @@ int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t m
     if (!rc) rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
     if (rc) return rc;
     GemmParams p;
-    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, nullptr, y, y_dtype, p);
-    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, p, pairs, err);
+    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, nullptr, false, y, y_dtype, p);
+    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, map_x, p, pairs, err);
 }
 
 // Plain f16 x f16 GEMM on raw operands: y[m, rows] = x[m, k] w[rows, k]^T, f32 accumulation (router logits).  Whole tiles only:
@@ -926,7 +997,7 @@ int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const _
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "f16 GEMM needs columns aligned to 8, got %zu", k);
     GemmParams p;
     clear_params(ctx, p);
-    plan_tokens(m, p);
+    plan_tokens(m, kBN, p);
     CUtensorMap map_w, map_x;
     int rc = make_f16_map(w, rows, k, kBM, &map_w, err);
     if (!rc) rc = make_f16_map(x, m, k, p.box_tok, &map_x, err);
@@ -937,23 +1008,23 @@ int launch_gemm_f16(zq_ctx *ctx, const __half *w, size_t rows, size_t k, const _
     p.k = (int)k;
     const size_t tiles = ((rows + kPairM - 1) / kPairM) * ((m + p.bn - 1) / p.bn);
     const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
-    return launch_src(ctx, 0, false, map_w, map_w, map_x, p, tiles < (size_t)pairs ? (int)tiles : pairs, err);
+    return launch_src(ctx, 0, false, map_w, map_w, map_x, map_x, p, tiles < (size_t)pairs ? (int)tiles : pairs, err);
 }
 
 // Grouped form for packed experts (MoE prefill): no f16 copy of the weights at all.  `w_maps` / `w2_maps`: device tables of the
 // experts' packed-weight tensor maps (one unit x 128 rows boxes, gated: 64 rows), indexed by the work items' z.
 int launch_gemm_fused_grouped(zq_ctx *ctx, uint32_t type, const CUtensorMap *w_maps, const CUtensorMap *w2_maps, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev,
-                              void *y, int y_dtype, zq_error *err) {
+                              bool wide, void *y, int y_dtype, zq_error *err) {
     if (n_items <= 0) return ZQ_OK;
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "grouped GEMM needs columns aligned to 8, got %zu", k);
-    CUtensorMap map_x;
-    int rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
-    if (rc) return rc;
     GemmParams p;
-    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, n_items_dev, y, y_dtype, p);
+    const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, n_items_dev, wide, y, y_dtype, p);
+    CUtensorMap map_x, map_x2;
+    int rc = make_token_maps(x, x_rows, k, p, &map_x, &map_x2, err);
+    if (rc) return rc;
     p.w_maps = w_maps;
     p.w2_maps = w2_maps;
-    return launch_src(ctx, type, w2_maps != nullptr, map_x, map_x, map_x, p, pairs, err);
+    return launch_src(ctx, type, w2_maps != nullptr, map_x, map_x, map_x, map_x2, p, pairs, err);
 }
 
 }  // namespace zq

@@ -478,12 +478,12 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_count_kernel(const 
     for (int e = threadIdx.x; e < E; e += kGroupThreads) hist[(size_t)blockIdx.x * E + e] = s_cnt[e];
 }
 
-// Tokens per tile when `count` tokens of an expert take `tiles` (= ceil(count / 256)) tiles: equal shares in whole MMA column
-// groups of 32.  270 tokens are 160 + 110, not 256 + 14: a tile costs at least its dequantisation, whatever its tokens.
+// Tokens per tile when `count` tokens of an expert take `tiles` (as few as their size allows) tiles: equal shares in whole MMA column
+// groups of 32.  330 tokens are 192 + 138, not 320 + 10: a tile costs at least its dequantisation, whatever its tokens.
 __host__ __device__ inline uint32_t moe_tile_tokens(uint32_t count, uint32_t tiles) { return ((count + tiles - 1) / tiles + 31u) & ~31u; }
 
 // counts: [0] items of the gated launch, [1] items of the down launch
-__global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_t *__restrict__ hist, int chunks, int E, uint32_t *__restrict__ offsets, int rt_gated, int rt_down, int4 *__restrict__ items_gated,
+__global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_t *__restrict__ hist, int chunks, int E, uint32_t *__restrict__ offsets, int rt_gated, int rt_down, int tile_tokens, int4 *__restrict__ items_gated,
                                                                          int4 *__restrict__ items_down, int *__restrict__ counts) {
     __shared__ uint32_t warp_tot[2][32];
     const int e = threadIdx.x, lane = e & 31, wid = e >> 5;
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(kGroupThreads) moe_prefill_scan_kernel(uint32_
             hist[(size_t)b * E + e] = c;
             c += v;
         }
-    const uint32_t nt = (c + 255u) / 256u;  // 256-token tiles of this expert
+    const uint32_t nt = (c + (uint32_t)tile_tokens - 1u) / (uint32_t)tile_tokens;  // token tiles of this expert
     uint32_t sc = c, st = nt;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
@@ -633,7 +633,9 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     const int tokens_per_chunk = (int)(kGroupThreads / top_k > 0 ? kGroupThreads / top_k : 1);
     const int chunks = (int)((m + tokens_per_chunk - 1) / tokens_per_chunk);
     const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 255) / 256);  // 128 gated outputs or 256 rows per tile
-    const size_t max_tiles = routes / 256 + E;  // sum over experts of ceil(count / 256)
+    const size_t max_tiles = routes / kGemmTileTokens + E;  // at least the sum over experts of ceil(count / tile)
+    // Wide tiles where experts get enough tokens for some to go past 256; below, the narrow kernel's deeper ring of packed boxes.
+    const bool wide = routes >= 128 * E;
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     // tables and f32 results
     const size_t o_hist = 0, o_offsets = o_hist + al((size_t)chunks * E * 4), o_counts = o_offsets + al((E + 1) * 4), o_token_slots = o_counts + al(16);
@@ -661,14 +663,14 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
         configured[ctx->device & 63] = true;
     }
     moe_prefill_count_kernel<<<chunks, kGroupThreads, E * 4, ctx->stream>>>(dev_ids, (int)m, (int)top_k, (int)E, tokens_per_chunk, d_hist, ctx->status_dev);
-    moe_prefill_scan_kernel<<<1, kGroupThreads, 0, ctx->stream>>>(d_hist, chunks, (int)E, d_offsets, rt_i, rt_h, d_items_g, d_items_d, d_counts);
+    moe_prefill_scan_kernel<<<1, kGroupThreads, 0, ctx->stream>>>(d_hist, chunks, (int)E, d_offsets, rt_i, rt_h, wide ? kGemmWideTokens : kGemmTileTokens, d_items_g, d_items_d, d_counts);
     moe_prefill_place_kernel<<<chunks, kGroupThreads, place_smem, ctx->stream>>>(dev_ids, dev_weights, (int)m, (int)top_k, (int)E, tokens_per_chunk, d_hist, d_offsets, d_token_slots, d_token_w);
     scatter_rows_f16_kernel<<<(unsigned)(m < (size_t)ctx->sm_count * 32 ? m : (size_t)ctx->sm_count * 32), 256, 0, ctx->stream>>>(dev_x, x_dtype, d_token_slots, (int)m, (int)top_k, (int)H, x16);
     ctx->launches += 4;
     ZQ_CUDA_CHECK(cudaGetLastError(), err);
-    rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, x16, routes, d_items_g, (int)(max_tiles * rt_i), d_counts, act16, ZQ_F16, err);
+    rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, x16, routes, d_items_g, (int)(max_tiles * rt_i), d_counts, wide, act16, ZQ_F16, err);
     if (rc) return rc;
-    rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items_d, (int)(max_tiles * rt_h), d_counts + 1, d_out, ZQ_F32, err);
+    rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items_d, (int)(max_tiles * rt_h), d_counts + 1, wide, d_out, ZQ_F32, err);
     if (rc) return rc;
     if (has_shared) {
         rc = zq_gated_mlp(ctx, shared_gate, shared_up, shared_down, dev_x, x_dtype, m, d_shared, ZQ_F32, nullptr, err);
@@ -1051,9 +1053,9 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
             if (rc) return rc;
             xin = x16;
         }
-        rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, xin, routes, d_items, n_gated, nullptr, act16, ZQ_F16, err);
+        rc = launch_gemm_fused_grouped(ctx, experts->gate_type, experts->d_gate_qmaps, experts->d_up_qmaps, I, H, xin, routes, d_items, n_gated, nullptr, false, act16, ZQ_F16, err);
         if (rc) return rc;
-        rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items + n_gated, n_down, nullptr, d_out, ZQ_F32, err);
+        rc = launch_gemm_fused_grouped(ctx, experts->down_type, experts->d_down_qmaps, nullptr, H, I, act16, routes, d_items + n_gated, n_down, nullptr, false, d_out, ZQ_F32, err);
         if (rc) return rc;
     } else if (grouped_gemm) {
         // Prefill: one grouped tensor-core GEMM per projection and chunk of experts instead of two launches per
