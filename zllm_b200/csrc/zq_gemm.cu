@@ -894,14 +894,22 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     const size_t n = w->rows, k = w->cols;
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM needs columns aligned to 8, got %zu", k);
     // Dequantising inside the kernel saves the operand pass (one read of the packed weight, one write and one read of its f16
-    // form); with many tokens the pass is amortised and what counts is that every token tile dequantises the weight again.  Both forms give
-    // the same bits.  Measured, inside / pass, us at 512, 1024, 1536, 2048, 4096 bf16 rows:
-    //   5120 -> 17408  Q4_K 69/122 131/178 191/236 252/296 539/615   Q6_K 101/134 175/183 269/259 376/335 728/533   Q8_0 71/116 132/173 196/268 280/334 510/560
-    //   4096 -> 4096   Q4_K 52/70 35/48 62/78 56/70 109/124          Q6_K 56/68 43/47 70/76 73/68 137/117            (Q5_K, Q4_0, IQ4_NL as Q4_K)
-    //   gated 4096 -> 11008  Q4_K 115/169 176/191 244/259 388/328 771/559   Q6_K 135/166 220/191 341/247   Q8_0 119/162 182/186 282/247 781/548
-    // One line for all types and both forms lies where the gated form of most types loses its advantage.  Past it plain projections of
-    // all types but Q6_K would still gain 10 to 25 %; below it gated Q6_K loses 7 to 15 % from 768 rows.
-    const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || m <= 1024) && has_i8_decode(w->type) && (!gated || w_up->type == w->type);
+    // form); against it stands that every token tile dequantises the weight again, which its MMAs hide unless there are few columns per
+    // output (a short tile's epilogue competes with the dequantisers for issue) or the type is Q6_K, which takes the most instructions.  Both
+    // forms give the same bits.  Measured, inside / pass, us:
+    //   rows                     700        1100       2048       4096       8192       16384
+    //   Q4_K 5120 -> 17408       91/143     142/191    249/301    500/579    944/1150   1863/2430
+    //   Q8_0 5120 -> 17408       102/156    151/205    282/342    519/619    1136/1158  2269/2539
+    //   Q6_K 5120 -> 17408       160/190    242/195    299/309    705/587    1361/1009
+    //   IQ4_NL 3840 -> 15360     100/147    139/191    217/265    330/366    673/708    1499/1615
+    //   gated Q4_K 4096 -> 11008 109/159    146/207    271/342    528/649    1064/1177  2241/2469
+    //   gated Q6_K 4096 -> 11008 185/224    258/282    349/333    679/580
+    //   gated Q4_K 3072 -> 4096             78/109     96/130     154/190    289/330
+    //   gated Q4_K 2048 -> 4096             58/72      76/89      123/131    232/212
+    //   gated Q5_K 1536 -> 4096             57/63      70/74      117/105    200/166
+    //   Q4_K 512 -> 4096                    24/25      26/28      50/39      55/47
+    const bool inside = w->type == ZQ_Q6_K ? m <= 1024 : m <= 2048 || k >= 3072;
+    const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || inside) && has_i8_decode(w->type) && (!gated || w_up->type == w->type);
     GemmParams p;
     clear_params(ctx, p);
     const int row_tiles = (int)((n + (gated ? kPairM / 2 : kPairM) - 1) / (gated ? kPairM / 2 : kPairM));
