@@ -109,6 +109,43 @@ def test_prefill_behind_a_reduce_that_waits_for_a_peer(rows, cols, m):
     c.close()
 
 
+@pytest.mark.parametrize("tensor_type,norm", [(H.Q8_0, True), (H.Q4_K, True), (H.Q4_K, False)])
+def test_decode_list_behind_a_reduce_that_waits_for_a_peer(tensor_type, norm):
+    """The same for the work-list decode kernel with records in shared memory: its producer loads the first weights under the reduce, and more
+    items per CTA than ring stages (9 and 17 of at most 5) make it wait for the consumers, which start when the reduce is over."""
+    from zllm_b200 import ffi
+    from zllm_b200.backend import B200Context
+
+    rows, cols = 20480, 4096
+    c = B200Context(0)
+    blob = (C.c_uint8 * ffi.DIST_HANDLE_BYTES)()
+    ffi.call("zq_dist_export", c.handle, 1 << 20, blob)
+    both = (C.c_uint8 * (2 * ffi.DIST_HANDLE_BYTES))(*(list(blob) * 2))
+    ffi.call("zq_dist_init", c.handle, 0, 2, both)
+    ffi.call("zq_dist_set_wait_ms", c.handle, 1000)
+    small = c.prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 256, 512, seed=3), 256, 512)
+    w = c.prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=5), rows, cols)
+    xs = [torch.randn((1, cols), device="cuda") for _ in range(2)]
+    gain = torch.rand(cols, device="cuda") + 0.5
+
+    def run():
+        return c.rmsnorm_linear_multi(xs[0], gain, 1e-6, [w]) if norm else c.linear_batch([(x, w) for x in xs])
+
+    before = c.launch_count
+    want = run()
+    assert c.launch_count - before == 1  # records inside the kernel
+    c.sync()
+    c.linear_row_parallel(torch.randn((1, 512), device="cuda"), small)
+    got = run()
+    with pytest.raises(ffi.ZqFailure) as info:
+        c.sync()
+    assert info.value.code == 5 and "peer" in info.value.message
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    small.release()
+    w.release()
+    c.close()
+
+
 EP = dict(experts=16, top_k=4, hidden=512, inter=256)
 
 

@@ -495,8 +495,10 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 issue_w(s, s);  // weights are constants: they may stream while the previous kernel still runs
             }
             pdl_launch_dependents();
+            // The records belong to the record pass, which waits for everything before it; and no bounded wait may count while an
+            // earlier kernel still runs (one that waits for another rank may take longer than any bound here).
+            pdl_wait_prior_grid();
             if constexpr (!RES) {
-                pdl_wait_prior_grid();  // the records belong to the record pass, which waits for everything before it
                 psi = 0;
                 for (int s = 0; s < pre; ++s) {
                     locate(s);
