@@ -189,8 +189,19 @@ template <bool KCLASS> __device__ __forceinline__ void wl_store_record(uint8_t *
     if (lane == 0) *reinterpret_cast<float *>(dst + kRecScale) = o.scale;
 }
 
+// The units of a source that a CTA needs: a range walks the chunks of a source's jobs from 0 to the end over and over, so it is one run of units
+// that may go round from the last chunk to the first.  (Everything between the lowest and the highest unit, which is the whole row wherever a
+// range goes on to the next tile: 4 x 17408 -> 5120 in Q4_K, one row, 42.7 us; a list of 2048 -> 300, 17408 -> 512, 1024 -> 9000 and 4096 -> 4096,
+// two rows, 17.8 us.  The record pass: 40.8 and 12.5.)
+struct WlRun {
+    int first, count;  // units; count goes round at `around`
+    int rec0;          // index of the first one's first record
+    int around;        // units per row, rounded up to whole chunks
+};
+__device__ __forceinline__ int wl_run_place(const WlRun &r, int unit) { return unit < r.first ? unit - r.first + r.around : unit - r.first; }
+
 // The records of this CTA's range, by the 16 consumer warps.
-template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(const WlArgs &a, uint8_t *records, const int *s_lo, const int *s_hi, const int *s_rec0, float *s_partial) {
+template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(const WlArgs &a, uint8_t *records, const WlRun *s_run, float *s_partial) {
     constexpr bool MIX = TYPE == 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto store = [&](const WlSrc &src, int rec, const float (&v)[8]) {
@@ -239,32 +250,37 @@ template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(con
         for (int i = 0; i < kWlNormTurns; ++i) {
             const int unit = warp + 16 * i;
             if (i >= turns) break;
+            if (unit * kUnitWeights >= s0.cols) break;  // warp-uniform, as all of this
             bool scaled = false;
             for (int s = 0; s < a.n_src; ++s) {  // the same row in one or both record formats
-                if (unit < s_lo[s] || unit >= s_hi[s]) continue;  // warp-uniform
+                const WlRun run = s_run[s];
+                const int place = wl_run_place(run, unit);
+                if (place >= run.count) continue;
                 if (!scaled) {
                     scaled = true;
 #pragma unroll
                     for (int j = 0; j < 8; ++j) v[i][j] = 8 * (tid + i * kWlConsumers) < s0.cols ? __fmul_rn(__fmul_rn(v[i][j], inv), a.norm.weight_offset == 0.0f ? w[i][j] : __fadd_rn(a.norm.weight_offset, w[i][j])) : 0.f;
                 }
-                store(a.src[s], s_rec0[s] + unit - s_lo[s], v[i]);
+                store(a.src[s], run.rec0 + place, v[i]);
             }
         }
     } else {
         for (int s = 0; s < a.n_src; ++s) {
             const WlSrc &src = a.src[s];
-            const int count = s_hi[s] > s_lo[s] ? (s_hi[s] - s_lo[s]) * src.m : 0;
+            const WlRun run = s_run[s];
+            const int count = run.count * src.m;
             constexpr int kBatch = 4;  // all loads of four records first, so that their latencies overlap
             for (int base = warp; base < count; base += 16 * kBatch) {
                 float v[kBatch][8];
 #pragma unroll
                 for (int b = 0; b < kBatch; ++b) {
-                    const int k = base + 16 * b, u = k / src.m, row = k - u * src.m, k0 = (s_lo[s] + u) * kUnitWeights + 8 * lane;
+                    const int k = base + 16 * b, place = k / src.m, row = k - place * src.m, unit = run.first + place < run.around ? run.first + place : run.first + place - run.around;
+                    const int k0 = unit * kUnitWeights + 8 * lane;
                     load_act8(src.x, a.x_dtype, (size_t)row * src.cols + k0, k < count && k0 < src.cols, v[b]);
                 }
 #pragma unroll
                 for (int b = 0; b < kBatch; ++b)
-                    if (base + 16 * b < count) store(src, s_rec0[s] + base + 16 * b, v[b]);  // warp-uniform
+                    if (base + 16 * b < count) store(src, run.rec0 + base + 16 * b, v[b]);  // warp-uniform
             }
         }
     }
@@ -283,7 +299,11 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     constexpr bool MIX = TYPE == 0;
     using S = WlSmem<MIX ? (uint32_t)ZQ_Q4_K : TYPE, NT>;
     using R = WlResSmem<TYPE>;
-    const int STAGES = RES ? a.stages : S::STAGES, STRIDE = RES ? a.stage_stride : S::STRIDE;
+    int STAGES = S::STAGES, STRIDE = S::STRIDE;
+    if constexpr (RES) {
+        STAGES = a.stages;
+        STRIDE = a.stage_stride;
+    }
     constexpr int STAGE_W = S::STAGE_W;  // not in a mixed list
     constexpr int OFF_XCH = RES ? R::OFF_XCH : S::OFF_XCH, OFF_SEG = RES ? R::OFF_SEG : S::OFF_SEG, OFF_BAR = RES ? R::OFF_BAR : S::OFF_BAR;
     constexpr int XCH_FLOATS = S::XCH_FLOATS, NACC = NT * 2;
@@ -298,7 +318,7 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     uint64_t *empty = full + 8;
     __shared__ uint32_t s_abort;
     __shared__ int s_nseg, s_last, s_c0, s_cl;
-    __shared__ int s_lo[RES ? kWlMaxJobs : 1], s_hi[RES ? kWlMaxJobs : 1], s_rec0[RES ? kWlMaxJobs : 1];  // units of a source that this CTA needs, index of their first record
+    __shared__ WlRun s_run[RES ? kWlMaxJobs : 1];
     __shared__ float s_partial[16];
     // Up to 4 activation rows a cut tile's partial sums are a few KB and one warp adds them up beside the consumers; with 9..16
     // that warp would need longer than the consumers themselves, so they do it together (and wait for it); with 5..8 rows the host
@@ -329,10 +349,17 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
         const int rel = q0 - a.jobs[j].q_begin;
         int tile = rel / a.jobs[j].chunks, cb = rel - tile * a.jobs[j].chunks;
         int q = q0, n = 0;
+        if constexpr (RES)
+            for (int i = 0; i < a.n_src; ++i) s_run[i].first = s_run[i].count = 0;
         while (q < q1 && n < kWlMaxSegs && j < a.n_jobs) {
             const int chunks = a.jobs[j].chunks;
             int ce = chunks;
             if (q + (ce - cb) > q1) ce = cb + (q1 - q);
+            if constexpr (RES) {  // first and count in chunks here
+                WlRun &run = s_run[a.jobs[j].src];
+                if (run.count == 0) run.first = cb;
+                run.count += ce - cb;
+            }
             segs[n++] = make_int4(j, tile, cb | (ce << 16), q - q0);
             q += ce - cb;
             cb = 0;
@@ -343,20 +370,13 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
         }
         if (q < q1) atomicMax(a.status, (uint32_t)kStatusBadIndex);  // the host sizes launches so that this never happens
         if constexpr (RES) {
-            for (int i = 0; i < a.n_src; ++i) {
-                s_lo[i] = INT32_MAX;
-                s_hi[i] = 0;
-            }
-            for (int k = 0; k < n; ++k) {
-                const WlJob &jb = a.jobs[segs[k].x];
-                const int lo = (segs[k].z & 0xFFFF) * kChunkUnits, hi = min((segs[k].z >> 16) * kChunkUnits, jb.units);
-                s_lo[jb.src] = min(s_lo[jb.src], lo);
-                s_hi[jb.src] = max(s_hi[jb.src], hi);
-            }
             int at = 0;
             for (int i = 0; i < a.n_src; ++i) {
-                s_rec0[i] = at;
-                if (s_hi[i] > s_lo[i]) at += (s_hi[i] - s_lo[i]) * a.src[i].m;
+                const int units = (a.src[i].cols + kUnitWeights - 1) / kUnitWeights, chunks = (units + kChunkUnits - 1) / kChunkUnits;
+                const bool all = s_run[i].count >= chunks;
+                const WlRun run = {all ? 0 : s_run[i].first * kChunkUnits, all ? units : s_run[i].count * kChunkUnits, at, chunks * kChunkUnits};
+                s_run[i] = run;
+                at += run.count * a.src[i].m;
             }
         }
         // Cut tiles first: a piece of a tile that a range boundary cuts (only the first and the last piece of a range can
@@ -536,13 +556,14 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
     uint32_t w_first = smem_u32(ws) + (uint32_t)((r0 * kChunkUnits + ul) * S::UB);
     const uint32_t rec_base = smem_u32(ws) + STAGE_W;
     const uint32_t xoff = (uint32_t)(16 * t + 8 * (g & 1));
-    if constexpr (RES) wl_resident_records<TYPE>(a, smem + a.off_rec, s_lo, s_hi, s_rec0, s_partial);
+    if constexpr (RES) wl_resident_records<TYPE>(a, smem + a.off_rec, s_run, s_partial);
 
     float yacc[NT][2];
     uint32_t moff[NT], soff[NT];
     uint32_t jtype = TYPE;
     int si = -1, seg_end = 0, chunk = 0, units = 0, M = 1, buf = 0, cut_k = 0;
     uint32_t rec_unit = 0;  // byte offset of this warp's unit inside a stage's records
+    WlRun run = {};         // resident records: where the piece's units lie
     int stage = 0;
     uint32_t phase = 0;
     for (int it = 0; it < total_items; ++it) {
@@ -564,7 +585,7 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
                 yacc[nt][0] = yacc[nt][1] = 0.f;
             }
             rec_unit = (uint32_t)(ul * M * kRec);
-            if constexpr (RES) rec_unit = smem_u32(smem) + (uint32_t)(a.off_rec + (s_rec0[jb.src] + (chunk * kChunkUnits + ul - s_lo[jb.src]) * M) * kRec);
+            if constexpr (RES) run = s_run[jb.src];
             if constexpr (MIX) {
                 jtype = jb.type;
                 ub = unit_bytes(jb);
@@ -575,7 +596,8 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
         if (chunk * kChunkUnits + ul < units) {
             const uint32_t soffs = (uint32_t)(stage * STRIDE);
             const uint32_t wq0 = w_first + soffs, wq1 = wq0 + (uint32_t)(8 * kChunkUnits * ub);
-            const uint32_t rb = RES ? rec_unit : rec_base + soffs + rec_unit;
+            uint32_t rb = rec_base + soffs + rec_unit;
+            if constexpr (RES) rb = smem_u32(smem) + (uint32_t)(a.off_rec + (run.rec0 + wl_run_place(run, chunk * kChunkUnits + ul) * M) * kRec);
             uint32_t rec[NT], srec[NT];
 #pragma unroll
             for (int nt = 0; nt < NT; ++nt) {
@@ -595,7 +617,6 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
             else if constexpr (is_kclass(TYPE)) consume_q4k_i8<NT, TYPE == ZQ_Q5_K>(wq0, wq1, t, rec, srec, xoff, yacc);
             else consume_b32_i8<TYPE, NT>(wq0, wq1, t, rec, srec, xoff, yacc);
         }
-        if constexpr (RES) rec_unit += (uint32_t)(kChunkUnits * M * kRec);
         __syncwarp();
         if (lane == 0) mbar_arrive(&empty[stage]);
         if (++stage == STAGES) {
@@ -752,9 +773,17 @@ static int launch_wl_resident(zq_ctx *ctx, uint32_t type, const WlArgs &wa, zq_e
     }
 }
 
-// A list of plain jobs of up to 4 rows in one launch with resident records; `taken` says whether it was.  It is where the records that a
-// CTA's range can need leave the ring three stages (Q8_0: two), and no result lies over an input (CTAs read inputs while others write results;
-// the record pass reads them all first).  A list of one input without a norm keeps the record pass: callers count on its two launches.
+// A list of plain jobs of up to 4 rows in one launch with resident records; `taken` says whether it was.  It is where a CTA's range needs few
+// records and they leave enough of a ring, and no result lies over an input (CTAs read inputs while others write results; the record pass reads
+// them all first).  A launch less is worth 2.5 to 3 us in a chain of calls, and a record costs some 30 ns of every CTA, in which the
+// ring stands still once it is full.  Record pass and resident records, us, calls back to back:
+//   records of a CTA   4          24         60         90         120        148
+//   Q4_K               14.8/11.9  14.0/12.3  20.6/19.3  21.8/21.1  21.2/22.9  41.3/46.3
+//   IQ4_NL             15.0/12.3  14.6/13.0  27.1/25.8  27.6/27.6  27.9/28.8  55.2/56.0
+// (8 of 1024 -> 512; 2048 -> 300, 17408 -> 512, 1024 -> 9000 and 4096 -> 4096 of 3 rows; 3840 -> 3840, 3840 -> 15360 and 15360 -> 3840 of 2, 3 and 4 rows; 4 of
+// 17408 -> 5120 of 2 rows.)  Less of a ring than the two stages of Q8_0 that the record pass has as well loses by itself: 4 of 17408 -> 5120 in Q5_K, one row,
+// three stages of 44 KB 49.0, four 47.9.  A list of one input without a norm keeps the record pass; resident records are not measured there.
+constexpr int kWlMostRecords = 96, kWlLeastRing = 136 << 10;
 static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, const WlNorm *norm, bool &taken, zq_error *err) {
     taken = false;
     if (n_jobs > (size_t)kWlMaxJobs || (norm && (jobs[0].m != 1 || jobs[0].w->cols > (size_t)kWlNormTurns * kWlConsumers * 8))) return ZQ_OK;
@@ -813,22 +842,23 @@ static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_
     wa.q_total = (int)q_total;
     const int grid = ctx->sm_count < wa.q_total ? ctx->sm_count : wa.q_total, per_cta = (wa.q_total + grid - 1) / grid;
     if (per_cta / min_chunks + 3 > kWlMaxSegs) return ZQ_OK;
-    // records a range can need: the sources of neighbouring jobs that one range reaches
+    // records a range can need: the sources of neighbouring jobs that one range reaches, but no more than two units of each item
     int most = 0;
     for (size_t i = 0; i < n_jobs; ++i) {
-        int need = 0, between = 0;
+        int need = 0, between = 0, rows = 0;
         uint32_t seen = 0;
         for (size_t k = i; k < n_jobs && between < per_cta; ++k) {
             if (!(seen >> wa.jobs[k].src & 1)) need += src_units[wa.jobs[k].src] * wa.jobs[k].m;
             seen |= 1u << wa.jobs[k].src;
+            rows = std::max(rows, wa.jobs[k].m);
             if (k > i) between += wa.jobs[k].tiles * wa.jobs[k].chunks;
         }
-        most = std::max(most, need);
+        most = std::max(most, (int)std::min<long long>(need, (long long)kChunkUnits * per_cta * rows));
     }
     wa.stage_stride = kTileRows * kChunkUnits * unit_bytes;
     const long long left = (long long)WlResSmem<0>::OFF_XCH - (long long)most * kRec;
     wa.stages = left < 0 ? 0 : (int)std::min<long long>(5, left / wa.stage_stride);
-    if (wa.stages < (unit_bytes == 272 ? 2 : 3)) return ZQ_OK;  // with Q8_0 the ring of the record pass has two stages as well
+    if (most > kWlMostRecords || wa.stages * wa.stage_stride < kWlLeastRing) return ZQ_OK;
     wa.off_rec = wa.stages * wa.stage_stride;
     wa.chunk_words = 0;
     wa.y_dtype = y_dtype;
