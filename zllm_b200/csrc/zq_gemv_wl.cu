@@ -42,8 +42,8 @@ struct WlJob {
     int tiles;                 // row tiles
     int q_begin;               // first ring item of the job in the launch's (job, tile, chunk) order
     int y_dtype;               // output (and residual) dtype of this job
-    int src;                   // resident records: index into WlArgs::src
-    uint32_t type;             // GGUF type (mixed lists)
+    uint16_t src;              // resident records: index into WlResArgs::src
+    uint16_t type;             // GGUF type (mixed lists)
 };
 
 // Resident records: a distinct input block of the list in one record format.
@@ -66,14 +66,18 @@ struct WlArgs {
     int chunk_words;   // 32-bit words per chunk of a weight row
     int y_dtype;
     int async_fix;     // 5..8 rows: the finisher warp completes cut tiles (otherwise the consumers together)
-    int stages, stage_stride, off_rec;  // resident records: ring stages, bytes of one, where the records start
-    int n_src, x_dtype;
-    WlSrc src[kWlMaxJobs];
-    WlNormArgs norm;
     float *partials;   // [2 * grid][kSlotFloats]: slot 2c + 1 = the tile CTA c begins, slot 2c = the tile it continues
     uint32_t *counters;  // [grid], zero at the start of the launch: arrivals at the cut tile that CTA c begins
     uint32_t *status;
 };
+struct WlResArgs : WlArgs {
+    int stages, stage_stride, off_rec;  // ring stages, bytes of one, where the records start
+    int n_src, x_dtype;
+    WlSrc src[kWlMaxJobs];
+    WlNormArgs norm;
+};
+template <bool RES> struct WlArgsOf { using type = WlArgs; };
+template <> struct WlArgsOf<true> { using type = WlResArgs; };
 
 struct WlQuantSrc {
     const void *x;
@@ -201,7 +205,7 @@ struct WlRun {
 __device__ __forceinline__ int wl_run_place(const WlRun &r, int unit) { return unit < r.first ? unit - r.first + r.around : unit - r.first; }
 
 // The records of this CTA's range, by the 16 consumer warps.
-template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(const WlArgs &a, uint8_t *records, const WlRun *s_run, float *s_partial) {
+template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(const WlResArgs &a, uint8_t *records, const WlRun *s_run, float *s_partial) {
     constexpr bool MIX = TYPE == 0;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     auto store = [&](const WlSrc &src, int rec, const float (&v)[8]) {
@@ -294,7 +298,7 @@ template <uint32_t TYPE> __device__ __forceinline__ void wl_resident_records(con
 // the exchange buffer is indexed by lane and the owning warp stores its 16 rows straight from its fragments.
 // RES: resident records.  TYPE 0 (with RES): the jobs' types differ, each brings its own.
 template <uint32_t TYPE, int NT, bool GATED, bool RES>
-__global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_constant__ WlArgs a) {
+__global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_constant__ typename WlArgsOf<RES>::type a) {
     static_assert(!RES || (NT == 1 && !GATED), "resident records: up to 4 rows, plain jobs");
     constexpr bool MIX = TYPE == 0;
     using S = WlSmem<MIX ? (uint32_t)ZQ_Q4_K : TYPE, NT>;
@@ -730,7 +734,7 @@ static int launch_wl_quantize(zq_ctx *ctx, const WlQuantArgs &qa, zq_error *err)
 }
 
 template <uint32_t TYPE, int NT, bool GATED, bool RES = false>
-static int launch_wl_one(zq_ctx *ctx, const WlArgs &wa, zq_error *err) {
+static int launch_wl_one(zq_ctx *ctx, const typename WlArgsOf<RES>::type &wa, zq_error *err) {
     constexpr int smem = RES ? WlResSmem<TYPE>::TOTAL : WlSmem<TYPE ? TYPE : (uint32_t)ZQ_Q4_K, NT>::TOTAL;
     auto kernel = gemv_wl_kernel<TYPE, NT, GATED, RES>;
     static bool configured[64] = {};
@@ -761,7 +765,7 @@ static int launch_wl_type(zq_ctx *ctx, const WlArgs &wa, int nt, bool gated, zq_
     return gated ? launch_wl_one<TYPE, 4, true>(ctx, wa, err) : launch_wl_one<TYPE, 4, false>(ctx, wa, err);
 }
 
-static int launch_wl_resident(zq_ctx *ctx, uint32_t type, const WlArgs &wa, zq_error *err) {
+static int launch_wl_resident(zq_ctx *ctx, uint32_t type, const WlResArgs &wa, zq_error *err) {
     switch (type) {
     case 0: return launch_wl_one<0, 1, false, true>(ctx, wa, err);
     case ZQ_Q4_K: return launch_wl_one<ZQ_Q4_K, 1, false, true>(ctx, wa, err);
@@ -788,7 +792,7 @@ static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_
     taken = false;
     if (n_jobs > (size_t)kWlMaxJobs || (norm && (jobs[0].m != 1 || jobs[0].w->cols > (size_t)kWlNormTurns * kWlConsumers * 8))) return ZQ_OK;
     if (!norm && std::all_of(jobs, jobs + n_jobs, [&](const WlHostJob &j) { return j.x == jobs[0].x; })) return ZQ_OK;
-    WlArgs wa;
+    WlResArgs wa;
     wa.n_jobs = (int)n_jobs;
     wa.n_src = 0;
     uint32_t type = jobs[0].w->type;
@@ -823,8 +827,8 @@ static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_
         d.tiles = (int)tiles;
         d.q_begin = (int)q_total;
         d.y_dtype = j.y_dtype >= 0 ? j.y_dtype : y_dtype;
-        d.src = s;
-        d.type = j.w->type;
+        d.src = (uint16_t)s;
+        d.type = (uint16_t)j.w->type;
         q_total += tiles * chunks;
         min_chunks = std::min(min_chunks, d.chunks);
     }
@@ -1051,7 +1055,7 @@ int launch_gemv_wl(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtyp
             d.q_begin = wa.q_total;
             d.y_dtype = j.y_dtype >= 0 ? j.y_dtype : y_dtype;
             d.src = 0;
-            d.type = type;
+            d.type = (uint16_t)type;
             wa.q_total += (int)(tiles * chunks);
             if ((int)chunks < min_chunks) min_chunks = (int)chunks;
             if ((int)chunks > max_chunks) max_chunks = (int)chunks;
