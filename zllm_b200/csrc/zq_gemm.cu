@@ -23,11 +23,15 @@
 // stores.  A gated tile is 64 gate and 64 up rows per SM (128 outputs per pair), 16 of one and 16 of the other in turn: gate and up of
 // an output meet in one warp of the epilogue, and the accumulator still fits twice.
 //
-// Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..9
-// epilogue; SRC != 0: warp 10 TMA of packed boxes, warps 11..26 dequantisers.  Eight epilogue warps and not four, because a tile's epilogue is
+// Roles: warp 0 TMA (activations, and A when it is in memory), warp 1 MMA issue (first SM of the pair), warps 2..9 (Q6_K: 2..5 or 2..9)
+// epilogue; SRC != 0: then a warp for the TMA of packed boxes and sixteen dequantisers.  Eight epilogue warps and not four, because a tile's epilogue is
 // a chain of some 5 (gated: 50) instructions per element in each, which short tiles (few columns of K) do not hide and which the
 // last tile of a pair shows in full: Q4_K gated 1536 -> 3840 at 256 tokens 95 us, now 26; 4096 -> 11008 at 256 tokens 75 us, now 47 (with the
-// exchange of gate and up inside a warp; before, through shared memory and a barrier per 16 columns).
+// exchange of gate and up inside a warp; before, through shared memory and a barrier per 16 columns).  27 warps leave 72 registers each.  Q6_K,
+// whose dequantisers set the pace of most tiles and need more, has four epilogue warps (23 warps, 80 registers) where the epilogue is cheap:
+// plain, and gated up to 64 tokens per tile.  Eight and four, us: 11008 -> 4096 at 24 / 128 / 512 tokens 28.6 / 31.7 / 51.2 and 26.3 / 30.6 / 48.7, 4096 -> 11008 gated
+// 37.7 / 43.0 / 93.9 and 36.9 / 44.4 / 99.6.  Of the others Q5_K spills four registers there, and every form with wide tiles
+// 18 (gated 25), in the epilogue and the way out of cut tiles.
 // Every wait is bounded, counted from the end of the previous kernel; a wait that runs out sets the CTA's state, all roles fall
 // through to the end, TMEM is released and the context status word reports it.
 #include <algorithm>
@@ -43,7 +47,6 @@ constexpr int kWideBN = kGemmWideTokens;  // 320: most tokens per wide tile (pac
 constexpr int kChunk = 32, kChunks = 512 / kChunk;  // accumulator columns of wide tiles are given back in chunks of 32
 constexpr int kBK = 64;       // K elements per ring stage (128 bytes of f16: one swizzle atom row)
 constexpr int kStepK = 256;   // K elements per step: one packed unit, the grain in which tiles are cut
-constexpr int kEpi = 8;       // epilogue warps
 constexpr int kDqWarps = 16;  // thread = (row, k-block of a unit): four warps per k-block
 
 struct GemmParams {
@@ -196,7 +199,7 @@ template <int DT> __device__ __forceinline__ float raw_as_f32(uint32_t r) {
 }
 
 // Shared-memory plan: a ring stage is 16 KB of weights and half a tile's tokens (16 KB, WIDE 20 KB); packed boxes take what the stages leave.
-template <uint32_t SRC, bool WIDE> struct GemmSmem {
+template <uint32_t SRC, bool WIDE, int EPI> struct GemmSmem {  // EPI: epilogue warps
     static constexpr int unit_bytes = SRC == ZQ_Q8_0 ? 272 : SRC == ZQ_Q6_K ? 224 : SRC == ZQ_Q5_K ? 176 : 144;
     static constexpr int a_bytes = kBM * kBK * 2;
     static constexpr int stage_bytes = a_bytes + (WIDE ? kWideBN : kBN) / 2 * kBK * 2;
@@ -207,7 +210,7 @@ template <uint32_t SRC, bool WIDE> struct GemmSmem {
     static constexpr int off_bar = off_p + pstages * p_bytes;
     static constexpr int bar_bytes = 256 + (WIDE ? kChunks * 8 : 0);
     static constexpr int total = off_bar + bar_bytes + 1024;    // barriers, slack for 1024-byte alignment
-    static constexpr int threads = (2 + kEpi + (SRC ? 1 + kDqWarps : 0)) * 32;
+    static constexpr int threads = (2 + EPI + (SRC ? 1 + kDqWarps : 0)) * 32;
     static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
     static_assert(off_p % 1024 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
 };
@@ -357,13 +360,13 @@ template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(co
 // got 257 to 320 tokens was two tiles (256 experts of 7168 x 2048 in Q4_K, 8192 tokens, 256 +- 16 to an expert: MoE layer 8.2 ms, now 7.1).
 // A form of its own because the second piece costs the issuing warp instructions in every k-block: with one form for both, 48
 // tokens of 5120 x 17408 up and down took 61.2 us instead of 56.7.
-template <uint32_t SRC, bool GATED, bool WIDE>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>::threads, 1)
+template <uint32_t SRC, bool GATED, bool WIDE, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, EPI>::threads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const GemmParams p) {
-    using S = GemmSmem<SRC, WIDE>;
+    using S = GemmSmem<SRC, WIDE, EPI>;
     constexpr int STAGES = S::stages, PST = S::pstages > 0 ? S::pstages : 1;
     constexpr int kRows = GATED ? kPairM / 2 : kPairM;  // output rows of a tile
-    constexpr int kPackedWarp = 2 + kEpi;
+    constexpr int kPackedWarp = 2 + EPI;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + S::off_bar);  // first SM: a stage's operands, both SMs' bytes and dequantiser warps
@@ -397,9 +400,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>:
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
-            mbar_init(&acc_empty[b], 2 * kEpi);
+            mbar_init(&acc_empty[b], 2 * EPI);
         }
-        for (int c = 0; WIDE && c < kChunks; ++c) mbar_init(&step_free[c], 2 * kEpi);
+        for (int c = 0; WIDE && c < kChunks; ++c) mbar_init(&step_free[c], 2 * EPI);
         fence_mbar_init();
         s_state = kStateAhead;
         s_cuts = 0;
@@ -527,7 +530,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>:
                 // bring the tile's residual rows into L2 while its MMAs run: a warp can only have a few KB of loads in flight below
                 const size_t esz = dtype_size(p.y_dtype), r0 = (size_t)sg.row0 + rank * kBM;
                 const size_t bytes = (size_t)p.n_out * esz;
-                for (int i = et; i < n_tok * (int)esz; i += 32 * kEpi) {  // 128 rows = esz lines of 128 bytes per token
+                for (int i = et; i < n_tok * (int)esz; i += 32 * EPI) {  // 128 rows = esz lines of 128 bytes per token
                     const size_t at = r0 * esz + (size_t)(i % (int)esz) * 128;
                     if (at < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(p.residual) + (size_t)(sg.tok0 + i / (int)esz) * bytes + at));
                 }
@@ -599,7 +602,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>:
                         if (c0 < n_tok) store16(dt, c0, v);
                     }
                 } else {
-                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {  // walked as above, 48 tokens of 5120 x 17408 up and down take 63.8 us instead of 57.7
+                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * EPI) {  // walked as above, 48 tokens of 5120 x 17408 up and down take 63.8 us instead of 57.7
                         uint32_t v[16];
                         tmem_ld16(acc + c0, v);
                         store16(dt, c0, v);
@@ -617,7 +620,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>:
                 const int c_first = (int)(((ts + 1) * G - 1) / Q), c_last = (int)(((ts + walk.steps) * G - 1) / Q);  // pairs that own the tile's first and last step
                 float *slot = p.partials + ((size_t)(2 * pair + (sg.k0 == 0 ? 1 : 0)) * 2 + rank) * ((size_t)p.bn * kBM) + q * 32 + lane;
                 if (ok) {
-                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * kEpi) {
+                    for (int c0 = 16 * part; c0 < n_tok; c0 += 4 * EPI) {
                         uint32_t v[16];
                         tmem_ld16(acc + c0, v);
 #pragma unroll
@@ -625,7 +628,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE>:
                     }
                 }
                 __threadfence();
-                asm volatile("bar.sync 3, %0;" ::"n"(32 * kEpi) : "memory");
+                asm volatile("bar.sync 3, %0;" ::"n"(32 * EPI) : "memory");
                 if (et == 0 && ok && atomicAdd(p.counters + 2 * c_first + rank, 1u) == (uint32_t)(c_last - c_first)) s_cut[s_cuts++] = {sg.row0, sg.tok0, n_tok, c_first, c_last};
             }
             if (WIDE)
@@ -783,12 +786,12 @@ int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n
     return ZQ_OK;
 }
 
-template <uint32_t SRC, bool GATED, bool WIDE>
+template <uint32_t SRC, bool GATED, bool WIDE, int EPI>
 static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
-    using S = GemmSmem<SRC, WIDE>;
+    using S = GemmSmem<SRC, WIDE, EPI>;
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED, WIDE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
         configured[ctx->device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -801,14 +804,16 @@ static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->disable_pdl ? 0 : 1;
-    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED, WIDE>, mw, mw2, mx, mx2, p), err);
+    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED, WIDE, EPI>, mw, mw2, mx, mx2, p), err);
     ctx->launches++;
     return ZQ_OK;
 }
 template <uint32_t SRC> static int launch_form(zq_ctx *ctx, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
     constexpr bool W = SRC != 0;  // operands in memory have no wide tiles
-    if (W && p.wide) return gated ? launch_one<SRC, true, W>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, W>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    return gated ? launch_one<SRC, true, false>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, false>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    constexpr int Q6 = SRC == ZQ_Q6_K ? 4 : 8;  // see the roles
+    if (W && p.wide) return gated ? launch_one<SRC, true, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    if (gated && (Q6 == 8 || p.bn > 64)) return launch_one<SRC, true, false, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    return gated ? launch_one<SRC, true, false, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, false, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
 }
 static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
 #define ZQ_GEMM_CASE(T) case T: return launch_form<T>(ctx, gated, mw, mw2, mx, mx2, p, pairs, err)

@@ -208,7 +208,8 @@ template <> struct DqBlock<ZQ_Q6_K> {
     }
     __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
 #pragma unroll
-        for (int c8 = 0; c8 < 8; ++c8) {  // eight columns: block G = 2 kb + c8 / 4, scale group h = (c8 / 2) & 1, t = 2 (c8 & 1) and t + 1
+        for (int i = 0; i < 8; ++i) {  // eight columns: block G = 2 kb + c8 / 4, scale group h = (c8 / 2) & 1, t = 2 (c8 & 1) and t + 1
+            const int c8 = 2 * (i & 3) + (i >> 2);  // all that t = 0, 1 serve first: fewer registers are live (no spills in 72)
             const int gb = c8 >> 2, hh = (c8 >> 1) & 1, x2 = 2 * (2 * gb + hh);
             const float s = __fmul_rn(d, (float)(int8_t)(sc >> (8 * (2 * gb + hh))));
             const uint64_t s2 = dq_pair(s), c2 = dq_pair(-160.0f * s);  // the byte below is q = c + 32 (0..63): 128 + q - 160 = q - 32
