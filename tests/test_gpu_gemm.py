@@ -179,7 +179,7 @@ def test_prefill_wide_tiles(tensor_type, rows, m, gated, dtype, gemm_variant):
     assert torch.equal(a, run())
 
 
-@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0])
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0, H.Q6_K])
 @pytest.mark.parametrize("m,rows,cols", [(31, 63, 512), (260, 130, 1024)])
 def test_prefill_gated_edges(tensor_type, m, rows, cols):
     """64 gate and 64 up rows share a tile: ragged row counts, one and two token tiles, shares of a tile.

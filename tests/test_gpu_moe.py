@@ -209,6 +209,34 @@ def test_moe_prefill_grouping_on_the_device_equals_grouping_on_the_host():
     assert H.max_rel_error(on_device, want) <= 2 * BOUND
 
 
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q6_K])
+def test_moe_prefill_wide_tiles_of_ragged_experts(tensor_type):
+    """Tiles of up to 320 tokens of different experts, several per pair of SMs: full and short ones in turn, whose accumulators overlap or
+    not.  The bits of tiles of up to 256 tokens, and of the host's grouping."""
+    from zllm_b200.backend import MoeExperts, moe_forward
+
+    counts = [310, 17, 300, 190, 5, 320, 270, 560] * 2  # token tiles of 10, 1, 10, 6, 1, 10, 9 and twice 9 chunks of 32
+    n_exp, hidden, inter, m = len(counts), 4096, 1536, sum(counts)
+    c = ctx()
+    made = [[c.prepare_weight(tensor_type, H.random_weight(tensor_type, r, k, seed=840 + 3 * e + i), r, k) for e in range(3)] for i, (r, k) in enumerate([(inter, hidden), (inter, hidden), (hidden, inter)])]
+    table = MoeExperts(c, *[[w[e % 3] for e in range(n_exp)] for w in made])
+    rng = np.random.default_rng(84)
+    ids = torch.from_numpy(rng.permutation(np.repeat(np.arange(n_exp, dtype=np.int32), counts)).reshape(m, 1)).cuda()
+    x, w = dev(rng.standard_normal((m, hidden)).astype(np.float32), torch.bfloat16), dev(np.ones((m, 1), np.float32))
+
+    def run(option):
+        c.set_option(option, 1)
+        try:
+            return moe_forward(c, table, x, ids, w, out_dtype=torch.float32).clone()
+        finally:
+            c.sync()
+            c.set_option(option, 0)
+
+    wide, narrow, grouped_on_host = (run(o) for o in ("force_wide_tiles", "disable_wide_tiles", "force_moe_host_grouping"))
+    assert torch.isfinite(wide).all() and float(wide.abs().max()) > 0
+    assert torch.equal(wide, narrow) and torch.equal(wide, grouped_on_host)
+
+
 def test_shared_expert_of_another_width_takes_its_own_launches():
     """A shared expert shaped like the routed ones rides along in the grouped launches; any other shape runs as a
     separate gated MLP (src/moe/topk_moe.rs:84-104) and is added in the combine."""

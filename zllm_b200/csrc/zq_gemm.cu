@@ -927,7 +927,7 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
         const auto time = [&](const GemmParams &g) { return (((long long)row_tiles * ((g.m + g.bn - 1) / g.bn) + pairs - 1) / pairs) * std::max(850, 56 * g.bn / 10); };
         GemmParams wide = p;
         plan_tokens(m, kWideBN, wide);
-        if (wide.wide && time(wide) <= time(p)) p = wide;
+        if (wide.wide && (ctx->wide_tiles > 0 || (!ctx->wide_tiles && time(wide) <= time(p)))) p = wide;
     }
     p.y = y;
     p.residual = residual;

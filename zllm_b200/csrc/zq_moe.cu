@@ -624,6 +624,31 @@ static int ensure_moe_ws(zq_ctx *ctx, size_t bytes, zq_error *err) {
     return ZQ_OK;
 }
 
+// Whether an MoE prefill takes tiles of up to 320 tokens: `mean` = routes per expert (absent ones count).  They save a tile's dequantisation and
+// epilogue where an expert has just over 256 tokens, and cost elsewhere: the wide form keeps two boxes of packed weights for three,
+// issues twice as many MMAs and gives its accumulator back in chunks, all of which shows with few columns.  Whole layers, top 8 of 32 or 64, wide against
+// narrow in % of the time (tokens dealt evenly, and by expert^-0.4):
+//   mean                 144       232       264       312       400       520       580       800
+//   Q4_K  2048 x 1024    +16 +20   +18  +7    +7 +21   +16  +9   +21 +19    +4 +19    +5 +17   +12 +13
+//         4096 x 1024     +9 +13    +8  +1    -4 +15    +7  +3    +9  +8    +3  +8    +1  +8    +4  +6
+//         4096 x 1536     +5  +4   +13  -1   -18  +1    -2  -2    +7  -2    -7  +6    -5 +11    -2  +2
+//         5120 x 2048     +5  +5    -4  -8   -15  +3    -5  -6    +9  -2    -5  +1    -4  +3    -8  -1
+//   Q8_0  4096 x 1536     +4   0    +4  +2   -15  -1    +2  -4    +5  -2    -5  +6    -1  +5    -8  +2
+//   Q5_K  2048 x 2048     +9 +12   +11  +3    -5 +15    +5  +8   +18  +9    +2 +14    +1 +15    +7 +12
+//         4096 x 1536     +2  +1    +7  -4   -20  +2   -13  -6    +4 -10   -12  +2   -13   0    -6  -4
+//   Q6_K  4096 x 1536      0  -3    +4  -7   -25  -6   -19 -11     0 -10   -15  -3   -10  -5   -11 -12
+//         4096 x 1024     +3  +4    +4  -6   -14  +8    -8  -3    +3  -2   -11   0   -14   0    -7  -1
+//         5120 x 2048      0  -3    -6 -13   -25  -6   -22 -12    -1 -11   -21  -8   -20  -2   -19  -6
+// So: enough columns, and either a type for which a dequantisation saved outweighs the rest, or a mean whose tiles are fewer at 320 tokens.
+static bool moe_wide_tiles(uint32_t gate_type, uint32_t down_type, size_t hidden, size_t inter, size_t mean) {
+    const auto both = [&](uint32_t a, uint32_t b) { return (gate_type == a || gate_type == b) && (down_type == a || down_type == b); };
+    const bool q6 = both(ZQ_Q6_K, ZQ_Q6_K), costly = both(ZQ_Q5_K, ZQ_Q6_K);  // to dequantise
+    if (hidden < 4096 || inter < (costly ? 1024u : 1536u) || mean < 232) return false;
+    if (q6 || (costly && inter >= 1536)) return true;
+    const size_t high = mean + mean / 16;  // an expert on the upper side of the mean
+    return mean < 960 && (high + kGemmTileTokens - 1) / kGemmTileTokens > (high + kGemmWideTokens - 1) / kGemmWideTokens;
+}
+
 // MoE prefill, everything on the device: grouping (three small kernels), one gather that also
 // converts to f16, the two grouped fused GEMMs (their item counts read from device memory), shared expert, combine.
 static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *shared_gate, const zq_weight *shared_up, const zq_weight *shared_down, const void *dev_x, int x_dtype, size_t m, const uint32_t *dev_ids,
@@ -634,8 +659,7 @@ static int moe_prefill_device(zq_ctx *ctx, const zq_moe_experts *experts, const 
     const int chunks = (int)((m + tokens_per_chunk - 1) / tokens_per_chunk);
     const int rt_i = (int)((I + 127) / 128), rt_h = (int)((H + 255) / 256);  // 128 gated outputs or 256 rows per tile
     const size_t max_tiles = routes / kGemmTileTokens + E;  // at least the sum over experts of ceil(count / tile)
-    // Wide tiles where experts get enough tokens for some to go past 256; below, the narrow kernel's deeper ring of packed boxes.
-    const bool wide = routes >= 128 * E;
+    const bool wide = ctx->wide_tiles ? ctx->wide_tiles > 0 : moe_wide_tiles(experts->gate_type, experts->down_type, H, I, routes / E);
     auto al = [](size_t v) { return (v + 255) & ~size_t(255); };
     // tables and f32 results
     const size_t o_hist = 0, o_offsets = o_hist + al((size_t)chunks * E * 4), o_counts = o_offsets + al((E + 1) * 4), o_token_slots = o_counts + al(16);
