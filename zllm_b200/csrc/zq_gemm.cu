@@ -124,21 +124,6 @@ __device__ __forceinline__ void pair_sync() {
 // fence.proxy.async) or was ordered by a tcgen05 fence (accumulators).  A release at cluster scope drains all of the thread's
 // memory traffic first, which cost more than a k-block's MMAs at every stage.
 __device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
-// The arrival that gives a wide tile's accumulator back.  The MMA warp tells the phases of step_free apart by one parity bit, which is
-// enough if it sees the arrivals there of the tile before last no later than that tile's arrivals here: both go to another SM's barriers, so
-// it takes release and acquire at cluster scope (once per tile and warp).
-__device__ __forceinline__ void pair_arrive_release(uint32_t cluster_bar) { asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory"); }
-__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Operand row of row r of a gated box (64 gate rows, then 64 up rows): 16 gate rows and the 16 up rows of the same outputs alternate, so
 // that they meet in one epilogue warp.
 __device__ __forceinline__ int gated_row(int r) { return ((r & 63) >> 4) * 32 + (r >> 6) * 16 + (r & 15); }
@@ -180,9 +165,9 @@ __device__ __forceinline__ bool elect_one() {
 enum : uint32_t { kStateRun = 0, kStateAbort = 1, kStateAhead = 2 };
 // `sleep_ns` > 0: roles that share a scheduler with working warps back off between polls (a bare poll loop re-issues
 // every few tens of nanoseconds).
-template <bool CLUSTER = false> __device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t state_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
+__device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32_t state_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
     for (uint32_t i = 0; i < (1u << 23);) {
-        if (CLUSTER ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         uint32_t state;
         asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(state) : "r"(state_addr));
         if (state == kStateAbort) return false;
@@ -223,7 +208,7 @@ template <uint32_t SRC, bool WIDE, int EPI> struct GemmSmem {  // EPI: epilogue 
     static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 || (SRC == ZQ_Q6_K && WIDE) ? 4 : 5;
     static constexpr int off_p = stages * stage_bytes;
     static constexpr int off_bar = off_p + pstages * p_bytes;
-    static constexpr int bar_bytes = 256 + (WIDE ? kChunks * 8 : 0);
+    static constexpr int bar_bytes = 256 + (WIDE ? 2 * kChunks * 8 : 0);
     static constexpr int total = off_bar + bar_bytes + 1024;    // barriers, slack for 1024-byte alignment
     static constexpr int threads = (2 + EPI + (SRC ? 1 + kDqWarps : 0)) * 32;
     static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
@@ -417,7 +402,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 2 * EPI);
         }
-        for (int c = 0; WIDE && c < kChunks; ++c) mbar_init(&step_free[c], 2 * EPI);
+        for (int c = 0; WIDE && c < 2 * kChunks; ++c) mbar_init(&step_free[c], 2 * EPI);
         fence_mbar_init();
         s_state = kStateAhead;
         s_cuts = 0;
@@ -501,8 +486,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
                 before = chunks;
                 const uint32_t idesc0 = (1u << 4) | ((uint32_t)(kPairM >> 4) << 24), idesc = idesc0 | ((uint32_t)(first * (kChunk >> 3)) << 17), idesc2 = idesc0 | ((uint32_t)(second * (kChunk >> 3)) << 17);
                 const int b = iter & 1;
-                if (iter >= 2) ok = wait_flag<WIDE>(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
-                if (WIDE && ok && shared > 0) ok = wait_flag(&step_free[shared - 1], (uint32_t)(iter - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
+                // WIDE: every chunk of the tile before last is waited for, a lane each, and then the one shared with the last tile.  A barrier of one of
+                // the two sets is thus never more than one phase ahead of or behind the one asked for, whatever the order in which arrivals at
+                // different barriers are seen.
+                if (iter >= 2) {
+                    if constexpr (WIDE) ok = __all_sync(0xffffffffu, wait_flag(&step_free[b * kChunks + (lane & (kChunks - 1))], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout));
+                    else ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
+                }
+                if (WIDE && ok && shared > 0) ok = wait_flag(&step_free[(b ^ 1) * kChunks + shared - 1], (uint32_t)((iter - 1) >> 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
                 tc_fence_after();
                 const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * kBN), acc2 = acc + (uint32_t)(first * kChunk);
@@ -556,7 +547,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             auto free_step = [&](int k) {  // this warp is through with the k-th chunk
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) pair_arrive(pair_first(smem_u32(&step_free[k])));
+                if (lane == 0) pair_arrive(pair_first(smem_u32(&step_free[b * kChunks + k])));
             };
             const bool whole = sg.k0 == 0 && sg.k1 == walk.steps;
             // output row of this lane; gated: lanes 0..15 hold gate rows, lanes 16..31 the up rows of the same outputs
@@ -650,10 +641,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
                 for (int k = whole && ok ? chunks : 0; k < kChunks; ++k) free_step(k);
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {  // this warp's part of the accumulator may be overwritten
-                if constexpr (WIDE) pair_arrive_release(pair_first(smem_u32(&acc_empty[b])));
-                else pair_arrive(pair_first(smem_u32(&acc_empty[b])));
-            }
+            if (!WIDE && lane == 0) pair_arrive(pair_first(smem_u32(&acc_empty[b])));  // this warp's part of the accumulator may be overwritten
         }
     } else if constexpr (SRC != 0) {
         if (warp == kPackedWarp) {
