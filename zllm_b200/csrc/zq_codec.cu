@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t *__restri
 // once (zq_gemm_dq.cuh forms the same bits).  Up to kDequantBatch matrices of one type and shape
 // per launch (MoE prefill dequantises the experts of a chunk together).  One warp per 256-weight unit, 8 consecutive elements per lane: the
 // unit's packed bytes are read once with coalesced loads, the 512 output bytes are one coalesced store, and the only
-// index division is one per warp.
+// index division is one per warp.  `paired`: the rows alternate with those of another matrix, 16 by 16.
 constexpr int kDequantBatch = 96;
 struct DequantBatch {
     const uint8_t *src[kDequantBatch];
@@ -371,7 +371,7 @@ struct DequantBatch {
 };
 
 template <uint32_t TYPE>
-__global__ void __launch_bounds__(256) dequantize_f16_batch_kernel(const __grid_constant__ DequantBatch batch, size_t row_pitch, int unit_bytes, int rows, int cols, int units_per_row) {
+__global__ void __launch_bounds__(256) dequantize_f16_batch_kernel(const __grid_constant__ DequantBatch batch, size_t row_pitch, int unit_bytes, int rows, int cols, int units_per_row, bool paired) {
     const uint8_t *resident = batch.src[blockIdx.y];
     __half *out = batch.dst[blockIdx.y];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -387,12 +387,12 @@ __global__ void __launch_bounds__(256) dequantize_f16_batch_kernel(const __grid_
         packed.y = h2_as_u32(__floats2half2_rn(v[2], v[3]));
         packed.z = h2_as_u32(__floats2half2_rn(v[4], v[5]));
         packed.w = h2_as_u32(__floats2half2_rn(v[6], v[7]));
-        *reinterpret_cast<uint4 *>(out + (size_t)row * cols + k0) = packed;
+        *reinterpret_cast<uint4 *>(out + (size_t)(paired ? row + (row & ~15) : row) * cols + k0) = packed;
     }
 }
 
 // weights[i] -> outs[i], all of one type and shape.
-int launch_dequantize_f16_batch(zq_ctx *ctx, const zq_weight *const *weights, __half *const *outs, size_t count, zq_error *err) {
+int launch_dequantize_f16_batch(zq_ctx *ctx, const zq_weight *const *weights, __half *const *outs, size_t count, zq_error *err, bool paired) {
     for (size_t first = 0; first < count; first += kDequantBatch) {
         const size_t n = count - first < (size_t)kDequantBatch ? count - first : (size_t)kDequantBatch;
         const zq_weight *w0 = weights[first];
@@ -411,7 +411,7 @@ int launch_dequantize_f16_batch(zq_ctx *ctx, const zq_weight *const *weights, __
         if (bx > cap) bx = cap;
         if (bx == 0) bx = 1;
         const int rc = with_type(w0->type, err, [&](auto t) {
-            dequantize_f16_batch_kernel<decltype(t)::value><<<dim3((unsigned)bx, (unsigned)n), 256, 0, ctx->stream>>>(batch, w0->row_pitch, f.unit_bytes, (int)w0->rows, (int)w0->cols, (int)w0->units_per_row);
+            dequantize_f16_batch_kernel<decltype(t)::value><<<dim3((unsigned)bx, (unsigned)n), 256, 0, ctx->stream>>>(batch, w0->row_pitch, f.unit_bytes, (int)w0->rows, (int)w0->cols, (int)w0->units_per_row, paired);
             return ZQ_OK;
         });
         if (rc) return rc;
@@ -421,9 +421,9 @@ int launch_dequantize_f16_batch(zq_ctx *ctx, const zq_weight *const *weights, __
     return ZQ_OK;
 }
 
-int launch_dequantize_f16(zq_ctx *ctx, const zq_weight *w, __half *out, zq_error *err) {
+int launch_dequantize_f16(zq_ctx *ctx, const zq_weight *w, __half *out, zq_error *err, bool paired) {
     if (w->rows == 0 || w->cols == 0) return ZQ_OK;
-    return launch_dequantize_f16_batch(ctx, &w, &out, 1, err);
+    return launch_dequantize_f16_batch(ctx, &w, &out, 1, err, paired);
 }
 
 int launch_dequantize(zq_ctx *ctx, const zq_weight *w, const uint32_t *row_ids, size_t n_rows, void *out, int out_dtype, zq_error *err) {

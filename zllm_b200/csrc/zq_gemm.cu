@@ -454,12 +454,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
                     const uint32_t bar = pair_first(smem_u32(&full[s]));
                     if (rank == 0) mbar_expect_tx(&full[s], bytes);
                     if constexpr (SRC == 0) {
-#pragma unroll
-                        for (int h = 0; h < (GATED ? 8 : 1); ++h) {  // gated: 16 rows of gate, 16 of up, and so on
-                            const CUtensorMap *m = GATED && (h & 1) ? &map_w2 : &map_w;
-                            if (p.items) tma_load_3d_pair(st + h * (S::a_bytes / 8), m, bar, kb * kBK, row + (h >> 1) * 16, sg.z);
-                            else tma_load_2d_pair(st + h * (S::a_bytes / 8), m, bar, kb * kBK, row + (h >> 1) * 16);
-                        }
+                        const int at = GATED ? 2 * row : row;  // gated: 16 rows of gate, 16 of up, and so on in memory already
+                        if (p.items) tma_load_3d_pair(st, &map_w, bar, kb * kBK, at, sg.z);
+                        else tma_load_2d_pair(st, &map_w, bar, kb * kBK, at);
                     }
                     tma_load_2d_pair(st + S::a_bytes, two ? &map_x2 : &map_x, bar, kb * kBK, tok);
                     if (two) tma_load_2d_pair(st + S::a_bytes + kWideBN / 4 * kBK * 2, &map_x2, bar, kb * kBK, tok2);
@@ -944,9 +941,10 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     const size_t tiles = ((n + rows_per_tile - 1) / rows_per_tile) * ((m + p.bn - 1) / p.bn);
     if (tiles > (size_t)INT32_MAX / 4) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM: %zu rows x %zu tokens are too many for one call", n, m);
     const int pairs = plan_cut(ctx, (int)tiles, (int)((k + kStepK - 1) / kStepK), fused, gated, ((gated ? 2 : 1) * n + m) * k * 2, p);
-    const size_t w_bytes = fused ? 0 : (n * k * 2 + 1023) & ~size_t(1023);
+    const size_t w_rows = gated ? 2 * ((n + 15) & ~size_t(15)) : n;  // rows of the operand in memory
+    const size_t w_bytes = fused ? 0 : (w_rows * k * 2 + 1023) & ~size_t(1023);
     const size_t x_bytes = x_dtype == ZQ_F16 ? 0 : (m * k * 2 + 1023) & ~size_t(1023);
-    int rc = ensure_workspace(ctx, (gated ? 2 : 1) * w_bytes + x_bytes, err);
+    int rc = ensure_workspace(ctx, w_bytes + x_bytes, err);
     if (rc) return rc;
     LaunchScratch scratch;
     rc = take_shares(ctx, p, scratch, err);
@@ -954,7 +952,7 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     uint8_t *ws = reinterpret_cast<uint8_t *>(ctx->workspace);
     const __half *xin = reinterpret_cast<const __half *>(x);
     if (x_dtype != ZQ_F16) {
-        __half *x16 = reinterpret_cast<__half *>(ws + (gated ? 2 : 1) * w_bytes);
+        __half *x16 = reinterpret_cast<__half *>(ws + w_bytes);
         rc = launch_to_f16(ctx, x, x_dtype, x16, m * k, err, p.counters, p.counters ? 2 * p.cut_pairs : 0);
         xin = x16;
     } else if (p.counters) {
@@ -965,15 +963,14 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     rc = make_token_maps(xin, m, k, p, &map_x, &map_x2, err);
     if (rc) return rc;
     if (fused) return launch_src(ctx, w->type, gated, gated ? w->unit_map_half : w->qmv_map, gated ? w_up->unit_map_half : w->qmv_map, map_x, map_x2, p, pairs, err);
-    __half *w16 = reinterpret_cast<__half *>(ws), *w16b = reinterpret_cast<__half *>(ws + w_bytes);
-    rc = launch_dequantize_f16(ctx, w, w16, err);
-    if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16b, err);
+    __half *w16 = reinterpret_cast<__half *>(ws);
+    rc = launch_dequantize_f16(ctx, w, w16, err, gated);
+    if (!rc && gated) rc = launch_dequantize_f16(ctx, w_up, w16 + 16 * k, err, true);
     if (rc) return rc;
-    CUtensorMap map_w, map_w2;
-    rc = make_f16_map(w16, n, k, gated ? 16 : kBM, &map_w, err);
-    if (!rc) rc = make_f16_map(gated ? w16b : w16, n, k, gated ? 16 : kBM, &map_w2, err);
+    CUtensorMap map_w;
+    rc = make_f16_map(w16, w_rows, k, kBM, &map_w, err);
     if (rc) return rc;
-    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, map_x2, p, pairs, err);
+    return launch_src(ctx, 0, gated, map_w, map_w, map_x, map_x2, p, pairs, err);
 }
 
 static int grouped_params(zq_ctx *ctx, size_t rows, size_t k, size_t x_rows, const int4 *items, int n_items, const int *n_items_dev, bool wide, void *y, int y_dtype, GemmParams &p) {
@@ -993,21 +990,20 @@ static int grouped_params(zq_ctx *ctx, size_t rows, size_t k, size_t x_rows, con
     return n_items < pairs ? n_items : pairs;
 }
 
-// Grouped GEMM (MoE prefill): `mats` f16 weight matrices [rows, k] stacked in one buffer (and a second stack for the
-// gated form), one f16 activation operand [x_rows, k] whose row ranges belong to the matrices, a device work list of
-// {matrix, first row, first token row, end token row}.  y[token row, rows] in y_dtype; gated: silu(w x) * (w2 x).
-int launch_gemm_grouped(zq_ctx *ctx, const __half *w, const __half *w2, size_t mats, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, void *y, int y_dtype, zq_error *err) {
+// Grouped GEMM (MoE prefill): `mats` f16 weight matrices [rows, k] stacked in one buffer (gated: gate and up of each as one matrix of twice
+// the rows, 16 and 16 in turn; rows a multiple of 16), one f16 activation operand [x_rows, k] whose row ranges belong to the matrices, a device work list of
+// {matrix, first row, first token row, end token row}.  y[token row, rows] in y_dtype; gated: silu(gate x) * (up x).
+int launch_gemm_grouped(zq_ctx *ctx, const __half *w, bool gated, size_t mats, size_t rows, size_t k, const __half *x, size_t x_rows, const int4 *items, int n_items, void *y, int y_dtype, zq_error *err) {
     if (n_items <= 0) return ZQ_OK;
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "grouped GEMM needs columns aligned to 8, got %zu", k);
-    const bool gated = w2 != nullptr;
-    CUtensorMap map_w, map_w2, map_x;
-    int rc = make_f16_map3(w, mats, rows, k, gated ? 16 : kBM, &map_w, err);
-    if (!rc) rc = make_f16_map3(gated ? w2 : w, mats, rows, k, gated ? 16 : kBM, &map_w2, err);
+    if (gated && rows % 16) return set_error(err, ZQ_ERR_SHAPE, "gated grouped GEMM needs rows aligned to 16, got %zu", rows);
+    CUtensorMap map_w, map_x;
+    int rc = make_f16_map3(w, mats, gated ? 2 * rows : rows, k, kBM, &map_w, err);
     if (!rc) rc = make_f16_map(x, x_rows, k, kBN / 2, &map_x, err);
     if (rc) return rc;
     GemmParams p;
     const int pairs = grouped_params(ctx, rows, k, x_rows, items, n_items, nullptr, false, y, y_dtype, p);
-    return launch_src(ctx, 0, gated, map_w, map_w2, map_x, map_x, p, pairs, err);
+    return launch_src(ctx, 0, gated, map_w, map_w, map_x, map_x, p, pairs, err);
 }
 
 // Plain f16 x f16 GEMM on raw operands: y[m, rows] = x[m, k] w[rows, k]^T, f32 accumulation (router logits).  Whole tiles only:

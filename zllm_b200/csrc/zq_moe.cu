@@ -770,7 +770,7 @@ int zq_moe_route_topk(zq_ctx *ctx, int scoring, const void *dev_x, int x_dtype, 
             router_items_kernel<<<(n_items + 255) / 256, 256, 0, ctx->stream>>>(chunks, row_tiles, tok_tiles, (int)m, d_items);
             ctx->launches += 3;
             ZQ_CUDA_CHECK(cudaGetLastError(), err);
-            rc = launch_gemm_grouped(ctx, w3, nullptr, (size_t)chunks, num_experts, (size_t)kc, x3, (size_t)chunks * m, d_items, n_items, logits_g, ZQ_F32, err);
+            rc = launch_gemm_grouped(ctx, w3, false, (size_t)chunks, num_experts, (size_t)kc, x3, (size_t)chunks * m, d_items, n_items, logits_g, ZQ_F32, err);
             if (rc) return rc;
         } else {
             split_f16_chunked_kernel<<<grid_for(ctx, m * hidden / 8, 256), 256, 0, ctx->stream>>>(dev_x, x_dtype, m, (int)hidden, 0, (int)(3 * hidden), x3);  // one slice: the plain [rows][3 K] layout
@@ -1084,7 +1084,7 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
     } else if (grouped_gemm) {
         // Prefill: one grouped tensor-core GEMM per projection and chunk of experts instead of two launches per
         // expert (an expert's own GEMM has 16-56 tiles for 148 SMs).  The chunk's packed weights are dequantised to
-        // f16 stacks [chunk][rows][K] in the workspace; the work list holds one item per (expert, token tile, row
+        // f16 stacks [chunk][rows][K] in the workspace (gate and up alternate, 16 rows each); the work list holds one item per (expert, token tile, row
         // tile); tokens are the gathered slot rows, so outputs land in slot order as the combine expects.
         const size_t per_expert = 3 * I * H * sizeof(__half);
         size_t chunk = (size_t(3) << 30) / per_expert;  // ~3 GB of f16 operands at a time
@@ -1112,7 +1112,7 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
         rc = ensure_workspace(ctx, 3 * w_stack + x16_bytes + act16_bytes + items_bytes, err);
         if (rc) return rc;
         uint8_t *wsb = reinterpret_cast<uint8_t *>(ctx->workspace);
-        __half *wg16 = reinterpret_cast<__half *>(wsb), *wu16 = reinterpret_cast<__half *>(wsb + w_stack), *wd16 = reinterpret_cast<__half *>(wsb + 2 * w_stack);
+        __half *wgu16 = reinterpret_cast<__half *>(wsb), *wd16 = reinterpret_cast<__half *>(wsb + 2 * w_stack);
         __half *x16 = reinterpret_cast<__half *>(wsb + 3 * w_stack), *act16 = reinterpret_cast<__half *>(wsb + 3 * w_stack + x16_bytes);
         int4 *d_items = reinterpret_cast<int4 *>(wsb + 3 * w_stack + x16_bytes + act16_bytes);
         ZQ_CUDA_CHECK(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice, ctx->stream), err);
@@ -1130,8 +1130,8 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
             for (size_t e = cp.e0; e < cp.e1; ++e) {
                 if (offsets[e + 1] == offsets[e]) continue;
                 const size_t z = e - cp.e0;
-                wl_gu.push_back(experts->gate[e]); ol_gu.push_back(wg16 + z * I * H);
-                wl_gu.push_back(experts->up[e]); ol_gu.push_back(wu16 + z * I * H);
+                wl_gu.push_back(experts->gate[e]); ol_gu.push_back(wgu16 + z * 2 * I * H);
+                wl_gu.push_back(experts->up[e]); ol_gu.push_back(wgu16 + z * 2 * I * H + 16 * H);
                 wl_d.push_back(experts->down[e]); ol_d.push_back(wd16 + z * H * I);
             }
             // gate and up share shape but may differ in type from expert to expert only if the table was built so;
@@ -1140,12 +1140,12 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
             for (const zq_weight *w : wl_gu) uniform = uniform && w->type == wl_gu[0]->type;
             for (const zq_weight *w : wl_d) uniform = uniform && w->type == wl_d[0]->type;
             if (uniform) {
-                rc = launch_dequantize_f16_batch(ctx, wl_gu.data(), ol_gu.data(), wl_gu.size(), err);
+                rc = launch_dequantize_f16_batch(ctx, wl_gu.data(), ol_gu.data(), wl_gu.size(), err, true);
                 if (!rc) rc = launch_dequantize_f16_batch(ctx, wl_d.data(), ol_d.data(), wl_d.size(), err);
                 if (rc) return rc;
             } else {
                 for (size_t i = 0; i < wl_gu.size(); ++i) {
-                    rc = launch_dequantize_f16(ctx, wl_gu[i], ol_gu[i], err);
+                    rc = launch_dequantize_f16(ctx, wl_gu[i], ol_gu[i], err, true);
                     if (rc) return rc;
                 }
                 for (size_t i = 0; i < wl_d.size(); ++i) {
@@ -1153,9 +1153,9 @@ int zq_moe_forward(zq_ctx *ctx, const zq_moe_experts *experts, const zq_weight *
                     if (rc) return rc;
                 }
             }
-            rc = launch_gemm_grouped(ctx, wg16, wu16, cp.e1 - cp.e0, I, H, xin, routes, d_items + cp.gated_first, cp.gated_n, act16, ZQ_F16, err);
+            rc = launch_gemm_grouped(ctx, wgu16, true, cp.e1 - cp.e0, I, H, xin, routes, d_items + cp.gated_first, cp.gated_n, act16, ZQ_F16, err);
             if (rc) return rc;
-            rc = launch_gemm_grouped(ctx, wd16, nullptr, cp.e1 - cp.e0, H, I, act16, routes, d_items + cp.down_first, cp.down_n, d_out, ZQ_F32, err);
+            rc = launch_gemm_grouped(ctx, wd16, false, cp.e1 - cp.e0, H, I, act16, routes, d_items + cp.down_first, cp.down_n, d_out, ZQ_F32, err);
             if (rc) return rc;
         }
     } else {
