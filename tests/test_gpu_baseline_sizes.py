@@ -32,13 +32,13 @@ def _device_weight(rows, cols, seed, std=0.02):
     return w, packed.cpu().numpy()
 
 
-def _sample_check(got, packed, rows, cols, x_f32, row_blocks, tok_blocks, bound=BOUND):
+def _sample_check(got, packed, rows, cols, x_f32, row_blocks, tok_blocks, tensor_type=H.Q4_K, bound=BOUND):
     """got: [m, rows] device result (f32, host); packed: GGUF bytes of the whole weight."""
-    row_bytes = orc.row_bytes(H.Q4_K, cols)
+    row_bytes = orc.row_bytes(tensor_type, cols)
     worst = 0.0
     for (r0, nr), (t0, nt) in zip(row_blocks, tok_blocks):
         sub = packed[r0 * row_bytes:(r0 + nr) * row_bytes]
-        want = orc.linear(H.Q4_K, sub, nr, cols, np.ascontiguousarray(x_f32[t0:t0 + nt]))
+        want = orc.linear(tensor_type, sub, nr, cols, np.ascontiguousarray(x_f32[t0:t0 + nt]))
         worst = max(worst, H.max_rel_error(got[t0:t0 + nt, r0:r0 + nr], want))
     assert worst <= bound, f"max relative error {worst} on the sampled blocks"
 
@@ -72,14 +72,22 @@ def test_prefill_gemm_at_benchmark_size(variant, rows, cols, m):
         torch.cuda.empty_cache()
 
 
-@pytest.mark.parametrize("m", [1024, 1025])
-def test_prefill_gemm_around_the_kernel_switch(m):
-    """Up to 1 024 tokens Q4_K prefill takes the fused kernel, above it the operand pass: both sides of the switch."""
+@pytest.mark.parametrize("tensor_type,m", [(H.Q4_K, 1024), (H.Q4_K, 1025), (H.Q6_K, 1536), (H.Q6_K, 1537), (H.Q5_K, 4096), (H.Q5_K, 4097)])
+def test_prefill_gemm_around_the_kernel_switch(tensor_type, m):
+    """Q6_K prefill takes the kernel that dequantises inside up to 1 536 tokens, Q5_K of 2 048 columns up to 4 096, and the operand pass above:
+    both sides of either switch (Q4_K: the same kernel on both sides of 1 024)."""
     rows, cols = 5120, 2048
-    w, packed = _device_weight(rows, cols, seed=m)
+    if tensor_type == H.Q4_K:
+        w, packed = _device_weight(rows, cols, seed=m)
+    else:
+        packed = H.random_weight(tensor_type, rows, cols, seed=m)
+        w = ctx().prepare_weight(tensor_type, packed, rows, cols)
     x = torch.randn((m, cols), device="cuda", dtype=torch.float32).to(torch.bfloat16)
+    before = ctx().launch_count
     y = host(ctx().linear(x, w, out_dtype=torch.float32))
-    _sample_check(y, packed, rows, cols, x.float().cpu().numpy(), [(0, 32), (rows - 32, 32)], [(0, 32), (m - 32, 32)])
+    inside = tensor_type == H.Q4_K or m in (1536, 4096)
+    assert ctx().launch_count - before == (2 if inside else 3)  # conversion of the rows and GEMM; the operand pass is one more
+    _sample_check(y, packed, rows, cols, x.float().cpu().numpy(), [(0, 32), (rows - 32, 32)], [(0, 32), (m - 32, 32)], tensor_type)
     w.release()
 
 

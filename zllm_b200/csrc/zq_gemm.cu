@@ -903,20 +903,26 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     if (k % 8) return set_error(err, ZQ_ERR_SHAPE, "prefill GEMM needs columns aligned to 8, got %zu", k);
     // Dequantising inside the kernel saves the operand pass (one read of the packed weight, one write and one read of its f16
     // form); against it stands that every token tile dequantises the weight again, which its MMAs hide unless there are few columns per
-    // output (a short tile's epilogue competes with the dequantisers for issue) or the type is Q6_K, which takes the most instructions.  Both
-    // forms give the same bits.  Measured, inside / pass, us:
-    //   rows                     700        1100       2048       4096       8192       16384
-    //   Q4_K 5120 -> 17408       91/143     142/191    249/301    500/579    944/1150   1863/2430
-    //   Q8_0 5120 -> 17408       102/156    151/205    282/342    519/619    1136/1158  2269/2539
-    //   Q6_K 5120 -> 17408       160/190    242/195    299/309    705/587    1361/1009
-    //   IQ4_NL 3840 -> 15360     100/147    139/191    217/265    330/366    673/708    1499/1615
-    //   gated Q4_K 4096 -> 11008 109/159    146/207    271/342    528/649    1064/1177  2241/2469
-    //   gated Q6_K 4096 -> 11008 185/224    258/282    349/333    679/580
-    //   gated Q4_K 3072 -> 4096             78/109     96/130     154/190    289/330
-    //   gated Q4_K 2048 -> 4096             58/72      76/89      123/131    232/212
-    //   gated Q5_K 1536 -> 4096             57/63      70/74      117/105    200/166
-    //   Q4_K 512 -> 4096                    24/25      26/28      50/39      55/47
-    const bool inside = w->type == ZQ_Q6_K ? m <= 1024 : m <= 2048 || k >= 3072;
+    // output (a short tile's epilogue competes with the dequantisers for issue) or the type takes many instructions (Q6_K, then Q5_K, then
+    // IQ4_NL) and the rows are so many that the power cap, not the idle tensor cores, pays for them.  The operands are the same bits, and so
+    // are results where the tiles are cut alike.  Measured in turn, inside / pass, us:
+    //   rows                 1100       1500       2048       3001       4096       8192       16384
+    //   Q4_K   1024 -> 4096  16/21      17/23      18/23      23/27      33/33
+    //   Q4_K   2048 -> 8192  34/47      41/55      57/73      79/95      100/117    193/212    403/411
+    //   Q4_K   5120 -> 17408 146/214    203/277    276/356    427/522    523/625    1092/1173  2227/2315
+    //   IQ4_NL 5120 -> 17408 159/218    221/288    271/334    423/508    595/663    1159/1230  2314/2368
+    //   Q5_K   2048 -> 8192  35/48      44/54      62/72      90/98      108/111    224/214    437/396
+    //   Q5_K   4096 -> 11008 89/114     131/173    149/181    222/251    312/338    596/596    1234/1187
+    //   Q6_K   4096 -> 11008 99/105     115/137    166/165    271/249    372/323    701/575    1442/1119
+    //   gated:
+    //   Q4_K   2048 -> 8192  67/86      86/105     108/123    171/179    223/219    477/416    961/792
+    //   Q4_K   4096 -> 11008 156/227    189/264    292/366    375/465    540/637    1107/1195  2269/2367
+    //   Q8_0   4096 -> 11008 169/213    190/255    291/348    405/471    531/603    1141/1192  2333/2401
+    //   IQ4_NL 5120 -> 17408 341/455    406/546    517/645    831/969    1049/1148  2283/2392  5309/5012
+    //   Q5_K   4096 -> 11008 200/256    204/264    305/355    458/499    602/625    1301/1240  2615/2369
+    //   Q6_K   4096 -> 11008 181/200    243/257    341/329    493/446    750/623    1472/1145  3050/2250
+    const size_t most = w->type == ZQ_Q5_K ? (gated ? 6000 : k >= 3072 ? 12000 : 4096) : w->type == ZQ_IQ4_NL && (gated || k < 3072) ? 12000 : SIZE_MAX;
+    const bool inside = w->type == ZQ_Q6_K ? m <= 1536 : m <= 2048 || (k >= (gated ? 3072 : 2048) && m <= most);
     const bool fused = !ctx->disable_fused_gemm && (ctx->force_fused_gemm || inside) && has_i8_decode(w->type) && (!gated || w_up->type == w->type);
     GemmParams p;
     clear_params(ctx, p);
