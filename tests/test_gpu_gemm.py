@@ -18,13 +18,21 @@ BOUND = 2e-3
 
 @pytest.fixture(autouse=True, params=["fused", "operand_pass"])
 def gemm_variant(request):
-    """Every decode type runs on the kernel that dequantises inside the GEMM and on the separate f16 operand pass + plain GEMM;
-    both must produce the same bits, so every case runs on both."""
+    """Every decode type runs on the kernel that dequantises inside the GEMM and on the separate f16 operand pass + plain GEMM, and every
+    case on both.  Their operands are the same bits; results are where both deal their tiles out alike."""
     ctx().set_option("disable_fused_gemm", 1 if request.param == "operand_pass" else 0)
     ctx().set_option("force_fused_gemm", 1 if request.param == "fused" else 0)
     yield request.param
     ctx().set_option("disable_fused_gemm", 0)
     ctx().set_option("force_fused_gemm", 0)
+
+
+@pytest.fixture
+def cut_tiles():
+    """Tiles are cut along K wherever they can be, whatever the rule makes of the times."""
+    ctx().set_option("force_cut_tiles", 1)
+    yield
+    ctx().set_option("force_cut_tiles", 0)
 
 
 def test_fused_and_operand_pass_kernels_agree_bit_for_bit(gemm_variant):
@@ -110,7 +118,7 @@ def test_prefill_full_width_slice():
     (40, 25600, 512),   # 100 tiles: every tile cut along K
     (40, 43520, 512),   # 170 tiles: 96 of them cut, 74 whole
 ])
-def test_prefill_tiles_and_shares(tensor_type, m, rows, cols):
+def test_prefill_tiles_and_shares(tensor_type, m, rows, cols, cut_tiles):
     """Edges of the pair's tile (32 tokens, 128 and 256 rows) and the three ways tiles are dealt (whole, cut, both), with a
     residual; block-32 types on columns that end inside a k-block.  Bound as above: both operands are rounded to f16 once."""
     if tensor_type in (H.Q4_0, H.IQ4_NL, H.Q8_0):
@@ -133,22 +141,35 @@ def test_prefill_tiles_and_shares(tensor_type, m, rows, cols):
     (H.Q4_K, 256, 511, 8192, False, torch.float32),   # whole 256-token tiles
     (H.Q4_K, 40, 43520, 3072, False, torch.float32),  # 170 tiles: 96 of them cut, 74 whole
     (H.Q4_K, 70, 700, 3072, True, torch.float32), (H.Q8_0, 256, 77, 8192, True, torch.float16), (H.IQ4_NL, 33, 1030, 4096, True, torch.bfloat16),
+    (H.Q6_K, 290, 2001, 2048, False, torch.float32), (H.Q4_K, 610, 900, 4096, False, torch.float32), (H.Q5_K, 280, 700, 2048, True, torch.float32),  # wide where dequantised inside
 ])
-def test_prefill_cut_tiles(tensor_type, m, rows, cols, gated, dtype):
+def test_prefill_cut_tiles(tensor_type, m, rows, cols, gated, dtype, cut_tiles):
     """Long rows and few tiles: cut along K and added up at the end, with residual, every output type, ragged rows and tokens.
-    Bounds as in the tests around this one, plus the rounding of a 16-bit output (2^-9 bf16, 2^-12 f16)."""
+    Bounds as in the tests around this one, plus the rounding of a 16-bit output (2^-9 bf16, 2^-12 f16).  That tiles were cut shows in
+    the last bits of f32 results, whose sums are in another order than those of whole tiles."""
     ws = [H.random_weight(tensor_type, rows, cols, seed=m + rows + i) for i in range(2 if gated else 1)]
     x = dev(np.random.default_rng(m).standard_normal((m, cols)).astype(np.float32), torch.float16)
     wd = [ctx().prepare_weight(tensor_type, w, rows, cols) for w in ws]
     sel = np.unique(np.concatenate([np.random.default_rng(m + 2).choice(m, size=min(m, 7), replace=False), [0, m - 1]]))
     xs = x.float().cpu().numpy()[sel]
     rounding = {torch.float32: 0.0, torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -8}[dtype]
+    r = None if gated else dev(np.random.default_rng(m + 1).standard_normal((m, rows)).astype(np.float32), dtype)
+
+    def run():
+        return host((ctx().gated_linear(x, *wd, out_dtype=dtype) if gated else ctx().linear(x, wd[0], out_dtype=dtype, residual=r)).float())
+
+    ctx().set_option("force_wide_tiles", 1)
+    try:
+        got = run()
+        if dtype == torch.float32:
+            ctx().set_option("disable_cut_tiles", 1)
+            whole = run()
+            assert not np.array_equal(got, whole) and H.max_rel_error(got, whole) <= 1e-4
+    finally:
+        ctx().set_option("force_wide_tiles", 0)
     if gated:
-        got = host(ctx().gated_linear(x, *wd, out_dtype=dtype).float())
         assert H.max_rel_error(got[sel], orc.gated_linear(tensor_type, *ws, rows, cols, xs)) <= 2.1 * BOUND + rounding
         return
-    r = dev(np.random.default_rng(m + 1).standard_normal((m, rows)).astype(np.float32), dtype)
-    got = host(ctx().linear(x, wd[0], out_dtype=dtype, residual=r).float())
     want = orc.linear(tensor_type, ws[0], rows, cols, xs) + r.float().cpu().numpy()[sel]
     assert H.max_rel_error(got[sel], want) <= BOUND + rounding
 

@@ -28,7 +28,9 @@ def _call(c, w, x):
 def _fresh():
     from zllm_b200.backend import B200Context
 
-    return B200Context(0, use_torch_stream=False)
+    c = B200Context(0, use_torch_stream=False)
+    c.set_option("force_cut_tiles", 1)  # the first three calls' tiles are cut whatever the rule makes of the times
+    return c
 
 
 def _bits(t):
@@ -87,9 +89,13 @@ def test_scratch_that_another_shape_has_used():
     """Shapes whose counters and partial sums lie at different places of the same scratch, in turn without a wait."""
     jobs = [_setup(ctx(), *call, seed=230 + 4 * i) for i, call in enumerate(CALLS)]
     want = []
-    for j in jobs:
-        want.append(_bits(_call(ctx(), *j)))
-    got = [[_call(ctx(), *j) for j in jobs] for _ in range(10)]
+    ctx().set_option("force_cut_tiles", 1)
+    try:
+        for j in jobs:
+            want.append(_bits(_call(ctx(), *j)))
+        got = [[_call(ctx(), *j) for j in jobs] for _ in range(10)]
+    finally:
+        ctx().set_option("force_cut_tiles", 0)
     ctx().sync()
     for outs in got:
         assert all(np.array_equal(_bits(y), bits) for y, bits in zip(outs, want))

@@ -301,6 +301,7 @@ struct zq_ctx {
     int narrow_gemv_tiles = 0;  // integer-MMA decode, up to 4 rows: 64-row tiles, two CTAs per SM (measured slower; off)
     int disable_pdl = 0;     // launch decode and prefill kernels without programmatic dependent launch
     int disable_worklist = 0;  // zq_linear_batch and the multi-weight entries: one launch per job instead of the work-list kernel
+    int cut_tiles = 0;             // prefill tiles cut along K: 0 by the rule, -1 never, 1 wherever whole tiles leave part of a round empty
     int wide_tiles = 0;            // tiles of up to 320 tokens of packed weights: 0 by the rules, -1 never, 1 wherever they hold more than 256
     int force_fused_gemm = 0;      // prefill of the decode types: dequantisation inside the GEMM for every token count (tests)
     int disable_fused_gemm = 0;    // prefill: always the separate f16 operand pass

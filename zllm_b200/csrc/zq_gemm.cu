@@ -869,14 +869,14 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool ga
     const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
     const int rounds = (tiles + pairs - 1) / pairs, whole = tiles < pairs ? tiles : pairs;
     p.cut_tiles = p.cut_pairs = 0;
-    if (steps < 2 || tiles % pairs == 0 || (!fused && operand_bytes > (size_t(128) << 20))) return whole;
+    if (ctx->cut_tiles < 0 || steps < 2 || tiles % pairs == 0 || (!ctx->cut_tiles && !fused && operand_bytes > (size_t(128) << 20))) return whole;
     const int full = tiles / pairs, cut = full >= 2 ? tiles - (full - 1) * pairs : tiles;
     long long shares = (long long)cut * steps / 2;
     if (shares > 8LL * cut) shares = 8LL * cut;
     const int cut_pairs = shares < pairs && cut == tiles ? (int)shares : pairs;
     const long long saved = (long long)(rounds - (tiles - cut) / pairs) * steps - ((long long)cut * steps + cut_pairs - 1) / cut_pairs;
     const long long step_ns = std::max(fused ? 850LL : 500LL, 56LL * p.bn / 10), cost_ns = 3000 + (fused ? (gated ? 30LL : 50LL) : 160LL) * p.bn;
-    if (saved * step_ns <= cost_ns) return whole;
+    if (!ctx->cut_tiles && saved * step_ns <= cost_ns) return whole;
     p.cut_tiles = cut;
     p.cut_pairs = cut_pairs;
     return cut_pairs;
