@@ -858,24 +858,26 @@ static int make_token_maps(const __half *x, size_t rows, size_t k, const GemmPar
 // How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; cut, the tiles beyond the full rounds and one
 // round more (all of them when there are fewer than two rounds) take equal shares of at least two steps, at most eight of a tile.
 // Cutting saves the steps that the busiest pair is ahead of the average one, at 0.85 us (a dequantised step of up to 152 tokens) or 5.6 ns
-// per token each; it costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the
-// addition by all warps takes the place of an epilogue that eight of them compute).  From operands in memory it also costs what the pairs
-// then read at different depths of K and no longer share in L2: three times as much, and nothing is cut past L2's size.  Of 127
-// random shapes of 17 to 1024 tokens (256 to 20000 rows, 512 to 17408 columns, three types, plain and gated) the rule is 1.5 % behind the
-// better choice on average, never cutting 15 %, always 12 %.  Whole and cut, us:
-//   Q4_K 5120 -> 5120, 64 tokens 23.5 / 18.0;  11008 -> 4096, 300 tokens 67.5 / 48.6;  2048 -> 8192, 700 tokens 29.4 / 34.3;  5120 -> 17408, 512 tokens 64.8 / 74.3
-//   operands in memory: 16896 -> 576, 1900 tokens 113 / 87;  15360 -> 3840, 3001 tokens 345 / 431
+// per token each.  It costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the
+// addition by all warps takes the place of an epilogue that eight of them compute), and 2 us for every round more, in which pairs no longer meet at
+// the same depth of K.  From operands in memory that costs most: 160 ns per token, 240 when they do not fit in L2 together.  Without the rounds'
+// share the rule cut 343 of 960 shapes (64 to 8192 tokens, 2048 to 17408 columns, three types, plain and gated) and was 0.3 % behind the better
+// choice for plain ones on average and 1.7 % for gated ones, up to 12 %; with it 0.2 and 0.3 %.  Whole and cut, us:
+//   Q4_K 15360 -> 3840, 64 tokens 57 / 25;  11008 -> 4096, 64 tokens 43 / 22;  Q6_K 15360 -> 3840, 300 tokens 92 / 53
+//   not any more: Q4_K gated 4096 -> 11008, 512 tokens 74 / 83;  3840 -> 15360, 3001 tokens 553 / 587;  5120 -> 17408, 800 tokens 241 / 263
+//   operands in memory past L2: 15360 -> 3840, 2500 tokens 383 / 305, 3600 tokens 460 / 390;  not 2048 tokens 252 / 339, 3001 tokens 372 / 429
 static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool gated, size_t operand_bytes, GemmParams &p) {
     const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
     const int rounds = (tiles + pairs - 1) / pairs, whole = tiles < pairs ? tiles : pairs;
     p.cut_tiles = p.cut_pairs = 0;
-    if (ctx->cut_tiles < 0 || steps < 2 || tiles % pairs == 0 || (!ctx->cut_tiles && !fused && operand_bytes > (size_t(128) << 20))) return whole;
+    if (ctx->cut_tiles < 0 || steps < 2 || tiles % pairs == 0) return whole;
     const int full = tiles / pairs, cut = full >= 2 ? tiles - (full - 1) * pairs : tiles;
     long long shares = (long long)cut * steps / 2;
     if (shares > 8LL * cut) shares = 8LL * cut;
     const int cut_pairs = shares < pairs && cut == tiles ? (int)shares : pairs;
     const long long saved = (long long)(rounds - (tiles - cut) / pairs) * steps - ((long long)cut * steps + cut_pairs - 1) / cut_pairs;
-    const long long step_ns = std::max(fused ? 850LL : 500LL, 56LL * p.bn / 10), cost_ns = 3000 + (fused ? (gated ? 30LL : 50LL) : 160LL) * p.bn;
+    const long long step_ns = std::max(fused ? 850LL : 500LL, 56LL * p.bn / 10);
+    const long long cost_ns = 3000 + (fused ? (gated ? 30LL : 50LL) * p.bn + 2000LL * (rounds - 1) : (operand_bytes > (size_t(128) << 20) ? 240LL : 160LL) * p.bn);
     if (!ctx->cut_tiles && saved * step_ns <= cost_ns) return whole;
     p.cut_tiles = cut;
     p.cut_pairs = cut_pairs;
