@@ -858,13 +858,14 @@ static int make_token_maps(const __half *x, size_t rows, size_t k, const GemmPar
 // How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; cut, the tiles beyond the full rounds and one
 // round more (all of them when there are fewer than two rounds) take equal shares of at least two steps, at most eight of a tile.
 // Cutting saves the steps that the busiest pair is ahead of the average one, at 0.85 us (a dequantised step of up to 152 tokens) or 5.6 ns
-// per token each.  It costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the
-// addition by all warps takes the place of an epilogue that eight of them compute), and 2 us for every round more, in which pairs no longer meet at
-// the same depth of K.  From operands in memory that costs most: 160 ns per token, 240 when they do not fit in L2 together.  Without the rounds'
-// share the rule cut 343 of 960 shapes (64 to 8192 tokens, 2048 to 17408 columns, three types, plain and gated) and was 0.3 % behind the better
-// choice for plain ones on average and 1.7 % for gated ones, up to 12 %; with it 0.2 and 0.3 %.  Whole and cut, us:
+// per token each.  It costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the addition
+// takes the place of an epilogue), and 8 ns per token for every round more, in which pairs no longer meet at the same depth of K.  From
+// operands in memory that costs most: 160 ns per token, and past L2 140 where the cut part is little more than a round, 400 where it is more and
+// nothing is shared for long.  Without the rounds' share the rule cut 343 of 960 shapes (64 to 8192 tokens, 2048 to 17408 columns, three types,
+// plain and gated) and was 0.3 % behind the better choice for plain ones on average and 1.7 % for gated ones, up to 12 %; with it 0.2 and
+// 0.3 %.  Whole and cut, us:
 //   Q4_K 15360 -> 3840, 64 tokens 57 / 25;  11008 -> 4096, 64 tokens 43 / 22;  Q6_K 15360 -> 3840, 300 tokens 92 / 53
-//   not any more: Q4_K gated 4096 -> 11008, 512 tokens 74 / 83;  3840 -> 15360, 3001 tokens 553 / 587;  5120 -> 17408, 800 tokens 241 / 263
+//   not: Q4_K gated 4096 -> 11008, 512 tokens 74 / 83;  3840 -> 15360, 3001 tokens 553 / 587;  5120 -> 17408, 800 tokens 241 / 263
 //   operands in memory past L2: 15360 -> 3840, 2500 tokens 383 / 305, 3600 tokens 460 / 390;  not 2048 tokens 252 / 339, 3001 tokens 372 / 429
 static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool gated, size_t operand_bytes, GemmParams &p) {
     const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
@@ -877,7 +878,8 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, bool fused, bool ga
     const int cut_pairs = shares < pairs && cut == tiles ? (int)shares : pairs;
     const long long saved = (long long)(rounds - (tiles - cut) / pairs) * steps - ((long long)cut * steps + cut_pairs - 1) / cut_pairs;
     const long long step_ns = std::max(fused ? 850LL : 500LL, 56LL * p.bn / 10);
-    const long long cost_ns = 3000 + (fused ? (gated ? 30LL : 50LL) * p.bn + 2000LL * (rounds - 1) : (operand_bytes > (size_t(128) << 20) ? 240LL : 160LL) * p.bn);
+    const long long token_ns = fused ? (gated ? 30 : 50) + 8 * (rounds - 1) : operand_bytes <= (size_t(128) << 20) ? 160 : 3 * cut <= 4 * pairs ? 140 : 400;
+    const long long cost_ns = 3000 + token_ns * p.bn;
     if (!ctx->cut_tiles && saved * step_ns <= cost_ns) return whole;
     p.cut_tiles = cut;
     p.cut_pairs = cut_pairs;
@@ -930,12 +932,18 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
     clear_params(ctx, p);
     const int row_tiles = (int)((n + (gated ? kPairM / 2 : kPairM) - 1) / (gated ? kPairM / 2 : kPairM));
     plan_tokens(m, kBN, p);
-    // Wide tiles where the rounds of whole tiles, at a step's time each (see plan_cut), come out no longer.  us, tiles of up to 256 and of up to 320:
-    //   Q4_K 5120 -> 17408  270 tokens 48.4 / 39.5, 560 80.8 / 76.3, 800 124 / 117;  4096 -> 4096  300 tokens 31.4 / 50.9 (not taken)
-    //   4096 -> 11008  Q6_K 270 tokens 54.1 / 45.2, 900 94.6 / 70.9;  Q8_0 560 tokens 41.6 / 55.1 (not taken), 800 72.2 / 66.2;  gated Q4_K 300 tokens 70.5 / 80.0 (not taken)
+    // Wide tiles where the rounds of whole tiles come out shorter: a step is the dequantisation of one, 1.5 us beside the wide form's MMAs, or 5.6 ns
+    // per token, and a wide tile costs up to 40 ns per token more at its end, where its accumulator is given back in chunks (gated: 20 more; 20 less
+    // for types that are costly to dequantise, whose pace hides it).  Over 863 shapes of four types it is 0.4 % behind the better choice on
+    // average; with 0.85 us and nothing for the end it was 1.7 %.  us, tiles of up to 256 and of up to 320:
+    //   taken: Q4_K 5120 -> 17408 320 tokens 52 / 46; Q5_K 3840 -> 15360 560 tokens 71 / 60; Q6_K 3840 -> 15360 900 tokens 118 / 97, gated 5120 -> 17408 560 tokens 232 / 181
+    //   not: gated Q4_K 2048 -> 8192 640 tokens 43 / 51, 3840 -> 15360 6000 tokens 1028 / 1247, gated Q8_0 4096 -> 4096 5000 tokens 240 / 284
     if (fused && m > kBN) {
-        const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1;
-        const auto time = [&](const GemmParams &g) { return (((long long)row_tiles * ((g.m + g.bn - 1) / g.bn) + pairs - 1) / pairs) * std::max(850, 56 * g.bn / 10); };
+        const int pairs = ctx->sm_count / 2 > 0 ? ctx->sm_count / 2 : 1, steps = (int)((k + kStepK - 1) / kStepK);
+        const int end_ns = (gated ? 40 : 20) - (w->type == ZQ_Q5_K || w->type == ZQ_Q6_K ? 20 : 0);
+        const auto time = [&](const GemmParams &g) {
+            return (((long long)row_tiles * ((g.m + g.bn - 1) / g.bn) + pairs - 1) / pairs) * ((long long)steps * std::max(1500, 56 * g.bn / 10) + (g.wide ? end_ns * g.bn : 0));
+        };
         GemmParams wide = p;
         plan_tokens(m, kWideBN, wide);
         if (wide.wide && (ctx->wide_tiles > 0 || (!ctx->wide_tiles && time(wide) <= time(p)))) p = wide;
