@@ -787,7 +787,7 @@ def bench_config3(ctx, device, hbm_peak, sustained_tflops):
         del y
     pre["all_seven"] = {"ms": round(total_ms, 3), "tflops": round(total_flop / total_ms / 1e9, 1)}
     pre["roofline"] = {"bound": "tensor", "achieved": round(total_flop / total_ms / 1e9, 1), "peak": sustained_tflops, "unit": "TFLOP/s", "frac": round(total_flop / total_ms / 1e9 / sustained_tflops, 4),
-                       "kernels": "f16 operand pass (dequantise to the workspace) + tcgen05 GEMM: past 1024 rows the weights are not unpacked inside the GEMM"}
+                       "kernels": "conversion of the bf16 rows + tcgen05 GEMM with the weights unpacked inside"}
     out["prefill_m4096"] = pre
     for layer in weights:
         for w in layer.values():

@@ -58,7 +58,7 @@ int zq_ctx_use_own_stream(zq_ctx *ctx, zq_error *err);
 int zq_ctx_sync(zq_ctx *ctx, zq_error *err);
 /* Diagnostic switches (the counterpart of the reference's ZLLM_CUDA_* environment switches, kept per context).
  * Known keys (0/1): "force_staged_gemv", "force_f16_gemv" (decode on the f16 kernels instead of the integer-MMA kernel),
- * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "disable_cut_tiles" / "force_cut_tiles" (prefill tiles cut along K: never / wherever whole ones leave part of a round empty), "disable_wide_tiles" / "force_wide_tiles" (prefill tiles of packed weights: never more than 256 tokens / up to 320 wherever that is more), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_fused_gemm" / "force_fused_gemm" (prefill of Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL and Q8_0 never / always with the dequantisation inside the GEMM; default: up to 1024 tokens and MoE prefill). */
+ * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "disable_cut_tiles" / "force_cut_tiles" (prefill tiles cut along K: never / wherever whole ones leave part of a round empty), "disable_wide_tiles" / "force_wide_tiles" (prefill tiles of packed weights: never more than 256 tokens / up to 320 wherever that is more), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_fused_gemm" / "force_fused_gemm" (prefill of Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL and Q8_0 never / always with the dequantisation inside the GEMM; default: by type, form, rows and columns as measured, always up to 1024 tokens, and MoE prefill). */
 int zq_ctx_set_option(zq_ctx *ctx, const char *key, int value, zq_error *err);
 int zq_ctx_sm_count(const zq_ctx *ctx);
 /* Number of kernels this library has launched on the context since creation (bench accounting). */
@@ -101,7 +101,7 @@ int zq_linear_multi(zq_ctx *ctx, const zq_weight *const *w, size_t n_weights, co
  * the projections of a decode step that are ready together (q, k, v; gate and up; the layers of several sequences)
  * stream through one persistent kernel whose TMA ring never drains between matrices.  Per job: y = W x (+ residual),
  * or y = silu(gate x) * (up x) when `w_up` is given (then `w` is the gate; no residual).  Jobs of Q4_K / Q5_K / Q6_K /
- * Q4_0 / IQ4_NL / Q8_0 weights with up to 16 rows share launches (one per weight type, row-count class 1-4 / 5-8 / 9-16 and plain / gated);
+ * Q4_0 / IQ4_NL / Q8_0 weights with up to 16 rows share launches (one for plain jobs of up to 4 rows, whatever their types, where few of the inputs' values are needed by any one SM; else one per weight type, row-count class 1-4 / 5-8 / 9-16 and plain / gated);
  * every other job runs as its own zq_linear / zq_gated_silu call.  All jobs share x_dtype and y_dtype.  Results do not
  * depend on how the jobs are grouped beyond f32 rounding of the split-tile sums, and are the same from run to run. */
 enum { ZQ_JOB_ROW_PARALLEL = 1 };  /* zq_linear_job.flags: sum this job's result over the ranks of the peer group (zq_dist_init) */

@@ -57,7 +57,7 @@ struct GemmParams {
     int m;       // tokens
     int n_out;   // output features (weight rows; gated: rows of gate)
     int k;       // input columns
-    int bn;      // tokens per tile (multiple of 32, at most 256)
+    int bn;      // tokens per tile (multiple of 32, at most 256; wide tiles 320)
     int box_tok; // token rows of one activation box (half a tile's)
     int wide;    // tiles may have up to kWideBN tokens; those with more than kBN take two boxes of 80 token rows
     int cut_tiles, cut_pairs;  // the first cut_tiles tiles are cut along K into cut_pairs equal shares
@@ -295,7 +295,7 @@ struct GemmCut {
 // every tile is cut: 17408 -> 5120 in Q4_K, 48 / 256 / 512 tokens 40 / 88 / 89 us, now 32 / 47 / 75.
 template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(const GemmParams &p, const GemmCut &t, uint32_t rank) {
     constexpr int OUT = GATED ? kBM / 2 : kBM, QUADS = OUT / 4, PARTS = GATED ? 2 : 1, LANES = THREADS / QUADS;  // LANES: columns that the CTA takes side by side
-    constexpr int COLS = (THREADS > 256 ? 4 : 16) / PARTS;
+    constexpr int COLS = 4 / PARTS;
     const int quad = (int)threadIdx.x % QUADS, lane_col = (int)threadIdx.x / QUADS, row = t.row0 + (int)rank * OUT + 4 * quad;
     const int at0 = GATED ? gated_row(4 * quad) : 4 * quad;  // operand row; gated: of gate, up lies 16 rows on
     const int rows = p.n_out - row < 4 ? p.n_out - row : 4, esz = (int)dtype_size(p.y_dtype);

@@ -9,7 +9,9 @@
 //
 //   wl_quantize_kernel   activation records (zq_i8.cuh) of every distinct input block of the list, once, into global
 //                        memory; each ring stage then brings the records of its two units along with the weights
-//   gemv_wl_kernel       integer-MMA decode (arithmetic of zq_gemv_i8.cu) over the CTA's range
+//   gemv_wl_kernel       integer-MMA decode (arithmetic of zq_gemv_i8.cu) over the CTA's range; in lists of plain jobs of up to 4 rows that
+//                        need few records per CTA it makes these itself, in shared memory, an RMSNorm of one row included, and
+//                        jobs of several types share the launch
 //
 // Tiles that a range boundary cuts are finished without any CTA waiting for another: each contributor leaves its
 // partial tile in its own slot of the context's scratch and bumps the tile's arrival counter; whoever arrives last
@@ -907,8 +909,9 @@ bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m) 
     return single > even && (single - even) * kTileRows * kChunkUnits * format_info(gate->type).unit_bytes >= (m > 8 && is_kclass(gate->type) ? 300 : 216) * 1024;
 }
 
-// Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one record
-// pass per record format, then one decode launch per (weight type, column-tile count, plain / gated) class.
+// Runs the jobs (all of them supported, see gemv_wl_supported) in as few launches as their classes allow: one launch with resident
+// records where launch_gemv_wl_resident takes the list, else one record pass per record format, then one decode launch per (weight type,
+// column-tile count, plain / gated) class.
 // `own_scratch` (one job): records, partial tiles and counters are scratch of the call instead of context memory.  gemv_i8_kernel, the
 // other route of a gated pair, uses no context memory up to 4 rows: such a call may be replayed from a graph after any later call
 // and run on two streams of a context at once, on either route.

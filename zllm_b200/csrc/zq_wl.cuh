@@ -1,6 +1,7 @@
 // Host-side interface of the work-list decode kernel (zq_gemv_wl.cu): a list of independent projections, each
 // y[m, rows] = x[m, cols] W^T (+ residual), or silu(x gate^T) * (x up^T) when `w_up` is given, run in as few launches as
-// their (weight type, row count, plain / gated) classes allow.
+// their (weight type, row count, plain / gated) classes allow: one for a list of plain jobs of up to 4 rows, whatever their types, that needs few
+// activation records per CTA.
 #pragma once
 #include "zq_common.cuh"
 
@@ -18,7 +19,7 @@ struct WlHostJob {
     int y_dtype;            // output dtype of this job, or -1 for the call's
 };
 
-// True when the job can ride in a work-list launch (Q4_K / Q4_0 / Q8_0, up to 16 activation rows).
+// True when the job can ride in a work-list launch (Q4_K / Q5_K / Q6_K / Q4_0 / IQ4_NL / Q8_0, up to 16 activation rows).
 bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &job);
 // True when one gated pair (supported) is better dealt out by this kernel than launched on gemv_i8_kernel.
 bool gated_prefers_worklist(const zq_ctx *ctx, const zq_weight *gate, size_t m);
