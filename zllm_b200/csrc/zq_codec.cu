@@ -494,8 +494,8 @@ __device__ __forceinline__ void q4k_codes(const float (&v)[32], float scale, flo
 // c ^ (group & 7), which keeps both the arriving 16-byte chunks and a lane's reads of its own 128 bytes free of bank conflicts.
 // VEC: values and blocks are 16-byte aligned (a block is 144 bytes, so every block then is).
 // Super-blocks are taken from the last to the first: what wrote the values (a dequantisation, usually) wrote the last of them last, and
-// some of those need not come back from HBM.  17408 x 5120 (356 MB of values) behind a dequantisation: 0.5 to 1.5 % off both together
-// (151.8 -> 151.1 and 150.0 -> 148.0 us on two cards).
+// some of those need not come back from HBM.  It is worth no more than runs differ by: 17408 x 5120 (356 MB of values) behind a dequantisation,
+// four comparisons, 150.9 -> 148.2, 151.8 -> 151.1, 150.0 -> 148.0 and 150.7 -> 151.5 us for both.
 constexpr int kEncWarps = 8, kEncTile = 4 * 1024;  // warps per CTA; bytes of a warp's tile (four super-blocks of f32)
 constexpr int kEncSmem = kEncWarps * 2 * kEncTile;
 template <bool VEC>

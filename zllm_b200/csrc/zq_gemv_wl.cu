@@ -788,7 +788,8 @@ static int launch_wl_resident(zq_ctx *ctx, uint32_t type, const WlResArgs &wa, z
 //   IQ4_NL             15.0/12.3  14.6/13.0  27.1/25.8  27.6/27.6  27.9/28.8  55.2/56.0
 // (8 of 1024 -> 512; 2048 -> 300, 17408 -> 512, 1024 -> 9000 and 4096 -> 4096 of 3 rows; 3840 -> 3840, 3840 -> 15360 and 15360 -> 3840 of 2, 3 and 4 rows; 4 of
 // 17408 -> 5120 of 2 rows.)  Less of a ring than the two stages of Q8_0 that the record pass has as well loses by itself: 4 of 17408 -> 5120 in Q5_K, one row,
-// three stages of 44 KB 49.0, four 47.9.  A list of one input without a norm keeps the record pass; resident records are not measured there.
+// three stages of 44 KB 49.0, four 47.9.  A list of one input without a norm keeps the record pass, whose two launches a
+// test pins; what resident records would give there is not measured.
 constexpr int kWlMostRecords = 96, kWlLeastRing = 136 << 10;
 static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_jobs, int x_dtype, int y_dtype, const WlNorm *norm, bool &taken, zq_error *err) {
     taken = false;
