@@ -61,6 +61,34 @@ def test_prefill_linear_matches_cpu_matmul(tensor_type, m, rows, cols):
     assert H.max_rel_error(got, want) <= BOUND
 
 
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+@pytest.mark.parametrize("m,rows,cols,gated", [
+    (17, 1, 256, False), (32, 300, 512, True), (64, 19300, 1280, False),  # four units of tokens in the ring; pairs that walk two tiles on an odd number of units
+    (65, 9800, 768, True), (96, 130, 2816, False), (128, 19300, 1536, False), (128, 9800, 1280, True), (129, 300, 1280, False),  # two units; past the largest short tile
+])
+def test_short_tiles_agree_with_the_operand_pass_bit_for_bit(gemm_variant, tensor_type, m, rows, cols, gated):
+    """The weight operand in tensor memory is the operand pass's, k for k: whole tiles have the same bits."""
+    if gemm_variant == "operand_pass":
+        pytest.skip("compares a fused variant with the operand pass in one go")
+    if tensor_type in (H.Q4_0, H.IQ4_NL, H.Q8_0):
+        cols -= 96
+    g = torch.Generator(device="cuda").manual_seed(m + rows)
+    make = lambda: ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=int(torch.randint(0, 1000, (1,), generator=g, device="cuda"))), rows, cols)
+    w = [make() for _ in range(2 if gated else 1)]
+    x = torch.randn((m, cols), generator=g, device="cuda").to(torch.float16)
+    run = lambda: ctx().gated_linear(x, *w, out_dtype=torch.float32) if gated else ctx().linear(x, w[0], out_dtype=torch.float32)
+    ctx().set_option("disable_cut_tiles", 1)
+    try:
+        a = run()
+        ctx().set_option("force_fused_gemm", 0)
+        ctx().set_option("disable_fused_gemm", 1)
+        b = run()
+    finally:
+        ctx().set_option("disable_cut_tiles", 0)
+    assert torch.isfinite(a).all()
+    assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
 def test_prefill_reference_generator_case():
     """src/kernel/cuda/linear.rs:2176-2206 shape (M = 9 runs the decode kernel; M = 33 the tensor-core path) with
     the reference's own device gate 0.05 + 0.002*|e| as an outer bound."""

@@ -8,8 +8,15 @@
 // One kernel in two forms of the weight operand A (f16 [rows, K]; every value rounded once to f16, 2^-12 relative, which
 // keeps layer outputs inside the 2e-3 bound; bf16 operands would not):
 //   SRC = 0     A was dequantised to memory before (launch_dequantize_f16) and arrives by TMA
-//   SRC = type  the packed rows arrive by TMA and dequantiser warps write A into the swizzled shared-memory tile
+//   SRC = type  the packed rows arrive by TMA and dequantiser warps write A into the swizzled shared-memory tile or, SHORT, into tensor memory
 //               (zq_gemm_dq.cuh): the weight crosses HBM once, packed, and no operand pass runs
+// Tiles of up to 128 tokens (SHORT) put that operand into tensor memory instead: two units of 128 columns behind the two accumulators,
+// so its way through shared memory (written once, read once, the larger part of that memory's traffic here) is gone and the ring holds
+// two units instead of five quarters of one.  What set their pace was the warp that issues the MMAs: 540 cycles per 64-column k-block (a
+// successful wait 180, four MMAs and a commit 360, at a fifth of its scheduler's issue slots) where its MMAs take 128 at 64 tokens.  It now
+// waits and commits once per unit, sixteen MMAs.  5120 -> 17408 / 17408 -> 5120 at 48 tokens, us: Q4_K 23.5 / 29.4, now 20.3 / 26.2; Q6_K 34.0 / 38.1,
+// now 26.7 / 31.2; Q8_0 26.4 / 29.6, now 20.3 / 28.2.  With 128 to 256 tokens (one accumulator, the epilogue no longer under the next tile)
+// plain shapes stay as they are and gated ones take 10 to 20 % longer.
 // Activations are f16 (exact for bf16 inputs in f16 range), converted before the kernel where they are not.
 //
 // The two SMs of a cluster work on one tile of 256 weight rows x up to 256 tokens (cta_group::2, M = 256): each holds half
@@ -45,6 +52,10 @@ constexpr int kPairM = 256;   // weight rows per pair
 constexpr int kBN = kGemmTileTokens;      // 256: most tokens per MMA, and per tile of operands in memory
 constexpr int kWideBN = kGemmWideTokens;  // 320: most tokens per wide tile (packed types): two MMAs (pieces) of up to 160 share a dequantised operand
 constexpr int kChunk = 32, kChunks = 512 / kChunk;  // accumulator columns of wide tiles are given back in chunks of 32
+constexpr int kShortBN = 128;  // most tokens per tile with the weight operand in tensor memory
+constexpr int kShortA = 256;   // its two units of 128 columns there, behind the two accumulators
+constexpr int kShortStages = 4;  // most units of tokens in shared memory (two of more than 64 tokens)
+constexpr int kFormPlain = 0, kFormWide = 1, kFormShort = 2;  // FORM of gemm_kernel: what the tiles may be
 constexpr int kBK = 64;       // K elements per ring stage (128 bytes of f16: one swizzle atom row)
 constexpr int kStepK = 256;   // K elements per step: one packed unit, the grain in which tiles are cut
 constexpr int kDqWarps = 16;  // thread = (row, k-block of a unit): four warps per k-block
@@ -60,6 +71,7 @@ struct GemmParams {
     int bn;      // tokens per tile (multiple of 32, at most 256; wide tiles 320)
     int box_tok; // token rows of one activation box (half a tile's)
     int wide;    // tiles may have up to kWideBN tokens; those with more than kBN take two boxes of 80 token rows
+    int a_tmem;  // host: the weight operand goes to tensor memory (tiles of at most kShortBN tokens)
     int cut_tiles, cut_pairs;  // the first cut_tiles tiles are cut along K into cut_pairs equal shares
     float *partials;           // [2 * pairs][2 SMs][bn columns][128 rows] f32
     uint32_t *counters;        // arrivals per (pair that begins a cut tile, SM), zero at the start of the launch
@@ -94,6 +106,16 @@ __device__ __forceinline__ void umma2_f16_ss(uint32_t tmem_d, uint64_t desc_a, u
         ::"r"(tmem_d), "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// the same with A in tensor memory: each SM's 128 rows in its own lanes, two K elements per column
+__device__ __forceinline__ void umma2_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // Load and wait in one statement: between two the compiler may copy or spill the destination registers, which do not hold the
 // values before the wait.
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -127,6 +149,8 @@ __device__ __forceinline__ void pair_arrive(uint32_t cluster_bar) { asm volatile
 // Operand row of row r of a gated box (64 gate rows, then 64 up rows): 16 gate rows and the 16 up rows of the same outputs alternate, so
 // that they meet in one epilogue warp.
 __device__ __forceinline__ int gated_row(int r) { return ((r & 63) >> 4) * 32 + (r >> 6) * 16 + (r & 15); }
+// The way back: the box's row behind operand row a.
+__device__ __forceinline__ int box_row(int a) { return ((a >> 4) & 1) * 64 + (a >> 5) * 16 + (a & 15); }
 // Loads into this SM's shared memory whose completion counts on a barrier of the pair's first SM.  No multicast.
 __device__ __forceinline__ void tma_load_2d_pair(void *dst, const CUtensorMap *map, uint32_t cluster_bar, int x, int y) {
     asm volatile("cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)),
@@ -199,13 +223,15 @@ template <int DT> __device__ __forceinline__ float raw_as_f32(uint32_t r) {
 }
 
 // Shared-memory plan: a ring stage is 16 KB of weights and half a tile's tokens (16 KB, WIDE 20 KB); packed boxes take what the stages leave.
-template <uint32_t SRC, bool WIDE, int EPI> struct GemmSmem {  // EPI: epilogue warps
+// SHORT: the ring is 64 KB of tokens, units of half a tile's.
+template <uint32_t SRC, int FORM, int EPI> struct GemmSmem {  // EPI: epilogue warps
+    static constexpr bool WIDE = FORM == kFormWide, SHORT = FORM == kFormShort;
     static constexpr int unit_bytes = SRC == ZQ_Q8_0 ? 272 : SRC == ZQ_Q6_K ? 224 : SRC == ZQ_Q5_K ? 176 : 144;
-    static constexpr int a_bytes = kBM * kBK * 2;
-    static constexpr int stage_bytes = a_bytes + (WIDE ? kWideBN : kBN) / 2 * kBK * 2;
+    static constexpr int a_bytes = SHORT ? 0 : kBM * kBK * 2;
+    static constexpr int stage_bytes = SHORT ? 16384 : a_bytes + (WIDE ? kWideBN : kBN) / 2 * kBK * 2;
     static constexpr int p_bytes = SRC ? kBM * unit_bytes : 0;  // one packed box
-    static constexpr int pstages = SRC == 0 ? 0 : unit_bytes <= 144 && !WIDE ? 3 : 2;
-    static constexpr int stages = SRC == 0 ? 6 : SRC == ZQ_Q8_0 || (SRC == ZQ_Q6_K && WIDE) ? 4 : 5;
+    static constexpr int pstages = SRC == 0 ? 0 : SHORT ? (unit_bytes <= 144 ? 6 : unit_bytes <= 176 ? 5 : 4) : unit_bytes <= 144 && !WIDE ? 3 : 2;
+    static constexpr int stages = SRC == 0 ? 6 : SHORT ? kShortStages : SRC == ZQ_Q8_0 || (SRC == ZQ_Q6_K && WIDE) ? 4 : 5;
     static constexpr int off_p = stages * stage_bytes;
     static constexpr int off_bar = off_p + pstages * p_bytes;
     static constexpr int bar_bytes = 256 + (WIDE ? 2 * kChunks * 8 : 0);
@@ -214,6 +240,12 @@ template <uint32_t SRC, bool WIDE, int EPI> struct GemmSmem {  // EPI: epilogue 
     static_assert(total <= 232448 - 64, "prefill GEMM: shared memory");
     static_assert(off_p % 1024 == 0 && off_bar % 8 == 0, "prefill GEMM: alignment");
 };
+
+// SHORT: units of tokens in the ring, from the bytes of a k-block of one
+template <class S> __device__ __forceinline__ int short_stages(uint32_t sub) {
+    const int fit = (int)((uint32_t)S::off_p / (4 * sub));
+    return fit < S::stages ? fit : S::stages;
+}
 
 constexpr int kTokGroup = 8;  // token tiles per raster group: a weight tile is reused by 8 token tiles while it is hot in L2
 
@@ -360,10 +392,11 @@ template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(co
 // got 257 to 320 tokens was two tiles (256 experts of 7168 x 2048 in Q4_K, 8192 tokens, 256 +- 16 to an expert: MoE layer 8.2 ms, now 7.1).
 // A form of its own because the second piece costs the issuing warp instructions in every k-block: with one form for both, 48
 // tokens of 5120 x 17408 up and down took 61.2 us instead of 56.7.
-template <uint32_t SRC, bool GATED, bool WIDE, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, EPI>::threads, 1)
+template <uint32_t SRC, bool GATED, int FORM, int EPI>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, EPI>::threads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const GemmParams p) {
-    using S = GemmSmem<SRC, WIDE, EPI>;
+    using S = GemmSmem<SRC, FORM, EPI>;
+    constexpr bool WIDE = S::WIDE, SHORT = S::SHORT;
     constexpr int STAGES = S::stages, PST = S::pstages > 0 ? S::pstages : 1;
     constexpr int kRows = GATED ? kPairM / 2 : kPairM;  // output rows of a tile
     constexpr int kPackedWarp = 2 + EPI;
@@ -375,6 +408,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
     uint64_t *p_empty = p_full + PST;
     uint64_t *acc_full = p_empty + PST;                                // each SM
     uint64_t *acc_empty = acc_full + 2;                                // first SM: both SMs' epilogue warps
+    uint64_t *a_full = acc_empty + 2, *a_empty = a_full + 2;           // SHORT: a unit of weights in tensor memory: first SM, both SMs' dequantiser warps; each SM, its MMAs are done
     uint64_t *step_free = acc_empty + 2;                               // WIDE, first SM: both SMs' epilogue warps are through with the k-th chunk of a tile; once per tile each
     __shared__ uint32_t s_tmem;
     __shared__ uint32_t s_state;
@@ -391,7 +425,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            mbar_init(&full[s], SRC ? 9 : 1);  // the TMA issuer, and four dequantiser warps of each SM
+            mbar_init(&full[s], SRC && !SHORT ? 9 : 1);  // the TMA issuer, and four dequantiser warps of each SM
             mbar_init(&empty[s], 1);
         }
         for (int s = 0; s < PST; ++s) {
@@ -401,6 +435,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
         for (int b = 0; b < 2; ++b) {
             mbar_init(&acc_full[b], 1);
             mbar_init(&acc_empty[b], 2 * EPI);
+        }
+        for (int b = 0; SHORT && b < 2; ++b) {
+            mbar_init(&a_full[b], 2 * kDqWarps);
+            mbar_init(&a_empty[b], 1);
         }
         for (int c = 0; WIDE && c < 2 * kChunks; ++c) mbar_init(&step_free[c], 2 * EPI);
         fence_mbar_init();
@@ -444,6 +482,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             const uint32_t bytes = 2u * (uint32_t)((SRC ? 0 : S::a_bytes) + (two ? kWideBN / 2 : p.box_tok) * kBK * 2);
             const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
             const int kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
+            if constexpr (SHORT) {  // a stage is a unit: four k-blocks side by side
+                const uint32_t sub = (uint32_t)p.box_tok * kBK * 2;
+                const int stages = short_stages<S>(sub);
+                for (int u = sg.k0; u < sg.k1; ++u) {
+                    if (!fresh && !wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout)) {
+                        ok = false;
+                        break;
+                    }
+                    if (elect_one()) {
+                        uint8_t *st = smem + (size_t)s * 4 * sub;
+                        const uint32_t bar = pair_first(smem_u32(&full[s]));
+                        if (rank == 0) mbar_expect_tx(&full[s], 8 * sub);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) tma_load_2d_pair(st + i * sub, &map_x, bar, u * kStepK + i * kBK, tok);
+                    }
+                    __syncwarp();
+                    if (++s == stages) {
+                        s = 0;
+                        ph ^= 1u;
+                        fresh = false;
+                    }
+                }
+                continue;
+            }
             for (int kb = sg.k0 * 4; kb < kb1; ++kb) {
                 if (!fresh && !wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout)) {
                     ok = false;
@@ -476,6 +538,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             uint32_t ph = 0;
             bool ok = true;
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
+            uint32_t ah = 0, aph = 0;  // SHORT: which unit of weights in tensor memory, and its phase
             int before = 0;  // chunks of the tile before
             for (; ok && walk.next(p, sg); ++iter) {
                 // f32 accumulator, f16 A and B, both K-major, M = 256, N = the piece's tokens
@@ -493,8 +556,37 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
                 if (WIDE && ok && shared > 0) ok = wait_flag(&step_free[(b ^ 1) * kChunks + shared - 1], (uint32_t)((iter - 1) >> 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * kBN), acc2 = acc + (uint32_t)(first * kChunk);
+                const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * (SHORT ? kShortBN : kBN)), acc2 = acc + (uint32_t)(first * kChunk);
                 const int kb0 = sg.k0 * 4, kb1 = sg.k1 * 4 < k_blocks ? sg.k1 * 4 : k_blocks;
+                if constexpr (SHORT) {
+                    const uint32_t sub = (uint32_t)p.box_tok * kBK * 2;  // as the TMA warp has them
+                    const int stages = short_stages<S>(sub);
+                    for (int u = sg.k0; u < sg.k1; ++u) {
+                        ok = wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout) && wait_flag(&a_full[ah], aph, state_addr, p.status, kStatusTmaTimeout);
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (elect_one()) {
+                            uint64_t db = desc0 + (uint32_t)s * (4 * sub / 16);
+                            const uint32_t a = tmem_base + (uint32_t)(kShortA + ah * (kStepK / 2));
+#pragma unroll
+                            for (int i = 0; i < kStepK / 16; ++i) {
+                                umma2_f16_ts(acc, a + 8 * i, db + 2 * (i & 3), idesc, (i > 0 || u > sg.k0) ? 1u : 0u);
+                                if ((i & 3) == 3) db += sub / 16;
+                            }
+                            tc_commit2(&a_empty[ah]);
+                            tc_commit2(&empty[s]);
+                            if (u + 1 == sg.k1) tc_commit2(&acc_full[b]);
+                        }
+                        __syncwarp();
+                        if (++s == stages) {
+                            s = 0;
+                            ph ^= 1u;
+                        }
+                        aph ^= ah;
+                        ah ^= 1u;
+                    }
+                    continue;
+                }
                 for (int kb = kb0; kb < kb1; ++kb) {
                     ok = wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout);
                     if (!ok) break;
@@ -540,7 +632,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             }
             const bool ok = wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0);
             tc_fence_after();
-            const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * kBN) + ((uint32_t)(q * 32) << 16);
+            const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * (SHORT ? kShortBN : kBN)) + ((uint32_t)(q * 32) << 16);
             auto free_step = [&](int k) {  // this warp is through with the k-th chunk
                 tc_fence_before();
                 __syncwarp();
@@ -671,42 +763,79 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, WIDE, 
             }
         } else {
             // ------------------------------------------------ dequantisers: thread = (row, k-block of the unit)
-            const int t = threadIdx.x - (kPackedWarp + 1) * 32, row = t & (kBM - 1), mine = t >> 7;  // row of the box; mine: warp-uniform
-            const int a_row = GATED ? gated_row(row) : row, sw = a_row & 7;
-            const uint32_t row0 = smem_u32(smem) + (uint32_t)((a_row >> 3) * 1024 + sw * 128), box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
-            int s = 0, ps = 0;  // ring positions: s walks the k-blocks of all warps, this warp serves one in four
-            uint32_t ph = 0, pph = 0;
-            bool ok = true, fresh = true;
-            DqBlock<SRC> dq;
-            auto advance = [&](int n) {
-                s += n;
-                if (s >= STAGES) {
-                    s -= STAGES;
-                    ph ^= 1u;
-                    fresh = false;
-                }
-            };
-            while (ok && walk.next(p, sg)) {
-                for (int u = sg.k0; u < sg.k1; ++u) {
-                    ok = wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
-                    if (!ok) break;
-                    dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
-                    // Everything the warp needs of the box is in registers once this vote has read them.  Without it the arrival
-                    // overtakes shared-memory loads still queued behind other warps' stores, and the next box lands under them.
-                    if (__any_sync(0xffffffffu, dq.mix() == 0x9E3779B9u)) __nanosleep(0);  // a no-op that keeps the vote
-                    if (lane == 0) mbar_arrive(&p_empty[ps]);
-                    if (++ps == PST) {
-                        ps = 0;
-                        pph ^= 1u;
+            const int t = threadIdx.x - (kPackedWarp + 1) * 32, mine = t >> 7;  // mine: k-block of the unit, warp-uniform
+            if constexpr (SHORT) {
+                // Operand in tensor memory: a warp reaches the 32 lanes of its own quarter (warp number modulo four) only.
+                const int a_row = (warp & 3) * 32 + lane, row = GATED ? box_row(a_row) : a_row;
+                const uint32_t box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
+                const uint32_t a0 = tmem_base + (uint32_t)(kShortA + mine * (kBK / 2)) + ((uint32_t)((warp & 3) * 32) << 16);
+                const uint32_t full0 = pair_first(smem_u32(&a_full[0]));
+                int ps = 0;
+                uint32_t pph = 0, ah = 0, aph = 0;
+                bool ok = true;
+                DqBlock<SRC> dq;
+                while (ok && walk.next(p, sg)) {
+                    for (int u = sg.k0; u < sg.k1; ++u) {
+                        ok = wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
+                        if (!ok) break;
+                        dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
+                        ok = wait_flag(&a_empty[ah], aph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
+                        if (!ok) break;
+                        tc_fence_after();  // behind the MMAs that read this half before
+                        dq.emit(DqTensorRow{a0 + ah * (kStepK / 2)});
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) {
+                            pair_arrive(full0 + ah * (uint32_t)sizeof(uint64_t));
+                            mbar_arrive(&p_empty[ps]);  // all that was read of the box has been stored by now
+                        }
+                        aph ^= ah;
+                        ah ^= 1u;
+                        if (++ps == PST) {
+                            ps = 0;
+                            pph ^= 1u;
+                        }
                     }
-                    advance(mine);
-                    if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
-                    if (!ok) break;
-                    dq.emit(row0 + (uint32_t)(s * S::stage_bytes), sw);
-                    fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores of the pair
-                    __syncwarp();
-                    if (lane == 0) pair_arrive(pair_first(smem_u32(&full[s])));
-                    advance(4 - mine);
+                }
+            } else {
+                const int row = t & (kBM - 1);  // row of the box
+                const int a_row = GATED ? gated_row(row) : row, sw = a_row & 7;
+                const uint32_t row0 = smem_u32(smem) + (uint32_t)((a_row >> 3) * 1024 + sw * 128), box0 = smem_u32(smem) + (uint32_t)(S::off_p + row * S::unit_bytes);
+                int s = 0, ps = 0;  // ring positions: s walks the k-blocks of all warps, this warp serves one in four
+                uint32_t ph = 0, pph = 0;
+                bool ok = true, fresh = true;
+                DqBlock<SRC> dq;
+                auto advance = [&](int n) {
+                    s += n;
+                    if (s >= STAGES) {
+                        s -= STAGES;
+                        ph ^= 1u;
+                        fresh = false;
+                    }
+                };
+                while (ok && walk.next(p, sg)) {
+                    for (int u = sg.k0; u < sg.k1; ++u) {
+                        ok = wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
+                        if (!ok) break;
+                        dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
+                        // Everything the warp needs of the box is in registers once this vote has read them.  Without it the arrival
+                        // overtakes shared-memory loads still queued behind other warps' stores, and the next box lands under them.
+                        if (__any_sync(0xffffffffu, dq.mix() == 0x9E3779B9u)) __nanosleep(0);  // a no-op that keeps the vote
+                        if (lane == 0) mbar_arrive(&p_empty[ps]);
+                        if (++ps == PST) {
+                            ps = 0;
+                            pph ^= 1u;
+                        }
+                        advance(mine);
+                        if (!fresh) ok = wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
+                        if (!ok) break;
+                        dq.emit(DqSharedRow{row0 + (uint32_t)(s * S::stage_bytes), sw});
+                        fence_proxy_async();  // generic-proxy stores -> visible to the tensor cores of the pair
+                        __syncwarp();
+                        if (lane == 0) pair_arrive(pair_first(smem_u32(&full[s])));
+                        advance(4 - mine);
+                    }
                 }
             }
         }
@@ -789,12 +918,12 @@ int launch_to_f16(zq_ctx *ctx, const void *x, int x_dtype, __half *out, size_t n
     return ZQ_OK;
 }
 
-template <uint32_t SRC, bool GATED, bool WIDE, int EPI>
+template <uint32_t SRC, bool GATED, int FORM, int EPI>
 static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
-    using S = GemmSmem<SRC, WIDE, EPI>;
+    using S = GemmSmem<SRC, FORM, EPI>;
     static bool configured[64] = {};
     if (!configured[ctx->device & 63]) {
-        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED, WIDE, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemm_kernel<SRC, GATED, FORM, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::total), err);
         configured[ctx->device & 63] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -807,16 +936,17 @@ static int launch_one(zq_ctx *ctx, const CUtensorMap &mw, const CUtensorMap &mw2
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->disable_pdl ? 0 : 1;
-    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED, WIDE, EPI>, mw, mw2, mx, mx2, p), err);
+    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_kernel<SRC, GATED, FORM, EPI>, mw, mw2, mx, mx2, p), err);
     ctx->launches++;
     return ZQ_OK;
 }
 template <uint32_t SRC> static int launch_form(zq_ctx *ctx, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
-    constexpr bool W = SRC != 0;  // operands in memory have no wide tiles
+    constexpr int W = SRC ? kFormWide : kFormPlain, H = SRC ? kFormShort : kFormPlain;  // operands in memory have no other form
     constexpr int Q6 = SRC == ZQ_Q6_K ? 4 : 8;  // see the roles
     if (W && p.wide) return gated ? launch_one<SRC, true, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    if (gated && (Q6 == 8 || p.bn > 64)) return launch_one<SRC, true, false, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    return gated ? launch_one<SRC, true, false, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, false, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    if (H && p.a_tmem) return gated ? launch_one<SRC, true, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    if (gated && (Q6 == 8 || p.bn > 64)) return launch_one<SRC, true, kFormPlain, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    return gated ? launch_one<SRC, true, kFormPlain, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, kFormPlain, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
 }
 static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
 #define ZQ_GEMM_CASE(T) case T: return launch_form<T>(ctx, gated, mw, mw2, mx, mx2, p, pairs, err)
@@ -948,6 +1078,7 @@ int launch_gemm(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const vo
         plan_tokens(m, kWideBN, wide);
         if (wide.wide && (ctx->wide_tiles > 0 || (!ctx->wide_tiles && time(wide) <= time(p)))) p = wide;
     }
+    p.a_tmem = fused && p.bn <= kShortBN;
     p.y = y;
     p.residual = residual;
     p.y_dtype = y_dtype;

@@ -3,7 +3,7 @@
 // A dequantiser thread owns one row of a packed box (one 256-weight unit per row) and one 64-column k-block of it.
 // DqBlock<TYPE>::load brings what it needs of the unit into registers (at the row pitches of these formats the eight rows of
 // a quarter-warp's 16-byte loads fall into eight different bank groups, Q6_K excepted), emit() turns it into eight 16-byte
-// chunks and stores them at their 128-byte-swizzle positions (chunk c of row r at c ^ (r & 7)).  mix() reads every loaded
+// chunks and gives them to its sink: the 128-byte-swizzle positions of a row in shared memory (chunk c of row r at c ^ (r & 7)), or a lane of tensor memory.  mix() reads every loaded
 // register: an instruction that uses it has waited for the loads, so the box may be given back to the TMA unit behind it.  Shared memory is addressed
 // by 32-bit shared addresses: as generic accesses the stores cost the fence behind them several times as much.
 //
@@ -107,6 +107,20 @@ __device__ __forceinline__ uint32_t dq_lds32(uint32_t addr) {
     return v;
 }
 
+// Where emit() puts chunk c (columns 8 c .. 8 c + 7 of the k-block): the swizzled row of the operand tile in shared memory, or the
+// thread's lane of the operand in tensor memory (two columns of K per 32-bit column; the whole warp stores together).
+struct DqSharedRow {
+    uint32_t row_base;
+    int sw;
+    __device__ __forceinline__ void put(int c, uint4 v) const { dq_store(row_base, sw, c, v); }
+};
+struct DqTensorRow {
+    uint32_t at;
+    __device__ __forceinline__ void put(int c, uint4 v) const {
+        asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(at + 4u * (uint32_t)c), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+    }
+};
+
 template <uint32_t TYPE> struct DqBlock;
 
 template <bool Q5> struct DqBlockK {
@@ -154,7 +168,7 @@ template <bool Q5> struct DqBlockK {
         dq_fma_halves(dq_hfma2(odd, s2, k2), d, cn, v1, v3);
         return make_uint2(dq_pack(v0, v1), dq_pack(v2, v3));
     }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
+    template <class Sink> __device__ __forceinline__ void emit(const Sink &sink) const {
         const uint32_t w[8] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w};
 #pragma unroll
         for (int n = 0; n < 2; ++n) {  // low nibbles: group 2 kb, high nibbles: group 2 kb + 1
@@ -181,7 +195,7 @@ template <bool Q5> struct DqBlockK {
                     }
                     r[i] = four(even, odd, s2, k2, c[n]);
                 }
-                dq_store(row_base, sw, 4 * n + c8, make_uint4(r[0].x, r[0].y, r[1].x, r[1].y));
+                sink.put(4 * n + c8, make_uint4(r[0].x, r[0].y, r[1].x, r[1].y));
             }
         }
     }
@@ -206,7 +220,7 @@ template <> struct DqBlock<ZQ_Q6_K> {
     __device__ __forceinline__ uint32_t mix() const {
         return lo[0].x ^ lo[0].y ^ lo[1].x ^ lo[1].y ^ lo[2].x ^ lo[2].y ^ lo[3].x ^ lo[3].y ^ hi[0] ^ hi[1] ^ hi[2] ^ hi[3] ^ sc ^ __float_as_uint(d);
     }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
+    template <class Sink> __device__ __forceinline__ void emit(const Sink &sink) const {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {  // eight columns: block G = 2 kb + c8 / 4, scale group h = (c8 / 2) & 1, t = 2 (c8 & 1) and t + 1
             const int c8 = 2 * (i & 3) + (i >> 2);  // all that t = 0, 1 serve first: fewer registers are live (no spills in 72)
@@ -221,7 +235,7 @@ template <> struct DqBlock<ZQ_Q6_K> {
                 const uint32_t l = (hh ? (lw >> 4) : lw) & 0x0F0F0F0Fu, u = (x2 >= 4 ? (hw >> (x2 - 4)) : (hw << (4 - x2))) & 0x30303030u;
                 m[w] = (l | u) ^ 0x20202020u;
             }
-            dq_store(row_base, sw, c8, dq_chunk_fma(m[0], m[1], s2, c2));
+            sink.put(c8, dq_chunk_fma(m[0], m[1], s2, c2));
         }
     }
 };
@@ -236,7 +250,7 @@ template <bool NL> struct DqBlock4 {
         for (int t = 0; t < 4; ++t) p[t] = dq_lds64(unit + 16 + 16 * (t + 4 * (kb >> 1)) + 8 * (kb & 1));
     }
     __device__ __forceinline__ uint32_t mix() const { return p[0].x ^ p[0].y ^ p[1].x ^ p[1].y ^ p[2].x ^ p[2].y ^ p[3].x ^ p[3].y ^ d; }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
+    template <class Sink> __device__ __forceinline__ void emit(const Sink &sink) const {
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const uint32_t d2 = dq_prmt(d, 0u, b ? 0x3232u : 0x1010u);
@@ -259,10 +273,10 @@ template <bool NL> struct DqBlock4 {
                 }
             }
             constexpr uint32_t bias2 = NL ? 0x64806480u : 0x64086408u;  // 1024 + 128, 1024 + 8
-            dq_store(row_base, sw, 4 * b + 0, dq_chunk_mul(lo[0], lo[1], bias2, d2));
-            dq_store(row_base, sw, 4 * b + 1, dq_chunk_mul(lo[2], lo[3], bias2, d2));
-            dq_store(row_base, sw, 4 * b + 2, dq_chunk_mul(hi[0], hi[1], bias2, d2));
-            dq_store(row_base, sw, 4 * b + 3, dq_chunk_mul(hi[2], hi[3], bias2, d2));
+            sink.put(4 * b + 0, dq_chunk_mul(lo[0], lo[1], bias2, d2));
+            sink.put(4 * b + 1, dq_chunk_mul(lo[2], lo[3], bias2, d2));
+            sink.put(4 * b + 2, dq_chunk_mul(hi[0], hi[1], bias2, d2));
+            sink.put(4 * b + 3, dq_chunk_mul(hi[2], hi[3], bias2, d2));
         }
     }
 };
@@ -283,7 +297,7 @@ template <> struct DqBlock<ZQ_Q8_0> {  // piece t of a k-block: words t (columns
         for (int t = 0; t < 4; ++t) m ^= p[t].x ^ p[t].y ^ p[t].z ^ p[t].w;
         return m;
     }
-    __device__ __forceinline__ void emit(uint32_t row_base, int sw) const {
+    template <class Sink> __device__ __forceinline__ void emit(const Sink &sink) const {
 #pragma unroll
         for (int b = 0; b < 2; ++b) {
             const uint32_t d2 = dq_prmt(d, 0u, b ? 0x3232u : 0x1010u);
@@ -291,7 +305,7 @@ template <> struct DqBlock<ZQ_Q8_0> {  // piece t of a k-block: words t (columns
             for (int c = 0; c < 4; ++c) {
                 const uint4 &a0 = p[2 * (c & 1)], &a1 = p[2 * (c & 1) + 1];
                 const uint32_t w0 = b ? ((c >> 1) ? a0.w : a0.z) : ((c >> 1) ? a0.y : a0.x), w1 = b ? ((c >> 1) ? a1.w : a1.z) : ((c >> 1) ? a1.y : a1.x);
-                dq_store(row_base, sw, 4 * b + c, dq_chunk_mul(w0 ^ 0x80808080u, w1 ^ 0x80808080u, 0x64806480u, d2));
+                sink.put(4 * b + c, dq_chunk_mul(w0 ^ 0x80808080u, w1 ^ 0x80808080u, 0x64806480u, d2));
             }
         }
     }
