@@ -335,3 +335,29 @@ def test_an_output_that_does_not_fit_is_an_out_of_memory_error():
         ctx().linear(torch.zeros((1, 256), device="cuda"), Huge())
     w = ctx().prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, 64, 256, seed=4), 64, 256)
     assert torch.equal(ctx().linear(torch.zeros((1, 256), device="cuda"), w), torch.zeros((1, 64), device="cuda"))
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q5_K, H.Q6_K, H.Q4_0, H.IQ4_NL, H.Q8_0])
+@pytest.mark.parametrize("rows,cols,dtype", [
+    (1, 256, torch.float32), (17, 512, torch.float16), (2400, 1536, torch.bfloat16),  # a unit; a ragged group; more than one group per CTA
+    (513, 4096, torch.float32), (300, 4352, torch.bfloat16), (40, 16384, torch.float16),  # 16 units, one per warp; 17, two per warp; 64, four per warp
+    (33, 16640, torch.float32),  # 65 units: past what the one-pass kernel holds
+])
+def test_one_row_through_small_matrices(gemv_variant, tensor_type, rows, cols, dtype):
+    """One row: plain with a residual and gated, at the edges of the groups (16 rows), warps (16) and turns (4) of the one-pass kernel.  Bounds:
+    16-bit activations of a slice (see above); the result rounded to the output type once."""
+    if gemv_variant != "i8":
+        pytest.skip("the one-pass kernel is a form of the integer-MMA path")
+    if tensor_type in (H.Q4_0, H.IQ4_NL, H.Q8_0) and cols > 256:
+        cols -= 96
+    data = [H.random_weight(tensor_type, rows, cols, seed=rows + i) for i in range(2)]
+    w = [ctx().prepare_weight(tensor_type, d, rows, cols) for d in data]
+    g = np.random.default_rng(rows + cols)
+    x = dev(g.standard_normal((1, cols)).astype(np.float32), dtype)
+    r = dev(g.standard_normal((1, rows)).astype(np.float32), dtype)
+    xf = x.float().cpu().numpy()
+    tol = 3e-4 + {torch.float32: 0.0, torch.float16: 2 ** -11, torch.bfloat16: 2 ** -8}[dtype]
+    want = orc.linear(tensor_type, data[0], rows, cols, xf) + r.float().cpu().numpy()
+    assert H.max_rel_error(host(ctx().linear_add(x, w[0], r)), want) <= tol
+    want = orc.gated_linear(tensor_type, data[0], data[1], rows, cols, xf)
+    assert H.max_rel_error(host(ctx().gated_linear(x, w[0], w[1], out_dtype=torch.float32)), want) <= 1e-3  # products of two sums

@@ -81,3 +81,20 @@ def test_rmsnorm_records_and_rows_at_edge_widths(cols, m, dtype, shift):
     xn = _rmsnorm(x.float().cpu().numpy(), nw.cpu().numpy(), eps, 0.0)
     for t, d, y in zip(types, data, got):
         assert H.max_rel_error(host(y), orc.linear(t, d, rows, cols, xn)) <= (3e-4 if m <= 16 else 2e-3)
+
+
+@pytest.mark.parametrize("cols", [256, 4352, 16384])  # one unit; two units of 256 columns in some warps; four in each
+@pytest.mark.parametrize("dtype,shift", [(torch.float32, 0), (torch.bfloat16, 0), (torch.float32, 1)])  # shift: a row that is not 16-byte aligned
+def test_norm_and_projections_of_several_types_in_one_launch(cols, dtype, shift):
+    types, rows, eps = (H.Q4_K, H.Q8_0, H.Q6_K), (300, 16, 33), 1e-6
+    rng = np.random.default_rng(cols + shift)
+    data = [H.random_weight(t, r, cols, seed=cols + r) for t, r in zip(types, rows)]
+    ws = [ctx().prepare_weight(t, d, r, cols) for t, d, r in zip(types, data, rows)]
+    x = dev((rng.standard_normal(cols + shift) * 3.0).astype(np.float32), dtype)[shift:].reshape(1, cols)
+    nw = (1.0 + 0.1 * rng.standard_normal(cols)).astype(np.float32)
+    before = ctx().launch_count
+    got = [host(y) for y in ctx().rmsnorm_linear_multi(x, dev(nw), eps, ws, out_dtype=torch.float32)]
+    assert ctx().launch_count - before == 1
+    xn = _rmsnorm(x.float().cpu().numpy(), nw, eps, 0.0)
+    for y, t, d, r in zip(got, types, data, rows):
+        assert H.max_rel_error(y, orc.linear(t, d, r, cols, xn)) <= 3e-4

@@ -34,6 +34,7 @@
 #include <tuple>
 
 #include "zq_i8.cuh"
+#include "zq_row.cuh"
 
 namespace zq {
 
@@ -495,6 +496,16 @@ static int launch_i8_type(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up
 int launch_gemv_i8(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const GemvParams &p, bool &taken, zq_error *err) {
     taken = false;
     if (p.m < 1 || p.m > kMaxGemvRows) return ZQ_OK;
+    if (p.m == 1 && !ctx->narrow_gemv_tiles) {  // one row: the one-pass kernel where the matrix fits into shared memory
+        RowCall c;
+        c.jobs[0] = {w, w_up, p.y, p.residual, p.y_dtype};
+        c.n_jobs = 1;
+        c.x = p.x;
+        c.x_dtype = p.x_dtype;
+        c.norm = nullptr;
+        const int rc = launch_gemv_row(ctx, c, taken, err);
+        if (rc || taken) return rc;
+    }
     switch (w->type) {
     case ZQ_Q4_K: return launch_i8_type<ZQ_Q4_K>(ctx, w, w_up, p, taken, err);
     case ZQ_Q5_K: return launch_i8_type<ZQ_Q5_K>(ctx, w, w_up, p, taken, err);

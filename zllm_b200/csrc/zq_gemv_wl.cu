@@ -25,6 +25,7 @@
 #include <algorithm>
 
 #include "zq_i8.cuh"
+#include "zq_row.cuh"
 #include "zq_wl.cuh"
 
 namespace zq {
@@ -845,6 +846,16 @@ static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_
         for (int s = 0; s < wa.n_src; ++s)
             if (!apart(wa.jobs[k].y, y_bytes, wa.src[s].x, (size_t)wa.src[s].m * wa.src[s].cols * xe)) return ZQ_OK;
         if (norm && !apart(wa.jobs[k].y, y_bytes, norm->weight, (size_t)wa.src[0].cols * sizeof(float))) return ZQ_OK;
+    }
+    if (norm && n_jobs <= (size_t)kRowMaxJobs) {  // small matrices: the one-pass kernel, norm included
+        RowCall c;
+        for (size_t k = 0; k < n_jobs; ++k) c.jobs[k] = {jobs[k].w, nullptr, jobs[k].y, jobs[k].residual, wa.jobs[k].y_dtype};
+        c.n_jobs = (int)n_jobs;
+        c.x = norm->x;
+        c.x_dtype = norm->x_dtype;
+        c.norm = norm;
+        const int rc = launch_gemv_row(ctx, c, taken, err);
+        if (rc || taken) return rc;
     }
     wa.q_total = (int)q_total;
     const int grid = ctx->sm_count < wa.q_total ? ctx->sm_count : wa.q_total, per_cta = (wa.q_total + grid - 1) / grid;

@@ -410,8 +410,7 @@ template <uint32_t TYPE> __device__ __forceinline__ RecLane quantize_record(cons
     float amax = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
-#pragma unroll
-    for (int s = 16; s >= 1; s >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, s));
+    amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));  // not negative and no NaN: ordered like their bits
     const bool live = amax > 0.f && amax < 3.0e38f;
     const float inv = live ? __fdividef(kActMax, amax) : 0.f;
     o.scale = live ? __fdividef(1.f, inv) : 0.f;  // the scale actually applied: x ~ x_q / inv
