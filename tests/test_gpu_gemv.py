@@ -361,3 +361,20 @@ def test_one_row_through_small_matrices(gemv_variant, tensor_type, rows, cols, d
     assert H.max_rel_error(host(ctx().linear_add(x, w[0], r)), want) <= tol
     want = orc.gated_linear(tensor_type, data[0], data[1], rows, cols, xf)
     assert H.max_rel_error(host(ctx().gated_linear(x, w[0], w[1], out_dtype=torch.float32)), want) <= 1e-3  # products of two sums
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q8_0])
+@pytest.mark.parametrize("value", [1e-40, 1e-36, 3.2e38, float("inf"), float("nan")])
+def test_slices_without_a_scale_count_as_zero(gemv_variant, tensor_type, value):
+    """A 256-column slice whose maximum has no finite reciprocal scale (infinite, or so small that 32512 / maximum overflows), and an element that is not
+    a number, add nothing; the other slices are as without them."""
+    if gemv_variant != "i8":
+        pytest.skip("the records of the integer-MMA path")
+    rows, cols = 40, 768
+    w = ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=3), rows, cols)
+    for m in (1, 5):
+        x = np.random.default_rng(4).standard_normal((m, cols)).astype(np.float32)
+        x[:, 256:512] = 0.0
+        want = host(ctx().linear(dev(x), w)).copy()
+        x[:, 300] = value
+        np.testing.assert_array_equal(host(ctx().linear(dev(x), w)), want)

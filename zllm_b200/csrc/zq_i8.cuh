@@ -107,10 +107,6 @@ __device__ __forceinline__ uint32_t lop3_and_xor(uint32_t a, uint32_t b, uint32_
     asm("lop3.b32 %0, %1, %2, %3, 0x6A;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
     return r;
 }
-__device__ __forceinline__ uint32_t pack_s8x4(int a, int b, int c, int d) {
-    return (uint32_t)(a & 0xFF) | ((uint32_t)(b & 0xFF) << 8) | ((uint32_t)(c & 0xFF) << 16) | ((uint32_t)(d & 0xFF) << 24);
-}
-
 // Reader side of a record: the B fragment (k 4t..4t+3 | k 16+4t..) of scale group G, limb l, for lane-in-quad t
 // sits at byte (4 G + t) * 16 + 8 l.  Which activation columns those k stand for is the format's business:
 //   Q4_K        k-th byte of the 32-byte nibble pair  ->  slot t holds columns 8t..8t+7 of the group
@@ -411,21 +407,24 @@ template <uint32_t TYPE> __device__ __forceinline__ RecLane quantize_record(cons
 #pragma unroll
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
     amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));  // not negative and no NaN: ordered like their bits
-    const bool live = amax > 0.f && amax < 3.0e38f;
-    const float inv = live ? __fdividef(kActMax, amax) : 0.f;
+    const float ratio = __fdividef(kActMax, amax);
+    const bool live = amax > 0.f && amax < 3.0e38f && ratio <= 3.4e38f;  // a slice whose ratio overflows is 0 at the scale 1 / ratio anyway
+    const float inv = live ? ratio : 0.f;
     o.scale = live ? __fdividef(1.f, inv) : 0.f;  // the scale actually applied: x ~ x_q / inv
-    int hi[8], lo[8], sum = 0;
+    // |v inv| <= 32512 up to a few parts in 2^22, so x_q rounds into the range; what is not a number becomes 0.  Limbs: with q = x_q + 128, hi is
+    // byte 1 of q and lo = byte 0 less 128, which is that byte with its top bit turned over.
+    uint32_t q[8];
+    int sum = 0;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        int xq = __float2int_rn(v[j] * inv);
-        xq = xq > 32512 ? 32512 : (xq < -32512 ? -32512 : xq);
-        hi[j] = (xq + 128) >> 8;
-        lo[j] = xq - (hi[j] << 8);
+        const int xq = __float2int_rn(v[j] * inv);
+        q[j] = (uint32_t)(xq + 128);
         sum += xq;
     }
     // the lane's two quads (columns 8 lane .. +3 and +4 .. +7) as packed limbs
-    o.ph0 = pack_s8x4(hi[0], hi[1], hi[2], hi[3]); o.ph1 = pack_s8x4(hi[4], hi[5], hi[6], hi[7]);
-    o.pl0 = pack_s8x4(lo[0], lo[1], lo[2], lo[3]); o.pl1 = pack_s8x4(lo[4], lo[5], lo[6], lo[7]);
+    auto bytes = [](uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t sel) { return __byte_perm(__byte_perm(a, b, sel), __byte_perm(c, d, sel), 0x5410); };
+    o.ph0 = bytes(q[0], q[1], q[2], q[3], 0x0051); o.ph1 = bytes(q[4], q[5], q[6], q[7], 0x0051);
+    o.pl0 = bytes(q[0], q[1], q[2], q[3], 0x0040) ^ 0x80808080u; o.pl1 = bytes(q[4], q[5], q[6], q[7], 0x0040) ^ 0x80808080u;
     if constexpr (is_kclass(TYPE)) {
         o.slot = (uint32_t)lane * 16;  // group lane / 4, slot t = lane % 4: both quads are this lane's
     } else {
