@@ -342,9 +342,11 @@ def test_an_output_that_does_not_fit_is_an_out_of_memory_error():
     (1, 256, torch.float32), (17, 512, torch.float16), (2400, 1536, torch.bfloat16),  # a unit; a ragged group; more than one group per CTA
     (513, 4096, torch.float32), (300, 4352, torch.bfloat16), (40, 16384, torch.float16),  # 16 units, one per warp; 17, two per warp; 64, four per warp
     (33, 16640, torch.float32),  # 65 units: past what the one-pass kernel holds
+    (11013, 3840, torch.bfloat16),  # streamed: 4 or 5 groups per SM (gated: twice as many stages), the last one ragged
+    (11013, 2048, torch.float32),   # gated: two lanes of eight warps over the groups of a ring
 ])
 def test_one_row_through_small_matrices(gemv_variant, tensor_type, rows, cols, dtype):
-    """One row: plain with a residual and gated, at the edges of the groups (16 rows), warps (16) and turns (4) of the one-pass kernel.  Bounds:
+    """One row: plain with a residual and gated, at the edges of the groups (16 rows), warps (16) and turns (4) of the one-row kernels.  Bounds:
     16-bit activations of a slice (see above); the result rounded to the output type once."""
     if gemv_variant != "i8":
         pytest.skip("the one-pass kernel is a form of the integer-MMA path")

@@ -98,3 +98,20 @@ def test_norm_and_projections_of_several_types_in_one_launch(cols, dtype, shift)
     xn = _rmsnorm(x.float().cpu().numpy(), nw, eps, 0.0)
     for y, t, d, r in zip(got, types, data, rows):
         assert H.max_rel_error(y, orc.linear(t, d, r, cols, xn)) <= 3e-4
+
+
+@pytest.mark.parametrize("types", [(H.Q4_K, H.Q6_K, H.Q5_K), (H.Q8_0, H.IQ4_NL, H.Q4_0)])
+def test_norm_and_large_projections_of_several_types_in_one_launch(types):
+    """More than the SMs' shared memory holds: a CTA streams groups of one projection and goes on to the next one's, of another type."""
+    cols, rows, eps = 3840, (7001, 3000, 1003), 1e-6
+    rng = np.random.default_rng(77)
+    data = [H.random_weight(t, r, cols, seed=r) for t, r in zip(types, rows)]
+    ws = [ctx().prepare_weight(t, d, r, cols) for t, d, r in zip(types, data, rows)]
+    x = dev((rng.standard_normal((1, cols)) * 3.0).astype(np.float32), torch.float16)
+    nw = (1.0 + 0.1 * rng.standard_normal(cols)).astype(np.float32)
+    before = ctx().launch_count
+    got = [host(y) for y in ctx().rmsnorm_linear_multi(x, dev(nw), eps, ws, out_dtype=torch.float32)]
+    assert ctx().launch_count - before == 1
+    xn = _rmsnorm(x.float().cpu().numpy(), nw, eps, 0.0)
+    for y, t, d, r in zip(got, types, data, rows):
+        assert H.max_rel_error(y, orc.linear(t, d, r, cols, xn)) <= 3e-4

@@ -1,4 +1,5 @@
-// Decode of one activation row through a small matrix: everything a CTA needs lies in shared memory, one pass, no ring, no cluster.
+// Decode of one activation row: whole rows of the weight per CTA, K over its warps, no cluster and nothing shared between CTAs.  Small matrices lie in
+// shared memory at once (gemv_row_kernel), larger ones go through a ring of row groups (gemv_row_stream_kernel).
 //
 // A projection of a few MB streams from HBM in a microsecond, and with programmatic dependent launch its weights arrive under the kernel before
 // it.  What is left is the chain from that kernel's end to this one's: 1536 -> 1536 in Q4_K took gemv_i8_kernel 4.7 us in a chain of its like, of
@@ -24,6 +25,7 @@ namespace zq {
 
 constexpr int kRowWarps = 16;      // most warps of a CTA
 constexpr int kRowMaxGroups = 16;  // most groups of 16 weight rows of a CTA
+constexpr int kRowSums = 4;        // groups whose sums may wait to be added up
 constexpr int kRowTurns = 4;       // most units per warp
 constexpr int kRowMaxSmem = 232448 - 1024;  // opt-in maximum minus static shared memory
 
@@ -41,7 +43,8 @@ struct RowArgs {
     int n_jobs;
     const void *x;
     int x_dtype, cols, units;
-    int groups;            // groups of 16 outputs per CTA
+    int groups;            // groups of 16 outputs per CTA; streamed: stages of the ring
+    int all_groups, stage_bytes;  // streamed: groups of all jobs (cta0: a job's first group), bytes of a stage
     int lanes_k, lanes_g;  // warps side by side along K, and over the groups
     int turns;             // most units per warp
     int off_rec, off_red;  // shared memory: weights at 0, records [warp][turn], partial sums [warp along K][group][16]
@@ -55,6 +58,107 @@ __host__ __device__ inline int row_unit_bytes(uint32_t type) { return type == ZQ
 // Bytes between rows in shared memory: whole 128-byte lines and a quarter (K-quants: eight-byte fragment loads of four rows) or a half (16-byte
 // ones of two) of one more, which spreads the rows that one access touches over the banks.
 __host__ __device__ inline int row_smem_pitch(uint32_t type, int units) { return ((units * row_unit_bytes(type) + 127) & ~127) + (type == ZQ_Q4_K || type == ZQ_Q5_K ? 32 : 64); }
+
+// The records of the units that this warp multiplies (unit ul, ul + lanes_k, ..), one after the other in its own place; with a norm in front all `threads` of
+// these warps meet once.
+template <uint32_t TYPE, bool GATED> __device__ __forceinline__ void row_records(const RowArgs &a, uint32_t type, uint8_t *rec_mine, int ul, int warp, int lane, int threads, float *s_partial) {
+    constexpr bool MIX = TYPE == 0;
+    auto store_rec = [&](int k, const float (&v)[8]) {
+        uint8_t *dst = rec_mine + k * kRec;
+        auto put = [&](auto kclass) {
+            constexpr uint32_t T = decltype(kclass)::value ? (uint32_t)ZQ_Q4_K : (uint32_t)ZQ_Q4_0;
+            const RecLane o = quantize_record<T>(v, lane);
+            *reinterpret_cast<uint4 *>(dst + o.slot) = make_uint4(o.ph0, o.ph1, o.pl0, o.pl1);
+            if (is_kclass(T) && (lane & 7) == 0) *reinterpret_cast<uint2 *>(dst + kRecSums + (lane >> 3) * 8) = make_uint2(o.sw0, o.sw1);
+            if (lane == 0) *reinterpret_cast<float *>(dst + kRecScale) = o.scale;
+        };
+        if (MIX ? is_kclass(type) : is_kclass(TYPE)) put(std::true_type());
+        else put(std::false_type());
+    };
+
+    if (!GATED && a.norm_weight) {  // the arithmetic of rmsnorm_kernel (zq_norm.cu)
+        float v[kRowTurns][8], w[kRowTurns][8];
+        auto load = [&](const void *p, int dtype, bool wide, int k0, float (&o)[8]) {
+            if (wide) {
+                load_act8(p, dtype, (size_t)k0, k0 < a.cols, o);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) o[e] = k0 < a.cols ? load_as_f32(p, dtype, (size_t)k0 + e) : 0.f;
+            }
+        };
+        float acc = 0.f;
+#pragma unroll
+        for (int k = 0; k < kRowTurns; ++k) {
+            const int u = ul + k * a.lanes_k;
+            if (u >= a.units) break;
+            load(a.x, a.x_dtype, a.x_wide, u * kUnitWeights + 8 * lane, v[k]);
+            load(a.norm_weight, ZQ_F32, a.w_wide, u * kUnitWeights + 8 * lane, w[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kRowTurns; ++k) {
+            if (ul + k * a.lanes_k >= a.units) break;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc = fmaf(v[k][e], v[k][e], acc);
+        }
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, s);
+        if (lane == 0) s_partial[warp] = acc;
+        asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
+        float total = (lane & 15) < a.lanes_k ? s_partial[lane & 15] : 0.f;
+#pragma unroll
+        for (int s = 8; s > 0; s >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, s);
+        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)a.cols), a.eps)));
+#pragma unroll
+        for (int k = 0; k < kRowTurns; ++k) {
+            const int u = ul + k * a.lanes_k;
+            if (u >= a.units) break;
+            const bool valid = u * kUnitWeights + 8 * lane < a.cols;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[k][e] = valid ? __fmul_rn(__fmul_rn(v[k][e], inv), a.weight_offset == 0.0f ? w[k][e] : __fadd_rn(a.weight_offset, w[k][e])) : 0.f;
+            store_rec(k, v[k]);
+        }
+    } else {
+        float v[8];
+        int k0 = ul * kUnitWeights + 8 * lane;
+        load_act8(a.x, a.x_dtype, (size_t)k0, k0 < a.cols, v);
+        store_rec(0, v);
+        for (int k = 1; ul + k * a.lanes_k < a.units; ++k) {
+            k0 += a.lanes_k * kUnitWeights;
+            load_act8(a.x, a.x_dtype, (size_t)k0, k0 < a.cols, v);
+            store_rec(k, v);
+        }
+    }
+}
+
+// One unit of 16 rows: wq0 is fragment row g of it, `pitch` bytes between rows.
+template <uint32_t TYPE> __device__ __forceinline__ void row_unit(uint32_t type, uint32_t wq0, int pitch, int t, uint32_t ru, uint32_t xoff, float (&yacc)[1][2]) {
+    const uint32_t wq1 = wq0 + (uint32_t)(8 * pitch);
+    const uint32_t rec[1] = {ru}, srec[1] = {ru};
+    if constexpr (TYPE == 0) {
+        switch (type) {
+        case ZQ_Q4_K: consume_q4k_i8<1, false>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        case ZQ_Q5_K: consume_q4k_i8<1, true>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        case ZQ_Q6_K: consume_q6k_i8<1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        case ZQ_Q4_0: consume_b32_i8<ZQ_Q4_0, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        case ZQ_IQ4_NL: consume_b32_i8<ZQ_IQ4_NL, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        default: consume_b32_i8<ZQ_Q8_0, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
+        }
+    } else if constexpr (TYPE == ZQ_Q6_K) consume_q6k_i8<1>(wq0, wq1, t, rec, srec, xoff, yacc);
+    else if constexpr (is_kclass(TYPE)) consume_q4k_i8<1, TYPE == ZQ_Q5_K>(wq0, wq1, t, rec, srec, xoff, yacc);
+    else consume_b32_i8<TYPE, 1>(wq0, wq1, t, rec, srec, xoff, yacc);
+}
+
+// The sum of one output over the warps along K, `stride` floats apart: pairs in turn, as the work-list kernel adds chunks of two units that are a CTA each.
+__device__ __forceinline__ float row_total(const float *p, int lanes_k, int stride) {
+    float s = 0.f;
+    for (int w = 0; w < lanes_k; w += 4) {
+        float q[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) q[e] = w + e < lanes_k ? p[(w + e) * stride] : 0.f;
+        s = (s + (q[0] + q[1])) + (q[2] + q[3]);
+    }
+    return s;
+}
 
 template <uint32_t TYPE, bool GATED>
 __global__ void __launch_bounds__(kRowWarps * 32, 1) gemv_row_kernel(const __grid_constant__ RowArgs a) {
@@ -94,72 +198,8 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1) gemv_row_kernel(const __gri
     for (; ul >= a.lanes_k; ul -= a.lanes_k) ++ug;
     const int g = lane >> 2, t = lane & 3;
     uint8_t *const rec_mine = smem + a.off_rec + warp * a.turns * kRec;
-    auto store_rec = [&](int k, const float (&v)[8]) {
-        uint8_t *dst = rec_mine + k * kRec;
-        auto put = [&](auto kclass) {
-            constexpr uint32_t T = decltype(kclass)::value ? (uint32_t)ZQ_Q4_K : (uint32_t)ZQ_Q4_0;
-            const RecLane o = quantize_record<T>(v, lane);
-            *reinterpret_cast<uint4 *>(dst + o.slot) = make_uint4(o.ph0, o.ph1, o.pl0, o.pl1);
-            if (is_kclass(T) && (lane & 7) == 0) *reinterpret_cast<uint2 *>(dst + kRecSums + (lane >> 3) * 8) = make_uint2(o.sw0, o.sw1);
-            if (lane == 0) *reinterpret_cast<float *>(dst + kRecScale) = o.scale;
-        };
-        if (MIX ? is_kclass(type) : is_kclass(TYPE)) put(std::true_type());
-        else put(std::false_type());
-    };
-
     pdl_wait_prior_grid();
-    if (!GATED && a.norm_weight) {  // the arithmetic of rmsnorm_kernel (zq_norm.cu)
-        float v[kRowTurns][8], w[kRowTurns][8];
-        auto load = [&](const void *p, int dtype, bool wide, int k0, float (&o)[8]) {
-            if (wide) {
-                load_act8(p, dtype, (size_t)k0, k0 < a.cols, o);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = k0 < a.cols ? load_as_f32(p, dtype, (size_t)k0 + e) : 0.f;
-            }
-        };
-        float acc = 0.f;
-#pragma unroll
-        for (int k = 0; k < kRowTurns; ++k) {
-            const int u = ul + k * a.lanes_k;
-            if (u >= a.units) break;
-            load(a.x, a.x_dtype, a.x_wide, u * kUnitWeights + 8 * lane, v[k]);
-            load(a.norm_weight, ZQ_F32, a.w_wide, u * kUnitWeights + 8 * lane, w[k]);
-        }
-#pragma unroll
-        for (int k = 0; k < kRowTurns; ++k) {
-            if (ul + k * a.lanes_k >= a.units) break;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) acc = fmaf(v[k][e], v[k][e], acc);
-        }
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, s);
-        if (lane == 0) s_partial[warp] = acc;
-        __syncthreads();
-        float total = (lane & 15) < a.lanes_k ? s_partial[lane & 15] : 0.f;
-#pragma unroll
-        for (int s = 8; s > 0; s >>= 1) total += __shfl_xor_sync(0xFFFFFFFFu, total, s);
-        const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(total, (float)a.cols), a.eps)));
-#pragma unroll
-        for (int k = 0; k < kRowTurns; ++k) {
-            const int u = ul + k * a.lanes_k;
-            if (u >= a.units) break;
-            const bool valid = u * kUnitWeights + 8 * lane < a.cols;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) v[k][e] = valid ? __fmul_rn(__fmul_rn(v[k][e], inv), a.weight_offset == 0.0f ? w[k][e] : __fadd_rn(a.weight_offset, w[k][e])) : 0.f;
-            store_rec(k, v[k]);
-        }
-    } else {
-        float v[8];
-        int k0 = ul * kUnitWeights + 8 * lane;
-        load_act8(a.x, a.x_dtype, (size_t)k0, k0 < a.cols, v);
-        store_rec(0, v);
-        for (int k = 1; ul + k * a.lanes_k < a.units; ++k) {
-            k0 += a.lanes_k * kUnitWeights;
-            load_act8(a.x, a.x_dtype, (size_t)k0, k0 < a.cols, v);
-            store_rec(k, v);
-        }
-    }
+    row_records<TYPE, GATED>(a, type, rec_mine, ul, warp, lane, (int)blockDim.x, s_partial);
     __syncwarp();
 
     const uint32_t rec0 = smem_u32(rec_mine), xoff = (uint32_t)(16 * t + 8 * (g & 1));
@@ -170,20 +210,7 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1) gemv_row_kernel(const __gri
         uint32_t w_at = smem_u32(smem) + (uint32_t)((16 * i + g) * pitch + ul * ub), ru = rec0;
         float yacc[1][2] = {{0.f, 0.f}};
         for (int u = ul; u < a.units; u += a.lanes_k) {
-            const uint32_t wq0 = w_at, wq1 = wq0 + (uint32_t)(8 * pitch);
-            const uint32_t rec[1] = {ru}, srec[1] = {ru};
-            if constexpr (MIX) {
-                switch (type) {
-                case ZQ_Q4_K: consume_q4k_i8<1, false>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                case ZQ_Q5_K: consume_q4k_i8<1, true>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                case ZQ_Q6_K: consume_q6k_i8<1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                case ZQ_Q4_0: consume_b32_i8<ZQ_Q4_0, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                case ZQ_IQ4_NL: consume_b32_i8<ZQ_IQ4_NL, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                default: consume_b32_i8<ZQ_Q8_0, 1>(wq0, wq1, t, rec, srec, xoff, yacc); break;
-                }
-            } else if constexpr (TYPE == ZQ_Q6_K) consume_q6k_i8<1>(wq0, wq1, t, rec, srec, xoff, yacc);
-            else if constexpr (is_kclass(TYPE)) consume_q4k_i8<1, TYPE == ZQ_Q5_K>(wq0, wq1, t, rec, srec, xoff, yacc);
-            else consume_b32_i8<MIX ? (uint32_t)ZQ_Q8_0 : TYPE, 1>(wq0, wq1, t, rec, srec, xoff, yacc);
+            row_unit<TYPE>(type, w_at, pitch, t, ru, xoff, yacc);
             w_at += (uint32_t)(a.lanes_k * ub);
             ru += kRec;
         }
@@ -197,33 +224,189 @@ __global__ void __launch_bounds__(kRowWarps * 32, 1) gemv_row_kernel(const __gri
         const int o = row0 + i;
         float res = 0.f;
         if (!GATED && jb.residual) res = load_as_f32(jb.residual, jb.y_dtype, (size_t)o);
-        auto total_of = [&](int at) {
-            const float *p = red + at;
-            const int stride = PARTS * a.groups * 16;
-            float s = 0.f;
-            for (int w = 0; w < a.lanes_k; w += 4) {
-                float q[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e) q[e] = w + e < a.lanes_k ? p[(w + e) * stride] : 0.f;
-                s = (s + (q[0] + q[1])) + (q[2] + q[3]);  // as the work-list kernel adds chunks of two units that are a CTA each
-            }
-            return s;
-        };
+        const int stride = PARTS * a.groups * 16;
         float v;
         if (GATED) {
-            const float gate = total_of(32 * (i >> 4) + (i & 15)), up = total_of(32 * (i >> 4) + 16 + (i & 15));
+            const float gate = row_total(red + 32 * (i >> 4) + (i & 15), a.lanes_k, stride), up = row_total(red + 32 * (i >> 4) + 16 + (i & 15), a.lanes_k, stride);
             v = (gate / (1.0f + expf(-gate))) * up;
         } else {
-            v = total_of(i) + res;
+            v = row_total(red + i, a.lanes_k, stride) + res;
         }
         store_from_f32(jb.y, jb.y_dtype, (size_t)o, v);
     }
 }
 
-// Takes a call where its weights fit into the shared memory of the SMs.  Two CTAs per SM where registers and shared memory let them: the
+// The same for matrices past the SMs' shared memory: one CTA per SM walks an equal share of the groups through a ring of groups (gated: of gate
+// and up rows in turn).  A producer warp copies, the warps along K multiply their units of every group, a warp of its own adds up and stores; nobody
+// meets anybody but at the stages' barriers.  Unlike the ring kernels it cuts no tile, quantises the row once per CTA and shares no result between CTAs.
+template <uint32_t TYPE, bool GATED>
+__global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kernel(const __grid_constant__ RowArgs a) {
+    constexpr bool MIX = TYPE == 0;
+    constexpr int PARTS = GATED ? 2 : 1;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
+    float *red = reinterpret_cast<float *>(smem + a.off_red);  // [buffer][part][warp along K][16]
+    __shared__ uint64_t s_full[kRowMaxGroups], s_empty[kRowMaxGroups], s_sums[kRowSums], s_free[kRowSums];
+    __shared__ int s_abort;
+    __shared__ float s_partial[kRowWarps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int consumers = a.lanes_k * a.lanes_g, S = a.groups;
+    const int g0 = (int)((long long)blockIdx.x * a.all_groups / gridDim.x), g1 = (int)((long long)(blockIdx.x + 1) * a.all_groups / gridDim.x);
+    if (tid == 0) {
+        for (int i = 0; i < S; ++i) {
+            mbar_init(&s_full[i], 1);
+            mbar_init(&s_empty[i], (uint32_t)a.lanes_k);
+        }
+        for (int i = 0; i < kRowSums; ++i) {
+            mbar_init(&s_sums[i], (uint32_t)(PARTS * a.lanes_k));
+            mbar_init(&s_free[i], 1);
+        }
+        fence_mbar_init();
+        s_abort = 0;
+    }
+    pdl_launch_dependents();
+    __syncthreads();
+    int j = 0;
+    auto job_of = [&](int g) -> const RowJob & {  // cta0: the job's first group
+        while (j + 1 < a.n_jobs && a.jobs[j + 1].cta0 <= g) ++j;
+        return a.jobs[j];
+    };
+    if (warp == consumers) {
+        // ------------------------------------------------ copies: a row per lane
+        int s = 0;
+        uint32_t ph = 0;
+        bool fresh = true;
+        for (int g = g0; g < g1; ++g) {
+            const RowJob &jb = job_of(g);
+            const int ub = MIX ? row_unit_bytes(jb.type) : Fmt<MIX ? (uint32_t)ZQ_Q4_K : TYPE>::unit_bytes, pitch = row_smem_pitch(MIX ? jb.type : TYPE, a.units);
+            const uint32_t row_bytes = (uint32_t)(a.units * ub);
+            const int row0 = (g - jb.cta0) * 16, rows = jb.n_out - row0 < 16 ? jb.n_out - row0 : 16;
+#pragma unroll
+            for (int part = 0; part < PARTS; ++part) {
+                if (!fresh) {
+                    i8_wait_or_abort(&s_empty[s], ph ^ 1u, &s_abort, a.status);
+                    if (*(volatile int *)&s_abort) return;  // never start a copy nobody will wait for
+                }
+                if (lane == 0) mbar_expect_tx(&s_full[s], (uint32_t)rows * row_bytes);
+                __syncwarp();
+                if (lane < rows) bulk_load_1d(smem + s * a.stage_bytes + lane * pitch, (part ? jb.w_up : jb.w) + (size_t)(row0 + lane) * row_bytes, row_bytes, &s_full[s]);
+                if (++s == S) {
+                    s = 0;
+                    ph ^= 1u;
+                    if (fresh) pdl_wait_prior_grid();  // weights are constants; but no bounded wait may count while an earlier kernel still runs
+                    fresh = false;
+                }
+            }
+        }
+        return;
+    }
+    pdl_wait_prior_grid();
+    if (warp == consumers + 1) {
+        // ------------------------------------------------ sums over the warps, epilogue
+        int b = 0;
+        uint32_t ph = 0;
+        for (int g = g0; g < g1; ++g) {
+            const RowJob &jb = job_of(g);
+            const int o = (g - jb.cta0) * 16 + (lane & 15);
+            const bool mine = lane < 16 && o < jb.n_out;
+            const float res = !GATED && mine && jb.residual ? load_as_f32(jb.residual, jb.y_dtype, (size_t)o) : 0.f;
+            i8_wait_or_abort(&s_sums[b], ph, &s_abort, a.status);
+            if (*(volatile int *)&s_abort) return;
+            // gated: lanes 0..15 add gate, lanes 16..31 up
+            float v = row_total(red + ((b * PARTS + (GATED ? lane >> 4 : 0)) * a.lanes_k) * 16 + (lane & 15), a.lanes_k, 16);
+            if (GATED) {
+                const float up = __shfl_down_sync(0xffffffffu, v, 16);
+                v = (v / (1.0f + expf(-v))) * up;
+            } else {
+                v += res;
+            }
+            if (mine) store_from_f32(jb.y, jb.y_dtype, (size_t)o, v);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[b]);
+            if (++b == kRowSums) {
+                b = 0;
+                ph ^= 1u;
+            }
+        }
+        return;
+    }
+    // ---------------------------------------------------- warps along K
+    int ul = warp, ug = 0;
+    for (; ul >= a.lanes_k; ul -= a.lanes_k) ++ug;
+    const int g = lane >> 2, t = lane & 3;
+    uint8_t *const rec_mine = smem + a.off_rec + warp * a.turns * kRec;
+    const uint32_t type0 = MIX ? job_of(g0).type : TYPE;
+    uint32_t rec_type = type0;
+    row_records<TYPE, GATED>(a, rec_type, rec_mine, ul, warp, lane, consumers * 32, s_partial);
+    __syncwarp();
+    const uint32_t rec0 = smem_u32(rec_mine), xoff = (uint32_t)(16 * t + 8 * (g & 1));
+    int s = ug;
+    uint32_t ph = 0;
+    for (int i = ug; i < PARTS * (g1 - g0); i += a.lanes_g) {
+        const int n = GATED ? i >> 1 : i, part = GATED ? i & 1 : 0, b = n & (kRowSums - 1);
+        const RowJob &jb = job_of(g0 + n);
+        const uint32_t type = MIX ? jb.type : TYPE;
+        const int ub = MIX ? row_unit_bytes(type) : Fmt<MIX ? (uint32_t)ZQ_Q4_K : TYPE>::unit_bytes, pitch = row_smem_pitch(type, a.units);
+        i8_wait_or_abort(&s_full[s], ph, &s_abort, a.status);
+        uint32_t w_at = smem_u32(smem) + (uint32_t)(s * a.stage_bytes + g * pitch + ul * ub), ru = rec0;
+        float yacc[1][2] = {{0.f, 0.f}};
+        for (int u = ul; u < a.units; u += a.lanes_k) {
+            row_unit<TYPE>(type, w_at, pitch, t, ru, xoff, yacc);
+            w_at += (uint32_t)(a.lanes_k * ub);
+            ru += kRec;
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_empty[s]);
+        if (n >= kRowSums) i8_wait_or_abort(&s_free[b], (uint32_t)(n / kRowSums - 1) & 1u, &s_abort, a.status);
+        if (*(volatile int *)&s_abort) return;
+        if (t == 0) {
+            float *at = red + ((b * PARTS + part) * a.lanes_k + ul) * 16 + g;
+            at[0] = yacc[0][0];
+            at[8] = yacc[0][1];
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&s_sums[b]);
+        s += a.lanes_g;
+        if (s >= S) {
+            s -= S;
+            ph ^= 1u;
+        }
+    }
+}
+
+// Whether matrices past the SMs' shared memory are streamed here, `all` groups of 16 outputs, n of them on the busiest SM.  Against the work list (a norm in
+// front) this form starts 2 us earlier and costs more per group, which shows where rows are short; us, work list / streamed:
+//   Q4_K  3840 -> 3 x 3840 12.5/8.5   3840 -> 32768 (n = 14) 19.4/18.4   3840 -> 50000 (n = 22) 23.8/25.9   2560 -> 16384 (n = 7) 11.5/9.0   2560 -> 32768 15.2/15.6   1536 -> 32768 12.0/13.9
+//   Q8_0  3840 -> 3 x 3840 14.6/11.3  3840 -> 32768 28.4/24.5  3840 -> 50000 36.5/34.5  2048 -> 50000 23.7/22.8  1536 -> 32768 15.4/15.0  1536 -> 50000 18.5/21.0
+//   Q6_K  3840 -> 50000 34.9/33.2  2560 -> 32768 19.8/18.5  2560 -> 50000 25.3/26.3  2048 -> 32768 17.1/18.4;   IQ4_NL  3840 -> 32768 26.1/25.1  5120 -> 32768 32.6/33.4
+// Against gemv_i8_kernel (one matrix, one pair) what counts is the busiest SM: its tiles of 128 rows cut along K as far as SMs are idle, in rounds of whole
+// slices, against n groups; rows times units there and here:
+//   Q4_K  5120 -> 11008 (0.63) 11.5/9.8  3840 -> 28672 (0.76) 18.8/17.0  5120 -> 28672 (0.81) 23.9/19.8  3840 -> 14336 (0.82) 9.8/10.3  3840 -> 17408 (0.94) 10.6/11.6  2048 -> 28672 (0.81) 12.6/14.0
+//   Q8_0  3072 -> 28672 (0.81) 22.1/18.3  3072 -> 14336 (0.88) 11.7/11.3  3840 -> 17408 (0.94) 15.1/15.4
+//   gated Q4_K  3840 -> 15360 (0.82) 20.3/17.1  3840 -> 17408 (0.94) 21.1/18.4  3072 -> 17408 (1.0) 18.7/18.2  2048 -> 14336 (0.88) 12.8/14.0;   IQ4_NL  3840 -> 15360 27.2/24.0  3840 -> 8192 (0.94) 14.6/14.7
+static bool row_stream_pays(const zq_ctx *ctx, const RowCall &c, uint32_t type, size_t lanes_k, size_t units, size_t all) {
+    const size_t sms = (size_t)ctx->sm_count, n = (all + sms - 1) / sms, row_bytes = units * row_unit_bytes(c.jobs[0].w->type);
+    for (int i = 1; i < c.n_jobs; ++i)
+        if (is_kclass(c.jobs[i].w->type) != is_kclass(c.jobs[0].w->type)) return false;  // a CTA's range may hold several jobs: one format of records
+    if (lanes_k < 4) return false;
+    if (c.norm) {
+        const bool eight = type == ZQ_Q8_0;
+        if (type == ZQ_IQ4_NL && units > (size_t)kRowWarps && n > 8) return false;
+        return n <= 7 || (n <= 14 ? row_bytes >= 2000 || (eight && row_bytes >= 1600) : row_bytes >= 3300 || (eight && row_bytes >= 2100));
+    }
+    const zq_weight *w = c.jobs[0].w;
+    const bool gated = c.jobs[0].w_up != nullptr;
+    const size_t per_tile = gated ? kTileRows / 2 : kTileRows, tiles = (w->rows + per_tile - 1) / per_tile, chunks = (units + kChunkUnits - 1) / kChunkUnits;
+    const size_t split = std::max<size_t>(1, std::min<size_t>(std::min<size_t>(sms / std::max<size_t>(tiles, 1), 8), chunks));
+    const size_t there = (tiles * split + sms - 1) / sms * ((chunks + split - 1) / split) * kTileRows * kChunkUnits, here = n * 16 * (gated ? 2 : 1) * units;
+    const auto within = [&](size_t percent) { return 100 * here <= percent * there; };
+    if (gated) return units >= 12 ? within(type == ZQ_IQ4_NL ? 90 : 95) : units >= 8 && within(70);
+    return (units >= 12 && within(type == ZQ_Q8_0 ? 90 : 70)) || (units >= 15 && within(81));
+}
+
+// Takes a call where its weights fit into the shared memory of the SMs, or else where streaming pays (above).  Two CTAs per SM where registers and shared memory let them: the
 // groups spread more evenly, and one copies while the other multiplies; else one CTA, up to 200 KB.  Two against one, us: Q4_K 512 -> 8192 2.9 / 3.2,
 // 2560 -> 8192 4.6 / 5.8, gated 1536 -> 3840 3.8 / 4.5, 2560 -> 3840 4.7 / 6.0; where the second does not fit beside the first (3840 -> 3840, 15 warps) 5.8 / 4.1.
-// What does not fit is a matter of bandwidth and stays with the ring kernels: Q4_K 3840 -> 8192 (17.7 MB) 7.7 there, 6.7 here; 5120 -> 8192 (23.6 MB) 8.9 and 8.7.
 template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, const RowCall &c, bool &taken, zq_error *err) {
     constexpr size_t PARTS = GATED ? 2 : 1;
     auto kernel = gemv_row_kernel<TYPE, GATED>;
@@ -233,6 +416,7 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         cudaFuncAttributes fa;
         ZQ_CUDA_CHECK(cudaFuncGetAttributes(&fa, kernel), err);
         ZQ_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxSmem), err);
+        ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemv_row_stream_kernel<TYPE, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxSmem), err);
         regs = (size_t)((fa.numRegs + 7) & ~7) * 32;
     }
     const size_t units = c.jobs[0].w->units_per_row, turns = (units + kRowWarps - 1) / kRowWarps, lanes_k = (units + turns - 1) / turns;
@@ -262,6 +446,11 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         const size_t w_bytes = 16 * groups * PARTS * row, rec = warps * turns * kRec;
         smem = w_bytes + rec + lanes_k * groups * PARTS * 16 * sizeof(float) + 128;
         if (per_sm * warps * regs > 65536 || smem > (per_sm == 2 ? (size_t)kRowMaxSmem / 2 - 1024 : (size_t)200 << 10)) continue;
+        // IQ4_NL's look-ups want more warps than two CTAs of six hold: 1536 -> 17408 7.5 us on gemv_i8_kernel, 8.6 here; gated 1024 -> 5120 5.3 / 5.9
+        if (TYPE == ZQ_IQ4_NL && (GATED && lanes_k <= 4 ? groups > 1 : groups > 2 && per_sm * warps < (size_t)kRowWarps)) break;
+        // much to copy and a busiest SM with far more of it than its share: Q8_0 1536 -> 14336 6.3 / 7.2, gated 1536 -> 5120 5.8 / 6.1
+        if (per_sm == 1 && w_bytes > 150 * 1024 && 100 * groups * ctx->sm_count > 112 * all) continue;
+        if (per_sm == 1 && groups >= 5 && row_stream_pays(ctx, c, TYPE, lanes_k, units, all)) break;
         ra.groups = (int)groups;
         ra.lanes_k = (int)lanes_k;
         ra.lanes_g = (int)lanes_g;
@@ -270,13 +459,36 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         ra.off_red = (int)(w_bytes + rec);
         taken = true;
     }
+    bool stream = false;
+    if (!taken) {
+        const bool pays = row_stream_pays(ctx, c, TYPE, lanes_k, units, all);
+        for (size_t lanes_g = 2; lanes_g >= 1 && !taken && pays; --lanes_g) {
+            if (lanes_g * lanes_k > (size_t)kRowWarps) continue;
+            warps = lanes_g * lanes_k;
+            const size_t rec = warps * turns * kRec, sums = kRowSums * PARTS * lanes_k * 16 * sizeof(float), stage = 16 * row;
+            size_t stages = std::min<size_t>(kRowMaxGroups, (kRowMaxSmem - 1024 - rec - sums - 128) / stage);
+            if (lanes_g == 2) stages &= ~size_t(1);  // a stage is always the same warps', so that their parities tell its phases apart
+            if (stages < (GATED ? 4 : 3)) continue;  // a pair takes two of them
+            ra.groups = (int)stages;
+            ra.lanes_k = (int)lanes_k;
+            ra.lanes_g = (int)lanes_g;
+            ra.turns = (int)turns;
+            ra.stage_bytes = (int)stage;
+            ra.off_rec = (int)(stages * stage);
+            ra.off_red = (int)(stages * stage + rec);
+            smem = stages * stage + rec + sums + 128;
+            taken = stream = true;
+        }
+    }
     if (!taken) return ZQ_OK;
     grid = 0;
     for (int i = 0; i < c.n_jobs; ++i) {
         const zq_weight *w = c.jobs[i].w;
         ra.jobs[i] = {w->data, GATED ? c.jobs[i].w_up->data : nullptr, c.jobs[i].y, c.jobs[i].residual, (int)w->rows, (int)grid, c.jobs[i].y_dtype, w->type};
-        grid += ((w->rows + 15) / 16 + ra.groups - 1) / ra.groups;
+        grid += stream ? (w->rows + 15) / 16 : ((w->rows + 15) / 16 + ra.groups - 1) / ra.groups;
     }
+    if (stream) grid = std::min<size_t>(all, (size_t)ctx->sm_count);
+    ra.all_groups = (int)all;
     ra.n_jobs = c.n_jobs;
     ra.x = c.x;
     ra.x_dtype = c.x_dtype;
@@ -290,7 +502,7 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
     ra.status = ctx->status_dev;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)(32 * warps));
+    cfg.blockDim = dim3((unsigned)(32 * (warps + (stream ? 2 : 0))));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
@@ -298,7 +510,7 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = ctx->disable_pdl ? 0 : 1;
-    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, ra), err);
+    ZQ_CUDA_CHECK(cudaLaunchKernelEx(&cfg, stream ? gemv_row_stream_kernel<TYPE, GATED> : kernel, ra), err);
     ctx->launches++;
     return ZQ_OK;
 }
