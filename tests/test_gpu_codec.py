@@ -164,6 +164,33 @@ def test_gather_rows_equals_f16_of_dequant(tensor_type):
     assert np.array_equal(got.cpu().numpy().view(np.uint16), want.view(np.uint16))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shape", [(1,), (7,), (2, 3)])
+def test_gather_rows_by_ids_on_the_device(shape, dtype):
+    """int32 ids that lie on the device take the native half alone; every other form of the ids gives the same rows.  The result
+    is allocated past the dispatcher unless a mode that watches it is on."""
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watch(TorchDispatchMode):
+        names = []
+
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            self.names.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    rows, cols = 33, 512
+    w = ctx().prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, rows, cols, seed=5), rows, cols)
+    ids = (torch.arange(int(np.prod(shape)), dtype=torch.int32) * 11).remainder(rows).reshape(shape)
+    on_device = ids.cuda()
+    strided = torch.stack([on_device, on_device * 0], dim=-1)[..., 0]
+    want = ctx().gather_rows(w, ids, dtype=dtype)
+    with Watch() as seen:
+        watched = ctx().gather_rows(w, on_device, dtype=dtype)
+    for got in (ctx().gather_rows(w, on_device, dtype=dtype), ctx().gather_rows(w, on_device.long(), dtype=dtype), ctx().gather_rows(w, strided, dtype=dtype), watched):
+        assert got.shape == (ids.numel(), cols) and got.dtype == dtype and torch.equal(got, want)
+    assert any("empty" in name for name in seen.names)
+
+
 def test_gather_rows_reports_bad_row_ids_without_faulting():
     from zllm_b200 import ffi
 

@@ -139,6 +139,8 @@ class B200Context:
         return out
 
     def gather_rows(self, w: Weight, row_ids: Optional[torch.Tensor], n_rows: Optional[int] = None, dtype=torch.float16) -> torch.Tensor:
+        if row_ids is not None and row_ids.dtype is torch.int32 and row_ids.device == self.device and row_ids.is_contiguous() and dtype in _DTYPES:
+            return self._native.gather_rows(self._h, w, row_ids, dtype)
         n = int(row_ids.numel()) if row_ids is not None else int(n_rows)
         if row_ids is not None:
             row_ids = row_ids.to(device=self.device, dtype=torch.int32).contiguous()
