@@ -9,6 +9,10 @@
 //   moe_quantize_kernel    activation records (zq_i8.cuh) of every routed row, grouped by expert
 //   moe_grouped_kernel     integer-MMA decode over the work list; CTA c takes items c, c + grid, ...; every ring
 //                          stage carries the weights of one (tile, 2 units) and the records of those units
+// The copies need the bytes of a ring all of the time: a stage that is free and not yet asked for is lost.  64 tokens, 256 experts of 7168 x 2048 in
+// Q4_K, top 8 and a shared one: gate/up 701 us and down 358 while the copying thread divided its 64-bit item number by the chunks of
+// a tile after each wait, 566 and 303 with the addresses ready before the wait (copies alone: 580 and 280).  A barrier of the consumer warps per
+// work item, which a warp of its own now stands in for, was 2 % of it.
 // Arithmetic per expert is that of zq_gemv_i8.cu (16-bit integer activations, exact integer weights), the combine
 // is the one of zq_moe.cu; an expert that received more than 8 rows is walked in passes of 8.
 #include <cstring>
@@ -22,7 +26,7 @@ constexpr int kPassRows = 8;                    // activation rows per pass (two
 constexpr int kPassUnitBytes = kPassRows * kRec;  // record slot of one unit inside a ring stage
 constexpr int kItemCache = 512;                 // work items whose descriptors a CTA keeps in shared memory
 constexpr int kPlanThreads = 1024;
-constexpr int kGroupedThreads = kI8Threads + 32;  // 16 consumer warps and a TMA producer warp
+constexpr int kGroupedThreads = kI8Threads + 64;  // 16 consumer warps, a TMA producer warp and a warp that finishes work items
 // ring depth: the wide Q8_0 rows leave room for two stages only
 __host__ __device__ constexpr int grouped_stages(uint32_t type) { return type == ZQ_Q8_0 ? 2 : (type == ZQ_Q5_K || type == ZQ_Q6_K) ? 3 : 4; }
 
@@ -230,6 +234,7 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
     uint4 *s_pass = reinterpret_cast<uint4 *>(smem + STAGES * STRIDE + 2 * RED_FLOATS * 4);
     uint64_t *full = reinterpret_cast<uint64_t *>(smem + STAGES * STRIDE + 2 * RED_FLOATS * 4 + kItemCache * 16);
     uint64_t *empty = full + 8;
+    __shared__ uint64_t s_sums[2], s_free[2];         // per buffer: all sums of an item are in; it may be written again
     __shared__ int s_abort;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -247,51 +252,75 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], kI8Threads / 32);
         }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(&s_sums[b], kI8Threads / 32);
+            mbar_init(&s_free[b], 1);
+        }
         fence_mbar_init();
         s_abort = 0;
     }
     __syncthreads();
     auto pass_of = [&](int k) -> uint4 { return k < kItemCache ? s_pass[k] : ga.passes[(bid + k * G) / ga.tiles]; };
 
-    // ring item q = (k-th work item of this CTA, chunk): weights of the tile's two units and their records
-    auto issue = [&](long long q, int stage) {
-        const int k = (int)(q / chunks), chunk = (int)(q - (long long)k * chunks);
-        const int tile = (bid + k * G) % ga.tiles;
-        const uint4 pe = pass_of(k);
-        const uint32_t e = pe.x, m0 = pe.y & 0xFFFFu, mc = pe.y >> 16, first = pe.z, cnt = pe.w;
-        int nu = ga.units - chunk * kChunkUnits;
-        if (nu > kChunkUnits) nu = kChunkUnits;
-        uint8_t *dst = ws + (size_t)stage * STRIDE;
-        mbar_expect_tx(&full[stage], (uint32_t)(STAGE_W + nu * mc * kRec));
-        const bool sh = (int)e == ga.shared_id;
-        const CUtensorMap *ma = sh ? &ga.shared_a : &ga.maps_a[e];
-        if (GATED) {
-            const CUtensorMap *mb = sh ? &ga.shared_b : &ga.maps_b[e];
-            tma_load_2d(dst, ma, &full[stage], chunk * ga.chunk_words, tile * out_rows);
-            tma_load_2d(dst + STAGE_W / 2, mb, &full[stage], chunk * ga.chunk_words, tile * out_rows);
-        } else {
-            tma_load_2d(dst, ma, &full[stage], chunk * ga.chunk_words, tile * out_rows);
-        }
-        for (int u = 0; u < nu; ++u) {
-            const size_t rec = (size_t)first * ga.units + (size_t)(chunk * kChunkUnits + u) * cnt + m0;
-            bulk_load_1d(dst + STAGE_W + u * kPassUnitBytes, ga.xq + rec * kRec, mc * kRec, &full[stage]);
-        }
-    };
     if (warp == kI8Threads / 32) {
         // ------------------------------------------------ producer warp: keeps the ring full; a stage is refilled as soon
-        // as all sixteen consumer warps have released it, whichever of them is late
+        // as all sixteen consumer warps have released it, whichever of them is late.  What stands between that release and
+        // the copies is dead time of the stage: addresses are ready before the wait, and only advance by constants in an item.
         if (lane == 0) {
             int pstage = 0;
-            uint32_t pphase = 0;
-            for (long long q = 0; q < total_q; ++q) {
-                if (q >= STAGES) i8_wait_or_abort(&empty[pstage], pphase ^ 1u, &s_abort, ga.status);
-                if (*(volatile int *)&s_abort) break;  // never start a copy nobody will wait for
-                issue(q, pstage);
-                if (++pstage == STAGES) {
-                    pstage = 0;
-                    pphase ^= 1u;
+            uint32_t pphase = 1;  // the first turn of the ring waits for nobody
+            for (int k = 0; k < my_count; ++k) {
+                const int tile = (bid + k * G) % ga.tiles;
+                const uint4 pe = pass_of(k);
+                const uint32_t e = pe.x, m0 = pe.y & 0xFFFFu, mc = pe.y >> 16, first = pe.z, cnt = pe.w;
+                const bool sh = (int)e == ga.shared_id;
+                const CUtensorMap *ma = sh ? &ga.shared_a : &ga.maps_a[e], *mb = sh ? &ga.shared_b : &ga.maps_b[e];
+                const int row = tile * out_rows;
+                const uint8_t *rec = ga.xq + ((size_t)first * ga.units + m0) * kRec;  // records of the rows of one pass of a unit are contiguous
+                const uint32_t rec_bytes = mc * kRec;
+                const size_t rec_step = (size_t)cnt * kRec;
+                for (int chunk = 0, left = ga.units, x = 0; chunk < chunks; ++chunk, left -= kChunkUnits, x += ga.chunk_words) {
+                    const int nu = left < kChunkUnits ? left : kChunkUnits;
+                    uint8_t *dst = ws + (size_t)pstage * STRIDE;
+                    const uint32_t bytes = STAGE_W + nu * rec_bytes;
+                    i8_wait_or_abort(&empty[pstage], pphase, &s_abort, ga.status);
+                    if (*(volatile int *)&s_abort) return;  // never start a copy nobody will wait for
+                    mbar_expect_tx(&full[pstage], bytes);
+                    tma_load_2d(dst, ma, &full[pstage], x, row);
+                    if (GATED) tma_load_2d(dst + STAGE_W / 2, mb, &full[pstage], x, row);
+                    for (int u = 0; u < nu; ++u, rec += rec_step) bulk_load_1d(dst + STAGE_W + u * kPassUnitBytes, rec, rec_bytes, &full[pstage]);
+                    if (++pstage == STAGES) {
+                        pstage = 0;
+                        pphase ^= 1u;
+                    }
                 }
             }
+        }
+        return;
+    }
+    if (warp == kI8Threads / 32 + 1) {
+        // ------------------------------------------------ finishing warp: adds the two unit halves of an item and stores it,
+        // while the consumer warps, which no barrier holds together, are in the next two
+        for (int k = 0; k < my_count; ++k) {
+            const float *sums = red + (k & 1) * RED_FLOATS;
+            const uint4 pe = pass_of(k);
+            const int mc = (int)(pe.y >> 16), n0 = (bid + k * G) % ga.tiles * out_rows;
+            float *out = ga.out + ((size_t)pe.z + (pe.y & 0xFFFFu)) * ga.n_out + n0;
+            i8_wait_or_abort(&s_sums[k & 1], (uint32_t)(k >> 1) & 1u, &s_abort, ga.status);
+            if (*(volatile int *)&s_abort) return;
+            for (int tok = 0; tok < mc; ++tok, sums += kTileRows, out += ga.n_out) {
+#pragma unroll
+                for (int row = lane; row < out_rows; row += 32) {
+                    float v = sums[row] + sums[RS * kTileRows + row];
+                    if (GATED) {
+                        const float up = sums[out_rows + row] + sums[RS * kTileRows + out_rows + row];
+                        v = (v / (1.0f + expf(-v))) * up;
+                    }
+                    if (n0 + row < ga.n_out) out[row] = v;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_free[k & 1]);
         }
         return;
     }
@@ -305,7 +334,7 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
 
     float yacc1[1][2], yacc2[2][2];
     uint32_t moff[2] = {0, 0}, soff[2] = {0, 0};
-    int mc = 0, chunk = 0, k = 0, stage = 0, buf = 0;
+    int mc = 0, chunk = 0, k = 0, stage = 0;
     uint32_t phase = 0;
     for (long long q = 0; q < total_q; ++q) {
         if (chunk == 0) {  // a new work item: rows of this pass, accumulators
@@ -346,8 +375,11 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
             phase ^= 1u;
         }
         if (++chunk == chunks) {
-            // ------------------------------------------------ end of the work item: add the two unit halves, store
-            float *rb_ = red + buf * RED_FLOATS;
+            // ------------------------------------------------ end of the work item: leave its sums to the finishing warp
+            const int b = k & 1;
+            float *rb_ = red + b * RED_FLOATS;
+            if (k >= 2) i8_wait_or_abort(&s_free[b], (uint32_t)((k >> 1) - 1) & 1u, &s_abort, ga.status);
+            if (*(volatile int *)&s_abort) return;
             if (mc <= 4) {
                 rb_[(ul * RS + t) * kTileRows + r0] = yacc1[0][0];
                 rb_[(ul * RS + t) * kTileRows + r0 + 8] = yacc1[0][1];
@@ -358,25 +390,8 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
                     rb_[(ul * RS + nt * 4 + t) * kTileRows + r0 + 8] = yacc2[nt][1];
                 }
             }
-            asm volatile("bar.sync 1, %0;" ::"n"(kI8Threads) : "memory");  // the consumer warps only; the other buffer is written next item, and read only after that item's barrier
-            const uint4 pe = pass_of(k);
-            const int tile = (bid + k * G) % ga.tiles;
-            const size_t slot0 = (size_t)pe.z + (pe.y & 0xFFFFu);
-            for (int i = tid; i < out_rows * mc; i += kI8Threads) {
-                const int row = i & (out_rows - 1), tok = i / out_rows;
-                const int n = tile * out_rows + row;
-                if (n >= ga.n_out) continue;
-                float v;
-                if (GATED) {
-                    const float gate = rb_[tok * kTileRows + row] + rb_[(RS + tok) * kTileRows + row];
-                    const float up = rb_[tok * kTileRows + out_rows + row] + rb_[(RS + tok) * kTileRows + out_rows + row];
-                    v = (gate / (1.0f + expf(-gate))) * up;
-                } else {
-                    v = rb_[tok * kTileRows + row] + rb_[(RS + tok) * kTileRows + row];
-                }
-                ga.out[(slot0 + tok) * ga.n_out + n] = v;
-            }
-            buf ^= 1;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&s_sums[b]);
             chunk = 0;
             ++k;
         }
