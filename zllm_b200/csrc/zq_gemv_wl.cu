@@ -491,35 +491,43 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
             auto locate = [&](int i) {
                 while (psi + 1 < nseg && segs[psi + 1].w <= i) ++psi;
             };
-            auto issue_w = [&](int i, int stage) {
+            // What stands between a stage's release and its copies is dead time of the stage: an item's addresses are ready before the wait.
+            const CUtensorMap *map_a = nullptr, *map_b = nullptr;
+            const uint8_t *rec = nullptr;
+            int x = 0, y = 0;
+            uint32_t w_bytes = 0, rec_bytes = 0;
+            auto prepare = [&](int i) {
+                locate(i);
                 const int4 sg = segs[psi];
                 const WlJob &jb = a.jobs[sg.x];
                 const int chunk = (sg.z & 0xFFFF) + (i - sg.w);
-                int nu = jb.units - chunk * kChunkUnits;
-                if (nu > kChunkUnits) nu = kChunkUnits;
-                uint8_t *dst = ws + (size_t)stage * STRIDE;
+                map_a = jb.map_a;
+                if (GATED) map_b = jb.map_b;
+                y = sg.y * out_rows;
                 if constexpr (RES) {
                     const int words = kChunkUnits * unit_bytes(jb) / 4;
-                    mbar_expect_tx(&full[stage], (uint32_t)(kTileRows * words * 4));
-                    tma_load_2d(dst, jb.map_a, &full[stage], chunk * words, sg.y * out_rows);
+                    w_bytes = (uint32_t)(kTileRows * words * 4);
+                    x = chunk * words;
                 } else {
-                    mbar_expect_tx(&full[stage], (uint32_t)(STAGE_W + nu * jb.m * kRec));
-                    tma_load_2d(dst, jb.map_a, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
-                    if (GATED) tma_load_2d(dst + STAGE_W / 2, jb.map_b, &full[stage], chunk * a.chunk_words, sg.y * out_rows);
+                    int nu = jb.units - chunk * kChunkUnits;
+                    if (nu > kChunkUnits) nu = kChunkUnits;
+                    w_bytes = STAGE_W;
+                    x = chunk * a.chunk_words;
+                    rec = jb.xq + (size_t)chunk * kChunkUnits * jb.m * kRec;
+                    rec_bytes = (uint32_t)(nu * jb.m * kRec);
                 }
             };
-            auto issue_x = [&](int i, int stage) {
-                const int4 sg = segs[psi];
-                const WlJob &jb = a.jobs[sg.x];
-                const int chunk = (sg.z & 0xFFFF) + (i - sg.w);
-                int nu = jb.units - chunk * kChunkUnits;
-                if (nu > kChunkUnits) nu = kChunkUnits;
-                bulk_load_1d(ws + (size_t)stage * STRIDE + STAGE_W, jb.xq + (size_t)chunk * kChunkUnits * jb.m * kRec, (uint32_t)(nu * jb.m * kRec), &full[stage]);
+            auto issue_w = [&](int stage) {
+                uint8_t *dst = ws + (size_t)stage * STRIDE;
+                mbar_expect_tx(&full[stage], w_bytes + rec_bytes);
+                tma_load_2d(dst, map_a, &full[stage], x, y);
+                if (GATED) tma_load_2d(dst + STAGE_W / 2, map_b, &full[stage], x, y);
             };
+            auto issue_x = [&](int stage) { bulk_load_1d(ws + (size_t)stage * STRIDE + STAGE_W, rec, rec_bytes, &full[stage]); };
             const int pre = total_items < STAGES ? total_items : STAGES;
             for (int s = 0; s < pre; ++s) {
-                locate(s);
-                issue_w(s, s);  // weights are constants: they may stream while the previous kernel still runs
+                prepare(s);
+                issue_w(s);  // weights are constants: they may stream while the previous kernel still runs
             }
             pdl_launch_dependents();
             // The records belong to the record pass, which waits for everything before it; and no bounded wait may count while an
@@ -528,20 +536,20 @@ __global__ void __launch_bounds__(kWlThreads, 1) gemv_wl_kernel(const __grid_con
             if constexpr (!RES) {
                 psi = 0;
                 for (int s = 0; s < pre; ++s) {
-                    locate(s);
-                    issue_x(s, s);
+                    prepare(s);
+                    issue_x(s);
                 }
             }
             int stage = 0;
             uint32_t phase = 0;
             for (int i = pre; i < total_items; ++i) {
+                prepare(i);
                 wl_wait(&empty[stage], phase, abort_addr, a.status);  // every consumer warp is done with the stage's previous item
                 uint32_t f;
                 asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(f) : "r"(abort_addr));
                 if (f) break;  // never start a copy nobody will wait for
-                locate(i);
-                issue_w(i, stage);
-                if constexpr (!RES) issue_x(i, stage);
+                issue_w(stage);
+                if constexpr (!RES) issue_x(stage);
                 if (++stage == STAGES) {
                     stage = 0;
                     phase ^= 1u;
