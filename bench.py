@@ -830,7 +830,7 @@ def bench_kquant_decode(ctx, device, hbm_peak=6545.9):
         gbs = n * k // e * b / ms / 1e6
         out[name] = {"us_per_launch": round(ms * 1e3, 2), "gbs": round(gbs, 1), "roofline": {"bound": "hbm", "achieved": round(gbs, 1), "peak": hbm_peak, "unit": "GB/s", "frac": round(gbs / hbm_peak, 4)}}
         del weights
-    out["kernel"] = "zq::gemv_i8_kernel<Q5_K / Q6_K, 1 column tile>"
+    out["kernel"] = "one-row decode: zq::gemv_row_stream_kernel, or zq::gemv_i8_kernel<Q5_K / Q6_K, 1 column tile> where the groups of rows come out uneven"
     return out
 
 

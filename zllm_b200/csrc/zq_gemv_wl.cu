@@ -143,8 +143,8 @@ template <uint32_t TYPE, int NT> struct WlSmem {
 // range needs, each once, into shared memory, while the first weights are on their way; an RMSNorm in front of the list (one
 // row) is computed there too, by every CTA for itself: a row is a few KB out of L2.  That takes a launch (of 4 to 5 us in a chain of
 // small ones) and the records' way through memory off a decode step; lists of several types go out as one launch instead of one per
-// type (TYPE 0).  Decode step of 12 layers of 1536 columns, q, k, v in Q4_K and Q6_K behind a norm: 434 us (81 launches), now 382 (62); 4 layers of
-// 3840 columns: 324, now 315; five Q4_K projections of five inputs: 38.7, now 37.9.
+// type (TYPE 0).  Five Q4_K projections of five inputs: 38.7 us, now 37.9.  Norm lists of one row come here where the one-row kernels do not take them
+// (zq_gemv_row.cu: too many columns for their groups, more than four projections).
 // The ring gets what the records leave, five stages at most.
 template <uint32_t TYPE> struct WlResSmem {
     static constexpr int XCH_FLOATS = 16 * 32 * 2;
@@ -913,6 +913,7 @@ bool gemv_wl_supported(const zq_ctx *ctx, const WlHostJob &j) {
 // same ring items out evenly, for a record pass, a longer start and the hand-over of cut tiles, ~5 us together.  It is taken when
 // the busiest SM would walk at least 216 KB of weights less, those 5 us at ~43 GB/s per SM; with 9..16 rows of Q4_K and Q5_K, where
 // arithmetic sets the pace of both kernels and the longer hand-over is not hidden, at least 300 KB.  Measured, gemv_i8 -> work list:
+// (one row comes here only where the one-row kernels of zq_gemv_row.cu do not take it)
 //   5120 -> 10240 (20 items on the busiest SM against 11)  1 row: Q4_K 21.5 -> 18.7 us, Q5_K 25.4 -> 21.1, IQ4_NL 30.2 -> 23.5, Q8_0 28.1 -> 25.8;
 //     8 rows: 26.4 -> 23.4, 29.5 -> 25.7, 35.5 -> 28.2, 33.9 -> 29.6;  16 rows: 36.9 -> 36.2, 40.9 -> 38.8, 45.1 -> 35.2, 42.0 -> 35.6, Q6_K 50.0 -> 40.8
 //   3840 -> 10240 (16 against 9)  16 rows: Q4_K 29.8 and 31.0 (258 KB: not taken), Q5_K 33.0 and 33.1, Q4_0 30.0 -> 26.5, IQ4_NL 36.0 -> 29.8, Q8_0 34.2 -> 29.9
