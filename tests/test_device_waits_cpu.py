@@ -1,0 +1,37 @@
+"""Rules of the kernels' bounded waits that no run shows: a wait that gives up must not part a warp in front of an instruction that wants all of it.
+
+What a kernel does after such a wait cannot be provoked without a fault, so the sources are read instead."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "zllm_b200", "csrc")
+
+
+def _source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def _between(text, first, last):
+    start = text.index(first)
+    return text[start:text.index(last, start)]
+
+
+def test_short_prefill_dequantisers_keep_the_warp_together():
+    """tcgen05.st and tcgen05.wait::st are .sync.aligned: no lane may leave the loop between the waits and them."""
+    roles = _source("zq_gemm.cu")
+    body = _between(roles[roles.index("DqTensorRow{") - 1500:], "while (", "pair_arrive(")
+    assert "wait_flag(" in body and "dq.emit(DqTensorRow{" in body
+    assert not re.search(r"\b(break|return|continue)\b|while \(ok", body)
+    assert body.count("ok = ok && wait_flag(") == body.count("wait_flag(") == 2
+
+
+def test_short_prefill_issuers_leave_by_a_vote():
+    """elect.sync and tcgen05.ld behind a wait: all lanes go on or none."""
+    roles = _source("zq_gemm.cu")
+    tokens = _between(roles, "const uint32_t sub = (uint32_t)p.box_tok * kBK * 2;", "elect_one()")
+    assert "wait_warp<true>(&empty" in tokens
+    mma = roles[roles.index("int before = 0;"):]
+    mma = _between(mma, "if constexpr (SHORT)", "elect_one()")
+    assert re.search(r"ok = __all_sync\(0xffffffffu, wait_flag\(&full.*wait_flag\(&a_full", mma)
+    assert "wait_warp<SHORT>(&acc_empty" in roles and "wait_warp<SHORT>(&acc_full" in roles and "wait_warp<SHORT>(&p_empty" in roles

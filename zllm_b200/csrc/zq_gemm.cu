@@ -202,6 +202,13 @@ __device__ __forceinline__ bool wait_flag(uint64_t *bar, uint32_t parity, uint32
     atomicMax(status, code);
     return false;
 }
+// The same where warp-wide instructions follow (elect.sync, tcgen05.ld, .st and tcgen05.wait want the whole warp).  Lanes poll each for itself: one
+// may see that the block gives up and another that the phase is complete, and with a way out of the loop between them nothing brings them together.
+// Short form: 2 % on gated IQ4_NL, nothing or less on the others.
+template <bool VOTE> __device__ __forceinline__ bool wait_warp(uint64_t *bar, uint32_t parity, uint32_t state_addr, uint32_t *status, uint32_t code, unsigned sleep_ns = 0) {
+    const bool ok = wait_flag(bar, parity, state_addr, status, code, sleep_ns);
+    return VOTE ? __all_sync(0xffffffffu, ok) : ok;
+}
 
 template <int DT> struct DtypeTag {
     static constexpr int value = DT;
@@ -486,7 +493,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                 const uint32_t sub = (uint32_t)p.box_tok * kBK * 2;
                 const int stages = short_stages<S>(sub);
                 for (int u = sg.k0; u < sg.k1; ++u) {
-                    if (!fresh && !wait_flag(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout)) {
+                    if (!fresh && !wait_warp<true>(&empty[s], ph ^ 1u, state_addr, p.status, kStatusMmaTimeout)) {
                         ok = false;
                         break;
                     }
@@ -551,7 +558,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                 // different barriers are seen.
                 if (iter >= 2) {
                     if constexpr (WIDE) ok = __all_sync(0xffffffffu, wait_flag(&step_free[b * kChunks + (lane & (kChunks - 1))], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout));
-                    else ok = wait_flag(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
+                    else ok = wait_warp<SHORT>(&acc_empty[b], (uint32_t)((iter >> 1) - 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 }
                 if (WIDE && ok && shared > 0) ok = wait_flag(&step_free[(b ^ 1) * kChunks + shared - 1], (uint32_t)((iter - 1) >> 1) & 1, state_addr, p.status, kStatusMmaTimeout);
                 if (!ok) break;
@@ -562,7 +569,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                     const uint32_t sub = (uint32_t)p.box_tok * kBK * 2;  // as the TMA warp has them
                     const int stages = short_stages<S>(sub);
                     for (int u = sg.k0; u < sg.k1; ++u) {
-                        ok = wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout) && wait_flag(&a_full[ah], aph, state_addr, p.status, kStatusTmaTimeout);
+                        ok = __all_sync(0xffffffffu, wait_flag(&full[s], ph, state_addr, p.status, kStatusTmaTimeout) && wait_flag(&a_full[ah], aph, state_addr, p.status, kStatusTmaTimeout));
                         if (!ok) break;
                         tc_fence_after();
                         if (elect_one()) {
@@ -630,7 +637,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                     if (at < bytes) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const uint8_t *>(p.residual) + (size_t)(sg.tok0 + i / (int)esz) * bytes + at));
                 }
             }
-            const bool ok = wait_flag(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0);
+            const bool ok = wait_warp<SHORT>(&acc_full[b], (uint32_t)(iter >> 1) & 1, state_addr, p.status, kStatusMmaTimeout, SRC ? 200 : 0);
             tc_fence_after();
             const uint32_t acc = tmem_base + (uint32_t)(WIDE ? tile_column(iter, chunks) : b * (SHORT ? kShortBN : kBN)) + ((uint32_t)(q * 32) << 16);
             auto free_step = [&](int k) {  // this warp is through with the k-th chunk
@@ -743,7 +750,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                 const CUtensorMap *mw2 = p.items ? (GATED ? &p.w2_maps[sg.z] : mw) : &map_w2;
                 const int row = sg.row0 + (int)rank * (GATED ? 64 : kBM);
                 for (int u = sg.k0; u < sg.k1; ++u) {
-                    if (!fresh && !wait_flag(&p_empty[ps], pph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 50)) {
+                    if (!fresh && !wait_warp<SHORT>(&p_empty[ps], pph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 50)) {
                         ok = false;
                         break;
                     }
@@ -774,13 +781,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, 
                 uint32_t pph = 0, ah = 0, aph = 0;
                 bool ok = true;
                 DqBlock<SRC> dq;
-                while (ok && walk.next(p, sg)) {
+                // tcgen05.st and its wait want every lane, so none leaves the loops: one whose wait has failed waits for nothing any more and walks on.  Costs
+                // nothing; a vote and a way out 1.5 % at 48 tokens of Q4_K, a __syncwarp here 4 % at 128.
+                while (walk.next(p, sg)) {
                     for (int u = sg.k0; u < sg.k1; ++u) {
-                        ok = wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
-                        if (!ok) break;
+                        ok = ok && wait_flag(&p_full[ps], pph, state_addr, p.status, kStatusTmaTimeout, 20);
                         dq.load(box0 + (uint32_t)(ps * S::p_bytes), mine);
-                        ok = wait_flag(&a_empty[ah], aph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
-                        if (!ok) break;
+                        ok = ok && wait_flag(&a_empty[ah], aph ^ 1u, state_addr, p.status, kStatusMmaTimeout, 20);
                         tc_fence_after();  // behind the MMAs that read this half before
                         dq.emit(DqTensorRow{a0 + ah * (kStepK / 2)});
                         tmem_st_wait();
