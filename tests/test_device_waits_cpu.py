@@ -35,3 +35,11 @@ def test_short_prefill_issuers_leave_by_a_vote():
     mma = _between(mma, "if constexpr (SHORT)", "elect_one()")
     assert re.search(r"ok = __all_sync\(0xffffffffu, wait_flag\(&full.*wait_flag\(&a_full", mma)
     assert "wait_warp<SHORT>(&acc_empty" in roles and "wait_warp<SHORT>(&acc_full" in roles and "wait_warp<SHORT>(&p_empty" in roles
+
+
+def test_streamed_row_groups_are_given_back_behind_their_sums():
+    """The arrival that frees a ring stage must not overtake the loads from it: it stands behind the store of the sums that need them all."""
+    kernel = _source("zq_gemv_row.cu")
+    consumer = _between(kernel[kernel.index("gemv_row_stream_kernel(const"):], "row_unit<TYPE>(", "s += a.lanes_g;")
+    assert consumer.count("mbar_arrive(&s_empty[s])") == 1
+    assert consumer.index("at[8] = yacc[0][1];") < consumer.index("__syncwarp();") < consumer.index("mbar_arrive(&s_empty[s])")

@@ -355,8 +355,6 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
             w_at += (uint32_t)(a.lanes_k * ub);
             ru += kRec;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&s_empty[s]);
         if (n >= kRowSums) i8_wait_or_abort(&s_free[b], (uint32_t)(n / kRowSums - 1) & 1u, &s_abort, a.status);
         if (*(volatile int *)&s_abort) return;
         if (t == 0) {
@@ -365,7 +363,10 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
             at[8] = yacc[0][1];
         }
         __syncwarp();
-        if (lane == 0) mbar_arrive(&s_sums[b]);
+        if (lane == 0) {
+            mbar_arrive(&s_empty[s]);  // behind the stores of the sums, whose MMAs have waited for all loads from the stage: an arrival may overtake queued loads (zq_gemm.cu)
+            mbar_arrive(&s_sums[b]);
+        }
         s += a.lanes_g;
         if (s >= S) {
             s -= S;
