@@ -43,3 +43,12 @@ def test_streamed_row_groups_are_given_back_behind_their_sums():
     consumer = _between(kernel[kernel.index("gemv_row_stream_kernel(const"):], "row_unit<TYPE>(", "s += a.lanes_g;")
     assert consumer.count("mbar_arrive(&s_empty[s])") == 1
     assert consumer.index("at[8] = yacc[0][1];") < consumer.index("__syncwarp();") < consumer.index("mbar_arrive(&s_empty[s])")
+
+
+def test_warps_leave_together_when_the_block_gives_up():
+    """A lane may return by its own reading of the flag only where it is alone (`lane == 0` of the MoE copies)."""
+    row, moe = _source("zq_gemv_row.cu"), _source("zq_moe_grouped.cu")
+    assert "(volatile int *)&s_abort" not in row and row.count("if (i8_warp_aborts(&s_abort)) return;") == 3
+    assert moe.count("(volatile int *)&s_abort") == 1 and moe.count("if (i8_warp_aborts(&s_abort)) return;") == 2
+    copies = _between(moe, "if (warp == kI8Threads / 32) {", "if (warp == kI8Threads / 32 + 1)")
+    assert copies.index("if (lane == 0) {") < copies.index("(volatile int *)&s_abort")

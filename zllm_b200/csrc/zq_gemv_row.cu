@@ -285,7 +285,7 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
             for (int part = 0; part < PARTS; ++part) {
                 if (!fresh) {
                     i8_wait_or_abort(&s_empty[s], ph ^ 1u, &s_abort, a.status);
-                    if (*(volatile int *)&s_abort) return;  // never start a copy nobody will wait for
+                    if (i8_warp_aborts(&s_abort)) return;  // never start a copy nobody will wait for
                 }
                 if (lane == 0) mbar_expect_tx(&s_full[s], (uint32_t)rows * row_bytes);
                 __syncwarp();
@@ -311,7 +311,7 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
             const bool mine = lane < 16 && o < jb.n_out;
             const float res = !GATED && mine && jb.residual ? load_as_f32(jb.residual, jb.y_dtype, (size_t)o) : 0.f;
             i8_wait_or_abort(&s_sums[b], ph, &s_abort, a.status);
-            if (*(volatile int *)&s_abort) return;
+            if (i8_warp_aborts(&s_abort)) return;
             // gated: lanes 0..15 add gate, lanes 16..31 up
             float v = row_total(red + ((b * PARTS + (GATED ? lane >> 4 : 0)) * a.lanes_k) * 16 + (lane & 15), a.lanes_k, 16);
             if (GATED) {
@@ -356,7 +356,7 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
             ru += kRec;
         }
         if (n >= kRowSums) i8_wait_or_abort(&s_free[b], (uint32_t)(n / kRowSums - 1) & 1u, &s_abort, a.status);
-        if (*(volatile int *)&s_abort) return;
+        if (i8_warp_aborts(&s_abort)) return;
         if (t == 0) {
             float *at = red + ((b * PARTS + part) * a.lanes_k + ul) * 16 + g;
             at[0] = yacc[0][0];

@@ -59,6 +59,8 @@ __device__ __forceinline__ void i8_wait_or_abort(uint64_t *bar, uint32_t parity,
     *abort_flag = 1;
     atomicMax(status, (uint32_t)kStatusTmaTimeout);
 }
+// Whether a whole warp leaves because the block has given up: lanes that read the flag each for itself could part in front of warp-wide instructions.
+__device__ __forceinline__ bool i8_warp_aborts(volatile int *abort_flag) { return __any_sync(0xffffffffu, *abort_flag != 0); }
 
 // Shared-memory loads by 32-bit shared address: no generic-address arithmetic, and the loads of one unit are issued
 // together ahead of the MMAs that consume them.

@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
             const int mc = (int)(pe.y >> 16), n0 = (bid + k * G) % ga.tiles * out_rows;
             float *out = ga.out + ((size_t)pe.z + (pe.y & 0xFFFFu)) * ga.n_out + n0;
             i8_wait_or_abort(&s_sums[k & 1], (uint32_t)(k >> 1) & 1u, &s_abort, ga.status);
-            if (*(volatile int *)&s_abort) return;
+            if (i8_warp_aborts(&s_abort)) return;
             for (int tok = 0; tok < mc; ++tok, sums += kTileRows, out += ga.n_out) {
 #pragma unroll
                 for (int row = lane; row < out_rows; row += 32) {
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
             const int b = k & 1;
             float *rb_ = red + b * RED_FLOATS;
             if (k >= 2) i8_wait_or_abort(&s_free[b], (uint32_t)((k >> 1) - 1) & 1u, &s_abort, ga.status);
-            if (*(volatile int *)&s_abort) return;
+            if (i8_warp_aborts(&s_abort)) return;
             if (mc <= 4) {
                 rb_[(ul * RS + t) * kTileRows + r0] = yacc1[0][0];
                 rb_[(ul * RS + t) * kTileRows + r0 + 8] = yacc1[0][1];
