@@ -380,3 +380,21 @@ def test_slices_without_a_scale_count_as_zero(gemv_variant, tensor_type, value):
         want = host(ctx().linear(dev(x), w)).copy()
         x[:, 300] = value
         np.testing.assert_array_equal(host(ctx().linear(dev(x), w)), want)
+
+
+@pytest.mark.parametrize("tensor_type", [H.Q4_K, H.Q6_K, H.Q8_0])
+@pytest.mark.parametrize("value", [8e37, 1e38, 2e38])  # below, and past 2^126, where an approximate division by the maximum gives 0
+def test_slices_of_very_large_values_are_scaled(gemv_variant, tensor_type, value):
+    """Up to 2e38: its products with these weights (up to 1.3) stay within f32."""
+    if gemv_variant != "i8":
+        pytest.skip("the records of the integer-MMA path")
+    rows, cols = 40, 768
+    data = H.random_weight(tensor_type, rows, cols, seed=3)
+    w = ctx().prepare_weight(tensor_type, data, rows, cols)
+    for m in (1, 5):
+        x = np.random.default_rng(4).standard_normal((m, cols)).astype(np.float32)
+        x[:, 300] = value
+        got = host(ctx().linear(dev(x), w)).astype(np.float64)
+        want = x.astype(np.float64) @ orc.dequantize(tensor_type, data, rows * cols).reshape(rows, cols).astype(np.float64).T
+        assert np.abs(want).max() < 3e38
+        _check(got / value, want / value)

@@ -409,7 +409,8 @@ template <uint32_t TYPE> __device__ __forceinline__ RecLane quantize_record(cons
 #pragma unroll
     for (int j = 0; j < 8; ++j) amax = fmaxf(amax, fabsf(v[j]));
     amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));  // not negative and no NaN: ordered like their bits
-    const float ratio = __fdividef(kActMax, amax);
+    // quarters of both: __fdividef gives 0 for a divisor past 2^126, and a maximum may be up to 3e38 (the bits of any other ratio are the same)
+    const float ratio = __fdividef(kActMax * 0.25f, amax * 0.25f);
     const bool live = amax > 0.f && amax < 3.0e38f && ratio <= 3.4e38f;  // a slice whose ratio overflows is 0 at the scale 1 / ratio anyway
     const float inv = live ? ratio : 0.f;
     o.scale = live ? __fdividef(1.f, inv) : 0.f;  // the scale actually applied: x ~ x_q / inv
