@@ -191,6 +191,20 @@ def test_gather_rows_by_ids_on_the_device(shape, dtype):
     assert any("empty" in name for name in seen.names)
 
 
+def test_profilers_see_the_results_being_allocated():
+    from torch.profiler import ProfilerActivity, profile
+
+    rows, cols = 33, 512
+    w = ctx().prepare_weight(H.Q4_K, H.random_weight(H.Q4_K, rows, cols, seed=5), rows, cols)
+    x, ids = torch.zeros((1, cols), device="cuda"), torch.arange(3, device="cuda", dtype=torch.int32)
+    calls = (lambda: ctx().linear(x, w), lambda: ctx().gated_linear(x, w, w), lambda: ctx().gather_rows(w, ids), lambda: ctx().linear_batch([(x, w)]), lambda: ctx().rmsnorm_linear_multi(x, x[0], 1e-6, [w]))
+    for call in calls:
+        call()
+        with profile(activities=[ProfilerActivity.CPU]) as seen:
+            call()
+        assert sum(e.count for e in seen.key_averages() if e.key == "aten::empty") == 1
+
+
 def test_gather_rows_reports_bad_row_ids_without_faulting():
     from zllm_b200 import ffi
 

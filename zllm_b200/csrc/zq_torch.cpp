@@ -9,6 +9,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
@@ -101,10 +102,11 @@ struct NoGil {
     ~NoGil() { PyEval_RestoreThread(s); }
 };
 // without the GIL.  On the GPU by the function that at::empty ends in
-// (0.4 us instead of 0.8), unless a mode is on that would see the call (dispatch modes, tracing, function transforms, autocast) or fill the tensor.
+// (0.4 us instead of 0.8), unless something is on that would see the call (dispatch modes, tracing, function transforms, autocast, the callbacks of
+// profilers) or fill the tensor.
 at::Tensor new_rows(const at::Tensor &like, size_t m, size_t n, at::ScalarType t) {
     const int64_t size[2] = {(int64_t)m, (int64_t)n};
-    const bool watched = !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty();
+    const bool watched = !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty() || at::hasCallbacks();
     if (like.is_cuda() && !watched && !at::globalContext().deterministicAlgorithms()) return at::Tensor(at::detail::empty_cuda(size, t, like.device(), std::nullopt));
     return at::empty(size, like.options().dtype(t));
 }
