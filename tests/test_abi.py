@@ -52,3 +52,10 @@ def test_product_package_does_not_touch_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h", ".cpp", ".hpp")):
                 text = open(os.path.join(dirpath, f), errors="replace").read()
                 assert "oracle" not in text.lower(), f"{f} mentions the oracle"
+
+
+def test_the_native_mirror_needs_no_cuda_build_of_torch():
+    """The CPU tests load it too: it is linked against torch's CPU libraries, and the CUDA allocator is reached through torch's hooks."""
+    with open(os.path.join(ROOT, "zllm_b200", "lib", "_zq_torch.so"), "rb") as f:
+        linked = f.read()
+    assert b"libtorch_cpu" in linked and b"libtorch_cuda" not in linked and b"libc10_cuda" not in linked

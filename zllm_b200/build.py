@@ -57,7 +57,7 @@ def _link_binding(force: bool):
     if not (force or _stale(BINDING, [obj])):
         return
     tlib = os.path.join(os.path.dirname(torch.__file__), "lib")
-    cmd = ["g++", "-shared", "-o", BINDING, obj, "-L", OUT_DIR, "-lzq_b200", "-L", tlib, "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-lc10", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"]
+    cmd = ["g++", "-shared", "-o", BINDING, obj, "-L", OUT_DIR, "-lzq_b200", "-L", tlib, "-ltorch_python", "-ltorch_cpu", "-lc10", "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{tlib}"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         sys.stderr.write(r.stdout + r.stderr)
