@@ -366,3 +366,27 @@ def test_norm_inside_the_decode_kernel_and_before_it(types):
         if len(types) == 1:
             assert np.array_equal(a[0].view(np.uint32), b[0].view(np.uint32))
         assert H.max_rel_error(a, b[:1]) <= 1e-5  # two types share a launch in one case: other ranges, other order of the f32 sums
+
+
+@pytest.mark.parametrize("offset", [0, 2560])  # the row at the front of the result's buffer, and inside it
+def test_gated_row_under_its_own_result_keeps_the_record_pass(offset):
+    """One row, its result over it: the records are made before anything is stored (two launches), not by CTAs that store side by side (one)."""
+    from zllm_b200 import ffi
+
+    rows, cols = 10240, 5120
+    data = [H.random_weight(H.Q4_K, rows, cols, seed=s) for s in (1, 2)]
+    w = [ctx().prepare_weight(H.Q4_K, d, rows, cols) for d in data]
+    x = torch.randn((1, cols), generator=torch.Generator().manual_seed(5)).cuda()
+    run = lambda src, dst: ffi.call("zq_gated_silu", ctx().handle, w[0].handle, w[1].handle, src.data_ptr(), 0, 1, dst.data_ptr(), 0)
+    apart = torch.empty((1, rows), device="cuda")
+    before = ctx().launch_count
+    run(x, apart)
+    assert ctx().launch_count - before == 1
+    buffer = torch.zeros((1, rows), device="cuda")
+    under = buffer[:, offset:offset + cols]
+    under.copy_(x)
+    before = ctx().launch_count
+    run(under, buffer)
+    assert ctx().launch_count - before == 2
+    want = orc.gated_linear(H.Q4_K, data[0], data[1], rows, cols, x.cpu().numpy())
+    assert H.max_rel_error(host(buffer), want) <= 1e-3 and H.max_rel_error(host(apart), want) <= 1e-3  # products of two sums

@@ -551,7 +551,10 @@ int zq_gated_silu(zq_ctx *ctx, const zq_weight *gate, const zq_weight *up, const
     if (!up || up->ctx != ctx) return set_error(err, ZQ_ERR_ARG, "gated linear: bad up weight");
     if (gate->rows != up->rows || gate->cols != up->cols || gate->type != up->type) return set_error(err, ZQ_ERR_SHAPE, "gated linear: gate [%zu, %zu] type %u and up [%zu, %zu] type %u differ", gate->rows, gate->cols, gate->type, up->rows, up->cols, up->type);
     const WlHostJob listed = {gate, up, dev_x, m, dev_y, nullptr, -1};
-    if (m == 1 && !ctx->narrow_gemv_tiles && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv) {
+    // The work list's record pass reads the row before anything is written; of the one-row kernels' CTAs one may store while another still reads.
+    const uint8_t *const xb = reinterpret_cast<const uint8_t *>(dev_x), *const yb = reinterpret_cast<const uint8_t *>(dev_y);
+    const bool apart = xb + m * gate->cols * dtype_size(x_dtype) <= yb || yb + m * gate->rows * dtype_size(y_dtype) <= xb;
+    if (m == 1 && apart && !ctx->narrow_gemv_tiles && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv) {
         RowCall one;
         one.jobs[0] = {gate, up, dev_y, nullptr, y_dtype};
         one.n_jobs = 1;
