@@ -551,21 +551,24 @@ int zq_gated_silu(zq_ctx *ctx, const zq_weight *gate, const zq_weight *up, const
     if (!up || up->ctx != ctx) return set_error(err, ZQ_ERR_ARG, "gated linear: bad up weight");
     if (gate->rows != up->rows || gate->cols != up->cols || gate->type != up->type) return set_error(err, ZQ_ERR_SHAPE, "gated linear: gate [%zu, %zu] type %u and up [%zu, %zu] type %u differ", gate->rows, gate->cols, gate->type, up->rows, up->cols, up->type);
     const WlHostJob listed = {gate, up, dev_x, m, dev_y, nullptr, -1};
-    // The work list's record pass reads the row before anything is written; of the one-row kernels' CTAs one may store while another still reads.
-    const uint8_t *const xb = reinterpret_cast<const uint8_t *>(dev_x), *const yb = reinterpret_cast<const uint8_t *>(dev_y);
-    const bool apart = xb + m * gate->cols * dtype_size(x_dtype) <= yb || yb + m * gate->rows * dtype_size(y_dtype) <= xb;
-    if (m == 1 && apart && !ctx->narrow_gemv_tiles && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv) {
-        RowCall one;
-        one.jobs[0] = {gate, up, dev_y, nullptr, y_dtype};
-        one.n_jobs = 1;
-        one.x = dev_x;
-        one.x_dtype = x_dtype;
-        one.norm = nullptr;
-        bool taken = false;
-        rc = launch_gemv_row(ctx, one, taken, err);
-        if (rc || taken) return rc;
+    if (!ctx->disable_worklist && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv && gemv_wl_supported(ctx, listed) && gated_prefers_worklist(ctx, gate, m)) {
+        // The one-row kernels first, as launch_gemv_i8 has them for the calls that do not come here; but the list's record pass reads the row before anything is
+        // written, and of their CTAs one may store while another still reads.
+        const uint8_t *const xb = reinterpret_cast<const uint8_t *>(dev_x), *const yb = reinterpret_cast<const uint8_t *>(dev_y);
+        const bool apart = xb + m * gate->cols * dtype_size(x_dtype) <= yb || yb + m * gate->rows * dtype_size(y_dtype) <= xb;
+        if (m == 1 && apart && !ctx->narrow_gemv_tiles) {
+            RowCall one;
+            one.jobs[0] = {gate, up, dev_y, nullptr, y_dtype};
+            one.n_jobs = 1;
+            one.x = dev_x;
+            one.x_dtype = x_dtype;
+            one.norm = nullptr;
+            bool taken = false;
+            rc = launch_gemv_row(ctx, one, taken, err);
+            if (rc || taken) return rc;
+        }
+        return launch_gemv_wl(ctx, &listed, 1, x_dtype, y_dtype, err, nullptr, true);
     }
-    if (!ctx->disable_worklist && !ctx->force_f16_gemv && !ctx->force_staged_gemv && !ctx->enable_tcgen05_gemv && gemv_wl_supported(ctx, listed) && gated_prefers_worklist(ctx, gate, m)) return launch_gemv_wl(ctx, &listed, 1, x_dtype, y_dtype, err, nullptr, true);
     if (m <= 16 && (!is_operand_pass_only(gate->type) || ((gate->type == ZQ_Q5_K || gate->type == ZQ_Q6_K) && !ctx->force_f16_gemv && !ctx->force_staged_gemv))) return launch_gemv(ctx, gate, up, dev_x, x_dtype, m, dev_y, y_dtype, nullptr, err);
     return launch_gemm(ctx, gate, up, dev_x, x_dtype, m, dev_y, y_dtype, nullptr, err);
 }

@@ -496,7 +496,7 @@ static int launch_i8_type(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up
 int launch_gemv_i8(zq_ctx *ctx, const zq_weight *w, const zq_weight *w_up, const GemvParams &p, bool &taken, zq_error *err) {
     taken = false;
     if (p.m < 1 || p.m > kMaxGemvRows) return ZQ_OK;
-    if (p.m == 1 && !ctx->narrow_gemv_tiles) {  // one row: the one-pass kernel where the matrix fits into shared memory
+    if (p.m == 1 && !ctx->narrow_gemv_tiles) {  // one row: the kernels of zq_gemv_row.cu where they fit and pay
         RowCall c;
         c.jobs[0] = {w, w_up, p.y, p.residual, p.y_dtype};
         c.n_jobs = 1;
