@@ -58,7 +58,7 @@ int zq_ctx_use_own_stream(zq_ctx *ctx, zq_error *err);
 int zq_ctx_sync(zq_ctx *ctx, zq_error *err);
 /* Diagnostic switches (the counterpart of the reference's ZLLM_CUDA_* environment switches, kept per context).
  * Known keys (0/1): "force_staged_gemv", "force_f16_gemv" (decode on the f16 kernels instead of the integer-MMA kernel),
- * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "disable_cut_tiles" / "force_cut_tiles" (prefill tiles cut along K: never / wherever whole ones leave part of a round empty), "disable_wide_tiles" / "force_wide_tiles" (prefill tiles of packed weights: never more than 256 tokens / up to 320 wherever that is more), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_fused_gemm" / "force_fused_gemm" (prefill of Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL and Q8_0 never / always with the dequantisation inside the GEMM; default: by type, form, rows and columns as measured, always up to 1024 tokens, and MoE prefill). */
+ * "enable_tcgen05_gemv" (Q4_K decode on the tcgen05 kernel), "disable_pdl" (decode and prefill kernels without programmatic dependent launch), "disable_worklist" (zq_linear_batch and the multi-weight entries launch one kernel per job), "force_moe_per_expert" (MoE forward always on the host-grouped path), "force_moe_host_grouping" (MoE prefill: routes grouped on the host instead of on the device), "disable_cut_tiles" / "force_cut_tiles" (prefill tiles cut along K: never / wherever whole ones leave part of a round empty), "disable_wide_tiles" / "force_wide_tiles" (prefill tiles of packed weights: never more than 256 tokens / up to 320 wherever that is more), "narrow_gemv_tiles" (decode, up to 4 rows: 64-row tiles, two CTAs per SM), "disable_row_gemv" / "force_row_resident" / "force_row_stream" (decode of one row: never on the one-row kernels / on the resident / on the streamed one wherever that form fits, and on no other), "disable_fused_gemm" / "force_fused_gemm" (prefill of Q4_K, Q5_K, Q6_K, Q4_0, IQ4_NL and Q8_0 never / always with the dequantisation inside the GEMM; default: by type, form, rows and columns as measured, always up to 1024 tokens, and MoE prefill). */
 int zq_ctx_set_option(zq_ctx *ctx, const char *key, int value, zq_error *err);
 int zq_ctx_sm_count(const zq_ctx *ctx);
 /* Number of kernels this library has launched on the context since creation (bench accounting). */

@@ -277,6 +277,10 @@ int zq_ctx_set_option(zq_ctx *ctx, const char *key, int value, zq_error *err) {
         ctx->narrow_gemv_tiles = value;
         return ZQ_OK;
     }
+    if (!strcmp(key, "disable_row_gemv") || !strcmp(key, "force_row_resident") || !strcmp(key, "force_row_stream")) {
+        ctx->row_form = !value ? 0 : key[0] == 'd' ? -1 : key[10] == 'r' ? 1 : 2;
+        return ZQ_OK;
+    }
     if (!strcmp(key, "disable_cut_tiles") || !strcmp(key, "force_cut_tiles")) {
         ctx->cut_tiles = !value ? 0 : key[0] == 'f' ? 1 : -1;
         return ZQ_OK;

@@ -298,6 +298,7 @@ struct zq_ctx {
     // parity-clean but, as measured, not yet faster than the warp-MMA path.
     int enable_tcgen05_gemv = 0;
     int force_f16_gemv = 0;  // skip the integer-MMA decode kernel (tests of the f16 kernels)
+    int row_form = 0;           // one-row decode kernels: by rule (0), never (-1), resident (1) or streamed (2) wherever that form fits
     int narrow_gemv_tiles = 0;  // integer-MMA decode, up to 4 rows: 64-row tiles, two CTAs per SM (measured slower; off)
     int disable_pdl = 0;     // launch decode and prefill kernels without programmatic dependent launch
     int disable_worklist = 0;  // zq_linear_batch and the multi-weight entries: one launch per job instead of the work-list kernel

@@ -385,11 +385,8 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
 //   Q4_K  5120 -> 11008 (0.63) 11.5/9.8  3840 -> 28672 (0.76) 18.8/17.0  5120 -> 28672 (0.81) 23.9/19.8  3840 -> 14336 (0.82) 9.8/10.3  3840 -> 17408 (0.94) 10.6/11.6  2048 -> 28672 (0.81) 12.6/14.0
 //   Q8_0  3072 -> 28672 (0.81) 22.1/18.3  3072 -> 14336 (0.88) 11.7/11.3  3840 -> 17408 (0.94) 15.1/15.4
 //   gated Q4_K  3840 -> 15360 (0.82) 20.3/17.1  3840 -> 17408 (0.94) 21.1/18.4  3072 -> 17408 (1.0) 18.7/18.2  2048 -> 14336 (0.88) 12.8/14.0;   IQ4_NL  3840 -> 15360 27.2/24.0  3840 -> 8192 (0.94) 14.6/14.7
-static bool row_stream_pays(const zq_ctx *ctx, const RowCall &c, uint32_t type, size_t lanes_k, size_t units, size_t all) {
+static bool row_stream_pays(const zq_ctx *ctx, const RowCall &c, uint32_t type, size_t units, size_t all) {
     const size_t sms = (size_t)ctx->sm_count, n = (all + sms - 1) / sms, row_bytes = units * row_unit_bytes(c.jobs[0].w->type);
-    for (int i = 1; i < c.n_jobs; ++i)
-        if (is_kclass(c.jobs[i].w->type) != is_kclass(c.jobs[0].w->type)) return false;  // a CTA's range may hold several jobs: one format of records
-    if (lanes_k < 4) return false;
     if (c.norm) {
         const bool eight = type == ZQ_Q8_0;
         if (type == ZQ_IQ4_NL && units > (size_t)kRowWarps && n > 8) return false;
@@ -424,15 +421,19 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
     if (turns > (size_t)kRowTurns) return ZQ_OK;
     // Gated pairs of many outputs from few columns, and IQ4_NL's of more than 16 units, are as fast or faster where a K slice is a CTA: IQ4_NL 1024 -> 8192 5.8 there,
     // 6.3 here, 8192 -> 512 6.9 / 7.3; Q6_K 512 -> 8192 4.3 / 4.4.
-    if (GATED && (c.jobs[0].w->rows >= 8 * c.jobs[0].w->cols || (TYPE == ZQ_IQ4_NL && turns > 1))) return ZQ_OK;
+    const int form = ctx->row_form;  // 0: by the rules below; else what fits
+    if (form == 0 && GATED && (c.jobs[0].w->rows >= 8 * c.jobs[0].w->cols || (TYPE == ZQ_IQ4_NL && turns > 1))) return ZQ_OK;
     size_t row = 0, all = 0;
     for (int i = 0; i < c.n_jobs; ++i) {
         row = std::max(row, (size_t)row_smem_pitch(c.jobs[i].w->type, (int)units));
         all += (c.jobs[i].w->rows + 15) / 16;
     }
+    bool streams = lanes_k >= 4;
+    for (int i = 1; i < c.n_jobs; ++i) streams &= is_kclass(c.jobs[i].w->type) == is_kclass(c.jobs[0].w->type);  // a CTA's range may hold several jobs: one format of records
+    const auto pays = [&]() { return form == 0 && streams && row_stream_pays(ctx, c, TYPE, units, all); };
     RowArgs ra;
     size_t grid = 0, warps = 0, smem = 0;
-    for (size_t per_sm = 2; per_sm >= 1 && !taken; --per_sm) {
+    for (size_t per_sm = 2; per_sm >= 1 && !taken && form != 2; --per_sm) {
         const size_t ctas = (size_t)ctx->sm_count * per_sm;
         size_t groups = (all + ctas - 1) / ctas;
         for (; groups <= (size_t)kRowMaxGroups; ++groups) {  // every job starts on a CTA of its own
@@ -448,10 +449,10 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         smem = w_bytes + rec + lanes_k * groups * PARTS * 16 * sizeof(float) + 128;
         if (per_sm * warps * regs > 65536 || smem > (per_sm == 2 ? (size_t)kRowMaxSmem / 2 - 1024 : (size_t)200 << 10)) continue;
         // IQ4_NL's look-ups want more warps than two CTAs of six hold: 1536 -> 17408 7.5 us on gemv_i8_kernel, 8.6 here; gated 1024 -> 5120 5.3 / 5.9
-        if (TYPE == ZQ_IQ4_NL && (GATED && lanes_k <= 4 ? groups > 1 : groups > 2 && per_sm * warps < (size_t)kRowWarps)) break;
+        if (form == 0 && TYPE == ZQ_IQ4_NL && (GATED && lanes_k <= 4 ? groups > 1 : groups > 2 && per_sm * warps < (size_t)kRowWarps)) break;
         // much to copy and a busiest SM with far more of it than its share: Q8_0 1536 -> 14336 6.3 / 7.2, gated 1536 -> 5120 5.8 / 6.1
-        if (per_sm == 1 && w_bytes > 150 * 1024 && 100 * groups * ctx->sm_count > 112 * all) continue;
-        if (per_sm == 1 && groups >= 5 && row_stream_pays(ctx, c, TYPE, lanes_k, units, all)) break;
+        if (form == 0 && per_sm == 1 && w_bytes > 150 * 1024 && 100 * groups * ctx->sm_count > 112 * all) continue;
+        if (form == 0 && per_sm == 1 && groups >= 5 && pays()) break;
         ra.groups = (int)groups;
         ra.lanes_k = (int)lanes_k;
         ra.lanes_g = (int)lanes_g;
@@ -461,9 +462,8 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         taken = true;
     }
     bool stream = false;
-    if (!taken) {
-        const bool pays = row_stream_pays(ctx, c, TYPE, lanes_k, units, all);
-        for (size_t lanes_g = 2; lanes_g >= 1 && !taken && pays; --lanes_g) {
+    if (!taken && (form == 2 ? streams : pays())) {
+        for (size_t lanes_g = 2; lanes_g >= 1 && !taken; --lanes_g) {
             if (lanes_g * lanes_k > (size_t)kRowWarps) continue;
             warps = lanes_g * lanes_k;
             const size_t rec = warps * turns * kRec, sums = kRowSums * PARTS * lanes_k * 16 * sizeof(float), stage = 16 * row;
@@ -518,7 +518,7 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
 
 int launch_gemv_row(zq_ctx *ctx, const RowCall &c, bool &taken, zq_error *err) {
     taken = false;
-    if (c.n_jobs < 1 || c.n_jobs > kRowMaxJobs) return ZQ_OK;
+    if (c.n_jobs < 1 || c.n_jobs > kRowMaxJobs || ctx->row_form < 0) return ZQ_OK;
     const bool gated = c.jobs[0].w_up != nullptr;
     uint32_t type = c.jobs[0].w->type;
     for (int i = 0; i < c.n_jobs; ++i) {
