@@ -26,8 +26,8 @@ def force():
     ctx().set_option("disable_row_gemv", 0)
 
 
-def kernels_of(call, tmp_path):
-    """Names of the library's kernels that a call launches."""
+def launches_of(call, tmp_path):
+    """(name, CTAs, threads) of the decode family's kernels that a call launches."""
     call()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     try:
@@ -38,9 +38,14 @@ def kernels_of(call, tmp_path):
         ctx().set_stream(torch.cuda.current_stream().cuda_stream)
     dot = tmp_path / "graph.dot"
     assert ctypes.CDLL("libcuda.so.1").cuGraphDebugDotPrint(ctypes.c_void_p(graph.raw_cuda_graph()), str(dot).encode(), 1) == 0
-    names = set(re.findall(r"(gemv_row_stream_kernel|gemv_row_kernel|gemv_i8_kernel|gemv_wl_kernel|wl_quantize_kernel|rmsnorm_kernel)", dot.read_text()))
-    assert names, "no kernel of the decode family in the graph"
-    return names
+    names = "gemv_row_stream_kernel|gemv_row_kernel|gemv_i8_kernel|gemv_wl_kernel|wl_quantize_kernel|rmsnorm_kernel"
+    found = [(name, int(ctas), int(threads)) for name, ctas, threads in re.findall(r"(%s)[^|]*?\\<\\<\\<(\d+),(\d+)," % names, dot.read_text())]
+    assert found, "no kernel of the decode family in the graph"
+    return found
+
+
+def kernels_of(call, tmp_path):
+    return {name for name, _, _ in launches_of(call, tmp_path)}
 
 
 def weights(types, rows, cols, seed):
@@ -131,3 +136,14 @@ def test_calls_of_a_decoder_step_take_the_form_they_were_measured_for(tmp_path, 
     x, nw = torch.randn((1, cols), device="cuda"), torch.rand(cols, device="cuda")
     call = (lambda: ctx().gated_linear(x, *ws)) if gated else (lambda: ctx().linear(x, ws[0])) if gated is False else (lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, ws))
     assert kernels_of(call, tmp_path) == {want}
+
+
+@pytest.mark.parametrize("types,rows,cols", [((H.Q6_K,), (3001,), 2304), ((H.Q4_K, H.Q6_K, H.Q5_K), (3436, 1718, 1718), 2304), ((H.Q6_K,), (4450,), 4608), ((H.Q8_0, H.Q4_K), (2500, 2500), 2048)])
+def test_two_ctas_of_an_sm_run_side_by_side(force, tmp_path, types, rows, cols):
+    """More CTAs than SMs only where two are resident together.  These kernels take more than 96 registers (Q6_K, several types): four warps per scheduler."""
+    ws = weights(types, rows, cols, 1)[1]
+    x, nw = torch.randn((1, cols), device="cuda"), torch.rand(cols, device="cuda")
+    force("resident")
+    for name, ctas, threads in launches_of((lambda: ctx().linear(x, ws[0])) if len(ws) == 1 else lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, ws), tmp_path):
+        assert name == "gemv_row_kernel"
+        assert ctas <= torch.cuda.get_device_properties(0).multi_processor_count or 2 * threads <= 16 * 32

@@ -417,6 +417,9 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         ZQ_CUDA_CHECK(cudaFuncSetAttribute(gemv_row_stream_kernel<TYPE, GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowMaxSmem), err);
         regs = (size_t)((fa.numRegs + 7) & ~7) * 32;
     }
+    // Warps that are resident at once: registers are a quarter of the SM's to each of its four schedulers.  Counted over the whole SM two CTAs of nine warps of 112
+    // registers were planned side by side and ran one after the other: three types 2304 -> 3436, 1718, 1718 8.9 us, now 6.4; Q6_K 2304 -> 3001 5.2, now 3.7.
+    const size_t slots = 4 * (16384 / regs);
     const size_t units = c.jobs[0].w->units_per_row, turns = (units + kRowWarps - 1) / kRowWarps, lanes_k = (units + turns - 1) / turns;
     if (turns > (size_t)kRowTurns) return ZQ_OK;
     // Gated pairs of many outputs from few columns, and IQ4_NL's of more than 16 units, are as fast or faster where a K slice is a CTA: IQ4_NL 1024 -> 8192 5.8 there,
@@ -443,11 +446,11 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         }
         if (groups > (size_t)kRowMaxGroups) continue;
         size_t lanes_g = 1;
-        while (2 * lanes_g * lanes_k <= (size_t)kRowWarps && 2 * lanes_g <= groups * PARTS && per_sm * 2 * lanes_g * lanes_k * regs <= 65536) lanes_g *= 2;
+        while (2 * lanes_g * lanes_k <= (size_t)kRowWarps && 2 * lanes_g <= groups * PARTS && per_sm * 2 * lanes_g * lanes_k <= slots) lanes_g *= 2;
         warps = lanes_k * lanes_g;
         const size_t w_bytes = 16 * groups * PARTS * row, rec = warps * turns * kRec;
         smem = w_bytes + rec + lanes_k * groups * PARTS * 16 * sizeof(float) + 128;
-        if (per_sm * warps * regs > 65536 || smem > (per_sm == 2 ? (size_t)kRowMaxSmem / 2 - 1024 : (size_t)200 << 10)) continue;
+        if (per_sm * warps > slots || smem > (per_sm == 2 ? (size_t)kRowMaxSmem / 2 - 1024 : (size_t)200 << 10)) continue;
         // IQ4_NL's look-ups want more warps than two CTAs of six hold: 1536 -> 17408 7.5 us on gemv_i8_kernel, 8.6 here; gated 1024 -> 5120 5.3 / 5.9
         if (form == 0 && TYPE == ZQ_IQ4_NL && (GATED && lanes_k <= 4 ? groups > 1 : groups > 2 && per_sm * warps < (size_t)kRowWarps)) break;
         // much to copy and a busiest SM with far more of it than its share: Q8_0 1536 -> 14336 6.3 / 7.2, gated 1536 -> 5120 5.8 / 6.1
