@@ -147,3 +147,14 @@ def test_two_ctas_of_an_sm_run_side_by_side(force, tmp_path, types, rows, cols):
     for name, ctas, threads in launches_of((lambda: ctx().linear(x, ws[0])) if len(ws) == 1 else lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, ws), tmp_path):
         assert name == "gemv_row_kernel"
         assert ctas <= torch.cuda.get_device_properties(0).multi_processor_count or 2 * threads <= 16 * 32
+
+
+@pytest.mark.parametrize("tensor_type,rows,cols,form", [
+    (H.Q4_K, 58000, 256, "norm"), (H.Q4_0, 33709, 512, "norm"), (H.Q4_0, 17408, 512, "plain"), (H.Q5_K, 15939, 2304, "plain"), (H.Q4_K, 6846, 2816, "gated"), (H.Q5_K, 5553, 2304, "gated"), (H.Q4_0, 7200, 3328, "gated"),
+])
+def test_calls_that_are_faster_elsewhere_are_left_alone(tmp_path, tensor_type, rows, cols, form):
+    """Many groups of one or two units, too much for one CTA, a ring for a few groups: 5 to 36 % slower on the one-row kernels."""
+    ws = weights((tensor_type,) * 2, (rows,) * (2 if form == "gated" else 1), cols, 1)[1]
+    x, nw = torch.randn((1, cols), device="cuda"), torch.rand(cols, device="cuda")
+    call = {"plain": lambda: ctx().linear(x, ws[0]), "gated": lambda: ctx().gated_linear(x, *ws), "norm": lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, ws)}[form]
+    assert not kernels_of(call, tmp_path) & {"gemv_row_kernel", "gemv_row_stream_kernel"}

@@ -398,7 +398,13 @@ static bool row_stream_pays(const zq_ctx *ctx, const RowCall &c, uint32_t type, 
     const size_t split = std::max<size_t>(1, std::min<size_t>(std::min<size_t>(sms / std::max<size_t>(tiles, 1), 8), chunks));
     const size_t there = (tiles * split + sms - 1) / sms * ((chunks + split - 1) / split) * kTileRows * kChunkUnits, here = n * 16 * (gated ? 2 : 1) * units;
     const auto within = [&](size_t percent) { return 100 * here <= percent * there; };
-    if (gated) return units >= 12 ? within(type == ZQ_IQ4_NL ? 90 : 95) : units >= 8 && within(70);
+    if (gated) {
+        // Few groups of few bytes do not pay for the ring's start: Q5_K 2304 -> 5553 (n = 3, 0.68) 7.7/8.3, 3328 -> 7514 (n = 4, 0.93) 11.0/12.2; Q4_0 3072 -> 5120 (n = 3, 0.75) 7.3/7.7, 3328 -> 7200
+        // (n = 4, 0.93) 8.9/10.2.  Types of more bytes or more instructions do: Q8_0 2816 -> 5352 (n = 3, 0.69) 10.1/8.9, IQ4_NL 2816 -> 6496 10.8/10.1
+        const bool few = (n == 3 || n == 4) && (type == ZQ_Q4_K || type == ZQ_Q5_K || type == ZQ_Q4_0);
+        if (units < 12 + (few && type == ZQ_Q4_0)) return units >= 8 && !few && within(70);
+        return within(type == ZQ_IQ4_NL || (few && type != ZQ_Q4_K) ? 90 : 95);
+    }
     return (units >= 12 && within(type == ZQ_Q8_0 ? 90 : 70)) || (units >= 15 && within(81));
 }
 
@@ -431,6 +437,7 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         row = std::max(row, (size_t)row_smem_pitch(c.jobs[i].w->type, (int)units));
         all += (c.jobs[i].w->rows + 15) / 16;
     }
+    const bool one_round = (c.jobs[0].w->rows + (GATED ? kTileRows / 2 : kTileRows) - 1) / (GATED ? kTileRows / 2 : kTileRows) <= (size_t)ctx->sm_count;  // of gemv_i8_kernel's tiles
     bool streams = lanes_k >= 4;
     for (int i = 1; i < c.n_jobs; ++i) streams &= is_kclass(c.jobs[i].w->type) == is_kclass(c.jobs[0].w->type);  // a CTA's range may hold several jobs: one format of records
     const auto pays = [&]() { return form == 0 && streams && row_stream_pays(ctx, c, TYPE, units, all); };
@@ -453,6 +460,13 @@ template <uint32_t TYPE, bool GATED> static int launch_row_one(zq_ctx *ctx, cons
         if (per_sm * warps > slots || smem > (per_sm == 2 ? (size_t)kRowMaxSmem / 2 - 1024 : (size_t)200 << 10)) continue;
         // IQ4_NL's look-ups want more warps than two CTAs of six hold: 1536 -> 17408 7.5 us on gemv_i8_kernel, 8.6 here; gated 1024 -> 5120 5.3 / 5.9
         if (form == 0 && TYPE == ZQ_IQ4_NL && (GATED && lanes_k <= 4 ? groups > 1 : groups > 2 && per_sm * warps < (size_t)kRowWarps)) break;
+        // One or two warps along K have all the look-ups and sums of many groups to themselves.  Norm in front, work list / here: 256 -> 18463 (6.2 groups) 5.4 / 4.4, 58465 (12.3) 6.9 / 9.3; 512 ->
+        // 22000 (4.6) 5.6 / 5.5, 27228 (5.8) 6.3 / 6.5, 33709 (7.1) 5.7 / 6.9, 3 x 18058 (11.4) 7.4 / 10.0.  Plain, two units, against one round of tiles: 512 -> 17408 Q4_0 3.5 / 3.9, Q4_K 3.7 / 4.0, Q8_0 4.0 / 4.1
+        if (form == 0 && c.norm && groups > (units == 1 ? 7 : 5) && units <= 2) break;
+        if (form == 0 && !c.norm && units == 2 && groups >= 4 && one_round) break;
+        // more than 150 KB of many groups in one CTA come too late against one round of tiles: Q5_K 2304 -> 15939 8.7 / 10.8, gated Q8_0 1536 -> 6462 6.2 / 6.9, Q4_K 3328 -> 6846 9.1 / 9.8;
+        // not of few: Q6_K 3072 -> 8870 (four) 8.7 / 7.7
+        if (form == 0 && !c.norm && per_sm == 1 && w_bytes > 150 * 1024 && groups * PARTS >= 5 && turns == 1 && one_round) break;
         // much to copy and a busiest SM with far more of it than its share: Q8_0 1536 -> 14336 6.3 / 7.2, gated 1536 -> 5120 5.8 / 6.1
         if (form == 0 && per_sm == 1 && w_bytes > 150 * 1024 && 100 * groups * ctx->sm_count > 112 * all) continue;
         if (form == 0 && per_sm == 1 && groups >= 5 && pays()) break;
