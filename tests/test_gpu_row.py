@@ -158,3 +158,11 @@ def test_calls_that_are_faster_elsewhere_are_left_alone(tmp_path, tensor_type, r
     x, nw = torch.randn((1, cols), device="cuda"), torch.rand(cols, device="cuda")
     call = {"plain": lambda: ctx().linear(x, ws[0]), "gated": lambda: ctx().gated_linear(x, *ws), "norm": lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, ws)}[form]
     assert not kernels_of(call, tmp_path) & {"gemv_row_kernel", "gemv_row_stream_kernel"}
+
+
+@pytest.mark.parametrize("types,rows,cols", [((H.Q8_0, H.Q4_0, H.Q4_0), (2000, 9000, 9000), 3328), ((H.Q4_0, H.Q6_K, H.IQ4_NL), (6000, 9000, 3000), 3328), ((H.Q5_K, H.Q4_K, H.Q4_K), (2000, 9000, 9000), 3584)])
+def test_a_lists_form_does_not_depend_on_its_order(tmp_path, types, rows, cols):
+    ws = weights(types, rows, cols, 1)[1]
+    x, nw = torch.randn((1, cols), device="cuda"), torch.rand(cols, device="cuda")
+    ran = [kernels_of(lambda: ctx().rmsnorm_linear_multi(x, nw, 1e-6, [ws[i] for i in order]), tmp_path) for order in ((0, 1, 2), (1, 2, 0), (2, 0, 1))]
+    assert ran[0] == ran[1] == ran[2]

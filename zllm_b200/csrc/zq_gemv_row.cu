@@ -386,9 +386,17 @@ __global__ void __launch_bounds__((kRowWarps + 2) * 32, 1) gemv_row_stream_kerne
 //   Q8_0  3072 -> 28672 (0.81) 22.1/18.3  3072 -> 14336 (0.88) 11.7/11.3  3840 -> 17408 (0.94) 15.1/15.4
 //   gated Q4_K  3840 -> 15360 (0.82) 20.3/17.1  3840 -> 17408 (0.94) 21.1/18.4  3072 -> 17408 (1.0) 18.7/18.2  2048 -> 14336 (0.88) 12.8/14.0;   IQ4_NL  3840 -> 15360 27.2/24.0  3840 -> 8192 (0.94) 14.6/14.7
 static bool row_stream_pays(const zq_ctx *ctx, const RowCall &c, uint32_t type, size_t units, size_t all) {
-    const size_t sms = (size_t)ctx->sm_count, n = (all + sms - 1) / sms, row_bytes = units * row_unit_bytes(c.jobs[0].w->type);
+    const size_t sms = (size_t)ctx->sm_count, n = (all + sms - 1) / sms;
     if (c.norm) {
+        size_t row_bytes = 0;  // of a list's average row, whatever its order
+        bool look_ups = false;
+        for (int i = 0; i < c.n_jobs; ++i) {
+            row_bytes += (c.jobs[i].w->rows + 15) / 16 * units * row_unit_bytes(c.jobs[i].w->type);
+            look_ups |= c.jobs[i].w->type == ZQ_IQ4_NL;
+        }
+        row_bytes /= all;
         const bool eight = type == ZQ_Q8_0;
+        if (type == 0 && look_ups && n > 8) return false;  // Q8_0, IQ4_NL, IQ4_NL 3328 -> 3 x 9707 (n = 13) 22.8/24.9, Q6_K, IQ4_NL, Q4_0 4352 -> 13133, 6566, 6566 (n = 12) 27.2/29.1
         if (type == ZQ_IQ4_NL && units > (size_t)kRowWarps && n > 8) return false;
         return n <= 7 || (n <= 14 ? row_bytes >= 2000 || (eight && row_bytes >= 1600) : row_bytes >= 3300 || (eight && row_bytes >= 2100));
     }
