@@ -362,3 +362,16 @@ def test_a_call_reads_what_the_call_directly_before_it_wrote(m, dtype):
     for _ in range(3):
         for a, b in zip(chain(False), want):
             assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+
+
+@pytest.mark.parametrize("m,epilogue_warps", [(24, 4), (64, 4), (96, 8), (128, 8), (200, 8)])
+def test_gated_q6k_has_the_epilogue_warps_it_was_measured_with(gemm_variant, tmp_path, m, epilogue_warps):
+    """Four up to 64 tokens per tile, where the dequantisers set the pace, eight above, where the epilogue does (2048 -> 8192 at 128 tokens 20.3 us with four, 17.8 with eight)."""
+    from tests.test_gpu_row import launches_of
+
+    if gemm_variant == "operand_pass":
+        pytest.skip("the dequantising form")
+    w = [ctx().prepare_weight(H.Q6_K, H.random_weight(H.Q6_K, 300, 512, seed=s), 300, 512) for s in (1, 2)]
+    x = torch.randn((m, 512), device="cuda", dtype=torch.float16)
+    (_, _, threads), = launches_of(lambda: ctx().gated_linear(x, *w), tmp_path, "gemm_kernel")
+    assert threads == 32 * (3 + 16 + epilogue_warps)  # tokens, MMAs and packed boxes; the dequantisers

@@ -26,8 +26,11 @@ def force():
     ctx().set_option("disable_row_gemv", 0)
 
 
-def launches_of(call, tmp_path):
-    """(name, CTAs, threads) of the decode family's kernels that a call launches."""
+DECODE = "gemv_row_stream_kernel|gemv_row_kernel|gemv_i8_kernel|gemv_wl_kernel|wl_quantize_kernel|rmsnorm_kernel"
+
+
+def launches_of(call, tmp_path, names=DECODE):
+    """(name, CTAs, threads) of the kernels of these names that a call launches."""
     call()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     try:
@@ -38,9 +41,8 @@ def launches_of(call, tmp_path):
         ctx().set_stream(torch.cuda.current_stream().cuda_stream)
     dot = tmp_path / "graph.dot"
     assert ctypes.CDLL("libcuda.so.1").cuGraphDebugDotPrint(ctypes.c_void_p(graph.raw_cuda_graph()), str(dot).encode(), 1) == 0
-    names = "gemv_row_stream_kernel|gemv_row_kernel|gemv_i8_kernel|gemv_wl_kernel|wl_quantize_kernel|rmsnorm_kernel"
     found = [(name, int(ctas), int(threads)) for name, ctas, threads in re.findall(r"(%s)[^|]*?\\<\\<\\<(\d+),(\d+)," % names, dot.read_text())]
-    assert found, "no kernel of the decode family in the graph"
+    assert found, "none of the kernels in the graph"
     return found
 
 

@@ -36,8 +36,8 @@
 // last tile of a pair shows in full: Q4_K gated 1536 -> 3840 at 256 tokens 95 us, now 26; 4096 -> 11008 at 256 tokens 75 us, now 47 (with the
 // exchange of gate and up inside a warp; before, through shared memory and a barrier per 16 columns).  27 warps leave 72 registers each.  Q6_K,
 // whose dequantisers set the pace of most tiles and need more, has four epilogue warps (23 warps, 80 registers) where the epilogue is cheap:
-// plain, and gated up to 64 tokens per tile.  Eight and four, us: 11008 -> 4096 at 24 / 128 / 512 tokens 28.6 / 31.7 / 51.2 and 26.3 / 30.6 / 48.7, 4096 -> 11008 gated
-// 37.7 / 43.0 / 93.9 and 36.9 / 44.4 / 99.6.  Of the others Q5_K spills four registers there, and every form with wide tiles
+// plain, and gated up to 64 tokens per tile.  Eight and four, us: 11008 -> 4096 at 512 tokens 51.2 and 48.7, 4096 -> 11008 gated at 512 tokens 93.9 and 99.6; SHORT,
+// gated at 24 / 64 / 128 tokens 5120 -> 17408 50.3 / 48.4 / 57 and 47.1 / 46.8 / 58, 2048 -> 8192 15.2 / 15.2 / 17.8 and 15.3 / 15.9 / 20.3.  Of the others Q5_K spills four registers there, and every form with wide tiles
 // 18 (gated 25), in the epilogue and the way out of cut tiles.
 // Every wait is bounded, counted from the end of the previous kernel; a wait that runs out sets the CTA's state, all roles fall
 // through to the end, TMEM is released and the context status word reports it.
@@ -951,9 +951,11 @@ template <uint32_t SRC> static int launch_form(zq_ctx *ctx, bool gated, const CU
     constexpr int W = SRC ? kFormWide : kFormPlain, H = SRC ? kFormShort : kFormPlain;  // operands in memory have no other form
     constexpr int Q6 = SRC == ZQ_Q6_K ? 4 : 8;  // see the roles
     if (W && p.wide) return gated ? launch_one<SRC, true, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, W, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    if (H && p.a_tmem) return gated ? launch_one<SRC, true, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    if (gated && (Q6 == 8 || p.bn > 64)) return launch_one<SRC, true, kFormPlain, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
-    return gated ? launch_one<SRC, true, kFormPlain, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, kFormPlain, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    if (H && p.a_tmem) {
+        if (gated && (Q6 == 8 || p.bn > 64)) return launch_one<SRC, true, H, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+        return gated ? launch_one<SRC, true, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, H, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
+    }
+    return gated ? launch_one<SRC, true, kFormPlain, 8>(ctx, mw, mw2, mx, mx2, p, pairs, err) : launch_one<SRC, false, kFormPlain, Q6>(ctx, mw, mw2, mx, mx2, p, pairs, err);
 }
 static int launch_src(zq_ctx *ctx, uint32_t src, bool gated, const CUtensorMap &mw, const CUtensorMap &mw2, const CUtensorMap &mx, const CUtensorMap &mx2, const GemmParams &p, int pairs, zq_error *err) {
 #define ZQ_GEMM_CASE(T) case T: return launch_form<T>(ctx, gated, mw, mw2, mx, mx2, p, pairs, err)
