@@ -375,3 +375,17 @@ def test_gated_q6k_has_the_epilogue_warps_it_was_measured_with(gemm_variant, tmp
     x = torch.randn((m, 512), device="cuda", dtype=torch.float16)
     (_, _, threads), = launches_of(lambda: ctx().gated_linear(x, *w), tmp_path, "gemm_kernel")
     assert threads == 32 * (3 + 16 + epilogue_warps)  # tokens, MMAs and packed boxes; the dequantisers
+
+
+@pytest.mark.parametrize("tensor_type,cols,cut", [(H.Q8_0, 3328, False), (H.Q4_0, 2816, False), (H.Q6_K, 3328, True), (H.Q4_K, 11008, True)])
+def test_short_tiles_are_cut_where_their_steps_take_longer_than_the_cut(gemm_variant, tmp_path, tensor_type, cols, cut):
+    """30 tiles of 256 rows and 32 tokens: whole they are a pair each, cut they are everybody's.  Q8_0 3328 -> 7537 whole 11.0 us, cut 14.6."""
+    from tests.test_gpu_row import launches_of
+
+    if gemm_variant == "operand_pass":
+        pytest.skip("the dequantising form")
+    rows = 7537
+    w = ctx().prepare_weight(tensor_type, H.random_weight(tensor_type, rows, cols, seed=1), rows, cols)
+    x = torch.randn((32, cols), device="cuda", dtype=torch.float16)
+    (_, ctas, _), = launches_of(lambda: ctx().linear(x, w), tmp_path, "gemm_kernel")
+    assert ctas == (torch.cuda.get_device_properties(0).multi_processor_count // 2 * 2 if cut else 2 * 30)
