@@ -108,7 +108,7 @@ struct NoGil {
 // profilers) or fill the tensor.
 at::Tensor new_rows(const at::Tensor &like, size_t m, size_t n, at::ScalarType t) {
     const int64_t size[2] = {(int64_t)m, (int64_t)n};
-    const bool watched = !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty() || at::hasCallbacks();
+    const bool watched = !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set).empty() || at::getStepCallbacksUnlessEmpty(at::RecordScope::FUNCTION).has_value();
     if (like.is_cuda() && !watched && !at::globalContext().deterministicAlgorithms()) {
         const c10::DeviceGuard on(like.device());
         return at::Tensor(at::detail::empty_generic(size, at::detail::getCUDAHooks().getCUDADeviceAllocator(), c10::DispatchKeySet(c10::DispatchKey::CUDA), t, std::nullopt));
