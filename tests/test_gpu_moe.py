@@ -366,3 +366,26 @@ def test_moe_prefill_takes_every_packed_type(gate_type, down_type, hidden, inter
                 want += weight * (mats[2][e] @ f16(g / (1.0 + np.exp(-g)) * u))
         error = np.linalg.norm(got[t] - want)
         assert error <= (2.0 ** -10 + (2.0 ** -9 if dtype == torch.bfloat16 else 2.0 ** -12 if dtype == torch.float16 else 0.0)) * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 8, 9, 19])  # of one expert: passes of up to 8, by one, two, three and more tokens of the finishing warps
+@pytest.mark.parametrize("hidden,inter", [(256, 256), (1024, 19200)])  # one item per CTA; several, an odd and an even number, in both buffers of sums
+def test_moe_decode_finishes_every_row_of_a_pass(rows, hidden, inter):
+    from zllm_b200.backend import MoeExperts, moe_forward
+
+    c = ctx()
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    make = lambda n, k: c.prepare_weight(H.Q4_0, c.quantize(H.Q4_0, torch.randn((n, k), generator=g, device="cuda") * 0.02), n, k)
+    experts = [[make(inter, hidden), make(inter, hidden), make(hidden, inter)] for _ in range(2)]
+    table = MoeExperts(c, *([e[i] for e in experts] for i in range(3)))
+    x = torch.randn((rows + 2, hidden), generator=g, device="cuda")
+    ids = torch.zeros((rows + 2, 1), dtype=torch.int32, device="cuda")
+    ids[-2:] = 1  # the other expert has two
+    weights = torch.rand((rows + 2, 1), generator=g, device="cuda") + 0.5
+    got = moe_forward(c, table, x, ids, weights)
+    want = torch.empty((rows + 2, hidden), dtype=torch.float64, device="cuda")
+    for e, part in ((0, slice(0, rows)), (1, slice(rows, rows + 2))):
+        gate, up, down = (c.dequantize(w).double() for w in experts[e])
+        xd = x[part].double()
+        want[part] = weights[part].double() * ((torch.nn.functional.silu(xd @ gate.T) * (xd @ up.T)) @ down.T)
+    assert H.max_rel_error(host(got), want.cpu().numpy()) <= BOUND

@@ -12,7 +12,10 @@
 // The copies need the bytes of a ring all of the time: a stage that is free and not yet asked for is lost.  64 tokens, 256 experts of 7168 x 2048 in
 // Q4_K, top 8 and a shared one: gate/up 701 us and down 358 while the copying thread divided its 64-bit item number by the chunks of
 // a tile after each wait, 566 and 303 with the addresses ready before the wait (copies alone: 580 and 280).  A barrier of the consumer warps per
-// work item, which a warp of its own now stands in for, was 2 % of it.
+// work item, which two warps of their own now stand in for, was 2 % of it.  They share the last item of a CTA, which nothing hides: layers of few or short items are little else.
+// Barrier, one warp, two, us: 16 experts of 512 x 1792 in Q8_0, 16 tokens of 8 experts 41.5, 45.6, 41.5;  32 of 512 x 256 in Q4_K, 61 tokens of 4 31.1, 33.2, 31.8
+// (90 layers of up to 64 tokens: one warp 0.992 of the barrier's time, 18 of them more than 2 % slower, the worst 1.10; two 0.981, 8, 1.03).  Finishing the last
+// item with all consumer warps gives small layers 1 % more and costs the large one 0.6 to 1.8.
 // Arithmetic per expert is that of zq_gemv_i8.cu (16-bit integer activations, exact integer weights), the combine
 // is the one of zq_moe.cu; an expert that received more than 8 rows is walked in passes of 8.
 #include <cstring>
@@ -26,7 +29,7 @@ constexpr int kPassRows = 8;                    // activation rows per pass (two
 constexpr int kPassUnitBytes = kPassRows * kRec;  // record slot of one unit inside a ring stage
 constexpr int kItemCache = 512;                 // work items whose descriptors a CTA keeps in shared memory
 constexpr int kPlanThreads = 1024;
-constexpr int kGroupedThreads = kI8Threads + 64;  // 16 consumer warps, a TMA producer warp and a warp that finishes work items
+constexpr int kGroupedThreads = kI8Threads + 96;  // 16 consumer warps, a TMA producer warp and two warps that finish work items
 // ring depth: the wide Q8_0 rows leave room for two stages only
 __host__ __device__ constexpr int grouped_stages(uint32_t type) { return type == ZQ_Q8_0 ? 2 : (type == ZQ_Q5_K || type == ZQ_Q6_K) ? 3 : 4; }
 
@@ -262,6 +265,27 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
     __syncthreads();
     auto pass_of = [&](int k) -> uint4 { return k < kItemCache ? s_pass[k] : ga.passes[(bid + k * G) / ga.tiles]; };
 
+    // Tokens first, first + step, .. of the CTA's k-th work item, by one warp once all sums are in; whether they are.
+    auto finish = [&](int k, int first, int step) -> bool {
+        const uint4 pe = pass_of(k);
+        const int mc = (int)(pe.y >> 16), n0 = (bid + k * G) % ga.tiles * out_rows;
+        const float *sums = red + (k & 1) * RED_FLOATS + first * kTileRows;
+        float *out = ga.out + ((size_t)pe.z + (pe.y & 0xFFFFu) + first) * ga.n_out + n0;
+        i8_wait_or_abort(&s_sums[k & 1], (uint32_t)(k >> 1) & 1u, &s_abort, ga.status);
+        if (i8_warp_aborts(&s_abort)) return false;
+        for (int tok = first; tok < mc; tok += step, sums += step * kTileRows, out += (size_t)step * ga.n_out) {
+#pragma unroll
+            for (int row = lane; row < out_rows; row += 32) {
+                float v = sums[row] + sums[RS * kTileRows + row];
+                if (GATED) {
+                    const float up = sums[out_rows + row] + sums[RS * kTileRows + out_rows + row];
+                    v = (v / (1.0f + expf(-v))) * up;
+                }
+                if (n0 + row < ga.n_out) out[row] = v;
+            }
+        }
+        return true;
+    };
     if (warp == kI8Threads / 32) {
         // ------------------------------------------------ producer warp: keeps the ring full; a stage is refilled as soon
         // as all sixteen consumer warps have released it, whichever of them is late.  What stands between that release and
@@ -298,30 +322,15 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
         }
         return;
     }
-    if (warp == kI8Threads / 32 + 1) {
-        // ------------------------------------------------ finishing warp: adds the two unit halves of an item and stores it,
+    if (warp > kI8Threads / 32) {
+        // ------------------------------------------------ finishing warps, one for each buffer of sums: add the two unit halves of an item and store it,
         // while the consumer warps, which no barrier holds together, are in the next two
-        for (int k = 0; k < my_count; ++k) {
-            const float *sums = red + (k & 1) * RED_FLOATS;
-            const uint4 pe = pass_of(k);
-            const int mc = (int)(pe.y >> 16), n0 = (bid + k * G) % ga.tiles * out_rows;
-            float *out = ga.out + ((size_t)pe.z + (pe.y & 0xFFFFu)) * ga.n_out + n0;
-            i8_wait_or_abort(&s_sums[k & 1], (uint32_t)(k >> 1) & 1u, &s_abort, ga.status);
-            if (i8_warp_aborts(&s_abort)) return;
-            for (int tok = 0; tok < mc; ++tok, sums += kTileRows, out += ga.n_out) {
-#pragma unroll
-                for (int row = lane; row < out_rows; row += 32) {
-                    float v = sums[row] + sums[RS * kTileRows + row];
-                    if (GATED) {
-                        const float up = sums[out_rows + row] + sums[RS * kTileRows + out_rows + row];
-                        v = (v / (1.0f + expf(-v))) * up;
-                    }
-                    if (n0 + row < ga.n_out) out[row] = v;
-                }
-            }
+        for (int k = warp - kI8Threads / 32 - 1; k + 1 < my_count; k += 2) {
+            if (!finish(k, 0, 1)) return;
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_free[k & 1]);
         }
+        if (my_count > 0) finish(my_count - 1, warp - kI8Threads / 32 - 1, 2);
         return;
     }
 
