@@ -997,12 +997,12 @@ static int make_token_maps(const __half *x, size_t rows, size_t k, const GemmPar
 // How many tiles are cut along K.  Whole tiles over P pairs take ceil(T / P) rounds; cut, the tiles beyond the full rounds and one
 // round more (all of them when there are fewer than two rounds) take equal shares of at least two steps, at most eight of a tile.
 // Cutting saves the steps that the busiest pair is ahead of the average one, at 0.85 us (a dequantised step of up to 152 tokens; of a SHORT
-// tile 0.5 us for Q4_K, Q4_0 and Q8_0, 0.9 for the others) or 5.6 ns per token each.  It costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the addition
+// tile 0.5 us for Q4_K, Q4_0 and Q8_0, gated 0.7, and 0.9 for the others) or 5.6 ns per token each.  It costs the shares' way out and in and their addition, 3 us and 50 ns per token of the tile (gated: 30, where the addition
 // takes the place of an epilogue), and 8 ns per token for every round more, in which pairs no longer meet at the same depth of K.  From
 // operands in memory that costs most: 160 ns per token, and past L2 140 where the cut part is little more than a round, 400 where it is more and
 // nothing is shared for long.  Without the rounds' share the rule cut 343 of 960 shapes (64 to 8192 tokens, 2048 to 17408 columns, three types,
 // plain and gated) and was 0.3 % behind the better choice for plain ones on average and 1.7 % for gated ones, up to 12 %; with it 0.2 and
-// 0.3 %.  800 shapes of 17 to 128 tokens, six types: 0.3 % behind, 17 of them more than 5 % (the worst 21, Q4_K gated 3072 -> 1154); with one step time for all 43.  Whole and cut, us:
+// 0.3 %.  800 shapes of 17 to 128 tokens, six types: 0.3 % behind, 14 of them more than 5 % (the worst 23); with one step time for all 43.  Whole and cut, us:
 //   Q4_K 15360 -> 3840, 64 tokens 47 / 22;  11008 -> 4096, 64 tokens 35 / 20;  Q6_K 15360 -> 3840, 300 tokens 91 / 52;  2560 -> 1434 gated, 115 tokens 18.2 / 16.1
 //   not: Q8_0 3328 -> 7537, 32 tokens 10.8 / 14.3;  Q4_0 2816 -> 7104, 30 tokens 9.9 / 14.3
 //   not: Q4_K gated 4096 -> 11008, 512 tokens 74 / 83;  3840 -> 15360, 3001 tokens 553 / 587;  5120 -> 17408, 800 tokens 241 / 263
@@ -1019,7 +1019,7 @@ static int plan_cut(const zq_ctx *ctx, int tiles, int steps, uint32_t src, bool 
     const int cut_pairs = shares < pairs && cut == tiles ? (int)shares : pairs;
     const long long saved = (long long)(rounds - (tiles - cut) / pairs) * steps - ((long long)cut * steps + cut_pairs - 1) / cut_pairs;
     const bool light = p.a_tmem && (src == ZQ_Q4_K || src == ZQ_Q4_0 || src == ZQ_Q8_0);
-    const long long step_ns = std::max(!fused || light ? 500LL : p.a_tmem ? 900LL : 850LL, 56LL * p.bn / 10);
+    const long long step_ns = std::max(!fused || (light && !gated) ? 500LL : light ? 700LL : p.a_tmem ? 900LL : 850LL, 56LL * p.bn / 10);
     const long long token_ns = fused ? (gated ? 30 : 50) + 8 * (rounds - 1) : operand_bytes <= (size_t(128) << 20) ? 160 : 3 * cut <= 4 * pairs ? 140 : 400;
     const long long cost_ns = 3000 + token_ns * p.bn;
     if (!ctx->cut_tiles && saved * step_ns <= cost_ns) return whole;
