@@ -398,7 +398,7 @@ template <bool GATED, int THREADS> __device__ __forceinline__ void add_up_cut(co
 // WIDE: tiles of up to 320 tokens.  What they are for: a tile of a packed type costs its dequantisation whatever its tokens, and an expert that
 // got 257 to 320 tokens was two tiles (256 experts of 7168 x 2048 in Q4_K, 8192 tokens, 256 +- 16 to an expert: MoE layer 8.2 ms, now 7.1).
 // A form of its own because the second piece costs the issuing warp instructions in every k-block: with one form for both, 48
-// tokens of 5120 x 17408 up and down took 61.2 us instead of 56.7.
+// tokens of 5120 x 17408 up and down took 61.2 us instead of 56.7 (before SHORT, which takes 46.5).
 template <uint32_t SRC, bool GATED, int FORM, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmSmem<SRC, FORM, EPI>::threads, 1)
     gemm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w2, const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_x2, const GemmParams p) {

@@ -148,7 +148,9 @@ template <uint32_t TYPE> __device__ __forceinline__ void row_unit(uint32_t type,
     else consume_b32_i8<TYPE, 1>(wq0, wq1, t, rec, srec, xoff, yacc);
 }
 
-// The sum of one output over the warps along K, `stride` floats apart: pairs in turn, as the work-list kernel adds chunks of two units that are a CTA each.
+// The sum of one output over the warps along K, `stride` floats apart: pairs in turn.  That is the order of the cluster and work-list kernels where each chunk of two
+// units is a CTA's there; where a CTA has several chunks they keep one running sum per half of a unit pair, and here a warp of several units (more
+// than 16 of a row) adds its own first, so that f32 sums differ in their last bits.
 __device__ __forceinline__ float row_total(const float *p, int lanes_k, int stride) {
     float s = 0.f;
     for (int w = 0; w < lanes_k; w += 4) {

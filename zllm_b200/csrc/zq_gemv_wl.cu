@@ -144,7 +144,7 @@ template <uint32_t TYPE, int NT> struct WlSmem {
 // row) is computed there too, by every CTA for itself: a row is a few KB out of L2.  That takes a launch (of 4 to 5 us in a chain of
 // small ones) and the records' way through memory off a decode step; lists of several types go out as one launch instead of one per
 // type (TYPE 0).  Five Q4_K projections of five inputs: 38.7 us, now 37.9.  Norm lists of one row come here where the one-row kernels do not take them
-// (zq_gemv_row.cu: too many columns for their groups, more than four projections).
+// (zq_gemv_row.cu: past the SMs' shared memory and short rows in many groups, both record formats or fewer than four units; many groups of one or two units).
 // The ring gets what the records leave, five stages at most.
 template <uint32_t TYPE> struct WlResSmem {
     static constexpr int XCH_FLOATS = 16 * 32 * 2;
@@ -855,7 +855,7 @@ static int launch_gemv_wl_resident(zq_ctx *ctx, const WlHostJob *jobs, size_t n_
             if (!apart(wa.jobs[k].y, y_bytes, wa.src[s].x, (size_t)wa.src[s].m * wa.src[s].cols * xe)) return ZQ_OK;
         if (norm && !apart(wa.jobs[k].y, y_bytes, norm->weight, (size_t)wa.src[0].cols * sizeof(float))) return ZQ_OK;
     }
-    if (norm && n_jobs <= (size_t)kRowMaxJobs) {  // small matrices: the one-pass kernel, norm included
+    if (norm && n_jobs <= (size_t)kRowMaxJobs) {  // one row: the kernels of zq_gemv_row.cu where they fit and pay, norm included
         RowCall c;
         for (size_t k = 0; k < n_jobs; ++k) c.jobs[k] = {jobs[k].w, nullptr, jobs[k].y, jobs[k].residual, wa.jobs[k].y_dtype};
         c.n_jobs = (int)n_jobs;

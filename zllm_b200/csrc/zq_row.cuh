@@ -1,10 +1,10 @@
-// Host-side interface of the one-pass decode kernel (zq_gemv_row.cu).
+// Host-side interface of the one-row decode kernels, resident and streamed (zq_gemv_row.cu).
 #pragma once
 #include "zq_wl.cuh"
 
 namespace zq {
 
-constexpr int kRowMaxJobs = 4;
+constexpr int kRowMaxJobs = 3;  // zq_rmsnorm_linear takes no more
 struct RowHostJob {
     const zq_weight *w, *w_up;  // w_up: gated pair
     void *y;
