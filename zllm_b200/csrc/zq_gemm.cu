@@ -15,7 +15,8 @@
 // two units instead of five quarters of one.  What set their pace was the warp that issues the MMAs: 540 cycles per 64-column k-block (a
 // successful wait 180, four MMAs and a commit 360, at a fifth of its scheduler's issue slots) where its MMAs take 128 at 64 tokens.  It now
 // waits and commits once per unit, sixteen MMAs.  5120 -> 17408 / 17408 -> 5120 at 48 tokens, us: Q4_K 23.5 / 29.4, now 20.3 / 26.2; Q6_K 34.0 / 38.1,
-// now 26.7 / 31.2; Q8_0 26.4 / 29.6, now 20.3 / 28.2.  With 128 to 256 tokens (one accumulator, the epilogue no longer under the next tile)
+// now 26.7 / 31.2; Q8_0 26.4 / 29.6, now 20.3 / 28.2.  Over 500 random shapes of 17 to
+// 128 tokens against the form before, with the cuts that go with each: Q4_K 0.91, Q5_K 0.88, Q6_K 0.87, Q4_0 0.87, IQ4_NL 0.95, Q8_0 0.88.  With 128 to 256 tokens (one accumulator, the epilogue no longer under the next tile)
 // plain shapes stay as they are and gated ones take 10 to 20 % longer.
 // Activations are f16 (exact for bf16 inputs in f16 range), converted before the kernel where they are not.
 //
