@@ -330,6 +330,8 @@ __global__ void __launch_bounds__(kGroupedThreads, 1) moe_grouped_kernel(const _
             __syncwarp();
             if (lane == 0) mbar_arrive(&s_free[k & 1]);
         }
+        // Parity tells the last item's phase apart for the warp of the other buffer too: it comes from item my_count - 2, whose sums every consumer left behind
+        // those of my_count - 3, the one before the last in this buffer.
         if (my_count > 0) finish(my_count - 1, warp - kI8Threads / 32 - 1, 2);
         return;
     }
