@@ -103,6 +103,7 @@ def test_norm_and_projections_of_several_types_in_one_launch(cols, dtype, shift)
 @pytest.mark.parametrize("types", [(H.Q4_K, H.Q6_K, H.Q5_K), (H.Q8_0, H.IQ4_NL, H.Q4_0)])
 def test_norm_and_large_projections_of_several_types_in_one_launch(types):
     """More than the SMs' shared memory holds: a CTA streams groups of one projection and goes on to the next one's, of another type."""
+    # The block-32 types do; Q4_K and Q5_K beside Q6_K need records of both formats and are one work-list launch (which runs which: tests/test_gpu_row.py).
     cols, rows, eps = 3840, (7001, 3000, 1003), 1e-6
     rng = np.random.default_rng(77)
     data = [H.random_weight(t, r, cols, seed=r) for t, r in zip(types, rows)]
